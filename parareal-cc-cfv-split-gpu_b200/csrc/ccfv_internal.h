@@ -126,13 +126,15 @@ constexpr size_t FD_BYTES = (sizeof(SweepField) + 63) & ~size_t(63);
 // SWEEP_CELL_COMPAT: the per-cell form with the reference's boundaries
 // (non-cyclic system).
 // SWEEP_FILTER_WIDE: the stencil form with the 13-tap right-hand side of the
-// reference scheme's third sweep (interior segments of compat lines).
+// reference scheme's third sweep, SWEEP_FILTER_SEG the eight-tap one of the
+// others (interior segments of compat lines; tiles of sweep_filter_kernel).
+// SWEEP_FILTER runs the streaming kernels (stream.cu).
 enum { SWEEP_GENERAL = 0, SWEEP_FAST = 1, SWEEP_FILTER = 2, SWEEP_GENERAL_SRC = 3,
        SWEEP_FILTER_EXACT = 4, SWEEP_CELL = 5, SWEEP_CELL_EXACT = 6, SWEEP_CELL_COMPAT = 7,
-       SWEEP_FILTER_WIDE = 8 };
-// Variants run by the filter kernel (factored solve).
+       SWEEP_FILTER_WIDE = 8, SWEEP_FILTER_SEG = 9 };
+// Variants run by the filter kernels (factored solve).
 inline bool filter_variant(int v) {
-  return v == SWEEP_FILTER || v == SWEEP_FILTER_EXACT || v == SWEEP_CELL ||
+  return v == SWEEP_FILTER || v == SWEEP_FILTER_SEG || v == SWEEP_FILTER_EXACT || v == SWEEP_CELL ||
          v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT || v == SWEEP_FILTER_WIDE;
 }
 // Warm-up (segmented) forms: lines longer than MAX_CLUSTER segments are
@@ -150,6 +152,38 @@ inline bool cell_filter_variant(int v) {
 inline bool exact_filter_variant(int v) { return v == SWEEP_FILTER_EXACT || v == SWEEP_CELL_EXACT; }
 constexpr int FILTER_JMAX = 64;  // longest recurrence warm-up of the filter kernel
 
+// Launch geometry shared by all fields of one sweep launch.
+struct LaunchGeom {
+  int cs = 1, lc_max = 0, halo = 0, groups = 0, variant = 0;
+  int dir = 0;            // sweep direction
+  int lanes = 0;          // streaming form: lanes per line
+  int rows = 0;           // streaming form: staged positions per line (at most)
+  int lc_fit = 0, halo_fit = 0;  // tile of the scan kernels: a step whose scan tile
+                                 // does not fit is refused whatever form runs it
+};
+
+// The fields of a plan's launch by value: they differ only in their buffers
+// and time origins, and field i's buffers lie i * stride bytes behind field
+// 0's.  tiles: tiles per field (0: not known to be so, read the descriptors).
+struct PlanFields {
+  SweepField f = {};
+  long long stride = 0;
+  int tiles = 0;
+  int seg = 0;  // streaming form: cells per segment
+};
+
+// Streaming form (stream.cu): positions per lane; cells per segment of a line
+// of L cells in cs segments (even: pairs of cells stay aligned); lines per CTA;
+// shared memory of a launch.
+constexpr int STREAM_CH = 17;
+__host__ __device__ inline int stream_seg(int L, int cs) { return ((L + cs - 1) / cs + 1) & ~1; }
+int stream_tile_lines(int dir, int lanes);
+size_t stream_smem_bytes(int dir, int lanes, int rows, bool fp64);
+// Lines per CTA of a launch geometry.
+inline int tile_lines(const LaunchGeom &G) {
+  return G.variant == SWEEP_FILTER ? stream_tile_lines(G.dir, G.lanes) : LPG;
+}
+
 // Shared-memory bytes of the sweep kernels for a launch.
 size_t sweep_smem_bytes(int lc_max, int halo, bool fp64, bool source = false);
 size_t sweep_fast_smem_bytes(int lc_max, int halo, bool fp64);
@@ -165,16 +199,17 @@ cudaError_t launch_filter_weights(bool fp64, const SweepField *d_field, void *wt
                                   int lines, cudaStream_t stream, bool wide = false);
 
 // Launches one fused sweep over all fields of `d_fields` (device array,
-// sorted by group0; tiles group_base .. group_base+groups_total-1).  All fields share the cluster size `cs`, their
-// max positions per CTA `lc_max` and the halo `halo`.  `toff` is added to
+// sorted by group0; tiles group_base .. group_base+groups_total-1).  All fields share G: the cluster size `cs`, their
+// max positions per CTA `lc_max` and the halo `halo` (LaunchGeom).  `toff` is added to
 // every field's ta_rel/tb_rel (the launch time); `data` (if non-null)
 // replaces fields[0].data (single-field launches).  `jstep` is the step of an
 // out-of-place sequence (SweepField::pp); `inplace` says whether any field
 // sweeps in place (the filter kernel's segments of a line then form a
-// cluster).
+// cluster).  `plan`: the same fields by value where they allow it (see
+// PlanFields; the streaming form then reads no descriptor).
 template <typename T>
-cudaError_t launch_sweep(int variant, const SweepField *d_fields, int nfields, int group_base,
-                         int groups_total, int cs, int lc_max, int halo, double toff, void *data,
+cudaError_t launch_sweep(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
+                         int nfields, int group_base, int groups_total, double toff, void *data,
                          unsigned *d_status, cudaStream_t stream, int jstep = 0,
                          bool inplace = true);
 
@@ -187,9 +222,16 @@ struct BatchStep {
   const int *g0idx = nullptr;  // the fields' group0 values (device), or null
 };
 template <typename T>
-cudaError_t launch_sweep_batch(int variant, const SweepField *d_fields, int nfields,
-                               int group_base, int groups_total, int cs, int lc_max, int halo,
-                               const BatchStep &bs, unsigned *d_status, cudaStream_t stream);
+cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, int nfields,
+                               int group_base, int groups_total, const BatchStep &bs,
+                               unsigned *d_status, cudaStream_t stream);
+// The streaming form's launch (SWEEP_FILTER), called by the two above.
+template <typename T>
+cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
+                          int nfields, int group_base, int groups_total, void *data,
+                          unsigned *d_status,
+                          int jstep, int nslice, const int *nlo, bool inplace,
+                          cudaStream_t stream, const int *g0idx, bool pdl);
 
 // Solver-table layout (T values): alpha[L] g[L] z[L] tP[L] tS[L]
 // aggA[cs*NCH] PA[cs*(NCH+1)], where, for the chunk partition the sweep

@@ -130,7 +130,6 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
         win[m] = line[q * sp];
         q = (q + 1 == L) ? 0 : q + 1;
       }
-      T w = T(0);
 #pragma unroll
       for (int i = 0; i < RG_CH; ++i) {
         win[7] = line[q * sp];
@@ -139,8 +138,7 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
 #pragma unroll
         for (int m = 0; m < 8; ++m) in += om[m] * win[m];
         if (k0 + i >= L) in = T(0);
-        w = in + mmu * w;
-        v[i] = w;
+        v[i] = in;
 #pragma unroll
         for (int m = 0; m < 7; ++m) win[m] = win[m + 1];
       }
@@ -163,88 +161,70 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
       }
       __syncwarp(fm);
       const T icw = T(F.sm_inv_den / 12.0);
-      T w = T(0);
 #pragma unroll
       for (int i = 0; i < RG_CH; ++i) {
         const int k = k0 + i;
         T in = T(0);
         if (k < L) in = icw * ((bl[k == 0 ? L - 1 : k - 1] + bl[k + 1 == L ? 0 : k + 1]) +
                                T(10.0) * bl[k]);
-        w = in + mmu * w;
-        v[i] = w;
+        v[i] = in;
       }
     }
-    // forward chunks joined by a shuffle scan of x -> pw x + e_c
-    {
-      T sa = pw, sb = v[RG_CH - 1];
-#pragma unroll
-      for (int d = 1; d < RG_LANES; d <<= 1) {
-        const T pa = __shfl_up_sync(fm, sa, d, RG_LANES);
-        const T pb = __shfl_up_sync(fm, sb, d, RG_LANES);
-        if (c >= d) {
-          sb = sa * pb + sb;
-          sa = sa * pa;
-        }
-      }
-      T cin = __shfl_up_sync(fm, sb, 1, RG_LANES);
-      if (c == 0) cin = T(0);
-#pragma unroll
-      for (int i = 0; i < RG_CH; ++i) {
-        cin *= mmu;
-        v[i] += cin;
-      }
-    }
-    // periodic closure of the forward filter: w_{-1} = w_{L-1} = E / (1 - (-mu)^L)
+    // Forward filter.  Each lane walks its chunk from zero for its end value;
+    // a shuffle scan of x -> pw x + e_c joins the chunks; the periodic closure
+    // w_{-1} = w_{L-1} = E / (1 - (-mu)^L) (E: the end of the line from a zero
+    // start) completes the carry, from which the lane walks again.  The
+    // second walk costs one multiply-add per position where adding
+    // carry * (-mu)^i to the first one's values costs two operations, and
+    // rounds like the recurrence itself, as the streaming sweeps do.
     {
       const int ce = (L - 1) / RG_CH, ie = (L - 1) - ce * RG_CH;
-      T e = T(0);
-#pragma unroll
-      for (int i = 0; i < RG_CH; ++i) e = (c == ce && i == ie) ? v[i] : e;
-      e = __shfl_sync(fm, e, ce, RG_LANES);
-      const T wl = e / (T(1) - pwa[L]);
+      T w = T(0), e = T(0);
 #pragma unroll
       for (int i = 0; i < RG_CH; ++i) {
-        const int k = k0 + i;
-        v[i] = k < L ? v[i] + wl * pwa[k + 1] : T(0);
+        w = v[i] + mmu * w;
+        e = i == ie ? w : e;
+      }
+      T pd = pw;
+#pragma unroll
+      for (int d = 1; d < RG_LANES; d <<= 1) {
+        const T t = __shfl_up_sync(fm, w, d, RG_LANES);
+        if (c >= d) w += pd * t;
+        pd *= pd;
+      }
+      T cin = __shfl_up_sync(fm, w, 1, RG_LANES);
+      if (c == 0) cin = T(0);
+      e = __shfl_sync(fm, e + cin * pwa[ie + 1], ce, RG_LANES);
+      w = cin + e / (T(1) - pwa[L]) * pwa[min(k0, L)];
+#pragma unroll
+      for (int i = 0; i < RG_CH; ++i) {
+        w = v[i] + mmu * w;
+        v[i] = k0 + i < L ? w : T(0);
       }
     }
-    // backward filter from a zero start at L
+    // backward filter from a zero start at L, closed by x_L = x_0 =
+    // X / (1 - (-mu)^L), then walked again from the true carry
     {
       T x = T(0);
 #pragma unroll
-      for (int i = RG_CH - 1; i >= 0; --i) {
-        x = v[i] + mmu * x;
-        v[i] = x;
-      }
-      T sa = pw, sb = v[0];
+      for (int i = RG_CH - 1; i >= 0; --i) x = v[i] + mmu * x;
+      T pd = pw;
 #pragma unroll
       for (int d = 1; d < RG_LANES; d <<= 1) {
-        const T pa = __shfl_down_sync(fm, sa, d, RG_LANES);
-        const T pb = __shfl_down_sync(fm, sb, d, RG_LANES);
-        if (c + d < RG_LANES) {
-          sb = sa * pb + sb;
-          sa = sa * pa;
-        }
+        const T t = __shfl_down_sync(fm, x, d, RG_LANES);
+        if (c + d < RG_LANES) x += pd * t;
+        pd *= pd;
       }
-      T cin = __shfl_down_sync(fm, sb, 1, RG_LANES);
+      T cin = __shfl_down_sync(fm, x, 1, RG_LANES);
       if (c == RG_LANES - 1) cin = T(0);
+      const T x0 = __shfl_sync(fm, x, 0, RG_LANES) / (T(1) - pwa[L]);
+      __syncwarp(fm);  // every read of this line is done
+      x = cin + x0 * pwa[max(L - k0 - RG_CH, 0)];
 #pragma unroll
       for (int i = RG_CH - 1; i >= 0; --i) {
-        cin *= mmu;
-        v[i] += cin;
-      }
-    }
-    // periodic closure of the backward filter: x_L = x_0 = X / (1 - (-mu)^L)
-    {
-      const T X = __shfl_sync(fm, v[0], 0, RG_LANES);
-      const T x0 = X / (T(1) - pwa[L]);
-      __syncwarp(fm);  // every read of this line is done
-      if (act) {
-#pragma unroll
-        for (int i = 0; i < RG_CH; ++i) {
-          const int k = k0 + i;
-          if (k < L) line[k * sp] = v[i] + x0 * pwa[L - k];
-        }
+        const int k = k0 + i;
+        x = k < L ? v[i] + mmu * x : x0;
+        if (act && k < L) line[k * sp] = x;
       }
       __syncwarp(fm);
     }

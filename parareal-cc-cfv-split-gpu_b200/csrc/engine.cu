@@ -291,14 +291,46 @@ int filter_lc(int L, bool fp64) {
   return ic == g_filter_lc_class.end() ? LC_MAX : ic->second;
 }
 
+// Streaming form: the tuned length of exactly these lines, else no limit (its
+// longest segment is the fastest but for rounding up to whole segments).  A
+// line class does not bound it, so a problem splits its lines alike alone and
+// in a batch and FP32 increments round alike.
+static int stream_lc(int L, bool fp64) {
+  if (g_lc_override > 0) return g_lc_override;
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  auto it = g_filter_lc.find({L, fp64 ? 1 : 0});
+  return it != g_filter_lc.end() ? it->second : L;
+}
+
 bool class_tuned(int L, bool fp64) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   return g_filter_lc_class.count({line_class(L), fp64 ? 1 : 0}) > 0;
 }
 
+// Streaming form of a warm-up sweep (stream.cu): segments as long as LN lanes
+// of STREAM_CH positions hold beside the warm-up J on both sides (longer
+// segments repeat less of it), or as the tuner found; a y line takes 32 lanes
+// unless 16 cover it with much fewer lanes in all (lines of one short segment):
+// a lane of the 16-lane kernel issues 1.37 times the instructions of one of the
+// 32-lane kernel (two lines' copies per warp, spills).
+static void stream_geom(LaunchGeom &G, int L, int J, int sh, int lc) {
+  G.lc_fit = G.lc_max;
+  G.halo_fit = G.halo;
+  auto segs = [&](int lanes) {
+    const int seg = std::min((lanes * STREAM_CH - 2 * J) & ~1, std::max(32, lc + (lc & 1)));
+    return (L + seg - 1) / seg;
+  };
+  G.lanes = G.dir == 1 && 3 * segs(32) <= 2 * segs(16) ? 32 : 16;
+  G.cs = segs(G.lanes);
+  G.lc_max = stream_seg(L, G.cs);
+  G.halo = (J + sh + 7) & ~1;
+  G.rows = (G.lanes * STREAM_CH + 2 * (G.halo - J) + 1) & ~1;
+}
+
 LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64, bool inplace,
                      double theta) {
   LaunchGeom G;
+  G.dir = dir;
   const int L = dir == 0 ? g.nx : g.ny;
   G.cs = (L + LC_MAX - 1) / LC_MAX;
   G.lc_max = (L + G.cs - 1) / G.cs;
@@ -336,6 +368,8 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
       if (inplace && G.cs > MAX_CLUSTER) {  // in place, a line's segments form one cluster
         G = general;
         if (uniform) G.variant = SWEEP_FAST;
+      } else if (uniform) {
+        stream_geom(G, L, J, sh, stream_lc(L, fp64));
       }
     } else if (uniform) {
       G.variant = SWEEP_FAST;
@@ -372,6 +406,10 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
         sweep_filter_smem_bytes(G.lc_max, G.halo, fp64, false, true) > 227 * 1024)
       G = general;
   }
+  if (!G.lc_fit) {
+    G.lc_fit = G.lc_max;
+    G.halo_fit = G.halo;
+  }
   return G;
 }
 
@@ -381,6 +419,14 @@ int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, 
   const ccfv_grid &g = ctx->grid;
   const size_t el = fp64 ? 8 : 4;
   const size_t NN = (size_t)g.nx * g.ny;
+  if (for_class) {  // streaming sweeps take no class length
+    bool uses = false;
+    for (int dir = 0; dir < 2; ++dir) {
+      const int v = step_geom(g, dir, dir == 0 ? 0.5 * dt : dt, 0, fp64, false).variant;
+      uses = uses || v != SWEEP_FILTER;
+    }
+    if (!uses) return CCFV_OK;
+  }
   if (!ctx->status.p) {  // contexts of the batched engine's problems have none
     CK(ctx->status.alloc(sizeof(unsigned) * 4));
     CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(unsigned) * 4, st));
@@ -506,9 +552,9 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
     if (ctx->force_general && G.variant != SWEEP_GENERAL_SRC) G.variant = SWEEP_GENERAL;
     if (G.cs > MAX_CLUSTER && !(warm_filter_variant(G.variant) && plan_pp))
       return set_error(ctx, CCFV_ERR_UNSUPPORTED, "line longer than 4096 cells");
-    if (std::max({sweep_smem_bytes(G.lc_max, G.halo, fp64, g.source != 0),
-                  sweep_fast_smem_bytes(G.lc_max, G.halo, fp64),
-                  sweep_filter_smem_bytes(G.lc_max, G.halo, fp64, true,
+    if (std::max({sweep_smem_bytes(G.lc_fit, G.halo_fit, fp64, g.source != 0),
+                  sweep_fast_smem_bytes(G.lc_fit, G.halo_fit, fp64),
+                  sweep_filter_smem_bytes(G.lc_fit, G.halo_fit, fp64, true,
                                           cell_filter_variant(G.variant))}) > 227 * 1024)
       return set_error(ctx, CCFV_ERR_UNSUPPORTED, "time step too large for the staged halo");
     for (int i = 0; i < nf; ++i) {
@@ -523,6 +569,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
       }
       if (filter_variant(G.variant)) filter_field(g, f, fp64);
       f.src_tb = kind == 2 ? 1 : 0;
+      f.groups = (f.M + tile_lines(G) - 1) / tile_lines(G);
       f.group0 = i * f.groups;
       f.cta0 = f.group0 * G.cs;
       f.halo_f = G.halo;
@@ -553,7 +600,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
       const int L = dir == 0 ? g.nx : g.ny;
       const bool wide = dsrc != 0;
       LaunchGeom G2 = G;
-      G2.variant = wide ? SWEEP_FILTER_WIDE : SWEEP_FILTER;
+      G2.variant = wide ? SWEEP_FILTER_WIDE : SWEEP_FILTER_SEG;
       G2.halo = wide ? Jc + 2 * shc + 12 : Jc + shc + 6;
       if ((L + G.cs - 1) / G.cs >= G2.halo &&
           sweep_filter_smem_bytes(G2.lc_max, G2.halo, fp64, false, false, wide) <= 227 * 1024) {
@@ -578,7 +625,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
   for (int kind = 0; kind < 3 && nf > 0; ++kind) {
     if (!stencil_filter_variant(plan->geom[kind].variant) && !plan->hyb[kind]) continue;
     any_hyb = any_hyb || plan->hyb[kind];
-    lines[kind] = h[(size_t)kind * nf].groups * LPG;
+    lines[kind] = h[(size_t)kind * nf].groups * tile_lines(plan->geom[kind]);
     CK(plan->wt[kind].alloc((fp64 ? 8 : 4) * (plan->wide[kind] ? 16 : 8) * (size_t)lines[kind]));
     CK(plan->nt[kind].alloc(sizeof(int) * (size_t)lines[kind]));
     for (int i = 0; i < nf; ++i) {
@@ -587,6 +634,21 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
         (*hv)[(size_t)kind * nf + i].nt = plan->nt[kind].as<int>();
       }
     }
+  }
+  for (int kind = 0; kind < 3 && nf > 0; ++kind) {
+    const SweepField *hk = h.data() + (size_t)kind * nf;
+    PlanFields &pv = plan->by_value[kind];
+    pv.f = hk[0];
+    pv.tiles = hk[0].groups;
+    pv.seg = plan->geom[kind].lc_max;
+    // buffers a constant stride apart (slices of one allocation)
+    auto at = [](const void *p) { return reinterpret_cast<long long>(p); };
+    pv.stride = nf > 1 ? at(hk[1].data) - at(hk[0].data) : 0;
+    for (int i = 1; i < nf; ++i)
+      if (at(hk[i].data) - at(hk[0].data) != i * pv.stride ||
+          (hk[i].pp && (at(hk[i].data2) - at(hk[0].data2) != i * pv.stride ||
+                        at(hk[i].in0) - at(hk[0].in0) != i * pv.stride || hk[i].par != hk[0].par)))
+        pv.tiles = 0;
   }
   CK(plan->fields.alloc(sizeof(SweepField) * h.size()));
   CK(cudaMemcpy(plan->fields.p, h.data(), sizeof(SweepField) * h.size(), cudaMemcpyHostToDevice));
@@ -615,21 +677,19 @@ int run_step_plan(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int
     const int gpf = plan.groups_per_field[kind];
     const SweepField *fk = base + (size_t)kind * plan.nf;
     cudaError_t e =
-        fp64 ? launch_sweep<double>(G.variant, fk, plan.nf, first * gpf, count * gpf, G.cs,
-                                    G.lc_max, G.halo, toff, data_override, status, st, jstep,
-                                    !plan.pp)
-             : launch_sweep<float>(G.variant, fk, plan.nf, first * gpf, count * gpf, G.cs,
-                                   G.lc_max, G.halo, toff, data_override, status, st, jstep,
-                                   !plan.pp);
+        fp64 ? launch_sweep<double>(G, plan.by_value[kind], fk, plan.nf, first * gpf,
+                                    count * gpf, toff, data_override, status, st, jstep, !plan.pp)
+             : launch_sweep<float>(G, plan.by_value[kind], fk, plan.nf, first * gpf, count * gpf,
+                                   toff, data_override, status, st, jstep, !plan.pp);
     CK(e);
     if (plan.hyb[kind]) {  // the interior segments of compat lines: stencil form
       const LaunchGeom &G2 = plan.geom2[kind];
       const SweepField *f2 = plan.fields2.as<SweepField>() + (size_t)kind * plan.nf;
-      e = fp64 ? launch_sweep<double>(G2.variant, f2, plan.nf, first * gpf, count * gpf, G2.cs,
-                                      G2.lc_max, G2.halo, toff, data_override, status, st, jstep,
+      e = fp64 ? launch_sweep<double>(G2, plan.by_value[kind], f2, plan.nf, first * gpf,
+                                      count * gpf, toff, data_override, status, st, jstep,
                                       !plan.pp)
-               : launch_sweep<float>(G2.variant, f2, plan.nf, first * gpf, count * gpf, G2.cs,
-                                     G2.lc_max, G2.halo, toff, data_override, status, st, jstep,
+               : launch_sweep<float>(G2, plan.by_value[kind], f2, plan.nf, first * gpf,
+                                     count * gpf, toff, data_override, status, st, jstep,
                                      !plan.pp);
       CK(e);
     }

@@ -38,17 +38,13 @@ struct SolverTable {
   double sm_fac = 0, sm_inv_den = 0;
 };
 
-// Launch geometry shared by all fields of one sweep launch.
-struct LaunchGeom {
-  int cs = 1, lc_max = 0, halo = 0, groups = 0, variant = 0;
-};
-
 // Three sweep launches (x dt/2, y dt, x dt/2) of one step over a set of fields.
 struct StepPlan {
   DevBuf fields;          // SweepField[3][nf]
   int nf = 0;
   int groups_per_field[3] = {0, 0, 0};
   LaunchGeom geom[3];
+  PlanFields by_value[3];  // the same fields as a kernel argument
   bool pp = false;        // out-of-place sequence (SweepField::pp)
   DevBuf wt[3], nt[3];    // filter kernel: per-line stencil tables per sub-step kind
   // compat lines split between two launches (SweepField::hyb): the second

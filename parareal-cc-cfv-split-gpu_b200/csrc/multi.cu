@@ -155,16 +155,20 @@ static void prepare_field(std::vector<PreparedField> &out, int kind, const ccfv_
   PreparedField pf;
   pf.G = step_geom(g, f0.dir, f0.Dt, f0.dsrc, fp64, /*inplace=*/false, f0.theta);
   const bool filt = filter_variant(pf.G.variant);
-  const int bucket = filt ? 0 : (pf.G.lc_max + 63) / 64;  // segment-length bucket bounds the tile
+  // segment-length bucket bounds the tile; streaming form: lanes per line
+  const int bucket = pf.G.variant == SWEEP_FILTER ? pf.G.lanes
+                     : filt                       ? 0
+                                                  : (pf.G.lc_max + 63) / 64;
   pf.key = KKey{kind, pf.G.variant, pf.G.cs, bucket, fp64 ? 1 : 0};
   pf.level = std::get<1>(tkey);
   pf.f = f0;
   pf.f.halo_f = pf.G.halo;
+  pf.f.groups = (pf.f.M + tile_lines(pf.G) - 1) / tile_lines(pf.G);
   if (filt) filter_field(g, pf.f, fp64);
   if (stencil_filter_variant(pf.G.variant)) {
     FilterTable &T = (*tabs)[tkey];  // shared by every field of this key
     if (!T.lines) {
-      T.lines = pf.f.groups * LPG;
+      T.lines = pf.f.groups * tile_lines(pf.G);
       T.fp64 = fp64;
       T.level = pf.level;
       T.wt.alloc((fp64 ? 8 : 4) * 8 * (size_t)T.lines);
@@ -181,11 +185,12 @@ static void place_field(std::map<KKey, SweepClass> &classes, const PreparedField
                         std::vector<FilterTable *> *pending) {
   SweepClass &K = classes[pf.key];
   K.kind = std::get<0>(pf.key);
-  K.variant = pf.G.variant;
-  K.cs = pf.G.cs;
   K.fp64 = std::get<4>(pf.key);
-  K.lc_max = std::max(K.lc_max, pf.G.lc_max);
-  K.halo = std::max(K.halo, pf.G.halo);
+  LaunchGeom G = pf.G;  // the tile of the class holds every field's
+  G.lc_max = std::max(K.G.lc_max, G.lc_max);
+  G.halo = std::max(K.G.halo, G.halo);
+  G.rows = std::max(K.G.rows, G.rows);
+  K.G = G;
   FilterTable *T = pf.T;
   if (T && !T->ready && (pending->empty() || pending->back() != T) &&
       std::find(pending->begin(), pending->end(), T) == pending->end()) {
@@ -212,7 +217,7 @@ static void finish_class(SweepClass &K) {
   for (size_t i = 0; i < K.h.size(); ++i) {
     SweepField &f = K.h[i];
     f.group0 = K.groups;
-    f.cta0 = K.groups * K.cs;
+    f.cta0 = K.groups * K.G.cs;
     K.groups += f.groups;
     K.bound[i] = step_bound(f);
     K.gpre[i + 1] = K.groups;
@@ -340,9 +345,9 @@ int MultiEngine::add(const ccfv_problem &pr, int *slot) {
                                      level == 0 ? 0.5 : th);
       if (!warm_filter_variant(G.variant) && G.cs > MAX_CLUSTER)
         return fail(CCFV_ERR_UNSUPPORTED, "line longer than 4096 cells");
-      if (std::max({sweep_smem_bytes(G.lc_max, G.halo, true, P->g.source != 0),
-                    sweep_fast_smem_bytes(G.lc_max, G.halo, true),
-                    sweep_filter_smem_bytes(G.lc_max, G.halo, true, true,
+      if (std::max({sweep_smem_bytes(G.lc_fit, G.halo_fit, true, P->g.source != 0),
+                    sweep_fast_smem_bytes(G.lc_fit, G.halo_fit, true),
+                    sweep_filter_smem_bytes(G.lc_fit, G.halo_fit, true, true,
                                             cell_filter_variant(G.variant))}) > 227 * 1024)
         return fail(CCFV_ERR_UNSUPPORTED, "time step too large for the staged halo");
     }
@@ -643,10 +648,8 @@ int MultiEngine::sweeps(std::map<KKey, SweepClass> &classes, int kind, int jstep
     bs.g0idx = idxbuf_.as<int>() + K.ioff;
     const SweepField *fd = classbuf_.as<SweepField>() + K.off;
     cudaError_t e =
-        K.fp64 ? launch_sweep_batch<double>(K.variant, fd, np, 0, K.gpre[np], K.cs, K.lc_max,
-                                            K.halo, bs, status, st_)
-               : launch_sweep_batch<float>(K.variant, fd, np, 0, K.gpre[np], K.cs, K.lc_max,
-                                           K.halo, bs, status, st_);
+        K.fp64 ? launch_sweep_batch<double>(K.G, fd, np, 0, K.gpre[np], bs, status, st_)
+               : launch_sweep_batch<float>(K.G, fd, np, 0, K.gpre[np], bs, status, st_);
     MCK(e);
   }
   return CCFV_OK;

@@ -87,7 +87,8 @@ int problem_setup(Problem &P, const ccfv_problem &p, std::string *err);
 // order, so the fields active at step j form a prefix: a launch covers only
 // that prefix's tiles.
 struct SweepClass {
-  int kind = 0, variant = 0, cs = 1, lc_max = 0, halo = 0, fp64 = 1;
+  int kind = 0, fp64 = 1;
+  LaunchGeom G;
   std::vector<SweepField> h;
   size_t off = 0, ioff = 0;
   int groups = 0;

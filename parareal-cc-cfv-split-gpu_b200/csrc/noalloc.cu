@@ -202,8 +202,8 @@ extern "C" int ccfv_step_noalloc(const ccfv_grid *grid, double *d_C, double tn, 
     e = cudaMemcpyAsync(d_fields, h_fields, sizeof(h_fields), cudaMemcpyHostToDevice, st);
   for (int kind = 0; kind < 3 && e == cudaSuccess; ++kind) {
     const LaunchGeom &G = geom[kind];
-    e = launch_sweep<double>(G.variant, d_fields + kind, 1, 0, h_fields[kind].groups, G.cs,
-                             G.lc_max, G.halo, tn, nullptr, d_status, st);
+    e = launch_sweep<double>(G, PlanFields(), d_fields + kind, 1, 0, h_fields[kind].groups, tn,
+                             nullptr, d_status, st);
   }
   unsigned flag = 0;
   if (e == cudaSuccess)

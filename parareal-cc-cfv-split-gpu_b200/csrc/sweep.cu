@@ -38,6 +38,7 @@
 #include <mutex>
 
 #include "ccfv_internal.h"
+#include "sweep_device.cuh"
 #include "sweep_math.cuh"
 
 namespace cg = cooperative_groups;
@@ -45,50 +46,6 @@ namespace cg = cooperative_groups;
 namespace ccfv {
 
 namespace {
-
-// Field of tile `tile` (fields sorted by group0): binary search on the
-// launch's compact group0 index when it has one (batched launches of
-// thousands of fields: a few cache lines instead of one descriptor line per
-// probe), else on the descriptors.
-__device__ __forceinline__ int find_field(const SweepField *__restrict__ fields,
-                                          const int *__restrict__ g0idx, int nfields, int tile) {
-  int lo = 0, hi = nfields - 1;
-  if (g0idx) {
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(g0idx + mid) <= tile) lo = mid; else hi = mid - 1;
-    }
-  } else {
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(&fields[mid].group0) <= tile) lo = mid; else hi = mid - 1;
-    }
-  }
-  return lo;
-}
-
-// A field's launch time offset (field_active, ccfv_internal.h, says whether
-// it takes part in a batched launch).
-__device__ __forceinline__ double field_time(const SweepField &f, double toff, int jstep,
-                                             int nslice) {
-  return toff + jstep * f.t_step + (f.slice < 0 ? nslice * f.t_slice : 0.0);
-}
-
-// Input and output of a field in a launch (SweepField::pp): in place, or the
-// ping-pong pair of an out-of-place sweep sequence.  Out of place, no CTA
-// reads what another CTA of the launch writes.
-__device__ __forceinline__ void field_io(const SweepField &f, int jstep, const void **src,
-                                         void **dst) {
-  if (!f.pp) {
-    *src = f.data;
-    *dst = f.data;
-    return;
-  }
-  const int s = 3 * jstep + f.kind;
-  const bool toA = ((s + f.par) & 1) != 0;
-  *dst = toA ? f.data : f.data2;
-  *src = s == 0 ? f.in0 : (toA ? f.data2 : f.data);
-}
 
 // Bounds-checked view of one line in the shared tile, indexed by position.
 template <typename T>
@@ -721,21 +678,6 @@ __global__ void __launch_bounds__(NTH, 2) sweep_kernel(const SweepField *__restr
 // fix-up and the backward recurrence fuse into a single reverse walk, and the
 // backward fix-up, the Sherman-Morrison correction and the store into a final
 // walk.
-
-__device__ __forceinline__ void cp_async8(void *sdst, const void *gsrc) {
-  unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *sdst, const void *gsrc) {
-  unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all_committed() {
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
 
 static_assert(sizeof(SweepField) % 8 == 0, "descriptor slot");
 
@@ -2138,12 +2080,27 @@ static FilterKernelT<T> filter_kernel_for(int variant) {
   }
 }
 
+// Programmatic dependent launch (the filter kernels wait for their predecessor
+// before reading cells) for the single-instance engine's launches: 1.4 % on
+// the 2048^2 Parareal solve, while the batched engine's back-to-back class
+// launches lost 14 % of their fine phase with it.  CCFV_PDL=0 turns it off.
+static bool pdl_enabled() {
+  static const bool on = [] {
+    const char *e = std::getenv("CCFV_PDL");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 template <typename T>
-static cudaError_t launch_impl(int variant, const SweepField *d_fields, int nfields,
-                               int group_base, int groups_total, int cs, int lc_max, int halo,
-                               double toff, void *data, unsigned *d_status, int jstep,
-                               int nslice, const int *nlo, bool inplace, cudaStream_t stream,
-                               const int *g0idx, bool pdl_ok) {
+static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
+                               const SweepField *d_fields, int nfields, int group_base, int groups_total, double toff, void *data,
+                               unsigned *d_status, int jstep, int nslice, const int *nlo,
+                               bool inplace, cudaStream_t stream, const int *g0idx, bool pdl_ok) {
+  const int variant = G.variant, cs = G.cs, lc_max = G.lc_max, halo = G.halo;
+  if (variant == SWEEP_FILTER)
+    return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, data, d_status,
+                            jstep, nslice, nlo, inplace, stream, g0idx, pdl_ok && pdl_enabled());
   const bool fast = (variant == SWEEP_FAST);
   const bool cell = cell_filter_variant(variant);
   const bool exact = exact_filter_variant(variant);
@@ -2169,7 +2126,7 @@ static cudaError_t launch_impl(int variant, const SweepField *d_fields, int nfie
       if (!configured[dev].load(std::memory_order_relaxed)) {
         for (const void *fn :
              {(const void *)sweep_kernel<T>, (const void *)sweep_fast_kernel<T>,
-              (const void *)filter_kernel_for<T>(SWEEP_FILTER),
+              (const void *)filter_kernel_for<T>(SWEEP_FILTER_SEG),
               (const void *)filter_kernel_for<T>(SWEEP_FILTER_EXACT),
               (const void *)filter_kernel_for<T>(SWEEP_CELL),
               (const void *)filter_kernel_for<T>(SWEEP_CELL_EXACT),
@@ -2210,16 +2167,7 @@ static cudaError_t launch_impl(int variant, const SweepField *d_fields, int nfie
       fattr[na++] = attr[0];
       clustered = exact ? 0 : 1;
     }
-    // programmatic dependent launch (the kernel waits for its predecessor
-    // before reading anything) for the single-instance engine's launches:
-    // 1.4 % on the 2048^2 Parareal solve, while the batched engine's
-    // back-to-back class launches lost 14 % of their fine phase with it.
-    // CCFV_PDL=0 turns it off.
-    static const bool pdl = [] {
-      const char *e = std::getenv("CCFV_PDL");
-      return !(e && e[0] == '0');
-    }();
-    if (pdl && pdl_ok) {
+    if (pdl_ok && pdl_enabled()) {
       fattr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       fattr[na].val.programmaticStreamSerializationAllowed = 1;
       ++na;
@@ -2238,29 +2186,31 @@ static cudaError_t launch_impl(int variant, const SweepField *d_fields, int nfie
 }
 
 template <typename T>
-cudaError_t launch_sweep(int variant, const SweepField *d_fields, int nfields, int group_base,
-                         int groups_total, int cs, int lc_max, int halo, double toff, void *data,
+cudaError_t launch_sweep(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
+                         int nfields, int group_base, int groups_total, double toff, void *data,
                          unsigned *d_status, cudaStream_t stream, int jstep, bool inplace) {
-  return launch_impl<T>(variant, d_fields, nfields, group_base, groups_total, cs, lc_max, halo,
-                        toff, data, d_status, jstep, 0, nullptr, inplace, stream, nullptr, true);
+  return launch_impl<T>(G, plan, d_fields, nfields, group_base, groups_total, toff, data,
+                        d_status, jstep, 0, nullptr, inplace, stream, nullptr, true);
 }
 
 template <typename T>
-cudaError_t launch_sweep_batch(int variant, const SweepField *d_fields, int nfields,
-                               int group_base, int groups_total, int cs, int lc_max, int halo,
-                               const BatchStep &bs, unsigned *d_status, cudaStream_t stream) {
-  return launch_impl<T>(variant, d_fields, nfields, group_base, groups_total, cs, lc_max, halo,
-                        0.0, nullptr, d_status, bs.jstep, bs.nslice, bs.nlo, bs.inplace, stream,
-                        bs.g0idx, false);
+cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, int nfields,
+                               int group_base, int groups_total, const BatchStep &bs,
+                               unsigned *d_status, cudaStream_t stream) {
+  return launch_impl<T>(G, PlanFields(), d_fields, nfields, group_base, groups_total, 0.0,
+                        nullptr, d_status,
+                        bs.jstep, bs.nslice, bs.nlo, bs.inplace, stream, bs.g0idx, false);
 }
 
-template cudaError_t launch_sweep<double>(int, const SweepField *, int, int, int, int, int, int,
-                                          double, void *, unsigned *, cudaStream_t, int, bool);
-template cudaError_t launch_sweep<float>(int, const SweepField *, int, int, int, int, int, int,
-                                         double, void *, unsigned *, cudaStream_t, int, bool);
-template cudaError_t launch_sweep_batch<double>(int, const SweepField *, int, int, int, int, int,
+template cudaError_t launch_sweep<double>(const LaunchGeom &, const PlanFields &,
+                                          const SweepField *, int, int, int, double, void *,
+                                          unsigned *, cudaStream_t, int, bool);
+template cudaError_t launch_sweep<float>(const LaunchGeom &, const PlanFields &,
+                                         const SweepField *, int, int, int, double, void *,
+                                         unsigned *, cudaStream_t, int, bool);
+template cudaError_t launch_sweep_batch<double>(const LaunchGeom &, const SweepField *, int, int,
                                                 int, const BatchStep &, unsigned *, cudaStream_t);
-template cudaError_t launch_sweep_batch<float>(int, const SweepField *, int, int, int, int, int,
+template cudaError_t launch_sweep_batch<float>(const LaunchGeom &, const SweepField *, int, int,
                                                int, const BatchStep &, unsigned *, cudaStream_t);
 
 }  // namespace ccfv

@@ -1,0 +1,53 @@
+"""Streaming sweep kernels (stream.cu) at the sizes where their tiles,
+segments and copies change: lines of one and of several segments, 16 and 32
+lanes per line, tiles with missing lines, odd row lengths and an odd base
+address (single-value copies instead of pairs)."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import periodic_field, rel_l2
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # FP64 parity bar of the sweeps against the oracle
+THREADS = min(32, os.cpu_count() or 1)
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64)).cuda()
+
+
+def _grids(oracle, ccfv, nx, ny, K, vp=(0.9, -1.7)):
+    return (oracle.grid(nx, ny, bc=1, vel=1, vp=vp, K=K, threads=THREADS, scheme=1),
+            ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=1, vel_params=vp, K=K, scheme=1)))
+
+
+@pytest.mark.parametrize("nx,ny", [(40, 41), (65, 233), (246, 250), (271, 258), (272, 520),
+                                   (500, 44), (42, 1025), (1030, 66)])
+@pytest.mark.parametrize("K", [1e-4, 4e-3])
+def test_stream_sizes_match_oracle(oracle, ccfv, nx, ny, K):
+    dt = 0.8 / max(nx, ny) / 1.7
+    C0 = periodic_field(nx, nx + ny, ny=ny)
+    g, s = _grids(oracle, ccfv, nx, ny, K)
+    assert [v for v, _ in s.sweep_plan(dt)] == ["filter"] * 3
+    c = dev(C0)
+    s.run(c, 0.0, dt, 2)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
+
+
+@pytest.mark.parametrize("nx,ny", [(96, 80), (300, 260)])
+def test_stream_odd_base_address_gives_the_same_values(ccfv, nx, ny):
+    import torch
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=1, vel_params=(0.9, -1.7), K=1e-3,
+                                   scheme=1))
+    C0 = dev(periodic_field(nx, 5, ny=ny))
+    a = C0.clone()
+    b = torch.empty(nx * ny + 1, dtype=torch.float64, device="cuda")[1:].view(nx, ny)
+    b.copy_(C0)
+    for c in (a, b):
+        s.run(c, 0.0, 1e-3, 3)
+    s.check()
+    assert torch.equal(a, b)
