@@ -261,7 +261,10 @@ int ccfv_sweep_plan(ccfv_ctx *ctx, double dt, int precision, int variant[3], int
     // as ccfv_step/ccfv_run and the Parareal engines sweep: out of place
     const LaunchGeom G = step_geom(ctx->grid, dir, Dt, dsrc, precision == CCFV_FP64, false);
     if (variant)
-      variant[kind] = (ctx->force_general && G.variant != SWEEP_GENERAL_SRC) ? SWEEP_GENERAL : G.variant;
+      variant[kind] = (ctx->force_general && G.variant != SWEEP_GENERAL_SRC) ? SWEEP_GENERAL
+                      : G.variant == SWEEP_COMPAT || G.variant == SWEEP_COMPAT_D
+                          ? CCFV_SWEEP_CELL_COMPAT
+                          : G.variant;
     if (segment) {
       // the cluster form runs whole-walk segments (and a shorter last one)
       // when its segment count is the least that covers the line

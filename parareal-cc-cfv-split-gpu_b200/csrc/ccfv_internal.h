@@ -53,9 +53,9 @@ struct SweepField {
   int cta0;              // filter kernel: first CTA of this field in the launch
                          // (a multiple of the launch's cluster size)
   int halo_f;            // filter kernel: staged halo (cells) of this field
-  int hyb;               // > 0: the line's segments are split between two launches,
-                         // those at least hyb cells from both ends run the stencil
-                         // form, the others the compat form; 0: one launch
+  int jd;                // cells over which a carry decays below rounding (jf, or more
+                         // where the recurrences need no warm-up)
+  int rk_tail;           // compat: the second term of the rank-one closure matters
   // Batched launches (all zero for single-instance launches):
   int inst;              // instance index into the launch's `nlo` array
   int slice;             // >= 0: fixed slice of this field; -1: the launch's slice
@@ -90,6 +90,7 @@ struct SweepField {
   double sm_inv_den;       // periodic, scan kernels: 1 / (1 + z0 + (a/gamma) z_{L-1});
                            // filter kernel: 1 / c
   const void *tab;         // T[3L]: alpha_k | g_k | z_k (solver factors)
+  double rk_a;             // compat: mu^2 / (1 - mu^(2L+2)), rank-one closure
   // Filter kernel: per-line stencil of w's input, computed once per plan
   // (the velocity fields it serves do not depend on time); null: computed
   // per tile.  wt: T[groups*LPG][8] taps -3..4; nt: int[groups*LPG] shifts.
@@ -125,25 +126,30 @@ constexpr size_t FD_BYTES = (sizeof(SweepField) + 63) & ~size_t(63);
 // per-cell right-hand side (feet that differ from edge to edge);
 // SWEEP_CELL_COMPAT: the per-cell form with the reference's boundaries
 // (non-cyclic system).
-// SWEEP_FILTER_WIDE: the stencil form with the 13-tap right-hand side of the
-// reference scheme's third sweep, SWEEP_FILTER_SEG the eight-tap one of the
-// others (interior segments of compat lines; tiles of sweep_filter_kernel).
-// SWEEP_FILTER runs the streaming kernels (stream.cu).
+// The streaming kernels (stream.cu) run SWEEP_FILTER and, with the reference's
+// boundaries, SWEEP_COMPAT and (the reference scheme's third sweep, derivative
+// of the remapped field) SWEEP_COMPAT_D.
 enum { SWEEP_GENERAL = 0, SWEEP_FAST = 1, SWEEP_FILTER = 2, SWEEP_GENERAL_SRC = 3,
        SWEEP_FILTER_EXACT = 4, SWEEP_CELL = 5, SWEEP_CELL_EXACT = 6, SWEEP_CELL_COMPAT = 7,
-       SWEEP_FILTER_WIDE = 8, SWEEP_FILTER_SEG = 9 };
+       SWEEP_COMPAT = 8, SWEEP_COMPAT_D = 9 };
+inline bool stream_variant(int v) {
+  return v == SWEEP_FILTER || v == SWEEP_COMPAT || v == SWEEP_COMPAT_D;
+}
 // Variants run by the filter kernels (factored solve).
 inline bool filter_variant(int v) {
-  return v == SWEEP_FILTER || v == SWEEP_FILTER_SEG || v == SWEEP_FILTER_EXACT || v == SWEEP_CELL ||
-         v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT || v == SWEEP_FILTER_WIDE;
+  return stream_variant(v) || v == SWEEP_FILTER_EXACT || v == SWEEP_CELL ||
+         v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT;
 }
 // Warm-up (segmented) forms: lines longer than MAX_CLUSTER segments are
 // allowed out of place.
 inline bool warm_filter_variant(int v) {
-  return v == SWEEP_FILTER || v == SWEEP_CELL || v == SWEEP_CELL_COMPAT;
+  return stream_variant(v) || v == SWEEP_CELL || v == SWEEP_CELL_COMPAT;
 }
-// Variants whose right-hand side is the per-line stencil table (SweepField::wt).
-inline bool stencil_filter_variant(int v) { return v == SWEEP_FILTER || v == SWEEP_FILTER_EXACT; }
+// Variants whose right-hand side is the per-line stencil table (SweepField::wt),
+// and its values per line.
+inline bool stencil_filter_variant(int v) { return stream_variant(v) || v == SWEEP_FILTER_EXACT; }
+constexpr int STREAM_TAPS_D = 24;  // 8 + 13 taps, padded
+inline int stencil_taps(int v) { return v == SWEEP_COMPAT_D ? STREAM_TAPS_D : 8; }
 // Variants with the per-cell right-hand side.
 inline bool cell_filter_variant(int v) {
   return v == SWEEP_CELL || v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT;
@@ -158,6 +164,8 @@ struct LaunchGeom {
   int dir = 0;            // sweep direction
   int lanes = 0;          // streaming form: lanes per line
   int rows = 0;           // streaming form: staged positions per line (at most)
+  int ends = 0;           // streaming form, reference's boundaries: scratch values per
+                          // line end (edges and cells next to it)
   int lc_fit = 0, halo_fit = 0;  // tile of the scan kernels: a step whose scan tile
                                  // does not fit is refused whatever form runs it
 };
@@ -178,25 +186,25 @@ struct PlanFields {
 constexpr int STREAM_CH = 17;
 __host__ __device__ inline int stream_seg(int L, int cs) { return ((L + cs - 1) / cs + 1) & ~1; }
 int stream_tile_lines(int dir, int lanes);
-size_t stream_smem_bytes(int dir, int lanes, int rows, bool fp64);
+size_t stream_smem_bytes(const LaunchGeom &G, bool fp64);
 // Lines per CTA of a launch geometry.
 inline int tile_lines(const LaunchGeom &G) {
-  return G.variant == SWEEP_FILTER ? stream_tile_lines(G.dir, G.lanes) : LPG;
+  return stream_variant(G.variant) ? stream_tile_lines(G.dir, G.lanes) : LPG;
 }
 
 // Shared-memory bytes of the sweep kernels for a launch.
 size_t sweep_smem_bytes(int lc_max, int halo, bool fp64, bool source = false);
 size_t sweep_fast_smem_bytes(int lc_max, int halo, bool fp64);
 size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact = false,
-                               bool cell = false, bool wide = false);
+                               bool cell = false);
 // Longest segment (cells per CTA along a line) of the filter kernel for a
 // recurrence warm-up of J cells.
 int filter_segment_max(int J);
 // Fills the per-line stencil table of the filter kernel for field `*d_field`
-// (device descriptor): wt = T[lines][8], nt = int[lines], lines = groups*LPG
+// (device descriptor): wt = T[lines][8] (deriv: [STREAM_TAPS_D]), nt = int[lines], lines = groups*LPG
 // (lines past M get zeros).
 cudaError_t launch_filter_weights(bool fp64, const SweepField *d_field, void *wt, int *nt,
-                                  int lines, cudaStream_t stream, bool wide = false);
+                                  int lines, cudaStream_t stream, bool deriv = false);
 
 // Launches one fused sweep over all fields of `d_fields` (device array,
 // sorted by group0; tiles group_base .. group_base+groups_total-1).  All fields share G: the cluster size `cs`, their
@@ -225,7 +233,7 @@ template <typename T>
 cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, int nfields,
                                int group_base, int groups_total, const BatchStep &bs,
                                unsigned *d_status, cudaStream_t stream);
-// The streaming form's launch (SWEEP_FILTER), called by the two above.
+// The streaming form's launch (stream_variant), called by the two above.
 template <typename T>
 cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
                           int nfields, int group_base, int groups_total, void *data,

@@ -312,10 +312,9 @@ bool class_tuned(int L, bool fp64) {
 // segments repeat less of it), or as the tuner found; a y line takes 32 lanes
 // unless 16 cover it with much fewer lanes in all (lines of one short segment):
 // a lane of the 16-lane kernel issues 1.37 times the instructions of one of the
-// 32-lane kernel (two lines' copies per warp, spills).
-static void stream_geom(LaunchGeom &G, int L, int J, int sh, int lc) {
-  G.lc_fit = G.lc_max;
-  G.halo_fit = G.halo;
+// 32-lane kernel (two lines' copies per warp, spills).  reach: cells a
+// right-hand side reads on either side.
+static void stream_geom(LaunchGeom &G, int L, int J, int reach, int lc) {
   auto segs = [&](int lanes) {
     const int seg = std::min((lanes * STREAM_CH - 2 * J) & ~1, std::max(32, lc + (lc & 1)));
     return (L + seg - 1) / seg;
@@ -323,8 +322,36 @@ static void stream_geom(LaunchGeom &G, int L, int J, int sh, int lc) {
   G.lanes = G.dir == 1 && 3 * segs(32) <= 2 * segs(16) ? 32 : 16;
   G.cs = segs(G.lanes);
   G.lc_max = stream_seg(L, G.cs);
-  G.halo = (J + sh + 7) & ~1;
-  G.rows = (G.lanes * STREAM_CH + 2 * (G.halo - J) + 1) & ~1;
+  G.halo = (J + reach + 1) & ~1;
+  G.rows = (G.lanes * STREAM_CH + 2 * (G.halo - J) + 2) & ~1;
+}
+
+// Streaming form with the reference's boundaries.  A line that the lanes of
+// one segment hold is solved without warm-up at any diffusion number (jok:
+// whether the warm-up is short enough for longer lines).  False: the other
+// forms take the sweep (steep steps whose line ends need more scratch than
+// fits, in place with too many segments).
+static bool stream_compat_geom(LaunchGeom &G, int L, int J, bool jok, int sh, int dsrc, bool fp64,
+                               bool inplace) {
+  LaunchGeom S = G;
+  S.variant = dsrc ? SWEEP_COMPAT_D : SWEEP_COMPAT;
+  S.ends = dsrc ? 2 * sh + 16 : sh + 8;
+  const int reach = dsrc ? 2 * sh + 12 : sh + 6;
+  if (L <= 16 * STREAM_CH || (S.dir == 1 && L <= 32 * STREAM_CH)) {
+    S.lanes = L <= 16 * STREAM_CH ? 16 : 32;
+    S.cs = 1;
+    S.lc_max = stream_seg(L, 1);
+    S.halo = (reach + 1) & ~1;
+    S.rows = (S.lanes * STREAM_CH + 2 * S.halo + 2) & ~1;
+  } else if (jok) {
+    stream_geom(S, L, J, reach, stream_lc(L, fp64));
+    if (inplace && S.cs > MAX_CLUSTER) return false;
+  } else {
+    return false;
+  }
+  if (stream_smem_bytes(S, fp64) > 227 * 1024) return false;
+  G = S;
+  return true;
 }
 
 LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64, bool inplace,
@@ -369,7 +396,9 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
         G = general;
         if (uniform) G.variant = SWEEP_FAST;
       } else if (uniform) {
-        stream_geom(G, L, J, sh, stream_lc(L, fp64));
+        G.lc_fit = G.lc_max;
+        G.halo_fit = G.halo;
+        stream_geom(G, L, J, sh + 6, stream_lc(L, fp64));
       }
     } else if (uniform) {
       G.variant = SWEEP_FAST;
@@ -405,6 +434,9 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
     if (G.variant == SWEEP_CELL_COMPAT &&
         sweep_filter_smem_bytes(G.lc_max, G.halo, fp64, false, true) > 227 * 1024)
       G = general;
+    G.lc_fit = G.lc_max;
+    G.halo_fit = G.halo;
+    if (uniform) stream_compat_geom(G, L, J, jok, sh, dsrc, fp64, inplace);
   }
   if (!G.lc_fit) {
     G.lc_fit = G.lc_max;
@@ -423,7 +455,7 @@ int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, 
     bool uses = false;
     for (int dir = 0; dir < 2; ++dir) {
       const int v = step_geom(g, dir, dir == 0 ? 0.5 * dt : dt, 0, fp64, false).variant;
-      uses = uses || v != SWEEP_FILTER;
+      uses = uses || !stream_variant(v);
     }
     if (!uses) return CCFV_OK;
   }
@@ -502,16 +534,19 @@ int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, 
   return CCFV_OK;
 }
 
-// Fills the filter-kernel constants of a field (its variant must be FILTER).
-void filter_field(const ccfv_grid &g, SweepField &f, bool fp64) {
+// Fills the filter-kernel constants of a field launched with geometry G.
+void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom &G) {
   double mu = 0, ic = 0;
   int J = 0;
   filter_params(g, f.dir, f.Dt, fp64, &mu, &ic, &J, f.theta);
   f.sm_fac = mu;
   f.sm_inv_den = ic;
+  f.jd = J;
   // compat lines of one segment: the non-cyclic recurrences start exactly at
   // the line's ends (no warm-up)
-  f.jf = (g.bc == CCFV_BC_COMPAT && f.L <= filter_segment_max(0)) ? 0 : J;
+  f.jf = (g.bc == CCFV_BC_COMPAT && G.cs == 1) ? 0 : J;
+  f.rk_a = mu * mu / (1.0 - std::pow(mu * mu, f.L + 1));
+  f.rk_tail = std::pow(std::fabs(mu), f.L) >= std::ldexp(1.0, -60) ? 1 : 0;
 }
 
 // Sub-steps of one split step: x(dt/2) over [t, t+dt/2], y(dt) over
@@ -567,7 +602,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
         f.in0 = pfi.in0;
         f.par = pfi.par;
       }
-      if (filter_variant(G.variant)) filter_field(g, f, fp64);
+      if (filter_variant(G.variant)) filter_field(g, f, fp64, G);
       f.src_tb = kind == 2 ? 1 : 0;
       f.groups = (f.M + tile_lines(G) - 1) / tile_lines(G);
       f.group0 = i * f.groups;
@@ -577,62 +612,22 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
       plan->groups_per_field[kind] = f.groups;
     }
     plan->geom[kind] = G;
-    // Compat lines, out of place: segments at least a halo from both line
-    // ends see no boundary (no clamps or ghosts, and the non-cyclic
-    // correction has decayed within the warm-up), so they run the stencil
-    // form (one tile) in a second launch and the compat form keeps the
-    // segments at the ends.  The reference scheme's third sweep, which
-    // differentiates the remapped field, takes the 13-tap stencil form
-    // (displacements of at most two cells).
-    plan->hyb[kind] = false;
-    plan->wide[kind] = false;
-    static const bool split_on = [] {
-      const char *e = std::getenv("CCFV_COMPAT_SPLIT");
-      return !(e && e[0] == '0');
-    }();
-    const bool uniform = g.velocity == CCFV_VEL_REF_ROT4 || g.velocity == CCFV_VEL_CONST ||
-                         g.velocity == CCFV_VEL_ROTATION;
-    int Jc = 0;
-    const int shc = shift_cells(g, dir, Dt);
-    if (split_on && plan_pp && uniform && g.bc == CCFV_BC_COMPAT && !g.source &&
-        G.variant == SWEEP_CELL_COMPAT && G.cs >= 3 && (dsrc == 0 || shc <= 2) &&
-        filter_params(g, dir, Dt, fp64, nullptr, nullptr, &Jc, theta) && Jc > 0) {
-      const int L = dir == 0 ? g.nx : g.ny;
-      const bool wide = dsrc != 0;
-      LaunchGeom G2 = G;
-      G2.variant = wide ? SWEEP_FILTER_WIDE : SWEEP_FILTER_SEG;
-      G2.halo = wide ? Jc + 2 * shc + 12 : Jc + shc + 6;
-      if ((L + G.cs - 1) / G.cs >= G2.halo &&
-          sweep_filter_smem_bytes(G2.lc_max, G2.halo, fp64, false, false, wide) <= 227 * 1024) {
-        plan->hyb[kind] = true;
-        plan->wide[kind] = wide;
-        plan->geom2[kind] = G2;
-        for (int i = 0; i < nf; ++i) h[(size_t)kind * nf + i].hyb = G2.halo;
-      }
-    }
   }
-  std::vector<SweepField> h2(h);  // the stencil launches' descriptors
-  for (int kind = 0; kind < 3; ++kind)
-    if (plan->hyb[kind])
-      for (int i = 0; i < nf; ++i) h2[(size_t)kind * nf + i].halo_f = plan->geom2[kind].halo;
   plan->nf = nf;
   plan->pp = nf > 0 && fields[0].B != nullptr;
   // filter sub-steps: one per-line stencil table per kind, shared by the
   // plan's fields (same grid and sub-step; the velocity fields of the filter
   // kernel do not depend on time)
   int lines[3] = {0, 0, 0};
-  bool any_hyb = false;
   for (int kind = 0; kind < 3 && nf > 0; ++kind) {
-    if (!stencil_filter_variant(plan->geom[kind].variant) && !plan->hyb[kind]) continue;
-    any_hyb = any_hyb || plan->hyb[kind];
+    if (!stencil_filter_variant(plan->geom[kind].variant)) continue;
     lines[kind] = h[(size_t)kind * nf].groups * tile_lines(plan->geom[kind]);
-    CK(plan->wt[kind].alloc((fp64 ? 8 : 4) * (plan->wide[kind] ? 16 : 8) * (size_t)lines[kind]));
+    CK(plan->wt[kind].alloc((fp64 ? 8 : 4) * stencil_taps(plan->geom[kind].variant) *
+                            (size_t)lines[kind]));
     CK(plan->nt[kind].alloc(sizeof(int) * (size_t)lines[kind]));
     for (int i = 0; i < nf; ++i) {
-      for (std::vector<SweepField> *hv : {&h, &h2}) {
-        (*hv)[(size_t)kind * nf + i].wt = plan->wt[kind].p;
-        (*hv)[(size_t)kind * nf + i].nt = plan->nt[kind].as<int>();
-      }
+      h[(size_t)kind * nf + i].wt = plan->wt[kind].p;
+      h[(size_t)kind * nf + i].nt = plan->nt[kind].as<int>();
     }
   }
   for (int kind = 0; kind < 3 && nf > 0; ++kind) {
@@ -652,18 +647,11 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
   }
   CK(plan->fields.alloc(sizeof(SweepField) * h.size()));
   CK(cudaMemcpy(plan->fields.p, h.data(), sizeof(SweepField) * h.size(), cudaMemcpyHostToDevice));
-  if (any_hyb) {
-    CK(plan->fields2.alloc(sizeof(SweepField) * h2.size()));
-    CK(cudaMemcpy(plan->fields2.p, h2.data(), sizeof(SweepField) * h2.size(),
-                  cudaMemcpyHostToDevice));
-  }
   for (int kind = 0; kind < 3; ++kind)
     if (lines[kind])
-      CK(launch_filter_weights(fp64,
-                               (plan->hyb[kind] ? plan->fields2 : plan->fields).as<SweepField>() +
-                                   (size_t)kind * nf,
+      CK(launch_filter_weights(fp64, plan->fields.as<SweepField>() + (size_t)kind * nf,
                                plan->wt[kind].p, plan->nt[kind].as<int>(), lines[kind], 0,
-                               plan->wide[kind]));
+                               plan->geom[kind].variant == SWEEP_COMPAT_D));
   CK(cudaStreamSynchronize(0));
   return CCFV_OK;
 }
@@ -682,17 +670,6 @@ int run_step_plan(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int
              : launch_sweep<float>(G, plan.by_value[kind], fk, plan.nf, first * gpf, count * gpf,
                                    toff, data_override, status, st, jstep, !plan.pp);
     CK(e);
-    if (plan.hyb[kind]) {  // the interior segments of compat lines: stencil form
-      const LaunchGeom &G2 = plan.geom2[kind];
-      const SweepField *f2 = plan.fields2.as<SweepField>() + (size_t)kind * plan.nf;
-      e = fp64 ? launch_sweep<double>(G2, plan.by_value[kind], f2, plan.nf, first * gpf,
-                                      count * gpf, toff, data_override, status, st, jstep,
-                                      !plan.pp)
-               : launch_sweep<float>(G2, plan.by_value[kind], f2, plan.nf, first * gpf,
-                                     count * gpf, toff, data_override, status, st, jstep,
-                                     !plan.pp);
-      CK(e);
-    }
   }
   return CCFV_OK;
 }

@@ -47,12 +47,6 @@ struct StepPlan {
   PlanFields by_value[3];  // the same fields as a kernel argument
   bool pp = false;        // out-of-place sequence (SweepField::pp)
   DevBuf wt[3], nt[3];    // filter kernel: per-line stencil tables per sub-step kind
-  // compat lines split between two launches (SweepField::hyb): the second
-  // launch's descriptors (stencil form) and geometry per sub-step kind
-  DevBuf fields2;         // SweepField[3][nf]
-  LaunchGeom geom2[3];
-  bool hyb[3] = {false, false, false};
-  bool wide[3] = {false, false, false};  // the stencil launch is the 13-tap form
 };
 
 // One field of a plan: swept in place on A (B == nullptr), or an out-of-place
@@ -112,7 +106,7 @@ double coarse_theta(const ccfv_parareal_opts &o, const ccfv_grid &g, double dtc)
 inline bool coarse_theta_ok(double th) {
   return th == 0.0 || th == CCFV_COARSE_THETA_AUTO || (th >= 0.5 && th <= 1.0);
 }
-void filter_field(const ccfv_grid &g, SweepField &f, bool fp64);
+void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom &G);
 // for_class: keep the choice for the line-length classes of this grid (the
 // batched engine) instead of its exact line lengths (ccfv_autotune).
 int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen,

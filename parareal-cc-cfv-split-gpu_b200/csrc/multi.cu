@@ -156,7 +156,7 @@ static void prepare_field(std::vector<PreparedField> &out, int kind, const ccfv_
   pf.G = step_geom(g, f0.dir, f0.Dt, f0.dsrc, fp64, /*inplace=*/false, f0.theta);
   const bool filt = filter_variant(pf.G.variant);
   // segment-length bucket bounds the tile; streaming form: lanes per line
-  const int bucket = pf.G.variant == SWEEP_FILTER ? pf.G.lanes
+  const int bucket = stream_variant(pf.G.variant) ? pf.G.lanes
                      : filt                       ? 0
                                                   : (pf.G.lc_max + 63) / 64;
   pf.key = KKey{kind, pf.G.variant, pf.G.cs, bucket, fp64 ? 1 : 0};
@@ -164,14 +164,15 @@ static void prepare_field(std::vector<PreparedField> &out, int kind, const ccfv_
   pf.f = f0;
   pf.f.halo_f = pf.G.halo;
   pf.f.groups = (pf.f.M + tile_lines(pf.G) - 1) / tile_lines(pf.G);
-  if (filt) filter_field(g, pf.f, fp64);
+  if (filt) filter_field(g, pf.f, fp64, pf.G);
   if (stencil_filter_variant(pf.G.variant)) {
     FilterTable &T = (*tabs)[tkey];  // shared by every field of this key
     if (!T.lines) {
       T.lines = pf.f.groups * tile_lines(pf.G);
       T.fp64 = fp64;
+      T.deriv = pf.G.variant == SWEEP_COMPAT_D;
       T.level = pf.level;
-      T.wt.alloc((fp64 ? 8 : 4) * 8 * (size_t)T.lines);
+      T.wt.alloc((fp64 ? 8 : 4) * stencil_taps(pf.G.variant) * (size_t)T.lines);
       T.nt.alloc(sizeof(int) * (size_t)T.lines);
     }
     pf.f.wt = T.wt.p;
@@ -190,6 +191,7 @@ static void place_field(std::map<KKey, SweepClass> &classes, const PreparedField
   G.lc_max = std::max(K.G.lc_max, G.lc_max);
   G.halo = std::max(K.G.halo, G.halo);
   G.rows = std::max(K.G.rows, G.rows);
+  G.ends = std::max(K.G.ends, G.ends);
   K.G = G;
   FilterTable *T = pf.T;
   if (T && !T->ready && (pending->empty() || pending->back() != T) &&
@@ -546,7 +548,7 @@ int MultiEngine::rebuild() {
     if (!T->wt.p || !T->nt.p) return fail(CCFV_ERR_NOMEM, "stencil table allocation failed");
     const SweepClass &K = (T->level == 0 ? fine_ : coarse_).at(T->cls);
     MCK(launch_filter_weights(T->fp64, classbuf_.as<SweepField>() + K.off + T->idx, T->wt.p,
-                              T->nt.as<int>(), T->lines, st_));
+                              T->nt.as<int>(), T->lines, st_, T->deriv));
     T->ready = true;
   }
   const int eb = 148;

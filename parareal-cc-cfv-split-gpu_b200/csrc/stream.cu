@@ -37,6 +37,7 @@
 
 #include "ccfv_internal.h"
 #include "sweep_device.cuh"
+#include "sweep_math.cuh"
 
 namespace ccfv {
 
@@ -77,45 +78,268 @@ __device__ __forceinline__ int wrap_pos(int pos, int L) {
   return pos;
 }
 
-// v[i] = sum_m o[m] C_{row + i + m}, the stencil input of SCH positions
-// (stride ES between positions).
-template <typename T, int ES>
-__device__ __forceinline__ void stencil8(const T *cp, const T (&o)[8], T (&v)[SCH]) {
-  T q[7];
+template <typename T>
+__device__ __forceinline__ void load_taps(T (&o)[8], const T *__restrict__ wt) {
 #pragma unroll
-  for (int m = 0; m < 7; ++m) q[m] = cp[m * ES];
+  for (int m = 0; m < 8; ++m) o[m] = __ldg(wt + m);
+}
+
+// v[i] (+)= sum_m o[m] C_{row + i + m}, NT taps of SCH positions (stride ES
+// between positions) through a register window.
+template <typename T, int ES, int NT, bool ADD>
+__device__ __forceinline__ void stencil(const T *cp, const T (&o)[8], T (&v)[SCH]) {
+  T q[NT];
+#pragma unroll
+  for (int m = 0; m < NT - 1; ++m) q[m] = cp[m * ES];
 #pragma unroll
   for (int i = 0; i < SCH; ++i) {
-    const T q7 = cp[(7 + i) * ES];
-    T t = o[0] * q[0];
+    q[NT - 1] = cp[(NT - 1 + i) * ES];
+    T t = ADD ? v[i] + o[0] * q[0] : o[0] * q[0];
 #pragma unroll
-    for (int m = 1; m < 7; ++m) t += o[m] * q[m];
-    v[i] = t + o[7] * q7;
+    for (int m = 1; m < NT; ++m) t += o[m] * q[m];
+    v[i] = t;
 #pragma unroll
-    for (int m = 0; m < 6; ++m) q[m] = q[m + 1];
-    q[6] = q7;
+    for (int m = 0; m < NT - 1; ++m) q[m] = q[m + 1];
   }
+}
+
+// ---- the reference's boundaries (BND 1, 2) ----
+//
+// Cells whose stencil reaches a clamped or ghost cell, a few at either end of
+// a line, take the reference's per-cell formulas; every other cell of the line
+// takes the stencil.  The recurrence inputs r_k of those positions are
+// prepared before the walk, the left end's by the first half of the line's
+// lanes and the right end's by the second half at the same time: one foot,
+// PPM integral and derivative per edge (not per cell and side), edges and
+// cells spread over the half's lanes.
+//
+// Region of one end: positions [ka, kb) need r; that needs b of [ba, bb), the
+// edges of those cells and, when the sweep differentiates the remapped field
+// (BND 2), the remapped cells [ra, rb).
+struct EndRegion {
+  int ka, kb, ba, bb, ra, rb;
+};
+
+// Cells of one line in shared memory: position -> staged value (zero outside
+// the line but for the four ghost cells).  near(k): whether the cells that a
+// foot in cell k reads, k - 3 .. k + 3, are staged.
+template <typename T, int ES>
+struct StagedLine {
+  T *c;  // cell 0
+  int b0, b1;
+  unsigned *status;
+  __device__ __forceinline__ T operator()(int pos) const { return c[pos * ES]; }
+  __device__ __forceinline__ bool near(int k) const {
+    if (k - 3 >= b0 && k + 3 < b1) return true;
+    atomicOr(status, STATUS_HALO);
+    return false;
+  }
+};
+
+// Ghost cells C_{-2}, C_{-1} (left) or C_L, C_{L+1} (3-point extrapolation,
+// T2S4:275-286) of the line ends: near to far cells a, b, d; ghosts at `g`.
+template <typename T>
+__device__ __forceinline__ void ghosts(T a, T b, T d, T &g1, T &g2) {
+  const T e = T(1.0 / 11.0);
+  g1 = e * (-d + T(3) * b + T(9) * a);
+  g2 = e * (T(-15) * d + T(56) * b - T(30) * a);
+}
+
+// PPM integral of a cell from its left edge to xi (d_intC_ppm4th, T2S4:63-65,
+// with the coefficients of T2S4:260-304).
+template <typename T, typename V>
+__device__ __forceinline__ T ppm_to(const V &c, int k, T xi) {
+  const T m2 = c(k - 2), m1 = c(k - 1), z = c(k), p1 = c(k + 1), p2 = c(k + 2);
+  const T cl = T(7.0 / 12.0) * (z + m1) - T(1.0 / 12.0) * (p1 + m2);
+  const T cr = T(7.0 / 12.0) * (p1 + z) - T(1.0 / 12.0) * (p2 + m1);
+  const T D = cr - cl, C6 = T(6.0) * (z - T(0.5) * (cl + cr));
+  const T xi2 = xi * xi;
+  return T(-1.0 / 3) * C6 * (xi2 * xi) + T(0.5) * (D + C6) * xi2 + cl * xi;
+}
+
+// Fourth-order derivative at a foot in cell k (T2S4:440-547) with the
+// reference's choice of ghosts at k = 1 (-2 tap reads C_{-2}) and k = L - 2
+// (+2 tap reads C_{L+1}).
+template <typename T, typename V>
+__device__ __forceinline__ T derivative_at(const V &c, int k, T xi, int L, T inv12h) {
+  const T m2 = c(k == 1 ? -2 : k - 2), m1 = c(k - 1), z = c(k), p1 = c(k + 1),
+          p2 = c(k == L - 2 ? L + 1 : k + 2);
+  const T xi2 = xi * xi, xi3 = xi2 * xi;
+  return inv12h * ((T(2.0) * xi3 - T(6.0) * xi2 + T(3.0) * xi + T(1.0)) * m2 +
+                   (T(-8.0) * xi3 + T(18.0) * xi2 + T(6.0) * xi - T(15.0)) * m1 +
+                   (T(12.0) * xi3 - T(18.0) * xi2 - T(24.0) * xi + T(15.0)) * z +
+                   (T(-8.0) * xi3 + T(6.0) * xi2 + T(18.0) * xi - T(1.0)) * p1 +
+                   (T(2.0) * xi3 - T(3.0) * xi) * p2);
+}
+
+// A foot in cell units: cell and offset, clamped by eps to the line
+// (T2S4:322-324, 414-415, 452-455).
+struct FootCell {
+  int k;
+  double xi;
+};
+__device__ __forceinline__ FootCell foot_cell(const SweepField &F, double f, double eps) {
+  const double x = fmin(fmax(f, F.s_min + eps), F.s_max - eps);
+  FootCell r;
+  // the cell decides between ghosts: the reference's quotient, rounded alike
+  r.k = (int)floor((x - F.s_min) / F.h);
+  r.xi = (x - (F.s_min + F.h * r.k)) * (12.0 * F.inv12h);
+  return r;
+}
+__device__ __forceinline__ double line_foot(const SweepField &F, int line, int e) {
+  const double tau0 = F.t_min + F.ht * (double)line;
+  return edge_foot(F, e, tau0, tau0 + F.ht, 0.0, 0.0);  // time-independent fields
+}
+
+// Remap of one cell over [fl, fr] (T2S4:306-347, 396-438), its left foot clamped
+// from below and its right one from above only: a left foot on the upper edge
+// itself lies in no cell and the right one still counts the last cell.
+template <typename T, typename V>
+__device__ __noinline__ T remap_at_end(const SweepField &F, const V &cells, double fl, double fr) {
+  const int L = F.L;
+  if (fl > F.s_max || fr < F.s_min || fl == fr) return T(0);
+  const double xl = fmax(fl, F.s_min + F.eps_remap), xr = fmin(fr, F.s_max - F.eps_remap);
+  const int kl = (int)floor((xl - F.s_min) / F.h), kr = (int)floor((xr - F.s_min) / F.h);
+  if (!cells.near(kl) || !cells.near(kr)) return T(0);
+  const T il = kl >= 0 && kl < L ? ppm_to(cells, kl, T((xl - (F.s_min + F.h * kl)) / F.h)) : T(0);
+  const T ir = kr >= 0 && kr < L ? ppm_to(cells, kr, T((xr - (F.s_min + F.h * kr)) / F.h)) : T(0);
+  if (kl == kr) return ir - il;
+  T v = (kl >= 0 && kl < L ? cells(kl) : T(0)) - il;
+  for (int j = kl + 1; j < min(kr, L); ++j) v += cells(j);
+  return v + ir;
+}
+
+// Marks of the feet that are in no cell of the line: below it (clamped to cell
+// 0), above it (added to the cell it is clamped to: L - 1, or L by rounding),
+// and within the clamp of one of its ends (remap_at_end).
+constexpr int FOOT_BELOW = -1, FOOT_ON_END = -2, FOOT_ABOVE = 1 << 30;
+
+// r_k = (1/12c)(b_{k-1} + 10 b_k + b_{k+1}) of the region's positions into
+// `r`, by HL lanes (this one: hc).  phi / d / tmp / kf: scratch of the half.
+// All lanes of the warp call it (empty region: nothing but the barriers).
+template <typename T, int ES, bool REMAPPED, int HL>
+__device__ __forceinline__ void end_inputs(const SweepField &F, const StagedLine<T, ES> &cells,
+                                           int line, const EndRegion &R, int hc, T *phi, T *d,
+                                           T *tmp, int *kf) {
+  const int L = F.L;
+  const T kbc = T(F.kb), inv12h = T(F.inv12h);
+  const bool any = R.ka < R.kb;
+  // feet of the edges [e0, e1]: PPM integral and cell, with a mark for feet
+  // outside the line (zero inflow), and the derivative of the staged cells
+  const int e0 = REMAPPED ? R.ra : R.ba, e1 = REMAPPED ? R.rb : R.bb;
+  // feet this far from the middle of the line are clamped by neither clamp
+  const double mid = 0.5 * (F.s_min + F.s_max), half = 0.5 * (F.s_max - F.s_min) - F.h;
+  if (any)
+    for (int e = e0 + hc; e <= e1; e += HL) {
+      const double f = line_foot(F, line, e);
+      FootCell p = foot_cell(F, f, F.eps_remap);
+      if (!cells.near(p.k)) p.k = 0, p.xi = 0.0;
+      phi[e - e0] = p.k >= 0 && p.k < L ? ppm_to(cells, p.k, T(p.xi)) : T(0);
+      kf[e - e0] = f < F.s_min               ? FOOT_BELOW
+                   : f > F.s_max             ? FOOT_ABOVE + p.k
+                   : f < F.s_min + F.eps_remap || f > F.s_max - F.eps_remap ? FOOT_ON_END
+                                                                            : p.k;
+      if (!REMAPPED) {
+        T dv = T(0);
+        if (f >= F.s_min && f <= F.s_max) {
+          const FootCell q = F.eps_remap == 1e-15 || fabs(f - mid) < half ? p : foot_cell(F, f, 1e-15);
+          dv = derivative_at(cells, q.k, T(q.xi), L, inv12h);
+        }
+        d[e - e0] = dv;
+      } else {
+        d[e - e0] = T(p.xi);  // until the derivative of the remapped field
+      }
+    }
+  __syncwarp();
+  // remapped cells: whole cells between the feet plus the two integrals
+  // (T2S4:306-347, 396-438); zero from outside the line
+  T *const b = REMAPPED ? phi : tmp;
+  const int c0 = REMAPPED ? R.ra : R.ba, c1 = REMAPPED ? R.rb : R.bb;
+  if (any)
+    for (int k = c0 + hc; k < c1; k += HL) {
+      const int kl = kf[k - e0], kr = kf[k + 1 - e0];
+      T v = T(0);
+      if (kl == FOOT_ON_END || kr == FOOT_ON_END) {
+        v = remap_at_end<T>(F, cells, line_foot(F, line, k), line_foot(F, line, k + 1));
+      } else if (kl < FOOT_ABOVE && kr != FOOT_BELOW) {
+        const int l = max(kl, 0), r = min(kr & (FOOT_ABOVE - 1), L);
+        for (int j = l; j < r; ++j) v += cells(j);
+        v = (v + phi[k + 1 - e0]) - phi[k - e0];
+      }
+      if (!REMAPPED) v += kbc * (d[k + 1 - e0] - d[k - e0]);
+      tmp[k - c0] = v;
+    }
+  __syncwarp();
+  if (REMAPPED) {
+    // derivative of the remapped field at the edges of [ba, bb)
+    // (T2S4:929-932), its ghosts from the three remapped end cells
+    auto remapped = [&](int k) -> T {
+      if (k < 0 || k >= L) {
+        T g1, g2;
+        if (k < 0) {
+          ghosts(tmp[0], tmp[1], tmp[2], g1, g2);  // ra = 0
+          return k == -1 ? g1 : g2;
+        }
+        const T *z = tmp + (L - 1 - R.ra);
+        ghosts(z[0], z[-1], z[-2], g1, g2);
+        return k == L ? g1 : g2;
+      }
+      return tmp[k - R.ra];
+    };
+    if (any)
+      for (int e = R.ba + hc; e <= R.bb; e += HL) {
+        int k = kf[e - e0];
+        T xi = d[e - e0], dv = T(0);
+        if (k == FOOT_ON_END) {  // inside [s_min, s_max], within the clamp
+          const FootCell q = foot_cell(F, line_foot(F, line, e), 1e-15);
+          k = q.k;
+          xi = T(q.xi);
+        }
+        if (k >= 0 && k < FOOT_ABOVE) dv = derivative_at(remapped, k, xi, L, inv12h);
+        d[e - e0] = dv;
+      }
+    __syncwarp();
+    if (any)
+      for (int k = R.ba + hc; k < R.bb; k += HL)
+        b[k - R.ba] = tmp[k - R.ra] + kbc * (d[k + 1 - e0] - d[k - e0]);
+    __syncwarp();
+  }
+  // compact mass matrix, b = 0 outside the line (T2S4:616-634)
+  if (any) {
+    const T icw = T(F.sm_inv_den / 12.0);
+    for (int k = R.ka + hc; k < R.kb; k += HL) {
+      const T bm = k > R.ba ? b[k - 1 - R.ba] : T(0), bp = k + 1 < R.bb ? b[k + 1 - R.ba] : T(0);
+      d[k - R.ka] = icw * ((bm + bp) + T(10.0) * b[k - R.ba]);
+    }
+  }
+  __syncwarp();
 }
 
 // What a CTA needs of its field.
 struct StreamField {
-  int L, M, J, H, groups, cta0;
+  int L, M, J, JD, H, groups, cta0;
   long long s_line, s_pos;
   double mu;
   const void *wt;
   const int *nt;
 };
 __device__ __forceinline__ StreamField stream_field(const SweepField &f) {
-  return StreamField{f.L, f.M, f.jf, f.halo_f, f.groups, f.cta0, f.s_line, f.s_pos, f.sm_fac,
+  return StreamField{f.L, f.M, f.jf, f.jd, f.halo_f, f.groups, f.cta0, f.s_line, f.s_pos, f.sm_fac,
                      f.wt, f.nt};
 }
 
-template <typename T, int DIR, int LN>
+// BND 0: periodic lines; 1: the reference's boundaries, derivative of the sweep
+// input; 2: the reference's third sweep, which differentiates the remapped
+// field.  Its interior right-hand side R_k + sum_t wq_t R_{k+n0-2+t} with R_j =
+// sum_s wr_s C_{j+n0-2+s} is two tap groups of the cells, 8 taps from k+n0-3
+// and 13 from k+2n0-5 with the mass matrix, in three windowed passes (8, 8, 5)
+// that keep the register window at eight values for any displacement.
+template <typename T, int DIR, int LN, int BND>
 __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 : 8)
     stream_kernel(const __grid_constant__ PlanFields plan, const SweepField *__restrict__ fields,
                   int nfields, int first, void *data_override, int rows, unsigned *status,
                   int jstep, int nslice, const int *nlo, int cs, int clustered,
-                  const int *g0idx) {
+                  const int *g0idx, int ends) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT = StreamCta<DIR, LN>::warps * 32;
   constexpr int LPW = StreamCta<DIR, LN>::lpw;
@@ -133,11 +357,13 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   // that the CTAs in flight cover whole rows of the field (x sweep of 4096^2:
   // 46.6 us against 48.3 us with a line's segments side by side).
   StreamField F;
+  const SweepField *D;  // whole descriptor (line ends only)
   int tile, rank;
   const void *vs;
   void *vd;
   if (plan.tiles > 0) {
     F = stream_field(plan.f);
+    D = &plan.f;
     tile = blockIdx.x;
     rank = blockIdx.y;
     field_io(plan.f, jstep, &vs, &vd, data_override);
@@ -150,6 +376,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     const int cta = (int)blockIdx.x + first;
     const SweepField &f = fields[find_field(fields, g0idx, nfields, cta / cs)];
     F = stream_field(f);
+    D = &f;
     const int q = cta - F.cta0;
     rank = clustered ? q % cs : q / F.groups;
     tile = clustered ? q / cs : q - rank * F.groups;
@@ -171,9 +398,14 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   // Positions p0-J .. p1+J-1 are walked by the first `act` lanes of a line, and
   // the cells of all positions of those lanes are staged: past p1+J they only
   // lengthen the backward warm-up, so nothing is masked inside a lane.
-  const int act = min(LN, (np + 2 * J + SCH - 1) / SCH);
-  const int nr = (act * SCH + 2 * (H - J) + 1) & ~1;
-  const int b0 = p0 - H;  // position of staged row 0
+  // (The reference's lines end: nothing is walked past position L - 1.)
+  const int walked = BND ? min(np + 2 * J, L - p0 + J) : np + 2 * J;
+  const int act = min(LN, (walked + SCH - 1) / SCH);
+  // first position of the first lane: p0 - J, or (BND) as much earlier as makes
+  // the last lane end with the line, so that nothing is masked there either
+  const int org = BND && p1 == L ? L - act * SCH : p0 - J;
+  const int nr = (act * SCH + 2 * (H - J) + 2) & ~1;
+  const int b0 = (org - (H - J)) & ~1;  // position of staged row 0
   const bool inside = b0 >= 0 && b0 + nr <= L;
   const bool pairs = ((DIR == 0 ? s_pos : s_line) & 1) == 0 && (DIR == 0 || (L & 1) == 0) &&
                      (((size_t)src | (size_t)dst) & (2 * sizeof(T) - 1)) == 0;
@@ -192,7 +424,12 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
         for (int r = r0; r < nr; r += NT / G, s += step, d += NT / G * X_PITCH) copy_pair(d, s);
       } else {
         for (int r = r0; r < nr; r += rs, d += rs * X_PITCH) {
-          const T *p = s + (long long)wrap_pos(b0 + r, L) * s_pos;
+          if (BND && (unsigned)(b0 + r) >= (unsigned)L) {
+            d[0] = T(0);
+            if (pairs) d[1] = T(0);
+            continue;
+          }
+          const T *p = s + (long long)(BND ? b0 + r : wrap_pos(b0 + r, L)) * s_pos;
           if (pairs) copy_pair(d, p); else copy_one(d, p);
         }
       }
@@ -209,9 +446,19 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
 #pragma unroll 5
           for (int e = 2 * lane; e < nr; e += 64) copy_pair(d + e, s + e);
         } else if (pairs) {
-          for (int e = 2 * lane; e < nr; e += 64) copy_pair(d + e, s + wrap_pos(b0 + e, L));
+          for (int e = 2 * lane; e < nr; e += 64) {
+            if (BND && (unsigned)(b0 + e) >= (unsigned)L)
+              d[e] = d[e + 1] = T(0);
+            else
+              copy_pair(d + e, s + (BND ? b0 + e : wrap_pos(b0 + e, L)));
+          }
         } else {
-          for (int e = lane; e < nr; e += 32) copy_one(d + e, s + wrap_pos(b0 + e, L));
+          for (int e = lane; e < nr; e += 32) {
+            if (BND && (unsigned)(b0 + e) >= (unsigned)L)
+              d[e] = T(0);
+            else
+              copy_one(d + e, s + (BND ? b0 + e : wrap_pos(b0 + e, L)));
+          }
         }
       }
     }
@@ -222,12 +469,10 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   const int lw = DIR == 0 ? (lane & 1) : lane / LN;          // line within the warp
   const int line = line0 + warp * LPW + lw;
   const T mmu = T(-F.mu);
+  const T *wt = reinterpret_cast<const T *>(F.wt) +  // padded past M
+                (size_t)line * (BND == 2 ? STREAM_TAPS_D : 8);
   T o[8];
-  {
-    const T *w = reinterpret_cast<const T *>(F.wt) + (size_t)line * 8;  // padded past M
-#pragma unroll
-    for (int m = 0; m < 8; ++m) o[m] = __ldg(w + m);
-  }
+  if (!BND) load_taps(o, wt);
   const int n0 = __ldg(F.nt + line);
   static_assert(SCH == 17, "pw");
   T pw = mmu * mmu;  // (-mu)^17
@@ -245,16 +490,102 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
 
   // ---- stencil and recurrences ----
   T *const col = DIR == 0 ? tile_s + warp * LPW + lw : tile_s + (size_t)(warp * LPW + lw) * rows;
-  const int k0 = H - J + c * SCH;  // staged row of this lane's first position
+  const int k0 = org - b0 + c * SCH;  // staged row of this lane's first position
   const int r0 = k0 + n0 - 3;
-  const bool ok = r0 >= 0 && r0 + SCH + 7 <= rows;
+  bool ok = r0 >= 0 && r0 + SCH + 7 <= rows;
+  if (BND == 2) ok = ok && k0 + 2 * n0 - 5 >= 0 && k0 + 2 * n0 + SCH + 8 <= rows;
   if (!ok && line < M) atomicOr(status, STATUS_HALO);
+  // inputs of the positions next to the line's ends (BND): the left region is
+  // r[k - lo.ka], k in [lo.ka, lo.kb), the right one likewise
+  EndRegion lo, hi;
+  T *rl = nullptr, *rr = nullptr;
+  if (BND) {
+    const int kend = org + act * SCH;  // first position not walked
+    // positions whose stencil, with the mass matrix's neighbours, stays clear
+    // of clamps and ghosts: [sl, sr)
+    int bl = max(2 - n0, 0), bh = min(L - 4 - n0, L - 1);
+    if (BND == 2) {
+      bl = max(bl, 4 - 2 * n0);
+      bh = min(bh, L - 7 - 2 * n0);
+    }
+    const int sl = min(bl + 1, L), sr = min(max(bh, sl), L);
+    auto region = [&](int ka, int kb) {
+      EndRegion e;
+      e.ka = ka;
+      e.kb = kb;
+      e.ba = max(0, ka - 1);
+      e.bb = min(L, kb + 1);
+      e.ra = max(0, min(e.ba, e.ba + n0 - 4));
+      e.rb = min(L, max(e.bb, e.bb + n0 + 5));
+      if (e.ra < 3) e.ra = 0;  // with the cells its ghosts come from
+      if (e.rb > L - 3) e.rb = L;
+      return e;
+    };
+    lo = region(max(0, org), min(sl, kend));
+    hi = region(max(sr, org), min(L, kend));
+    if (line >= M) lo.kb = lo.ka, hi.kb = hi.ka;
+    // scratch: per line and end 3 arrays of `ends` values and one of cells
+    T *sc = tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows;
+    int *kf = reinterpret_cast<int *>(sc + (size_t)StreamCta<DIR, LN>::lines * 6 * ends);
+    const int li = warp * LPW + lw, side = c >= LN / 2;
+    sc += (size_t)li * 6 * ends;
+    kf += (size_t)(2 * li + side) * ends;
+    rl = sc + ends;
+    rr = sc + 4 * ends;
+    const StagedLine<T, ES> cells{col - b0 * ES, b0, b0 + nr, status};
+    if (c == 0 && line < M) {  // ghost cells of the staged line
+      T g1, g2;
+      if (b0 <= -2) {
+        ghosts(cells(0), cells(1), cells(2), g1, g2);
+        col[(-1 - b0) * ES] = g1;
+        col[(-2 - b0) * ES] = g2;
+      }
+      if (L + 2 - b0 <= nr && L - 3 >= b0) {
+        ghosts(cells(L - 1), cells(L - 2), cells(L - 3), g1, g2);
+        col[(L - b0) * ES] = g1;
+        col[(L + 1 - b0) * ES] = g2;
+      }
+    }
+    __syncwarp();
+    {
+      T *h = sc + side * 3 * ends;
+      end_inputs<T, ES, BND == 2, LN / 2>(*D, cells, line, side ? hi : lo, c % (LN / 2), h,
+                                          h + ends, h + 2 * ends, kf);
+    }
+  }
   // doubling steps that bring a carry in from every chunk of the warm-up (FP32:
   // one more, so that what is left out, |mu|^J of it at every chunk start, is
   // far below a rounding and not a share of one with the same sign everywhere)
-  const int ns = (J <= SCH ? 0 : J <= 2 * SCH ? 1 : 2) + (sizeof(T) == 4 ? 1 : 0);
+  // (the reference's lines of one segment: no warm-up, any decay length).
+  int ns = (F.JD <= SCH ? 0 : F.JD <= 2 * SCH ? 1 : 2) + (sizeof(T) == 4 ? 1 : 0);
+  if (BND && F.JD > 4 * SCH) ns = LN == 32 ? 5 : 4;
   T v[SCH];
-  stencil8<T, ES>(col + (ok ? r0 : 0) * ES, o, v);
+  if (BND) load_taps(o, wt);
+  stencil<T, ES, 8, false>(col + (ok ? r0 : 0) * ES, o, v);
+  if (BND == 2) {
+    load_taps(o, wt + 8);
+    stencil<T, ES, 8, true>(col + (ok ? k0 + 2 * n0 - 5 : 0) * ES, o, v);
+    load_taps(o, wt + 16);
+    stencil<T, ES, 5, true>(col + (ok ? k0 + 2 * n0 + 3 : 0) * ES, o, v);
+  }
+  const int kp = org + c * SCH;  // this lane's first position
+  if (BND) {
+    // lanes next to the line's ends take the prepared inputs (zero before the
+    // line) through their own rows: a loop over a few positions instead of 17
+    // predicated selects
+    __syncwarp();  // the cells of these rows have been read
+    if (kp < lo.kb || kp < 0 || kp + SCH > hi.ka) {
+      T *row = col + k0 * ES;
+#pragma unroll
+      for (int i = 0; i < SCH; ++i) row[i * ES] = v[i];
+      for (int k = kp; k < min(kp + SCH, lo.kb); ++k)
+        row[(k - kp) * ES] = k < 0 ? T(0) : rl[k - lo.ka];
+      for (int k = max(kp, hi.ka); k < min(kp + SCH, hi.kb); ++k)
+        row[(k - kp) * ES] = rr[k - hi.ka];
+#pragma unroll
+      for (int i = 0; i < SCH; ++i) v[i] = row[i * ES];
+    }
+  }
   T w = T(0);
 #pragma unroll
   for (int i = 0; i < SCH; ++i) w = v[i] + mmu * w;
@@ -288,12 +619,40 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     if (c == LN - 1) x = T(0);
   }
   __syncwarp();  // every lane of the line has read its cells
-  {
-    T *xp = col + k0 * ES;
+  T *xp = col + k0 * ES;
 #pragma unroll
-    for (int i = SCH - 1; i >= 0; --i) {
-      x = v[i] + mmu * x;
-      xp[i * ES] = x;
+  for (int i = SCH - 1; i >= 0; --i) {
+    x = v[i] + mmu * x;
+    if (BND) v[i] = x;
+    xp[i * ES] = x;
+  }
+  if (BND && p0 == 0) {
+    // non-cyclic system: A = c (1 + mu S^-1)(1 + mu S) + c mu^2 e_0 e_0^T, so
+    // x = y - y_0 g with g_k = mu^2 ((-mu)^k - (-mu)^(2L-k)) / (1 - mu^(2L+2))
+    // (Sherman-Morrison); y_0 is this segment's value at position 0, and g has
+    // decayed below rounding within the segment
+    __syncwarp();
+    const double q = -F.mu, a = (double)col[-b0 * ES] * D->rk_a;
+    __syncwarp();
+    if (kp < F.JD) {
+      double g = -a * powi(q, max(kp, 0));
+#pragma unroll
+      for (int i = 0; i < SCH; ++i)
+        if (kp + i >= 0) {
+          v[i] += T(g);
+          g *= q;
+        }
+      if (D->rk_tail) {
+        g = a * powi(q, 2 * L - min(kp + SCH, L) + 1);
+#pragma unroll
+        for (int i = SCH - 1; i >= 0; --i)
+          if (kp + i < L) {
+            v[i] += T(g);
+            g *= q;
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < SCH; ++i) xp[i * ES] = v[i];
     }
   }
   if (DIR == 0) __syncthreads(); else __syncwarp();
@@ -306,7 +665,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       const int g = 2 * ((int)threadIdx.x % G);
       if (line0 + g < M) {
         T *d = dst + (long long)p0 * s_pos + line0 + g;
-        const T *s = tile_s + H * X_PITCH + g;
+        const T *s = tile_s + (p0 - b0) * X_PITCH + g;
 #pragma unroll 4
         for (int r = (int)threadIdx.x / G; r < np; r += NT / G)
           *reinterpret_cast<Pair<T> *>(d + (long long)r * s_pos) =
@@ -316,7 +675,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       const int g = (int)threadIdx.x % X_LINES;
       if (line0 + g < M)
         for (int r = (int)threadIdx.x / X_LINES; r < np; r += NT / X_LINES)
-          dst[(long long)(p0 + r) * s_pos + line0 + g] = tile_s[(r + H) * X_PITCH + g];
+          dst[(long long)(p0 + r) * s_pos + line0 + g] = tile_s[(r + p0 - b0) * X_PITCH + g];
     }
   } else {
 #pragma unroll
@@ -324,7 +683,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       const int gl = line0 + warp * LPW + l;
       if (gl < M) {
         T *d = dst + (long long)gl * s_line + p0;
-        const T *s = tile_s + (size_t)(warp * LPW + l) * rows + H;
+        const T *s = tile_s + (size_t)(warp * LPW + l) * rows + p0 - b0;
         if (pairs)
           for (int e = 2 * lane; e < np; e += 64)
             *reinterpret_cast<Pair<T> *>(d + e) = *reinterpret_cast<const Pair<T> *>(s + e);
@@ -337,12 +696,18 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
 
 template <typename T>
 using StreamKernelT = void (*)(const PlanFields, const SweepField *, int, int, void *, int,
-                               unsigned *, int, int, const int *, int, int, const int *);
+                               unsigned *, int, int, const int *, int, int, const int *, int);
 
+template <typename T, int BND>
+StreamKernelT<T> stream_kernel_of(int dir, int lanes) {
+  if (dir == 0) return stream_kernel<T, 0, 16, BND>;
+  return lanes == 32 ? stream_kernel<T, 1, 32, BND> : stream_kernel<T, 1, 16, BND>;
+}
 template <typename T>
-StreamKernelT<T> stream_kernel_for(int dir, int lanes) {
-  if (dir == 0) return stream_kernel<T, 0, 16>;
-  return lanes == 32 ? stream_kernel<T, 1, 32> : stream_kernel<T, 1, 16>;
+StreamKernelT<T> stream_kernel_for(int variant, int dir, int lanes) {
+  return variant == SWEEP_COMPAT     ? stream_kernel_of<T, 1>(dir, lanes)
+         : variant == SWEEP_COMPAT_D ? stream_kernel_of<T, 2>(dir, lanes)
+                                     : stream_kernel_of<T, 0>(dir, lanes);
 }
 
 }  // namespace
@@ -351,18 +716,17 @@ int stream_tile_lines(int dir, int lanes) {
   return dir == 0 ? X_LINES : Y_WARPS * (32 / lanes);
 }
 
-size_t stream_smem_bytes(int dir, int lanes, int rows, bool fp64) {
-  const size_t n = dir == 0 ? (size_t)X_PITCH * rows
-                            : (size_t)stream_tile_lines(dir, lanes) * rows;
-  return n * (fp64 ? 8 : 4);
+size_t stream_smem_bytes(const LaunchGeom &G, bool fp64) {
+  const size_t el = fp64 ? 8 : 4, lines = stream_tile_lines(G.dir, G.lanes);
+  return (G.dir == 0 ? (size_t)X_PITCH : lines) * G.rows * el +
+         lines * 2 * (size_t)G.ends * (3 * el + sizeof(int));
 }
 
 template <typename T>
 cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
                           int nfields, int group_base, int groups_total, void *data,
-                          unsigned *d_status,
-                          int jstep, int nslice, const int *nlo, bool inplace,
-                          cudaStream_t stream, const int *g0idx, bool pdl) {
+                          unsigned *d_status, int jstep, int nslice, const int *nlo,
+                          bool inplace, cudaStream_t stream, const int *g0idx, bool pdl) {
   // Function attributes apply to the device that is current when they are
   // set: configure each device once (several host threads may launch).
   int dev = 0;
@@ -374,15 +738,14 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   if (!configured[dev].load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lk(config_mu);
     if (!configured[dev].load(std::memory_order_relaxed)) {
-      for (auto fn : {stream_kernel_for<T>(0, 16), stream_kernel_for<T>(1, 16),
-                      stream_kernel_for<T>(1, 32)}) {
-        err = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   227 * 1024);
-        if (err != cudaSuccess) return err;
-        err = cudaFuncSetAttribute((const void *)fn,
-                                   cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (err != cudaSuccess) return err;
-      }
+      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D})
+        for (int l : {0, 16, 32}) {
+          const void *fn = (const void *)stream_kernel_for<T>(v, l ? 1 : 0, l);
+          err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+          if (err != cudaSuccess) return err;
+          err = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+          if (err != cudaSuccess) return err;
+        }
       configured[dev].store(true, std::memory_order_release);
     }
   }
@@ -393,7 +756,7 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
                                 (unsigned)(groups_total / plan.tiles))
                          : dim3((unsigned)(groups_total * G.cs), 1, 1);
   cfg.blockDim = dim3((unsigned)((G.dir == 0 ? X_WARPS : Y_WARPS) * 32), 1, 1);
-  cfg.dynamicSmemBytes = stream_smem_bytes(G.dir, G.lanes, G.rows, sizeof(T) == 8);
+  cfg.dynamicSmemBytes = stream_smem_bytes(G, sizeof(T) == 8);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   unsigned na = 0;
@@ -414,9 +777,9 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   cfg.attrs = attr;
   cfg.numAttrs = na;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, stream_kernel_for<T>(G.dir, G.lanes), plan, d_fields, nfields,
+  return cudaLaunchKernelEx(&cfg, stream_kernel_for<T>(G.variant, G.dir, G.lanes), plan, d_fields, nfields,
                             by_value ? group_base / plan.tiles : group_base * G.cs, data, G.rows, d_status, jstep, nslice, nlo, G.cs,
-                            clustered, g0idx);
+                            clustered, g0idx, G.ends);
 }
 
 template cudaError_t launch_stream<double>(const LaunchGeom &, const PlanFields &,

@@ -1042,11 +1042,6 @@ __host__ __device__ inline int filter_tile_rows(int lc_max, int H) {
 // Exact (cluster) form: powers (-mu)^e for e = 0 .. FPW - 1 (a segment of at
 // most FLANES * FCH cells needs exponents up to FLANES * FCH).
 constexpr int FPW = FLANES * FCH + 8;
-// Wide stencil form (the reference scheme's third sweep, whose right-hand
-// side differentiates the remapped field): 13 taps, a table row of 16.
-constexpr int WIDE_TAPS = 13;
-constexpr int WIDE_TAPS_PAD = 16;
-
 template <typename T>
 struct FiltSmem {
   T *C;      // [filter_tile_rows * PITCH]  input cells, then w, then x
@@ -1061,13 +1056,13 @@ struct FiltSmem {
   int rows;
 };
 
-template <typename T, bool EXACT, bool CELL, bool WIDE>
+template <typename T, bool EXACT, bool CELL>
 __device__ __forceinline__ FiltSmem<T> carve_filt(unsigned char *raw, int lc_max, int H) {
   FiltSmem<T> s;
   s.fd = reinterpret_cast<SweepField *>(raw);
   s.n0 = reinterpret_cast<int *>(raw + FD_BYTES);
   T *p = reinterpret_cast<T *>(raw + FD_BYTES + 64 * sizeof(int));
-  s.om = p; p += (WIDE ? WIDE_TAPS_PAD : 8) * LPG;
+  s.om = p; p += 8 * LPG;
   s.pwt = p; p += 32;
   s.pwa = nullptr;
   s.ex = nullptr;
@@ -1084,17 +1079,6 @@ __device__ __forceinline__ FiltSmem<T> carve_filt(unsigned char *raw, int lc_max
     s.et = reinterpret_cast<double *>((a + 7) & ~uintptr_t(7));
   }
   return s;
-}
-
-// x^n (n >= 0) by binary powering, in FP64.
-__device__ __forceinline__ double powi(double x, int n) {
-  double r = 1.0;
-  while (n > 0) {
-    if (n & 1) r *= x;
-    x *= x;
-    n >>= 1;
-  }
-  return r;
 }
 
 // Per-cell right-hand side of the filter kernel (velocity fields whose feet
@@ -1224,47 +1208,41 @@ __device__ __forceinline__ T compat_remap(const SweepField &F, const CompatEdge<
   return remap_cell(F, vc, l.f, r.f);
 }
 
-// The per-line stencil table of one field (one thread per line).  Wide
-// (the reference scheme's third sweep, uniform displacement): b_k = R_k +
-// sum_t wq_t R_{k+n0-2+t} with R_j = sum_s wr_s C_{j+n0-2+s} (the compat
-// form's interior formulas) composes into 11 taps from C_{k+2n0-4}, valid for
-// n0 in [-3, 2]; with the mass matrix 13 taps from C_{k+2n0-5}, stored with
-// the shift 2n0-2 so that the kernel's first tap row is k + shift - 3.
+// The per-line stencil table of one field (one thread per line): eight taps
+// from C_{k+n0-3}.  deriv (the reference scheme's third sweep, uniform
+// displacement): b_k = R_k + sum_t wq_t R_{k+n0-2+t} with R_j = sum_s wr_s
+// C_{j+n0-2+s} (the interior formulas of the line) is two groups of taps, with
+// the mass matrix 8 from C_{k+n0-3} and 13 from C_{k+2n0-5}.
 template <typename T>
 __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__restrict__ wt,
-                                      int *__restrict__ nt, int lines, int wide) {
+                                      int *__restrict__ nt, int lines, int deriv) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= lines) return;
   const SweepField F = *f;
-  if (wide) {
-    double om[WIDE_TAPS_PAD];
-    for (int m = 0; m < WIDE_TAPS_PAD; ++m) om[m] = 0.0;
-    int shift = 0;
+  if (deriv) {
+    double om[STREAM_TAPS_D];
+    for (int m = 0; m < STREAM_TAPS_D; ++m) om[m] = 0.0;
+    int n0 = 0;
     if (l < F.M) {
       const double tau0 = F.t_min + F.ht * (double)l;
       const double f0 = edge_foot(F, 0, tau0, tau0 + F.ht, F.ta_rel, F.tb_rel);
-      double wr[6], wq[6];
-      int n0 = 0;
+      double wr[6], wq[6], wd[11];
       uniform_weights<double>(F, f0, wr, wq, &n0);
-      double bt[11];
-      for (int j = 0; j < 11; ++j) bt[j] = 0.0;
-      for (int sidx = 0; sidx < 6; ++sidx) {
-        const int j = sidx - n0 + 2;
-        if (j >= 0 && j < 11) bt[j] += wr[sidx];
-      }
+      for (int j = 0; j < 11; ++j) wd[j] = 0.0;
       for (int t = 0; t < 6; ++t)
-        for (int sidx = 0; sidx < 6; ++sidx) bt[t + sidx] += wq[t] * wr[sidx];
+        for (int s = 0; s < 6; ++s) wd[t + s] += wq[t] * wr[s];
+      // mass matrix (1/12c)(b_{k-1} + 10 b_k + b_{k+1}) of n taps at w
       const double icw = F.sm_inv_den / 12.0;
-      for (int m = 0; m < WIDE_TAPS; ++m) {
-        const double bm = m < 11 ? bt[m] : 0.0;                       // b_{k-1}
-        const double bc = (m >= 1 && m < 12) ? bt[m - 1] : 0.0;       // b_k
-        const double bp = m >= 2 ? bt[m - 2] : 0.0;                   // b_{k+1}
-        om[m] = icw * (bm + 10.0 * bc + bp);
-      }
-      shift = 2 * n0 - 2;
+      auto mass = [&](const double *w, int n, double *out) {
+        for (int m = 0; m < n + 2; ++m)
+          out[m] = icw * ((m < n ? w[m] : 0.0) + 10.0 * (m >= 1 && m <= n ? w[m - 1] : 0.0) +
+                          (m >= 2 ? w[m - 2] : 0.0));
+      };
+      mass(wr, 6, om);
+      mass(wd, 11, om + 8);
     }
-    for (int m = 0; m < WIDE_TAPS_PAD; ++m) wt[(size_t)l * WIDE_TAPS_PAD + m] = T(om[m]);
-    nt[l] = shift;
+    for (int m = 0; m < STREAM_TAPS_D; ++m) wt[(size_t)l * STREAM_TAPS_D + m] = T(om[m]);
+    nt[l] = n0;
     return;
   }
   if (l < F.M) {
@@ -1303,8 +1281,8 @@ __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__res
 // and the per-edge arithmetic: two CTAs per SM.
 // COMPAT (per-cell form only): the reference's boundaries, a separate
 // instantiation so that the periodic per-cell form carries none of their code.
-template <typename T, bool EXACT, bool CELL, bool COMPAT, bool WIDE = false>
-__global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
+template <typename T, bool EXACT, bool CELL, bool COMPAT>
+__global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
     sweep_filter_kernel(const SweepField *__restrict__ fields, int nfields, int group_base,
                         double toff, void *data_override, int lc_max, int H, unsigned *status,
                         int jstep, int nslice, const int *nlo, int cs, int clustered,
@@ -1321,7 +1299,7 @@ __global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
   // of different segment lengths share one launch (lc_max and H size the
   // shared memory only)
   const int cta = (int)blockIdx.x + group_base;
-  FiltSmem<T> S = carve_filt<T, EXACT, CELL, WIDE>(smem_raw, lc_max, H);
+  FiltSmem<T> S = carve_filt<T, EXACT, CELL>(smem_raw, lc_max, H);
   {
     // a field's CTAs start at cta0 = group0 * cs (cs is uniform over a launch);
     // only the threads that copy the descriptor search for it
@@ -1355,12 +1333,6 @@ __global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
   const int p1 = min(L, p0 + Lc);
   const int np = p1 - p0;
   const int nrows = np + 2 * H;
-  // compat lines split between two launches (SweepField::hyb): each launch
-  // keeps its own segments (uniform over the CTA, before any barrier)
-  if (!EXACT && F.hyb > 0 && !clustered) {
-    const bool interior = p0 >= F.hyb && p1 + F.hyb <= L;
-    if (CELL ? interior : !interior) return;
-  }
   const int J = EXACT ? 0 : F.jf;
   const T mu = T(F.sm_fac), ic = T(F.sm_inv_den);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1443,11 +1415,6 @@ __global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
   }
   if (CELL) {
     // per-cell form: no per-line stencil (b is computed per cell below)
-  } else if (WIDE) {  // wide stencil rows (WIDE_TAPS_PAD per line) and shifts
-    static_assert(WIDE_TAPS_PAD * LPG == NTH, "one table entry per thread");
-    const T *src = reinterpret_cast<const T *>(F.wt) + line0 * WIDE_TAPS_PAD + threadIdx.x;
-    if (sizeof(T) == 8) cp_async8(S.om + threadIdx.x, src); else cp_async4(S.om + threadIdx.x, src);
-    if (threadIdx.x < LPG) cp_async4(S.n0 + threadIdx.x, F.nt + line0 + threadIdx.x);
   } else if (F.wt) {  // per-line stencil from the plan's table, copied with the cells
     if (threadIdx.x < 8 * LPG) {
       const T *src = reinterpret_cast<const T *>(F.wt) + line0 * 8 + threadIdx.x;
@@ -1458,7 +1425,7 @@ __global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
     }
   }
   cp_async_commit();
-  if (!CELL && !WIDE && !F.wt && threadIdx.x < LPG) {
+  if (!CELL && !F.wt && threadIdx.x < LPG) {
     filter_line_stencil<T>(F, line0 + threadIdx.x, toff, S.om + 8 * threadIdx.x,
                            S.n0 + threadIdx.x);
   } else if (threadIdx.x == 9 * LPG) {
@@ -1739,7 +1706,7 @@ __global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
     const int qb = p1 + J;
     const int k0 = p0 - J + c * FCH;
     const int r0 = CELL ? k0 - 1 + rb : k0 + S.n0[ln] - 3 + rb;  // row of the first tap
-    const bool ok = r0 >= 0 && r0 + FCH + (CELL ? 2 : WIDE ? WIDE_TAPS - 1 : 7) <= S.rows;
+    const bool ok = r0 >= 0 && r0 + FCH + (CELL ? 2 : 7) <= S.rows;
     if (!ok) atomicOr(status, STATUS_HALO);
     T v[FCH];
     if (CELL) {
@@ -1758,27 +1725,6 @@ __global__ void __launch_bounds__(NTH, (CELL || WIDE) ? 2 : 4)
         v[i] = w;
         b0 = b1;
         b1 = b2;
-      }
-    } else if constexpr (WIDE) {
-      // w_k = sum of WIDE_TAPS taps of the cells from row r0 - mu w_{k-1}
-      const T *omp = S.om + WIDE_TAPS_PAD * ln;
-      T o[WIDE_TAPS], wv[WIDE_TAPS];
-#pragma unroll
-      for (int m = 0; m < WIDE_TAPS; ++m) o[m] = omp[m];
-      const T *cp = S.C + (ok ? r0 : 0) * PITCH + ln;
-#pragma unroll
-      for (int m = 0; m < WIDE_TAPS - 1; ++m) wv[m] = cp[m * PITCH];
-      T w = T(0);
-#pragma unroll
-      for (int i = 0; i < FCH; ++i) {
-        wv[WIDE_TAPS - 1] = cp[(WIDE_TAPS - 1 + i) * PITCH];
-        T mb = o[0] * wv[0];
-#pragma unroll
-        for (int m = 1; m < WIDE_TAPS; ++m) mb += o[m] * wv[m];
-        w = mb + mmu * w;
-        v[i] = w;
-#pragma unroll
-        for (int m = 0; m < WIDE_TAPS - 1; ++m) wv[m] = wv[m + 1];
       }
     } else {
       const T *omp = S.om + 8 * ln;
@@ -2032,11 +1978,10 @@ size_t sweep_smem_bytes(int lc_max, int halo, bool fp64, bool source) {
   return FD_BYTES + n * el;
 }
 
-size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact, bool cell,
-                               bool wide) {
+size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact, bool cell) {
   size_t el = fp64 ? 8 : 4;
   return FD_BYTES + 64 * sizeof(int) +
-         ((wide ? WIDE_TAPS_PAD : 8) * (size_t)LPG + 32 + (exact ? (size_t)FPW + 2 * LPG : 0) +
+         (8 * (size_t)LPG + 32 + (exact ? (size_t)FPW + 2 * LPG : 0) +
           (cell ? 2 : 1) * (size_t)filter_tile_rows(lc_max, halo) * PITCH) * el +
          (cell ? 8 * (size_t)FPW + 8 : 0);
 }
@@ -2044,15 +1989,15 @@ size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact, bool
 int filter_segment_max(int J) { return filter_seg_max(J); }
 
 cudaError_t launch_filter_weights(bool fp64, const SweepField *d_field, void *wt, int *nt,
-                                  int lines, cudaStream_t stream, bool wide) {
+                                  int lines, cudaStream_t stream, bool deriv) {
   const int bt = 128, grid = (lines + bt - 1) / bt;
   count_launch();
   if (fp64)
     filter_weights_kernel<double><<<grid, bt, 0, stream>>>(d_field, static_cast<double *>(wt), nt,
-                                                           lines, wide ? 1 : 0);
+                                                           lines, deriv ? 1 : 0);
   else
     filter_weights_kernel<float><<<grid, bt, 0, stream>>>(d_field, static_cast<float *>(wt), nt,
-                                                          lines, wide ? 1 : 0);
+                                                          lines, deriv ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -2075,8 +2020,7 @@ static FilterKernelT<T> filter_kernel_for(int variant) {
     case SWEEP_CELL: return sweep_filter_kernel<T, false, true, false>;
     case SWEEP_CELL_EXACT: return sweep_filter_kernel<T, true, true, false>;
     case SWEEP_CELL_COMPAT: return sweep_filter_kernel<T, false, true, true>;
-    case SWEEP_FILTER_WIDE: return sweep_filter_kernel<T, false, false, false, true>;
-    default: return sweep_filter_kernel<T, false, false, false>;
+    default: return nullptr;
   }
 }
 
@@ -2098,7 +2042,7 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
                                unsigned *d_status, int jstep, int nslice, const int *nlo,
                                bool inplace, cudaStream_t stream, const int *g0idx, bool pdl_ok) {
   const int variant = G.variant, cs = G.cs, lc_max = G.lc_max, halo = G.halo;
-  if (variant == SWEEP_FILTER)
+  if (stream_variant(variant))
     return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, data, d_status,
                             jstep, nslice, nlo, inplace, stream, g0idx, pdl_ok && pdl_enabled());
   const bool fast = (variant == SWEEP_FAST);
@@ -2106,8 +2050,7 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
   const bool exact = exact_filter_variant(variant);
   const bool filt = filter_variant(variant);
   const bool src = (variant == SWEEP_GENERAL_SRC);
-  const size_t smem = filt ? sweep_filter_smem_bytes(lc_max, halo, sizeof(T) == 8, exact, cell,
-                                                     variant == SWEEP_FILTER_WIDE)
+  const size_t smem = filt ? sweep_filter_smem_bytes(lc_max, halo, sizeof(T) == 8, exact, cell)
                       : fast ? sweep_fast_smem_bytes(lc_max, halo, sizeof(T) == 8)
                              : sweep_smem_bytes(lc_max, halo, sizeof(T) == 8, src);
   {
@@ -2126,12 +2069,10 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
       if (!configured[dev].load(std::memory_order_relaxed)) {
         for (const void *fn :
              {(const void *)sweep_kernel<T>, (const void *)sweep_fast_kernel<T>,
-              (const void *)filter_kernel_for<T>(SWEEP_FILTER_SEG),
               (const void *)filter_kernel_for<T>(SWEEP_FILTER_EXACT),
               (const void *)filter_kernel_for<T>(SWEEP_CELL),
               (const void *)filter_kernel_for<T>(SWEEP_CELL_EXACT),
-              (const void *)filter_kernel_for<T>(SWEEP_CELL_COMPAT),
-              (const void *)filter_kernel_for<T>(SWEEP_FILTER_WIDE)}) {
+              (const void *)filter_kernel_for<T>(SWEEP_CELL_COMPAT)}) {
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      227 * 1024);
           if (err != cudaSuccess) return err;

@@ -71,4 +71,15 @@ __device__ __forceinline__ void cp_async16(void *sdst, const void *gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
 }
 
+// x^n (n >= 0) by binary powering, in FP64.
+__device__ __forceinline__ double powi(double x, int n) {
+  double r = 1.0;
+  while (n > 0) {
+    if (n & 1) r *= x;
+    x *= x;
+    n >>= 1;
+  }
+  return r;
+}
+
 }  // namespace ccfv

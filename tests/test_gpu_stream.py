@@ -51,3 +51,39 @@ def test_stream_odd_base_address_gives_the_same_values(ccfv, nx, ny):
         s.run(c, 0.0, 1e-3, 3)
     s.check()
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,cfl", [(18, 0.7), (34, 2.6), (271, 0.8), (273, 0.8), (290, 12.8),
+                                   (545, 1.7), (1100, 3.3)])
+@pytest.mark.parametrize("vel,vp", [(0, ()), (1, (3.0, -3.7))], ids=["rot4", "const"])
+@pytest.mark.parametrize("scheme", [0, 1])
+def test_reference_boundaries_match_oracle(oracle, ccfv, N, cfl, vel, vp, scheme):
+    """Line ends of the reference's setting: inflow and outflow, feet several
+    cells away, both schemes (the reference's third sweep differentiates the
+    remapped field), lines of one lane group, one segment and several."""
+    from conftest import seeded_field
+    K, dt = 2e-3, cfl * (2.0 / N) / 4.0
+    C0 = seeded_field(N, N)
+    g = oracle.grid(N, K=K, vel=vel, vp=vp, threads=THREADS, scheme=scheme)
+    s = ccfv.Solver(ccfv.make_grid(N, K=K, velocity=vel, vel_params=vp, scheme=scheme))
+    assert [v for v, _ in s.sweep_plan(dt)] == ["cell_compat"] * 3
+    c = dev(C0)
+    s.run(c, 0.0, dt, 2)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
+
+
+def test_reference_boundaries_one_segment_any_diffusion(oracle, ccfv):
+    """A y line of one 32-lane segment needs no recurrence warm-up: diffusion
+    numbers far above the warm-up limit, on a grid whose x lines fit 16 lanes."""
+    from conftest import seeded_field
+    nx, ny, K = 200, 500, 0.5
+    dt = 0.8 * (2.0 / ny) / 4.0
+    C0 = seeded_field(nx, 3, ny=ny)
+    g = oracle.grid(nx, ny, K=K, threads=THREADS)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, K=K))
+    assert s.sweep_plan(dt)[1] == ("cell_compat", ny)
+    c = dev(C0)
+    s.run(c, 0.0, dt, 2)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
