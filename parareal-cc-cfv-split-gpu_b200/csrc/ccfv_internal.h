@@ -62,10 +62,11 @@ struct SweepField {
   int jmax;              // the field takes part while jstep < jmax (0: always)
   int smax;              // slice-indexed fields: while slice < smax
   int gskip;             // slice-indexed fields: skip slice == nlo (zero increment)
-  int kind;              // sub-step of the split step: 0 x(dt/2), 1 y(dt), 2 x(dt/2)
-  int pp;                // 1: out-of-place sequence: sweep s = 3 jstep + kind writes A
-                         // when s + par is odd, else B, and reads the other buffer
-                         // (in0 for s = 0); 0: in place on `data`
+  int jmin;              // ... and while jstep >= jmin
+  int s0, sj;            // pass of the launch in an out-of-place sequence: s0 + sj jstep
+  int pp;                // 1: out-of-place sequence: pass s writes A when s + par is
+                         // odd, else B, and reads the other buffer (in0 for s = 0);
+                         // 0: in place on `data`
   int par;               // pp = 1: parity offset (chosen so the last sweep writes A)
   int phase;             // slice-indexed fields: 0 every launch, 1 only while the
                          // instance's nlo < 0 (first coarse sweep), 2 only while
@@ -104,7 +105,7 @@ struct SweepField {
 // same rule on the host to skip launches in which no field is active.
 __host__ __device__ inline bool field_active(const SweepField &f, int jstep, int nslice,
                                              const int *nlo) {
-  if (f.jmax > 0 && jstep >= f.jmax) return false;
+  if ((f.jmax > 0 && jstep >= f.jmax) || jstep < f.jmin) return false;
   if (!nlo) return true;
   const int lo = nlo[f.inst];
   if (f.slice >= 0) return f.slice >= lo;
@@ -128,12 +129,13 @@ constexpr size_t FD_BYTES = (sizeof(SweepField) + 63) & ~size_t(63);
 // (non-cyclic system).
 // The streaming kernels (stream.cu) run SWEEP_FILTER and, with the reference's
 // boundaries, SWEEP_COMPAT and (the reference scheme's third sweep, derivative
-// of the remapped field) SWEEP_COMPAT_D.
+// of the remapped field) SWEEP_COMPAT_D.  SWEEP_FILTER_XX: the last x sweep of
+// a step and the first of the next one in one pass over the field.
 enum { SWEEP_GENERAL = 0, SWEEP_FAST = 1, SWEEP_FILTER = 2, SWEEP_GENERAL_SRC = 3,
        SWEEP_FILTER_EXACT = 4, SWEEP_CELL = 5, SWEEP_CELL_EXACT = 6, SWEEP_CELL_COMPAT = 7,
-       SWEEP_COMPAT = 8, SWEEP_COMPAT_D = 9 };
+       SWEEP_COMPAT = 8, SWEEP_COMPAT_D = 9, SWEEP_FILTER_XX = 10 };
 inline bool stream_variant(int v) {
-  return v == SWEEP_FILTER || v == SWEEP_COMPAT || v == SWEEP_COMPAT_D;
+  return v == SWEEP_FILTER || v == SWEEP_COMPAT || v == SWEEP_COMPAT_D || v == SWEEP_FILTER_XX;
 }
 // Variants run by the filter kernels (factored solve).
 inline bool filter_variant(int v) {
@@ -148,8 +150,11 @@ inline bool warm_filter_variant(int v) {
 // Variants whose right-hand side is the per-line stencil table (SweepField::wt),
 // and its values per line.
 inline bool stencil_filter_variant(int v) { return stream_variant(v) || v == SWEEP_FILTER_EXACT; }
-constexpr int STREAM_TAPS_D = 24;  // 8 + 13 taps, padded
-inline int stencil_taps(int v) { return v == SWEEP_COMPAT_D ? STREAM_TAPS_D : 8; }
+constexpr int STREAM_TAPS_D = 24;   // 8 + 13 taps, padded
+constexpr int STREAM_TAPS_XX = 16;  // 15 taps, padded
+inline int stencil_taps(int v) {
+  return v == SWEEP_COMPAT_D ? STREAM_TAPS_D : v == SWEEP_FILTER_XX ? STREAM_TAPS_XX : 8;
+}
 // Variants with the per-cell right-hand side.
 inline bool cell_filter_variant(int v) {
   return v == SWEEP_CELL || v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT;
@@ -168,6 +173,15 @@ struct LaunchGeom {
                           // line end (edges and cells next to it)
   int lc_fit = 0, halo_fit = 0;  // tile of the scan kernels: a step whose scan tile
                                  // does not fit is refused whatever form runs it
+};
+
+// Buffers of a single-field launch that replace its descriptor's, and how the
+// pass uses them (launch_sweep).
+enum { IO_IN_PLACE = 1, IO_FLIP = 2 };
+struct FieldIo {
+  void *data = nullptr;
+  const void *in = nullptr;
+  int mode = 0;
 };
 
 // The fields of a plan's launch by value: they differ only in their buffers
@@ -201,25 +215,27 @@ size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact = fal
 // recurrence warm-up of J cells.
 int filter_segment_max(int J);
 // Fills the per-line stencil table of the filter kernel for field `*d_field`
-// (device descriptor): wt = T[lines][8] (deriv: [STREAM_TAPS_D]), nt = int[lines], lines = groups*LPG
+// (device descriptor): wt = T[lines][stencil_taps(variant)], nt = int[lines], lines = groups*LPG
 // (lines past M get zeros).
 cudaError_t launch_filter_weights(bool fp64, const SweepField *d_field, void *wt, int *nt,
-                                  int lines, cudaStream_t stream, bool deriv = false);
+                                  int lines, cudaStream_t stream, int variant = SWEEP_FILTER);
 
 // Launches one fused sweep over all fields of `d_fields` (device array,
 // sorted by group0; tiles group_base .. group_base+groups_total-1).  All fields share G: the cluster size `cs`, their
 // max positions per CTA `lc_max` and the halo `halo` (LaunchGeom).  `toff` is added to
 // every field's ta_rel/tb_rel (the launch time); `data` (if non-null)
-// replaces fields[0].data (single-field launches).  `jstep` is the step of an
-// out-of-place sequence (SweepField::pp); `inplace` says whether any field
+// replaces fields[0].data and `in` (if non-null, else `data`) its in0
+// (single-field launches).  `jstep` is the step of an out-of-place sequence
+// (SweepField::pp); `mode`: IO_IN_PLACE writes this pass over its input,
+// IO_FLIP exchanges the two buffers of a pass; `inplace` says whether any field
 // sweeps in place (the filter kernel's segments of a line then form a
 // cluster).  `plan`: the same fields by value where they allow it (see
 // PlanFields; the streaming form then reads no descriptor).
 template <typename T>
 cudaError_t launch_sweep(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
-                         int nfields, int group_base, int groups_total, double toff, void *data,
-                         unsigned *d_status, cudaStream_t stream, int jstep = 0,
-                         bool inplace = true);
+                         int nfields, int group_base, int groups_total, double toff,
+                         const FieldIo &io, unsigned *d_status, cudaStream_t stream,
+                         int jstep = 0, bool inplace = true);
 
 // Batched form: `jstep` / `nslice` select the step and slice of this launch,
 // `nlo[inst]` the first active slice of every instance (see SweepField).
@@ -236,7 +252,7 @@ cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, 
 // The streaming form's launch (stream_variant), called by the two above.
 template <typename T>
 cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
-                          int nfields, int group_base, int groups_total, void *data,
+                          int nfields, int group_base, int groups_total, const FieldIo &io,
                           unsigned *d_status,
                           int jstep, int nslice, const int *nlo, bool inplace,
                           cudaStream_t stream, const int *g0idx, bool pdl);

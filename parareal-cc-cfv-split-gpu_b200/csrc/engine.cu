@@ -326,6 +326,15 @@ static void stream_geom(LaunchGeom &G, int L, int J, int reach, int lc) {
   G.rows = (G.lanes * STREAM_CH + 2 * (G.halo - J) + 2) & ~1;
 }
 
+// Warm-up of a first-order recurrence run twice in a row: started from zero J
+// cells early, what is missing is (J (1 - |mu|) + 1) |mu|^J of the result.
+static int double_warm_up(double mu, bool fp64) {
+  const double eps = std::ldexp(1.0, fp64 ? -56 : -27), m = std::fabs(mu);
+  int J = 1;
+  while (J < 4 * FILTER_JMAX && (J * (1.0 - m) + 1.0) * std::pow(m, J) > eps) ++J;
+  return J;
+}
+
 // Streaming form with the reference's boundaries.  A line that the lanes of
 // one segment hold is solved without warm-up at any diffusion number (jok:
 // whether the warm-up is short enough for longer lines).  False: the other
@@ -445,6 +454,26 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
   return G;
 }
 
+bool fused_x_geom(const ccfv_grid &g, double dt, bool fp64, bool inplace, double theta,
+                  LaunchGeom *G) {
+  // periodic lines on the stencil, every sweep alike (the reference's third
+  // sweep is not, and velocity fields with feet of their own depend on time).
+  // FP32 increments keep the two sweeps: the rounding of 15 composed taps
+  // biases a smooth field more than that of 8 taps twice (2e-7 against 2e-8 of
+  // the increment on a 100^2 problem).
+  if (!fp64) return false;
+  *G = step_geom(g, 0, 0.5 * dt, 0, fp64, inplace, theta);
+  if (G->variant != SWEEP_FILTER || g.scheme != CCFV_SCHEME_CONSISTENT) return false;
+  double mu = 0;
+  filter_params(g, 0, 0.5 * dt, fp64, &mu, nullptr, nullptr, theta);
+  const int J = double_warm_up(mu, fp64);
+  if (g.nx <= 2 * J || 2 * J + 64 > 16 * STREAM_CH) return false;
+  G->variant = SWEEP_FILTER_XX;
+  stream_geom(*G, g.nx, J, 2 * shift_cells(g, 0, 0.5 * dt) + 10, stream_lc(g.nx, fp64));
+  if (inplace && G->cs > MAX_CLUSTER) return false;
+  return stream_smem_bytes(*G, fp64) <= 227 * 1024;
+}
+
 // Times the filter kernel's candidate segment lengths on this grid (x and y
 // sweeps of one step of dt on a scratch field) and keeps the fastest.
 int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, bool for_class) {
@@ -494,11 +523,10 @@ int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, 
       g_lc_override = 0;
       break;  // nothing to tune: this grid does not use the filter kernel
     }
-    if (rc == CCFV_OK) rc = run_step_plan(ctx, plan, fp64, 0, (int)nf, 0.0, nullptr, st, 0);
+    if (rc == CCFV_OK) rc = run_steps(ctx, plan, fp64, 0, (int)nf, 0.0, dt, 1, st);
     if (rc == CCFV_OK) {
       cudaEventRecord(a, st);
-      for (int r = 0; r < 5 && rc == CCFV_OK; ++r)
-        rc = run_step_plan(ctx, plan, fp64, 0, (int)nf, 0.0, nullptr, st, r);
+      rc = run_steps(ctx, plan, fp64, 0, (int)nf, 0.0, dt, 5, st);
       cudaEventRecord(b, st);
       cudaEventSynchronize(b);
       float ms = 0;
@@ -541,6 +569,7 @@ void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom
   filter_params(g, f.dir, f.Dt, fp64, &mu, &ic, &J, f.theta);
   f.sm_fac = mu;
   f.sm_inv_den = ic;
+  if (G.variant == SWEEP_FILTER_XX) J = double_warm_up(mu, fp64);
   f.jd = J;
   // compat lines of one segment: the non-cyclic recurrences start exactly at
   // the line's ends (no warm-up)
@@ -552,7 +581,7 @@ void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom
 // Sub-steps of one split step: x(dt/2) over [t, t+dt/2], y(dt) over
 // [t, t+dt], x(dt/2) over [t+dt/2, t+dt] (GpuOneStep, T2S4:785-968).
 static void sweep_kind(int kind, double dt, int *dir, double *Dt, double *ta, double *tb) {
-  if (kind == 0) { *dir = 0; *Dt = 0.5 * dt; *ta = 0.0; *tb = 0.5 * dt; }
+  if (kind == 0 || kind == 3) { *dir = 0; *Dt = 0.5 * dt; *ta = 0.0; *tb = 0.5 * dt; }
   else if (kind == 1) { *dir = 1; *Dt = dt; *ta = 0.0; *tb = dt; }
   else { *dir = 0; *Dt = 0.5 * dt; *ta = 0.5 * dt; *tb = dt; }
 }
@@ -573,8 +602,12 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
   ccfv_grid g = ctx->grid;
   if (homogeneous) g.source = CCFV_SRC_NONE;
   const int nf = (int)fields.size();
-  std::vector<SweepField> h(3 * (size_t)nf);
-  for (int kind = 0; kind < 3; ++kind) {
+  const bool plan_pp = !fields.empty() && fields[0].B != nullptr;
+  LaunchGeom GX;
+  plan->fused = !ctx->force_general && fused_x_geom(g, dt, fp64, !plan_pp, theta, &GX);
+  const int kinds = plan->fused ? 4 : 3;
+  std::vector<SweepField> h(kinds * (size_t)nf);
+  for (int kind = 0; kind < kinds; ++kind) {
     int dir;
     double Dt, ta, tb;
     sweep_kind(kind, dt, &dir, &Dt, &ta, &tb);
@@ -582,8 +615,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
     int st = CCFV_OK;
     const SolverTable *tab = get_table(ctx, dir, Dt, fp64, &st, theta);
     if (!tab) return st;
-    const bool plan_pp = !fields.empty() && fields[0].B != nullptr;
-    LaunchGeom G = step_geom(g, dir, Dt, dsrc, fp64, !plan_pp, theta);
+    LaunchGeom G = kind == 3 ? GX : step_geom(g, dir, Dt, dsrc, fp64, !plan_pp, theta);
     if (ctx->force_general && G.variant != SWEEP_GENERAL_SRC) G.variant = SWEEP_GENERAL;
     if (G.cs > MAX_CLUSTER && !(warm_filter_variant(G.variant) && plan_pp))
       return set_error(ctx, CCFV_ERR_UNSUPPORTED, "line longer than 4096 cells");
@@ -595,12 +627,13 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
     for (int i = 0; i < nf; ++i) {
       const PlanField &pfi = fields[i];
       SweepField f = make_field(g, dir, Dt, ta + pfi.t0, tb + pfi.t0, pfi.A, tab, dsrc, theta);
-      f.kind = kind;
+      f.s0 = kind == 3 ? 2 : kind;
+      f.sj = plan->fused ? 2 : 3;
       if (pfi.B) {
         f.pp = 1;
         f.data2 = pfi.B;
         f.in0 = pfi.in0;
-        f.par = pfi.par;
+        f.par = plan_passes(plan->fused, pfi.ends) & (pfi.ends > 0 ? 1 : 0);
       }
       if (filter_variant(G.variant)) filter_field(g, f, fp64, G);
       f.src_tb = kind == 2 ? 1 : 0;
@@ -614,12 +647,12 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
     plan->geom[kind] = G;
   }
   plan->nf = nf;
-  plan->pp = nf > 0 && fields[0].B != nullptr;
+  plan->pp = plan_pp;
   // filter sub-steps: one per-line stencil table per kind, shared by the
   // plan's fields (same grid and sub-step; the velocity fields of the filter
   // kernel do not depend on time)
-  int lines[3] = {0, 0, 0};
-  for (int kind = 0; kind < 3 && nf > 0; ++kind) {
+  int lines[4] = {0, 0, 0, 0};
+  for (int kind = 0; kind < kinds && nf > 0; ++kind) {
     if (!stencil_filter_variant(plan->geom[kind].variant)) continue;
     lines[kind] = h[(size_t)kind * nf].groups * tile_lines(plan->geom[kind]);
     CK(plan->wt[kind].alloc((fp64 ? 8 : 4) * stencil_taps(plan->geom[kind].variant) *
@@ -630,7 +663,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
       h[(size_t)kind * nf + i].nt = plan->nt[kind].as<int>();
     }
   }
-  for (int kind = 0; kind < 3 && nf > 0; ++kind) {
+  for (int kind = 0; kind < kinds && nf > 0; ++kind) {
     const SweepField *hk = h.data() + (size_t)kind * nf;
     PlanFields &pv = plan->by_value[kind];
     pv.f = hk[0];
@@ -647,29 +680,36 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
   }
   CK(plan->fields.alloc(sizeof(SweepField) * h.size()));
   CK(cudaMemcpy(plan->fields.p, h.data(), sizeof(SweepField) * h.size(), cudaMemcpyHostToDevice));
-  for (int kind = 0; kind < 3; ++kind)
+  for (int kind = 0; kind < kinds; ++kind)
     if (lines[kind])
       CK(launch_filter_weights(fp64, plan->fields.as<SweepField>() + (size_t)kind * nf,
                                plan->wt[kind].p, plan->nt[kind].as<int>(), lines[kind], 0,
-                               plan->geom[kind].variant == SWEEP_COMPAT_D));
+                               plan->geom[kind].variant));
   CK(cudaStreamSynchronize(0));
   return CCFV_OK;
 }
 
-int run_step_plan(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int count,
-                  double toff, void *data_override, cudaStream_t st, int jstep) {
-  const SweepField *base = plan.fields.as<SweepField>();
+int run_steps(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int count, double t0,
+              double dt, int nsteps, cudaStream_t st, const FieldIo &io0, bool y_in_place) {
   unsigned *status = ctx->status.as<unsigned>();
-  for (int kind = 0; kind < 3; ++kind) {
+  auto launch = [&](int kind, int n, const FieldIo &io, bool inplace) {
     const LaunchGeom &G = plan.geom[kind];
     const int gpf = plan.groups_per_field[kind];
-    const SweepField *fk = base + (size_t)kind * plan.nf;
-    cudaError_t e =
-        fp64 ? launch_sweep<double>(G, plan.by_value[kind], fk, plan.nf, first * gpf,
-                                    count * gpf, toff, data_override, status, st, jstep, !plan.pp)
-             : launch_sweep<float>(G, plan.by_value[kind], fk, plan.nf, first * gpf, count * gpf,
-                                   toff, data_override, status, st, jstep, !plan.pp);
-    CK(e);
+    const SweepField *fk = plan.fields.as<SweepField>() + (size_t)kind * plan.nf;
+    const double toff = t0 + n * dt;
+    return fp64 ? launch_sweep<double>(G, plan.by_value[kind], fk, plan.nf, first * gpf,
+                                       count * gpf, toff, io, status, st, n, inplace)
+                : launch_sweep<float>(G, plan.by_value[kind], fk, plan.nf, first * gpf,
+                                      count * gpf, toff, io, status, st, n, inplace);
+  };
+  for (int n = 0; n < nsteps; ++n) {
+    const bool last = n == nsteps - 1;
+    FieldIo io = io0;
+    if (n == 0 || !plan.fused) CK(launch(0, n, io, !plan.pp));
+    if (last && y_in_place) io.mode = io0.mode | IO_IN_PLACE;
+    CK(launch(1, n, io, !plan.pp || (last && y_in_place)));
+    if (last && y_in_place) io.mode = io0.mode ^ IO_FLIP;
+    CK(launch(plan.fused && !last ? 3 : 2, n, io, !plan.pp));
   }
   return CCFV_OK;
 }
@@ -703,23 +743,33 @@ static StepPlan *single_plan(ccfv_ctx *ctx, double dt, bool fp64, int *status, d
   return res;
 }
 
-// nsteps split steps on one field: 3 nsteps sweeps alternating between the
-// field and the scratch field; an odd count ends in the scratch field and is
-// copied back.
+// nsteps split steps on one field, passes alternating between the field and the
+// scratch field.  A second field to start from only sets the parity that ends
+// in d_C.  In place, an odd number of passes would end in the scratch field:
+// the last y sweep then writes over its input (a line's segments form one
+// cluster), which costs nothing where copying the result back was one more
+// pass over the field (4096^2 step: 208 us with the copy, 172 us without);
+// lines of more segments than a cluster holds are copied.
 int steps(ccfv_ctx *ctx, void *d_C, bool fp64, double t0, double dt, int nsteps, cudaStream_t st,
-          double theta) {
+          double theta, const void *src) {
   int status = CCFV_OK;
+  const size_t bytes =
+      (fp64 ? sizeof(double) : sizeof(float)) * (size_t)ctx->grid.nx * ctx->grid.ny;
+  if (nsteps <= 0) {
+    if (src) CK(cudaMemcpyAsync(d_C, src, bytes, cudaMemcpyDeviceToDevice, st));
+    return CCFV_OK;
+  }
   StepPlan *plan = single_plan(ctx, dt, fp64, &status, theta);
   if (!plan) return status;
-  for (int n = 0; n < nsteps; ++n) {
-    int rc = run_step_plan(ctx, *plan, fp64, 0, 1, t0 + n * dt, d_C, st, n);
-    if (rc) return rc;
-  }
-  if ((3 * nsteps) & 1) {
-    const size_t el = fp64 ? sizeof(double) : sizeof(float);
-    CK(cudaMemcpyAsync(d_C, (fp64 ? ctx->pp64 : ctx->pp32).p,
-                       el * (size_t)ctx->grid.nx * ctx->grid.ny, cudaMemcpyDeviceToDevice, st));
-  }
+  const bool odd = plan_passes(plan->fused, nsteps) & 1;
+  FieldIo io;
+  io.data = d_C;
+  io.in = src;
+  if (src && odd) io.mode = IO_FLIP;
+  const bool y_in_place = !src && odd && plan->geom[1].cs <= MAX_CLUSTER;
+  if (int rc = run_steps(ctx, *plan, fp64, 0, 1, t0, dt, nsteps, st, io, y_in_place)) return rc;
+  if (!src && odd && !y_in_place)
+    CK(cudaMemcpyAsync(d_C, (fp64 ? ctx->pp64 : ctx->pp32).p, bytes, cudaMemcpyDeviceToDevice, st));
   return CCFV_OK;
 }
 
@@ -874,7 +924,7 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
       fl[n].t0 = o->t0 + n * DT;
       fl[n].B = FS + (size_t)n * NN;
       fl[n].in0 = U + (size_t)n * NN;
-      fl[n].par = pp_parity(J);
+      fl[n].ends = J;
     }
     int rc = build_step_plan(ctx, plan.get(), dt, true, fl);
     if (rc) return rc;
@@ -907,7 +957,7 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
   }
   const StepPlan *dplan =
       (o->form == CCFV_FORM_DELTA && g.source != CCFV_SRC_NONE) ? &hplan : &cplan;
-  const TG *Wres = ((3 * m) & 1) ? W2 : W;
+  const TG *Wres = (plan_passes(dplan->fused, m) & 1) ? W2 : W;
 
   cudaEvent_t ev0, ev1;
   CK(cudaEventCreate(&ev0));
@@ -917,18 +967,13 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
   CK(cudaMemcpyAsync(U, C0, fb, k_in, st));
 
   auto coarse_on_W = [&](int n, const StepPlan *plan) -> int {
-    for (int i = 0; i < m; ++i) {
-      int rc = run_step_plan(ctx, *plan, g64, 0, 1, o->t0 + n * DT + i * dtc, nullptr, st, i);
-      if (rc) return rc;
-    }
-    return CCFV_OK;
+    return run_steps(ctx, *plan, g64, 0, 1, o->t0 + n * DT, dtc, m, st);
   };
 
   // k = 0: coarse sweep U[n+1] = G(U[n])  (T2S4:1271-1280), FP64
   for (int n = 0; n < S; ++n) {
     double *un1 = U + (size_t)(n + 1) * NN;
-    CK(cudaMemcpyAsync(un1, U + (size_t)n * NN, fb, cudaMemcpyDeviceToDevice, st));
-    int rc = steps(ctx, un1, true, o->t0 + n * DT, dtc, m, st, th);
+    int rc = steps(ctx, un1, true, o->t0 + n * DT, dtc, m, st, th, U + (size_t)n * NN);
     if (rc) return rc;
     if (Gold) CK(cudaMemcpyAsync(Gold + (size_t)(n + 1) * NN, un1, fb, cudaMemcpyDeviceToDevice, st));
   }
@@ -947,22 +992,21 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
     const int act = S - nlo;
     // F-phase: F[n+1] = F(U[n]) for every active slice, out of place
     CK(cudaEventRecord(fa, st));
-    for (int j = 0; j < J; ++j) {
-      int rc = run_step_plan(ctx, *ctx->fine_plan, true, nlo, act, j * dt, nullptr, st, j);
-      if (rc) return rc;
-    }
+    if (int rc = run_steps(ctx, *ctx->fine_plan, true, nlo, act, 0.0, dt, J, st)) return rc;
     CK(cudaEventRecord(fb_, st));
     fine_cu += (double)act * J * NN;
-    fine_launches += 3LL * J;
-    fine_cells += 3LL * J * act * NN;
+    fine_launches += plan_passes(ctx->fine_plan->fused, J);
+    fine_cells += (long long)plan_passes(ctx->fine_plan->fused, J) * act * NN;
     // G-phase + correction
     CK(cudaMemsetAsync(norms, 0, sizeof(double) * 2 * (S + 1), st));
     for (int n = nlo; n < S; ++n) {
       int rc;
       const TG *Gn = Wres;  // where this slice's G value ends up
       if (o->form == CCFV_FORM_STANDARD) {
-        CK(cudaMemcpyAsync(W, U + (size_t)n * NN, fb, cudaMemcpyDeviceToDevice, st));
-        if ((rc = coarse_on_W(n, &cplan))) return rc;
+        FieldIo io;  // from U[n] (already updated) through the pair W / W2
+        io.data = W;
+        io.in = U + (size_t)n * NN;
+        if ((rc = run_steps(ctx, cplan, g64, 0, 1, o->t0 + n * DT, dtc, m, st, io))) return rc;
         coarse_cu += (double)m * NN;
       } else if (n == nlo) {
         CK(cudaMemsetAsync(W, 0, sizeof(TG) * NN, st));  // G(0) = 0
@@ -1071,8 +1115,7 @@ int fine_slices(ccfv_ctx *ctx, double *d_fields, int n, double t0, double slice_
   for (int i = 0; i < n; ++i) fl.push_back({d_fields + (size_t)i * NN, t0 + i * slice_dt});
   int rc = build_step_plan(ctx, &plan, dt, true, fl);
   if (rc) return rc;
-  for (int j = 0; j < J; ++j)
-    if ((rc = run_step_plan(ctx, plan, true, 0, n, j * dt, nullptr, st))) return rc;
+  if ((rc = run_steps(ctx, plan, true, 0, n, 0.0, dt, J, st))) return rc;
   CK(cudaStreamSynchronize(st));  // the plan's descriptors are released on return
   return CCFV_OK;
 }

@@ -38,30 +38,33 @@ struct SolverTable {
   double sm_fac = 0, sm_inv_den = 0;
 };
 
-// Three sweep launches (x dt/2, y dt, x dt/2) of one step over a set of fields.
+// The sweep launches of a sequence of steps over a set of fields: kinds x(dt/2),
+// y(dt), x(dt/2), and, where the x sweeps of neighbouring steps fuse
+// (SWEEP_FILTER_XX), the last one of a step with the first of the next.
 struct StepPlan {
-  DevBuf fields;          // SweepField[3][nf]
+  DevBuf fields;          // SweepField[kinds][nf]
   int nf = 0;
-  int groups_per_field[3] = {0, 0, 0};
-  LaunchGeom geom[3];
-  PlanFields by_value[3];  // the same fields as a kernel argument
+  bool fused = false;     // steps run x y (xx y)* x: 2 n + 1 passes, else 3 n
+  int groups_per_field[4] = {0, 0, 0, 0};
+  LaunchGeom geom[4];
+  PlanFields by_value[4];  // the same fields as a kernel argument
   bool pp = false;        // out-of-place sequence (SweepField::pp)
-  DevBuf wt[3], nt[3];    // filter kernel: per-line stencil tables per sub-step kind
+  DevBuf wt[4], nt[4];    // filter kernel: per-line stencil tables per sub-step kind
 };
 
 // One field of a plan: swept in place on A (B == nullptr), or an out-of-place
-// sequence of steps over the pair A/B that starts from in0 and, with parity
-// offset par, ends in A (SweepField::pp).  t0: the field's time origin.
+// sequence of passes over the pair A/B that starts from in0 (SweepField::pp).
+// ends: > 0, a sequence of that many steps ends in A (the parity offset is
+// chosen so); 0: its first pass writes B.  t0: the field's time origin.
 struct PlanField {
   void *A = nullptr;
   double t0 = 0.0;
   void *B = nullptr;
   const void *in0 = nullptr;
-  int par = 0;
+  int ends = 0;
 };
-// Parity offset that makes a sequence of `steps` split steps (3 sweeps each)
-// end in buffer A.
-inline int pp_parity(int steps) { return (3 * steps) & 1; }
+// Passes over the field of n steps.
+inline int plan_passes(bool fused, int n) { return fused ? 2 * n + 1 : 3 * n; }
 
 }  // namespace ccfv
 
@@ -125,11 +128,20 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
 int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
                     const std::vector<PlanField> &fields, bool homogeneous = false,
                     double theta = 0.5);
-// jstep: the step's index in an out-of-place sequence (selects the buffers).
-int run_step_plan(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int count,
-                  double toff, void *data_override, cudaStream_t st, int jstep = 0);
+// nsteps steps of dt from t0 on fields first .. first+count-1 of a plan.  io:
+// buffers of a single field that replace the plan's; y_in_place: the last
+// step's y sweep writes over its input, so that the sequence ends in the
+// other buffer than its number of passes says.
+int run_steps(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int count, double t0,
+              double dt, int nsteps, cudaStream_t st, const FieldIo &io = FieldIo(),
+              bool y_in_place = false);
+// nsteps steps of the field `src` into d_C (null: d_C in place).
 int steps(ccfv_ctx *ctx, void *d_C, bool fp64, double t0, double dt, int nsteps, cudaStream_t st,
-          double theta = 0.5);
+          double theta = 0.5, const void *src = nullptr);
+// Whether the x sweeps of neighbouring steps of dt fuse into one pass, and its
+// geometry.
+bool fused_x_geom(const ccfv_grid &g, double dt, bool fp64, bool inplace, double theta,
+                  LaunchGeom *G);
 int coarse_fp32(ccfv_ctx *ctx, double *d_C, double tn, double DT, int m, cudaStream_t st,
                 double theta = 0.5);
 int fine_slices(ccfv_ctx *ctx, double *d_fields, int n, double t0, double slice_dt, double DT,

@@ -153,7 +153,10 @@ static void prepare_field(std::vector<PreparedField> &out, int kind, const ccfv_
                           const SweepField &f0, bool fp64, FilterTables *tabs,
                           std::tuple<int, int, int> tkey) {
   PreparedField pf;
-  pf.G = step_geom(g, f0.dir, f0.Dt, f0.dsrc, fp64, /*inplace=*/false, f0.theta);
+  if (kind == 3)
+    fused_x_geom(g, 2.0 * f0.Dt, fp64, /*inplace=*/false, f0.theta, &pf.G);
+  else
+    pf.G = step_geom(g, f0.dir, f0.Dt, f0.dsrc, fp64, /*inplace=*/false, f0.theta);
   const bool filt = filter_variant(pf.G.variant);
   // segment-length bucket bounds the tile; streaming form: lanes per line
   const int bucket = stream_variant(pf.G.variant) ? pf.G.lanes
@@ -170,7 +173,7 @@ static void prepare_field(std::vector<PreparedField> &out, int kind, const ccfv_
     if (!T.lines) {
       T.lines = pf.f.groups * tile_lines(pf.G);
       T.fp64 = fp64;
-      T.deriv = pf.G.variant == SWEEP_COMPAT_D;
+      T.variant = pf.G.variant;
       T.level = pf.level;
       T.wt.alloc((fp64 ? 8 : 4) * stencil_taps(pf.G.variant) * (size_t)T.lines);
       T.nt.alloc(sizeof(int) * (size_t)T.lines);
@@ -428,8 +431,27 @@ int MultiEngine::rebuild() {
     Problem *P = slots_[i].get();
     if (!live(P)) continue;
     const ccfv_grid &g = P->g;
-    // coarse sequences start in W and end in W2 when 3m is odd
-    he[i] = BElem{P->U, P->F, P->Gold, P->W, ((3 * P->m) & 1) ? P->W2 : P->W, P->NN, P->S,
+    // The x sweeps of neighbouring steps in one pass (kind 3), where the form
+    // allows it: the first x sweep then runs in step 0 only and the last one in
+    // the last step.  A coarse sequence has one parity for the states of the
+    // first sweep (FP64) and the increments of the iterations, so FP32
+    // increments (not fused) keep both as they are.
+    LaunchGeom gx;
+    const bool fuse_f = P->J > 1 && fused_x_geom(g, P->dt, true, false, 0.5, &gx);
+    const bool fuse_c =
+        P->m > 1 && P->g64 && fused_x_geom(g, P->dtc, true, false, P->theta, &gx);
+    // where kind's field of an n-step sequence takes part, and its pass
+    auto place_pass = [](SweepField &f, int kind, int n, bool fused) {
+      f.jmax = n;
+      f.s0 = kind == 3 ? 2 : kind;
+      f.sj = fused ? 2 : 3;
+      if (fused && kind == 0) f.jmax = 1;
+      if (fused && kind == 2) f.jmin = n - 1;
+      if (kind == 3) f.jmax = n - 1;
+    };
+    // coarse sequences start in W and end in W2 when their passes are odd
+    const int cpass = plan_passes(fuse_c, P->m);
+    he[i] = BElem{P->U, P->F, P->Gold, P->W, (cpass & 1) ? P->W2 : P->W, P->NN, P->S,
                   P->o.form, P->g64 ? 1 : 0, 0, norms_d_.as<double>() + norm_off_[i]};
     // resident coarse propagator: delta form, periodic, the coarse field in
     // one SM's shared memory (CCFV_RESIDENT_G=0 keeps every problem in the
@@ -440,10 +462,10 @@ int MultiEngine::rebuild() {
                          resident_g_fits(g.nx, g.ny, P->g64,
                                          g.velocity == CCFV_VEL_SWIRL);
     std::vector<PreparedField> rg_prep;  // its iterations' coarse fields, if resident
-    for (int kind = 0; kind < 3 && !P->prepared; ++kind) {
+    for (int kind = 0; kind < 4 && !P->prepared; ++kind) {
       const int dir = kind == 1 ? 1 : 0;
       const int dsrc = (kind == 2 && g.scheme == CCFV_SCHEME_REFERENCE) ? 1 : 0;
-      {  // fine: field s = F[s+1], time t0 + s DT (+ j dt per launch step)
+      if (kind < 3 || fuse_f) {  // fine: field s = F[s+1], time t0 + s DT (+ j dt per launch step)
         const double Dt = kind == 1 ? P->dt : 0.5 * P->dt;
         const double ta = kind == 2 ? 0.5 * P->dt : 0.0, tb = kind == 0 ? 0.5 * P->dt : P->dt;
         for (int s = 0; s < P->S; ++s) {
@@ -452,33 +474,31 @@ int MultiEngine::rebuild() {
           f.inst = i;
           f.slice = s;
           f.src_tb = kind == 2 ? 1 : 0;
-          f.jmax = P->J;
+          place_pass(f, kind, P->J, fuse_f);
           f.t_step = P->dt;
           // out of place: U[s] -> ... -> F[s+1] through the pair F[s+1] / FS[s]
-          f.kind = kind;
           f.pp = 1;
           f.data2 = P->FS + (size_t)s * P->NN;
           f.in0 = P->U + (size_t)s * P->NN;
-          f.par = pp_parity(P->J);
+          f.par = plan_passes(fuse_f, P->J) & 1;
           prepare_field(P->prep, kind, g, f, true, &P->ftab, std::make_tuple(kind, 0, 1));
         }
       }
-      {  // coarse: the work field W, slice from the launch (t0 + n DT + i dtc)
-        const double Dt = kind == 1 ? P->dtc : 0.5 * P->dtc;
+      if (kind < 3 || fuse_c) {  // coarse: the work field W, slice from the launch (t0 + n DT + i dtc)
+        const double Dt = kind == 1 ? P->dtc : 0.5 * P->dtc;  // kind 3: as 0
         const double ta = kind == 2 ? 0.5 * P->dtc : 0.0, tb = kind == 0 ? 0.5 * P->dtc : P->dtc;
         auto coarse_field = [&](const ccfv_grid &gg, const SolverTable *tab, int phase) {
           SweepField f = make_field(gg, dir, Dt, ta + P->o.t0, tb + P->o.t0, P->W, tab, dsrc,
                                     P->theta);
           f.inst = i;
           f.slice = -1;
-          f.jmax = P->m;
+          place_pass(f, kind, P->m, fuse_c);
           f.smax = P->S;
           f.gskip = P->o.form == CCFV_FORM_DELTA ? 1 : 0;
           f.t_step = P->dtc;
           f.t_slice = P->DT;
           f.phase = phase;
           f.src_tb = kind == 2 ? 1 : 0;
-          f.kind = kind;
           f.pp = 1;  // W -> ... -> W or W2 through the pair W / W2
           f.data2 = P->W2;
           f.in0 = P->W;
@@ -497,8 +517,10 @@ int MultiEngine::rebuild() {
                         std::make_tuple(kind, 1, 1));
           ccfv_grid gh = g;
           if (P->o.form == CCFV_FORM_DELTA) gh.source = CCFV_SRC_NONE;
-          prepare_field(want_rg ? rg_prep : P->prep, kind, gh, coarse_field(gh, P->tab[2 + dir], 2),
-                        P->g64, &P->ftab, std::make_tuple(kind, 1, P->g64 ? 1 : 0));
+          if (kind < 3 || !want_rg)
+            prepare_field(want_rg ? rg_prep : P->prep, kind, gh,
+                          coarse_field(gh, P->tab[2 + dir], 2), P->g64, &P->ftab,
+                          std::make_tuple(kind, 1, P->g64 ? 1 : 0));
         }
       }
     }
@@ -548,7 +570,7 @@ int MultiEngine::rebuild() {
     if (!T->wt.p || !T->nt.p) return fail(CCFV_ERR_NOMEM, "stencil table allocation failed");
     const SweepClass &K = (T->level == 0 ? fine_ : coarse_).at(T->cls);
     MCK(launch_filter_weights(T->fp64, classbuf_.as<SweepField>() + K.off + T->idx, T->wt.p,
-                              T->nt.as<int>(), T->lines, st_, T->deriv));
+                              T->nt.as<int>(), T->lines, st_, T->variant));
     T->ready = true;
   }
   const int eb = 148;
@@ -644,14 +666,23 @@ int MultiEngine::sweeps(std::map<KKey, SweepClass> &classes, int kind, int jstep
     const int np = (int)(std::partition_point(K.bound.begin(), K.bound.end(),
                                               [&](int b) { return b > jstep; }) -
                          K.bound.begin());
-    bool any = false;  // the kernel's own guard, evaluated here on the host copy of nlo
-    for (int i = 0; i < np && !any; ++i) any = field_active(K.h[i], jstep, nslice, nlo_.data());
-    if (!any) continue;
+    // first and last field that take part: the kernel's own guard, evaluated
+    // here on the host copy of nlo (the last x sweep of fused sequences is
+    // active in one step only: a short range at the prefix's end)
+    int lo = 0, hi = np;
+    while (lo < hi && !field_active(K.h[lo], jstep, nslice, nlo_.data())) ++lo;
+    if (lo == hi) continue;
+    if (K.kind == 2)
+      while (!field_active(K.h[hi - 1], jstep, nslice, nlo_.data())) --hi;
+    else
+      lo = 0;
     bs.g0idx = idxbuf_.as<int>() + K.ioff;
     const SweepField *fd = classbuf_.as<SweepField>() + K.off;
     cudaError_t e =
-        K.fp64 ? launch_sweep_batch<double>(K.G, fd, np, 0, K.gpre[np], bs, status, st_)
-               : launch_sweep_batch<float>(K.G, fd, np, 0, K.gpre[np], bs, status, st_);
+        K.fp64 ? launch_sweep_batch<double>(K.G, fd, hi, K.gpre[lo], K.gpre[hi] - K.gpre[lo], bs,
+                                            status, st_)
+               : launch_sweep_batch<float>(K.G, fd, hi, K.gpre[lo], K.gpre[hi] - K.gpre[lo], bs,
+                                           status, st_);
     MCK(e);
   }
   return CCFV_OK;
@@ -659,7 +690,7 @@ int MultiEngine::sweeps(std::map<KKey, SweepClass> &classes, int kind, int jstep
 
 int MultiEngine::coarse_slice(int s, int mmax) {
   for (int i = 0; i < mmax; ++i)
-    for (int kind = 0; kind < 3; ++kind)
+    for (int kind : {0, 1, 3, 2})
       if (int rc = sweeps(coarse_, kind, i, s)) return rc;
   return CCFV_OK;
 }
@@ -729,7 +760,7 @@ int MultiEngine::iterate(std::vector<int> *finished) {
     // F[s+1] = F(U[s]): the fine sequences read U[s] in their first sweep
     MCK(cudaEventRecord(ef, st_));
     for (int j = 0; j < Jmax; ++j)
-      for (int kind = 0; kind < 3; ++kind)
+      for (int kind : {0, 1, 3, 2})
         if (int rc = sweeps(fine_, kind, j, 0)) return rc;
     MCK(cudaEventRecord(ef2, st_));
     if (resident) {

@@ -20,7 +20,7 @@ struct FilterTable {
   DevBuf wt, nt;
   int lines = 0;
   bool fp64 = true;
-  bool deriv = false;  // table of SWEEP_COMPAT_D
+  int variant = SWEEP_FILTER;  // form whose taps it holds
   bool ready = false;
   int level = 0;  // 0: fine class, 1: coarse class
   std::tuple<int, int, int, int, int> cls;

@@ -203,7 +203,7 @@ extern "C" int ccfv_step_noalloc(const ccfv_grid *grid, double *d_C, double tn, 
   for (int kind = 0; kind < 3 && e == cudaSuccess; ++kind) {
     const LaunchGeom &G = geom[kind];
     e = launch_sweep<double>(G, PlanFields(), d_fields + kind, 1, 0, h_fields[kind].groups, tn,
-                             nullptr, d_status, st);
+                             FieldIo(), d_status, st);
   }
   unsigned flag = 0;
   if (e == cudaSuccess)

@@ -333,11 +333,17 @@ __device__ __forceinline__ StreamField stream_field(const SweepField &f) {
 // field.  Its interior right-hand side R_k + sum_t wq_t R_{k+n0-2+t} with R_j =
 // sum_s wr_s C_{j+n0-2+s} is two tap groups of the cells, 8 taps from k+n0-3
 // and 13 from k+2n0-5 with the mass matrix, in three windowed passes (8, 8, 5)
-// that keep the register window at eight values for any displacement.
+// that keep the register window at eight values for any displacement.  BND 3
+// (x sweeps, periodic): the last x sweep of a step and the first of the next
+// one in one pass.  Both solve the same circulant systems, so their operators
+// commute: the two stencils compose into 15 taps from k+2n0-6 and the forward
+// recurrence runs twice, then the backward one; the warm-up of such a double
+// recurrence is a few cells longer.  2048^2: one pass of 21.3 us for two of
+// 18.2 us (eight steps 317 -> 255 us).
 template <typename T, int DIR, int LN, int BND>
-__global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 : 8)
+__global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 : 6)
     stream_kernel(const __grid_constant__ PlanFields plan, const SweepField *__restrict__ fields,
-                  int nfields, int first, void *data_override, int rows, unsigned *status,
+                  int nfields, int first, const FieldIo io, int rows, unsigned *status,
                   int jstep, int nslice, const int *nlo, int cs, int clustered,
                   const int *g0idx, int ends) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -346,6 +352,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   constexpr int ES = DIR == 0 ? X_PITCH : 1;    // element stride of a position
   constexpr int LS = DIR == 0 ? 2 : 1;          // lane stride of a chunk
   constexpr unsigned FULL = 0xffffffffu;
+  constexpr bool ENDS = BND == 1 || BND == 2;  // the reference's boundaries
+  constexpr bool XX = BND == 3;
   T *tile_s = reinterpret_cast<T *>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
@@ -366,7 +374,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     D = &plan.f;
     tile = blockIdx.x;
     rank = blockIdx.y;
-    field_io(plan.f, jstep, &vs, &vd, data_override);
+    field_io(plan.f, jstep, io, &vs, &vd);
     const long long off = (first + (int)blockIdx.z) * plan.stride;
     vs = static_cast<const char *>(vs) + off;
     vd = static_cast<char *>(vd) + off;
@@ -380,7 +388,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     const int q = cta - F.cta0;
     rank = clustered ? q % cs : q / F.groups;
     tile = clustered ? q / cs : q - rank * F.groups;
-    field_io(f, jstep, &vs, &vd, data_override);
+    field_io(f, jstep, io, &vs, &vd);
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (!field_active(f, jstep, nslice, nlo)) return;  // uniform over a cluster
@@ -399,13 +407,14 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   // the cells of all positions of those lanes are staged: past p1+J they only
   // lengthen the backward warm-up, so nothing is masked inside a lane.
   // (The reference's lines end: nothing is walked past position L - 1.)
-  const int walked = BND ? min(np + 2 * J, L - p0 + J) : np + 2 * J;
+  const int walked = ENDS ? min(np + 2 * J, L - p0 + J) : np + 2 * J;
   const int act = min(LN, (walked + SCH - 1) / SCH);
   // first position of the first lane: p0 - J, or (BND) as much earlier as makes
   // the last lane end with the line, so that nothing is masked there either
-  const int org = BND && p1 == L ? L - act * SCH : p0 - J;
-  const int nr = (act * SCH + 2 * (H - J) + 2) & ~1;
-  const int b0 = (org - (H - J)) & ~1;  // position of staged row 0
+  const int org = ENDS && p1 == L ? L - act * SCH : p0 - J;
+  const int nr = (act * SCH + 2 * (H - J) + (ENDS ? 2 : 1)) & ~1;
+  // position of staged row 0, row of position p0 (both even with p0 and H)
+  const int b0 = ENDS ? (org - (H - J)) & ~1 : p0 - H, h0 = ENDS ? p0 - b0 : H;
   const bool inside = b0 >= 0 && b0 + nr <= L;
   const bool pairs = ((DIR == 0 ? s_pos : s_line) & 1) == 0 && (DIR == 0 || (L & 1) == 0) &&
                      (((size_t)src | (size_t)dst) & (2 * sizeof(T) - 1)) == 0;
@@ -424,12 +433,12 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
         for (int r = r0; r < nr; r += NT / G, s += step, d += NT / G * X_PITCH) copy_pair(d, s);
       } else {
         for (int r = r0; r < nr; r += rs, d += rs * X_PITCH) {
-          if (BND && (unsigned)(b0 + r) >= (unsigned)L) {
+          if (ENDS && (unsigned)(b0 + r) >= (unsigned)L) {
             d[0] = T(0);
             if (pairs) d[1] = T(0);
             continue;
           }
-          const T *p = s + (long long)(BND ? b0 + r : wrap_pos(b0 + r, L)) * s_pos;
+          const T *p = s + (long long)(ENDS ? b0 + r : wrap_pos(b0 + r, L)) * s_pos;
           if (pairs) copy_pair(d, p); else copy_one(d, p);
         }
       }
@@ -447,17 +456,17 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
           for (int e = 2 * lane; e < nr; e += 64) copy_pair(d + e, s + e);
         } else if (pairs) {
           for (int e = 2 * lane; e < nr; e += 64) {
-            if (BND && (unsigned)(b0 + e) >= (unsigned)L)
+            if (ENDS && (unsigned)(b0 + e) >= (unsigned)L)
               d[e] = d[e + 1] = T(0);
             else
-              copy_pair(d + e, s + (BND ? b0 + e : wrap_pos(b0 + e, L)));
+              copy_pair(d + e, s + (ENDS ? b0 + e : wrap_pos(b0 + e, L)));
           }
         } else {
           for (int e = lane; e < nr; e += 32) {
-            if (BND && (unsigned)(b0 + e) >= (unsigned)L)
+            if (ENDS && (unsigned)(b0 + e) >= (unsigned)L)
               d[e] = T(0);
             else
-              copy_one(d + e, s + (BND ? b0 + e : wrap_pos(b0 + e, L)));
+              copy_one(d + e, s + (ENDS ? b0 + e : wrap_pos(b0 + e, L)));
           }
         }
       }
@@ -470,9 +479,9 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   const int line = line0 + warp * LPW + lw;
   const T mmu = T(-F.mu);
   const T *wt = reinterpret_cast<const T *>(F.wt) +  // padded past M
-                (size_t)line * (BND == 2 ? STREAM_TAPS_D : 8);
+                (size_t)line * (BND == 2 ? STREAM_TAPS_D : XX ? STREAM_TAPS_XX : 8);
   T o[8];
-  if (!BND) load_taps(o, wt);
+  if (!ENDS) load_taps(o, wt);
   const int n0 = __ldg(F.nt + line);
   static_assert(SCH == 17, "pw");
   T pw = mmu * mmu;  // (-mu)^17
@@ -490,16 +499,16 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
 
   // ---- stencil and recurrences ----
   T *const col = DIR == 0 ? tile_s + warp * LPW + lw : tile_s + (size_t)(warp * LPW + lw) * rows;
-  const int k0 = org - b0 + c * SCH;  // staged row of this lane's first position
-  const int r0 = k0 + n0 - 3;
-  bool ok = r0 >= 0 && r0 + SCH + 7 <= rows;
+  const int k0 = (ENDS ? org - b0 : H - J) + c * SCH;  // staged row of this lane's first position
+  const int r0 = XX ? k0 + 2 * n0 - 6 : k0 + n0 - 3;  // row of the first tap
+  bool ok = r0 >= 0 && r0 + SCH + (XX ? 14 : 7) <= rows;
   if (BND == 2) ok = ok && k0 + 2 * n0 - 5 >= 0 && k0 + 2 * n0 + SCH + 8 <= rows;
   if (!ok && line < M) atomicOr(status, STATUS_HALO);
   // inputs of the positions next to the line's ends (BND): the left region is
   // r[k - lo.ka], k in [lo.ka, lo.kb), the right one likewise
   EndRegion lo, hi;
   T *rl = nullptr, *rr = nullptr;
-  if (BND) {
+  if (ENDS) {
     const int kend = org + act * SCH;  // first position not walked
     // positions whose stencil, with the mass matrix's neighbours, stays clear
     // of clamps and ghosts: [sl, sr)
@@ -558,10 +567,14 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   // far below a rounding and not a share of one with the same sign everywhere)
   // (the reference's lines of one segment: no warm-up, any decay length).
   int ns = (F.JD <= SCH ? 0 : F.JD <= 2 * SCH ? 1 : 2) + (sizeof(T) == 4 ? 1 : 0);
-  if (BND && F.JD > 4 * SCH) ns = LN == 32 ? 5 : 4;
+  if (ENDS && F.JD > 4 * SCH) ns = LN == 32 ? 5 : 4;
   T v[SCH];
-  if (BND) load_taps(o, wt);
+  if (ENDS) load_taps(o, wt);
   stencil<T, ES, 8, false>(col + (ok ? r0 : 0) * ES, o, v);
+  if (XX) {
+    load_taps(o, wt + 8);
+    stencil<T, ES, 7, true>(col + (ok ? r0 + 8 : 0) * ES, o, v);
+  }
   if (BND == 2) {
     load_taps(o, wt + 8);
     stencil<T, ES, 8, true>(col + (ok ? k0 + 2 * n0 - 5 : 0) * ES, o, v);
@@ -569,7 +582,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     stencil<T, ES, 5, true>(col + (ok ? k0 + 2 * n0 + 3 : 0) * ES, o, v);
   }
   const int kp = org + c * SCH;  // this lane's first position
-  if (BND) {
+  if (ENDS) {
     // lanes next to the line's ends take the prepared inputs (zero before the
     // line) through their own rows: a loop over a few positions instead of 17
     // predicated selects
@@ -586,10 +599,12 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       for (int i = 0; i < SCH; ++i) v[i] = row[i * ES];
     }
   }
-  T w = T(0);
+  // one recurrence over the line: the chunk from zero for its end value, the
+  // carry into it by doubling steps over the lanes, the chunk again
+  auto forward = [&] {
+    T w = T(0);
 #pragma unroll
-  for (int i = 0; i < SCH; ++i) w = v[i] + mmu * w;
-  {
+    for (int i = 0; i < SCH; ++i) w = v[i] + mmu * w;
     T pd = pw;
     for (int s = 0; s < ns; ++s) {
       const T t = __shfl_up_sync(FULL, w, LS << s, DIR == 0 ? 32 : LN);
@@ -598,17 +613,18 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     }
     w = __shfl_up_sync(FULL, w, LS, DIR == 0 ? 32 : LN);
     if (c == 0) w = T(0);
-  }
 #pragma unroll
-  for (int i = 0; i < SCH; ++i) {
-    w = v[i] + mmu * w;
-    v[i] = w;
-  }
-  T x = T(0);
+    for (int i = 0; i < SCH; ++i) {
+      w = v[i] + mmu * w;
+      v[i] = w;
+    }
+  };
+  // carry of the backward recurrence from the right of this chunk
+  auto backward_carry = [&] {
+    T x = T(0);
 #pragma unroll
-  for (int i = SCH - 1; i >= 0; --i) x = v[i] + mmu * x;
-  if (c >= act) x = T(0);  // lanes whose cells are not staged
-  {
+    for (int i = SCH - 1; i >= 0; --i) x = v[i] + mmu * x;
+    if (c >= act) x = T(0);  // lanes whose cells are not staged
     T pd = pw;
     for (int s = 0; s < ns; ++s) {
       const T t = __shfl_down_sync(FULL, x, LS << s, DIR == 0 ? 32 : LN);
@@ -616,17 +632,28 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       pd *= pd;
     }
     x = __shfl_down_sync(FULL, x, LS, DIR == 0 ? 32 : LN);
-    if (c == LN - 1) x = T(0);
+    return c == LN - 1 ? T(0) : x;
+  };
+  forward();
+  if (XX) {
+    forward();
+    T x = backward_carry();
+#pragma unroll
+    for (int i = SCH - 1; i >= 0; --i) {
+      x = v[i] + mmu * x;
+      v[i] = x;
+    }
   }
+  T x = backward_carry();
   __syncwarp();  // every lane of the line has read its cells
   T *xp = col + k0 * ES;
 #pragma unroll
   for (int i = SCH - 1; i >= 0; --i) {
     x = v[i] + mmu * x;
-    if (BND) v[i] = x;
+    if (ENDS) v[i] = x;
     xp[i * ES] = x;
   }
-  if (BND && p0 == 0) {
+  if (ENDS && p0 == 0) {
     // non-cyclic system: A = c (1 + mu S^-1)(1 + mu S) + c mu^2 e_0 e_0^T, so
     // x = y - y_0 g with g_k = mu^2 ((-mu)^k - (-mu)^(2L-k)) / (1 - mu^(2L+2))
     // (Sherman-Morrison); y_0 is this segment's value at position 0, and g has
@@ -665,7 +692,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       const int g = 2 * ((int)threadIdx.x % G);
       if (line0 + g < M) {
         T *d = dst + (long long)p0 * s_pos + line0 + g;
-        const T *s = tile_s + (p0 - b0) * X_PITCH + g;
+        const T *s = tile_s + h0 * X_PITCH + g;
 #pragma unroll 4
         for (int r = (int)threadIdx.x / G; r < np; r += NT / G)
           *reinterpret_cast<Pair<T> *>(d + (long long)r * s_pos) =
@@ -675,7 +702,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       const int g = (int)threadIdx.x % X_LINES;
       if (line0 + g < M)
         for (int r = (int)threadIdx.x / X_LINES; r < np; r += NT / X_LINES)
-          dst[(long long)(p0 + r) * s_pos + line0 + g] = tile_s[(r + p0 - b0) * X_PITCH + g];
+          dst[(long long)(p0 + r) * s_pos + line0 + g] = tile_s[(r + h0) * X_PITCH + g];
     }
   } else {
 #pragma unroll
@@ -683,7 +710,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
       const int gl = line0 + warp * LPW + l;
       if (gl < M) {
         T *d = dst + (long long)gl * s_line + p0;
-        const T *s = tile_s + (size_t)(warp * LPW + l) * rows + p0 - b0;
+        const T *s = tile_s + (size_t)(warp * LPW + l) * rows + h0;
         if (pairs)
           for (int e = 2 * lane; e < np; e += 64)
             *reinterpret_cast<Pair<T> *>(d + e) = *reinterpret_cast<const Pair<T> *>(s + e);
@@ -695,7 +722,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
 }
 
 template <typename T>
-using StreamKernelT = void (*)(const PlanFields, const SweepField *, int, int, void *, int,
+using StreamKernelT = void (*)(const PlanFields, const SweepField *, int, int, const FieldIo, int,
                                unsigned *, int, int, const int *, int, int, const int *, int);
 
 template <typename T, int BND>
@@ -705,6 +732,7 @@ StreamKernelT<T> stream_kernel_of(int dir, int lanes) {
 }
 template <typename T>
 StreamKernelT<T> stream_kernel_for(int variant, int dir, int lanes) {
+  if (variant == SWEEP_FILTER_XX) return stream_kernel<T, 0, 16, 3>;
   return variant == SWEEP_COMPAT     ? stream_kernel_of<T, 1>(dir, lanes)
          : variant == SWEEP_COMPAT_D ? stream_kernel_of<T, 2>(dir, lanes)
                                      : stream_kernel_of<T, 0>(dir, lanes);
@@ -724,7 +752,7 @@ size_t stream_smem_bytes(const LaunchGeom &G, bool fp64) {
 
 template <typename T>
 cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
-                          int nfields, int group_base, int groups_total, void *data,
+                          int nfields, int group_base, int groups_total, const FieldIo &io,
                           unsigned *d_status, int jstep, int nslice, const int *nlo,
                           bool inplace, cudaStream_t stream, const int *g0idx, bool pdl) {
   // Function attributes apply to the device that is current when they are
@@ -738,7 +766,7 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   if (!configured[dev].load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lk(config_mu);
     if (!configured[dev].load(std::memory_order_relaxed)) {
-      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D})
+      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D, SWEEP_FILTER_XX})
         for (int l : {0, 16, 32}) {
           const void *fn = (const void *)stream_kernel_for<T>(v, l ? 1 : 0, l);
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -778,16 +806,16 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   cfg.numAttrs = na;
   count_launch();
   return cudaLaunchKernelEx(&cfg, stream_kernel_for<T>(G.variant, G.dir, G.lanes), plan, d_fields, nfields,
-                            by_value ? group_base / plan.tiles : group_base * G.cs, data, G.rows, d_status, jstep, nslice, nlo, G.cs,
-                            clustered, g0idx, G.ends);
+                            by_value ? group_base / plan.tiles : group_base * G.cs, io, G.rows,
+                            d_status, jstep, nslice, nlo, G.cs, clustered, g0idx, G.ends);
 }
 
 template cudaError_t launch_stream<double>(const LaunchGeom &, const PlanFields &,
-                                           const SweepField *, int, int, int, void *, unsigned *,
+                                           const SweepField *, int, int, int, const FieldIo &, unsigned *,
                                            int, int, const int *, bool, cudaStream_t, const int *,
                                            bool);
 template cudaError_t launch_stream<float>(const LaunchGeom &, const PlanFields &,
-                                          const SweepField *, int, int, int, void *, unsigned *,
+                                          const SweepField *, int, int, int, const FieldIo &, unsigned *,
                                           int, int, const int *, bool, cudaStream_t, const int *,
                                           bool);
 

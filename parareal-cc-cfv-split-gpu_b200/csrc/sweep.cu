@@ -304,7 +304,7 @@ __device__ __forceinline__ Smem<T> carve(unsigned char *raw, int lc_max, int H) 
 template <typename T>
 __global__ void __launch_bounds__(NTH, 2) sweep_kernel(const SweepField *__restrict__ fields,
                                                     int nfields, int group_base, double toff,
-                                                    void *data_override, int lc_max, int H,
+                                                    const FieldIo io, int lc_max, int H,
                                                     unsigned *status, int jstep, int nslice,
                                                     const int *nlo, const int *g0idx) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -317,10 +317,6 @@ __global__ void __launch_bounds__(NTH, 2) sweep_kernel(const SweepField *__restr
   // ---- descriptor of this tile's field (binary search on group0) ----
   if (threadIdx.x == 0) {
     *S.fd = fields[find_field(fields, g0idx, nfields, tile)];
-    if (data_override) {
-      S.fd->data = data_override;
-      if (S.fd->pp) S.fd->in0 = data_override;
-    }
   }
   __syncthreads();
   const SweepField &F = *S.fd;
@@ -340,7 +336,7 @@ __global__ void __launch_bounds__(NTH, 2) sweep_kernel(const SweepField *__restr
   {
     const void *vs;
     void *vd;
-    field_io(F, jstep, &vs, &vd);
+    field_io(F, jstep, io, &vs, &vd);
     gsrc = reinterpret_cast<const T *>(vs);
     gdst = reinterpret_cast<T *>(vd);
   }
@@ -723,7 +719,7 @@ __device__ __forceinline__ FastSmem<T> carve_fast(unsigned char *raw, int lc_max
 template <typename T>
 __global__ void __launch_bounds__(NTH, 2)
     sweep_fast_kernel(const SweepField *__restrict__ fields, int nfields, int group_base,
-                      double toff, void *data_override, int lc_max, int H, unsigned *status,
+                      double toff, const FieldIo io, int lc_max, int H, unsigned *status,
                       int jstep, int nslice, const int *nlo, const int *g0idx) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -738,11 +734,6 @@ __global__ void __launch_bounds__(NTH, 2)
     if (threadIdx.x < NW8)
       reinterpret_cast<long long *>(S.fd)[threadIdx.x] =
           __ldg(reinterpret_cast<const long long *>(&fields[lo]) + threadIdx.x);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && data_override) {
-    S.fd->data = data_override;
-    if (S.fd->pp) S.fd->in0 = data_override;
   }
   __syncthreads();
   const SweepField &F = *S.fd;
@@ -762,7 +753,7 @@ __global__ void __launch_bounds__(NTH, 2)
   {
     const void *vs;
     void *vd;
-    field_io(F, jstep, &vs, &vd);
+    field_io(F, jstep, io, &vs, &vd);
     gsrc = reinterpret_cast<const T *>(vs);
     gdst = reinterpret_cast<T *>(vd);
   }
@@ -1209,17 +1200,18 @@ __device__ __forceinline__ T compat_remap(const SweepField &F, const CompatEdge<
 }
 
 // The per-line stencil table of one field (one thread per line): eight taps
-// from C_{k+n0-3}.  deriv (the reference scheme's third sweep, uniform
+// from C_{k+n0-3}.  SWEEP_COMPAT_D (the reference scheme's third sweep, uniform
 // displacement): b_k = R_k + sum_t wq_t R_{k+n0-2+t} with R_j = sum_s wr_s
 // C_{j+n0-2+s} (the interior formulas of the line) is two groups of taps, with
-// the mass matrix 8 from C_{k+n0-3} and 13 from C_{k+2n0-5}.
+// the mass matrix 8 from C_{k+n0-3} and 13 from C_{k+2n0-5}.  SWEEP_FILTER_XX:
+// the eight taps twice, 15 from C_{k+2n0-6}.
 template <typename T>
 __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__restrict__ wt,
-                                      int *__restrict__ nt, int lines, int deriv) {
+                                      int *__restrict__ nt, int lines, int variant) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= lines) return;
   const SweepField F = *f;
-  if (deriv) {
+  if (variant == SWEEP_COMPAT_D) {
     double om[STREAM_TAPS_D];
     for (int m = 0; m < STREAM_TAPS_D; ++m) om[m] = 0.0;
     int n0 = 0;
@@ -1242,6 +1234,18 @@ __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__res
       mass(wd, 11, om + 8);
     }
     for (int m = 0; m < STREAM_TAPS_D; ++m) wt[(size_t)l * STREAM_TAPS_D + m] = T(om[m]);
+    nt[l] = n0;
+    return;
+  }
+  if (variant == SWEEP_FILTER_XX) {
+    double o[8], om[STREAM_TAPS_XX];
+    int n0 = 0;
+    for (int m = 0; m < 8; ++m) o[m] = 0.0;
+    if (l < F.M) filter_line_stencil<double>(F, l, 0.0, o, &n0);
+    for (int m = 0; m < STREAM_TAPS_XX; ++m) om[m] = 0.0;
+    for (int m = 0; m < 8; ++m)
+      for (int t = 0; t < 8; ++t) om[m + t] += o[m] * o[t];
+    for (int m = 0; m < STREAM_TAPS_XX; ++m) wt[(size_t)l * STREAM_TAPS_XX + m] = T(om[m]);
     nt[l] = n0;
     return;
   }
@@ -1284,7 +1288,7 @@ __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__res
 template <typename T, bool EXACT, bool CELL, bool COMPAT>
 __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
     sweep_filter_kernel(const SweepField *__restrict__ fields, int nfields, int group_base,
-                        double toff, void *data_override, int lc_max, int H, unsigned *status,
+                        double toff, const FieldIo io, int lc_max, int H, unsigned *status,
                         int jstep, int nslice, const int *nlo, int cs, int clustered,
                         const int *g0idx) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1309,11 +1313,6 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
       reinterpret_cast<long long *>(S.fd)[threadIdx.x] =
           __ldg(reinterpret_cast<const long long *>(&fields[lo]) + threadIdx.x);
     }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && data_override) {
-    S.fd->data = data_override;
-    if (S.fd->pp) S.fd->in0 = data_override;
   }
   __syncthreads();
   const SweepField &F = *S.fd;
@@ -1341,7 +1340,7 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
   {
     const void *vs;
     void *vd;
-    field_io(F, jstep, &vs, &vd);
+    field_io(F, jstep, io, &vs, &vd);
     gsrc = reinterpret_cast<const T *>(vs);
     gdst = reinterpret_cast<T *>(vd);
   }
@@ -1989,15 +1988,15 @@ size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact, bool
 int filter_segment_max(int J) { return filter_seg_max(J); }
 
 cudaError_t launch_filter_weights(bool fp64, const SweepField *d_field, void *wt, int *nt,
-                                  int lines, cudaStream_t stream, bool deriv) {
+                                  int lines, cudaStream_t stream, int variant) {
   const int bt = 128, grid = (lines + bt - 1) / bt;
   count_launch();
   if (fp64)
     filter_weights_kernel<double><<<grid, bt, 0, stream>>>(d_field, static_cast<double *>(wt), nt,
-                                                           lines, deriv ? 1 : 0);
+                                                           lines, variant);
   else
     filter_weights_kernel<float><<<grid, bt, 0, stream>>>(d_field, static_cast<float *>(wt), nt,
-                                                          lines, deriv ? 1 : 0);
+                                                          lines, variant);
   return cudaGetLastError();
 }
 
@@ -2009,7 +2008,7 @@ size_t sweep_fast_smem_bytes(int lc_max, int halo, bool fp64) {
 }
 
 template <typename T>
-using FilterKernelT = void (*)(const SweepField *, int, int, double, void *, int, int, unsigned *,
+using FilterKernelT = void (*)(const SweepField *, int, int, double, const FieldIo, int, int, unsigned *,
                                int, int, const int *, int, int, const int *);
 
 // The filter kernel's instantiation of a variant.
@@ -2038,12 +2037,13 @@ static bool pdl_enabled() {
 
 template <typename T>
 static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
-                               const SweepField *d_fields, int nfields, int group_base, int groups_total, double toff, void *data,
+                               const SweepField *d_fields, int nfields, int group_base, int groups_total, double toff,
+                               const FieldIo &io,
                                unsigned *d_status, int jstep, int nslice, const int *nlo,
                                bool inplace, cudaStream_t stream, const int *g0idx, bool pdl_ok) {
   const int variant = G.variant, cs = G.cs, lc_max = G.lc_max, halo = G.halo;
   if (stream_variant(variant))
-    return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, data, d_status,
+    return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, io, d_status,
                             jstep, nslice, nlo, inplace, stream, g0idx, pdl_ok && pdl_enabled());
   const bool fast = (variant == SWEEP_FAST);
   const bool cell = cell_filter_variant(variant);
@@ -2084,7 +2084,6 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
     }
   }
   if (groups_total <= 0) return cudaSuccess;
-  if (exact && inplace) return cudaErrorInvalidValue;  // the exact form sweeps out of place
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(groups_total * cs), 1, 1);
   cfg.blockDim = dim3(NTH, 1, 1);
@@ -2116,21 +2115,22 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
     cfg.attrs = fattr;
     cfg.numAttrs = na;
     FilterKernelT<T> fn = filter_kernel_for<T>(variant);
-    return cudaLaunchKernelEx(&cfg, fn, d_fields, nfields, group_base * cs, toff, data, lc_max,
+    return cudaLaunchKernelEx(&cfg, fn, d_fields, nfields, group_base * cs, toff, io, lc_max,
                               halo, d_status, jstep, nslice, nlo, cs, clustered, g0idx);
   }
   if (fast)
     return cudaLaunchKernelEx(&cfg, sweep_fast_kernel<T>, d_fields, nfields, group_base, toff,
-                              data, lc_max, halo, d_status, jstep, nslice, nlo, g0idx);
-  return cudaLaunchKernelEx(&cfg, sweep_kernel<T>, d_fields, nfields, group_base, toff, data,
+                              io, lc_max, halo, d_status, jstep, nslice, nlo, g0idx);
+  return cudaLaunchKernelEx(&cfg, sweep_kernel<T>, d_fields, nfields, group_base, toff, io,
                             lc_max, halo, d_status, jstep, nslice, nlo, g0idx);
 }
 
 template <typename T>
 cudaError_t launch_sweep(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
-                         int nfields, int group_base, int groups_total, double toff, void *data,
+                         int nfields, int group_base, int groups_total, double toff,
+                               const FieldIo &io,
                          unsigned *d_status, cudaStream_t stream, int jstep, bool inplace) {
-  return launch_impl<T>(G, plan, d_fields, nfields, group_base, groups_total, toff, data,
+  return launch_impl<T>(G, plan, d_fields, nfields, group_base, groups_total, toff, io,
                         d_status, jstep, 0, nullptr, inplace, stream, nullptr, true);
 }
 
@@ -2139,15 +2139,15 @@ cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, 
                                int group_base, int groups_total, const BatchStep &bs,
                                unsigned *d_status, cudaStream_t stream) {
   return launch_impl<T>(G, PlanFields(), d_fields, nfields, group_base, groups_total, 0.0,
-                        nullptr, d_status,
+                        FieldIo(), d_status,
                         bs.jstep, bs.nslice, bs.nlo, bs.inplace, stream, bs.g0idx, false);
 }
 
 template cudaError_t launch_sweep<double>(const LaunchGeom &, const PlanFields &,
-                                          const SweepField *, int, int, int, double, void *,
+                                          const SweepField *, int, int, int, double, const FieldIo &,
                                           unsigned *, cudaStream_t, int, bool);
 template cudaError_t launch_sweep<float>(const LaunchGeom &, const PlanFields &,
-                                         const SweepField *, int, int, int, double, void *,
+                                         const SweepField *, int, int, int, double, const FieldIo &,
                                          unsigned *, cudaStream_t, int, bool);
 template cudaError_t launch_sweep_batch<double>(const LaunchGeom &, const SweepField *, int, int,
                                                 int, const BatchStep &, unsigned *, cudaStream_t);

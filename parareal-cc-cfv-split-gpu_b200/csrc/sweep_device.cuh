@@ -36,20 +36,20 @@ __device__ __forceinline__ double field_time(const SweepField &f, double toff, i
 
 // Input and output of a field in a launch (SweepField::pp): in place, or the
 // ping-pong pair of an out-of-place sweep sequence.  Out of place, no CTA
-// reads what another CTA of the launch writes.  `data` (if non-null) replaces
-// f.data and, out of place, f.in0 (single-field launches).
-__device__ __forceinline__ void field_io(const SweepField &f, int jstep, const void **src,
-                                         void **dst, void *data = nullptr) {
-  void *A = data ? data : f.data;
+// reads what another CTA of the launch writes.  FieldIo: see launch_sweep.
+__device__ __forceinline__ void field_io(const SweepField &f, int jstep, const FieldIo &io,
+                                         const void **src, void **dst) {
+  void *A = io.data ? io.data : f.data;
   if (!f.pp) {
     *src = A;
     *dst = A;
     return;
   }
-  const int s = 3 * jstep + f.kind;
-  const bool toA = ((s + f.par) & 1) != 0;
-  *dst = toA ? A : f.data2;
-  *src = s == 0 ? (data ? data : f.in0) : (toA ? f.data2 : A);
+  const int s = f.s0 + f.sj * jstep;
+  const bool toA = ((s + f.par + (io.mode >> 1)) & 1) != 0;
+  const void *in0 = io.in ? io.in : io.data ? io.data : f.in0;
+  *src = s == 0 ? in0 : (toA ? f.data2 : A);
+  *dst = (io.mode & IO_IN_PLACE) ? const_cast<void *>(*src) : toA ? A : f.data2;
 }
 
 __device__ __forceinline__ void cp_async8(void *sdst, const void *gsrc) {

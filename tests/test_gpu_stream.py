@@ -87,3 +87,22 @@ def test_reference_boundaries_one_segment_any_diffusion(oracle, ccfv):
     s.run(c, 0.0, dt, 2)
     s.check()
     assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
+
+
+@pytest.mark.parametrize("nx,ny,K", [(60, 52, 1e-3), (272, 300, 5e-3), (1500, 40, 2e-4),
+                                     (24, 8400, 1e-6), (70, 64, 0.3)])
+@pytest.mark.parametrize("n", [1, 2, 5])
+def test_step_sequences_match_oracle(oracle, ccfv, nx, ny, K, n):
+    """Sequences of one, an even and an odd number of steps: x sweeps of
+    neighbouring steps in one pass, the last y sweep over its own input (lines
+    of more segments than a cluster holds: 8400 cells, copied back), strong
+    diffusion (cluster form), against the oracle's separate sweeps."""
+    dt = 0.8 / max(nx, ny) / 1.7
+    C0 = periodic_field(nx, nx + ny, ny=ny)
+    g, s = _grids(oracle, ccfv, nx, ny, K)
+    c = dev(C0)
+    s.run(c, 0.0, dt, n)
+    s.check()
+    out = c.cpu().numpy()
+    assert rel_l2(out, oracle.run(g, C0, 0.0, dt, n)) < TOL
+    assert abs(out.sum() - C0.sum()) < 1e-12 * np.abs(C0).sum()
