@@ -150,10 +150,13 @@ inline bool warm_filter_variant(int v) {
 // Variants whose right-hand side is the per-line stencil table (SweepField::wt),
 // and its values per line.
 inline bool stencil_filter_variant(int v) { return stream_variant(v) || v == SWEEP_FILTER_EXACT; }
-constexpr int STREAM_TAPS_D = 24;   // 8 + 13 taps, padded
+constexpr int STREAM_TAPS_C = 10;   // 8 taps, the feet's offset in a cell last
+constexpr int STREAM_TAPS_D = 24;   // 8 + 13 taps, likewise
 constexpr int STREAM_TAPS_XX = 16;  // 15 taps, padded
 inline int stencil_taps(int v) {
-  return v == SWEEP_COMPAT_D ? STREAM_TAPS_D : v == SWEEP_FILTER_XX ? STREAM_TAPS_XX : 8;
+  return v == SWEEP_COMPAT_D ? STREAM_TAPS_D
+         : v == SWEEP_COMPAT ? STREAM_TAPS_C
+         : v == SWEEP_FILTER_XX ? STREAM_TAPS_XX : 8;
 }
 // Variants with the per-cell right-hand side.
 inline bool cell_filter_variant(int v) {
@@ -243,6 +246,7 @@ struct BatchStep {
   int jstep = 0, nslice = 0;
   const int *nlo = nullptr;
   bool inplace = true;
+  bool pdl = false;            // programmatic dependent launch
   const int *g0idx = nullptr;  // the fields' group0 values (device), or null
 };
 template <typename T>
@@ -290,7 +294,9 @@ size_t resident_g_smem_bytes(int nx, int ny, bool fp64, bool cell);
 // Whether an nx x ny coarse field can be resident (lines of at most 272
 // cells, the field in shared memory).
 bool resident_g_fits(int nx, int ny, bool fp64, bool cell);
-cudaError_t launch_resident_g(bool fp64, const ResidentG *d_rg, int n, size_t smem,
+// cell: the instances' right-hand side is per cell (else SweepField::wt / nt
+// hold their stencil tables).
+cudaError_t launch_resident_g(bool fp64, bool cell, const ResidentG *d_rg, int n, size_t smem,
                               const int *nlo, cudaStream_t st);
 
 // Counts kernel launches made by the library.

@@ -98,8 +98,18 @@ __device__ __forceinline__ T rg_rhs(const RgEdge<T> &l, const RgEdge<T> &r, cons
   return remap + kbc * (r.d - l.d);
 }
 
+// Threads of a resident CTA.  One CTA runs a chain of dependent sweeps, so its
+// time is the latency of a round of lines times the rounds: as many half-warps
+// as the register file holds (212^2 FP32, 64 slices: one launch of 15.1 ms with
+// 256 threads, @RG@ ms with 1024).  The per-cell form keeps 16 lines a round,
+// whose right-hand sides have a scratch row each.
+template <typename T, bool CELL>
+constexpr int rg_threads() {
+  return CELL ? 256 : sizeof(T) == 4 ? 1024 : 512;
+}
+
 // One sweep of the resident field E ([nx][P], P odd) for every line.
-template <typename T>
+template <typename T, bool CELL>
 __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr, double toff) {
   const int L = F.L, M = F.M;
   const int sp = F.dir == 0 ? P : 1, sl = F.dir == 0 ? 1 : P;
@@ -109,7 +119,6 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
   const unsigned fm = 0xffffffffu;
   const T mu = T(F.sm_fac), mmu = -mu;
   const T pw = pwa[RG_CH];  // (-mu)^17
-  const bool cell = !F.uniform;
   const int nh = (blockDim.x / 32) * 2;  // half-warps (lines per round)
   for (int r = 0; r * nh < M; ++r) {
     const int gl = r * nh + hw;
@@ -118,11 +127,11 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
     T *line = E + (size_t)g * sl;
     const int k0 = c * RG_CH;
     T v[RG_CH];
-    const double tau0 = F.t_min + F.ht * (double)g;
-    if (!cell) {
-      T om[8];
-      int n0 = 0;
-      filter_line_stencil<T>(F, g, toff, om, &n0);
+    if (!CELL) {
+      T om[8];  // the plan's stencil table (the fields do not depend on time)
+#pragma unroll
+      for (int m = 0; m < 8; ++m) om[m] = __ldg(reinterpret_cast<const T *>(F.wt) + 8 * g + m);
+      const int n0 = __ldg(F.nt + g);
       int q = wrapi(k0 + n0 - 3, L);
       T win[8];
 #pragma unroll
@@ -150,6 +159,7 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
       const int mm = (L + RG_LANES - 1) / RG_LANES;
       const int s0 = c * mm, s1 = min(L, s0 + mm);
       const T kbc = T(F.kb);
+      const double tau0 = F.t_min + F.ht * (double)g;
       const LineFeet lf(F, tau0, tau0 + F.ht, toff + F.ta_rel, toff + F.tb_rel);
       if (s0 < s1) {
         RgEdge<T> el = rg_edge<T>(F, line, sp, L, lf.foot(F, s0));
@@ -231,12 +241,12 @@ __device__ void rg_sweep(const SweepField &F, T *E, int P, const T *pwa, T *bscr
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, bool CELL>
+__global__ void __launch_bounds__(rg_threads<T, CELL>())
     resident_g_kernel(const ResidentG *__restrict__ rg, const int *__restrict__ nlo) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SweepField fd[3];
-  __shared__ double red[2][8];
+  __shared__ double red[2][32];
   const ResidentG &R = rg[blockIdx.x];
   constexpr int NW8 = (int)(sizeof(SweepField) / 8);
   for (int i = threadIdx.x; i < 3 * NW8; i += blockDim.x)
@@ -273,7 +283,7 @@ __global__ void __launch_bounds__(256)
       for (int j = 0; j < m; ++j)
         for (int kind = 0; kind < 3; ++kind) {
           const SweepField &F = fd[kind];
-          rg_sweep<T>(F, E, P, F.dir == 0 ? pwx : pwy, bscr, j * F.t_step + s * F.t_slice);
+          rg_sweep<T, CELL>(F, E, P, F.dir == 0 ? pwx : pwy, bscr, j * F.t_step + s * F.t_slice);
           __syncthreads();
         }
     }
@@ -281,15 +291,19 @@ __global__ void __launch_bounds__(256)
     const double *Fs = R.F + (long long)(s + 1) * NN;
     double *Us = R.U + (long long)(s + 1) * NN;
     double se = 0.0, su = 0.0;
-    for (long long idx = threadIdx.x; idx < NN; idx += blockDim.x) {
-      const int i = (int)(idx / ny), jj = (int)(idx - (long long)i * ny);
-      T &e = E[(size_t)i * P + jj];
-      const double un = Fs[idx] + (s > lo ? (double)e : 0.0);
-      const double d = un - Us[idx];
-      Us[idx] = un;
-      e = T(d);
-      se += d * d;
-      su += un * un;
+    for (int i = threadIdx.x >> 5; i < nx; i += (int)(blockDim.x >> 5)) {
+      T *er = E + (size_t)i * P;
+      const double *fr = Fs + (long long)i * ny;
+      double *ur = Us + (long long)i * ny;
+#pragma unroll 4
+      for (int jj = threadIdx.x & 31; jj < ny; jj += 32) {
+        const double un = fr[jj] + (s > lo ? (double)er[jj] : 0.0);
+        const double d = un - ur[jj];
+        ur[jj] = un;
+        er[jj] = T(d);
+        se += d * d;
+        su += un * un;
+      }
     }
     for (int o = 16; o > 0; o >>= 1) {
       se += __shfl_down_sync(0xffffffffu, se, o);
@@ -326,20 +340,25 @@ bool resident_g_fits(int nx, int ny, bool fp64, bool cell) {
          resident_g_smem_bytes(nx, ny, fp64, cell) <= 200 * 1024;
 }
 
-cudaError_t launch_resident_g(bool fp64, const ResidentG *d_rg, int n, size_t smem,
-                              const int *nlo, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  const void *fn = fp64 ? (const void *)resident_g_kernel<double>
-                        : (const void *)resident_g_kernel<float>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+template <typename T, bool CELL>
+static cudaError_t launch_rg(const ResidentG *d_rg, int n, size_t smem, const int *nlo,
+                             cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute((const void *)resident_g_kernel<T, CELL>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   count_launch();
-  if (fp64)
-    resident_g_kernel<double><<<n, 256, smem, st>>>(d_rg, nlo);
-  else
-    resident_g_kernel<float><<<n, 256, smem, st>>>(d_rg, nlo);
+  resident_g_kernel<T, CELL><<<n, rg_threads<T, CELL>(), smem, st>>>(d_rg, nlo);
   return cudaGetLastError();
+}
+
+cudaError_t launch_resident_g(bool fp64, bool cell, const ResidentG *d_rg, int n, size_t smem,
+                              const int *nlo, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  if (fp64)
+    return cell ? launch_rg<double, true>(d_rg, n, smem, nlo, st)
+                : launch_rg<double, false>(d_rg, n, smem, nlo, st);
+  return cell ? launch_rg<float, true>(d_rg, n, smem, nlo, st)
+              : launch_rg<float, false>(d_rg, n, smem, nlo, st);
 }
 
 }  // namespace ccfv

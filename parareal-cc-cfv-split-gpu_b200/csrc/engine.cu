@@ -344,7 +344,7 @@ static bool stream_compat_geom(LaunchGeom &G, int L, int J, bool jok, int sh, in
                                bool inplace) {
   LaunchGeom S = G;
   S.variant = dsrc ? SWEEP_COMPAT_D : SWEEP_COMPAT;
-  S.ends = dsrc ? 2 * sh + 16 : sh + 8;
+  S.ends = dsrc ? 2 * sh + 20 : sh + 10;
   const int reach = dsrc ? 2 * sh + 12 : sh + 6;
   if (L <= 16 * STREAM_CH || (S.dir == 1 && L <= 32 * STREAM_CH)) {
     S.lanes = L <= 16 * STREAM_CH ? 16 : 32;

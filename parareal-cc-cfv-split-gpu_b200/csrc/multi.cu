@@ -577,7 +577,7 @@ int MultiEngine::rebuild() {
   MCK(elems_.alloc(sizeof(BElem) * std::max(n, 1)));
   if (n) MCK(cudaMemcpyAsync(elems_.p, he.data(), sizeof(BElem) * n, cudaMemcpyHostToDevice, st_));
   {
-    std::vector<ResidentG> hr[2];
+    std::vector<ResidentG> hr[4];
     for (int i = 0; i < n; ++i) {
       Problem *P = slots_[i].get();
       if (!live(P) || !P->resident) continue;
@@ -593,17 +593,27 @@ int MultiEngine::rebuild() {
       r.nx = P->g.nx;
       r.ny = P->g.ny;
       r.pitch = P->g.ny | 1;
-      const int q = P->g64 ? 1 : 0;
-      rgsmem_[q] = std::max(rgsmem_[q], resident_g_smem_bytes(P->g.nx, P->g.ny, P->g64,
-                                                              P->g.velocity == CCFV_VEL_SWIRL));
+      const bool cell = P->g.velocity == CCFV_VEL_SWIRL;
+      const int q = (cell ? 2 : 0) + (P->g64 ? 1 : 0);
+      rgsmem_[q] = std::max(rgsmem_[q], resident_g_smem_bytes(P->g.nx, P->g.ny, P->g64, cell));
       hr[q].push_back(r);
     }
-    for (int q = 0; q < 2; ++q) {
+    for (int q = 0; q < 4; ++q) {
       rgn_[q] = (int)hr[q].size();
-      if (rgn_[q]) {
-        MCK(rgbuf_[q].alloc(sizeof(ResidentG) * hr[q].size()));
-        MCK(cudaMemcpyAsync(rgbuf_[q].p, hr[q].data(), sizeof(ResidentG) * hr[q].size(),
-                            cudaMemcpyHostToDevice, st_));
+      if (!rgn_[q]) continue;
+      MCK(rgbuf_[q].alloc(sizeof(ResidentG) * hr[q].size()));
+      MCK(cudaMemcpyAsync(rgbuf_[q].p, hr[q].data(), sizeof(ResidentG) * hr[q].size(),
+                          cudaMemcpyHostToDevice, st_));
+      for (int i = 0; i < rgn_[q]; ++i) {
+        Problem *P = slots_[hr[q][i].inst].get();
+        if (q >= 2 || P->rg_tables) continue;  // per cell, or filled before
+        for (const SweepField &f : hr[q][i].f) {
+          if (!f.wt || !f.nt) return fail(CCFV_ERR_NOMEM, "stencil table allocation failed");
+          const size_t k = &f - hr[q][i].f;
+          MCK(launch_filter_weights(q == 1, rgbuf_[q].as<ResidentG>()[i].f + k,
+                                    const_cast<void *>(f.wt), const_cast<int *>(f.nt), f.M, st_));
+        }
+        P->rg_tables = true;
       }
     }
   }
@@ -657,6 +667,7 @@ int MultiEngine::sweeps(std::map<KKey, SweepClass> &classes, int kind, int jstep
   bs.nslice = nslice;
   bs.nlo = nlo_d_.as<int>();
   bs.inplace = false;  // every batched field sweeps out of place
+  bs.pdl = true;
   unsigned *status = status_.as<unsigned>();
   for (auto &kv : classes) {
     SweepClass &K = kv.second;
@@ -771,9 +782,9 @@ int MultiEngine::iterate(std::vector<int> *finished) {
         MCK(cudaEventCreateWithFlags(&side_ev_[0], cudaEventDisableTiming));
       }
       MCK(cudaStreamWaitEvent(side_, ef2, 0));
-      for (int q = 0; q < 2; ++q)
+      for (int q = 0; q < 4; ++q)
         if (rgn_[q])
-          MCK(launch_resident_g(q == 1, rgbuf_[q].as<ResidentG>(), rgn_[q], rgsmem_[q],
+          MCK(launch_resident_g((q & 1) != 0, q >= 2, rgbuf_[q].as<ResidentG>(), rgn_[q], rgsmem_[q],
                                 nlo_d_.as<int>(), side_));
       MCK(cudaEventRecord(side_ev_[0], side_));
     }

@@ -66,6 +66,7 @@ struct Problem {
   // the field in shared memory; rgf = its coarse sweep descriptors of the
   // iterations (not placed in the launch classes)
   bool resident = false;
+  bool rg_tables = false;    // its stencil tables are filled
   SweepField rgf[3];
   enum { NEW, RUNNING, DONE } state = NEW;
   int k = 0;                 // iterations done
@@ -158,9 +159,10 @@ class MultiEngine {
   // resident coarse propagators: descriptors per coarse precision (FP32,
   // FP64), their shared memory, and the side stream they run on beside the
   // shared coarse launches of the other problems
-  DevBuf rgbuf_[2];
-  int rgn_[2] = {0, 0};
-  size_t rgsmem_[2] = {0, 0};
+  // (index 2 cell + fp64)
+  DevBuf rgbuf_[4];
+  int rgn_[4] = {0, 0, 0, 0};
+  size_t rgsmem_[4] = {0, 0, 0, 0};
   cudaStream_t side_ = nullptr;
   cudaEvent_t side_ev_[2] = {nullptr, nullptr};
   long long allocs_ = 0;  // problem allocations attempted (fault injection counts them)

@@ -186,17 +186,33 @@ __device__ __forceinline__ FootCell foot_cell(const SweepField &F, double f, dou
   r.xi = (x - (F.s_min + F.h * r.k)) * (12.0 * F.inv12h);
   return r;
 }
+// edge_foot (sweep_math.cuh) of the velocity fields that do not depend on the
+// position along the line, nor on time: Heun's two speeds are one.
 __device__ __forceinline__ double line_foot(const SweepField &F, int line, int e) {
+  const double s = F.s_min + F.h * e;
+  auto corner = [&](double tau) {
+    const double w = F.vel == VEL_REF_ROT4 ? (F.dir == 0 ? -4 * tau : 4 * tau)
+                     : F.vel == VEL_CONST
+                         ? (F.dir == 0 ? F.vp[0] : F.vp[1])
+                         : (F.dir == 0 ? -F.vp[0] * (tau - F.vp[2]) : F.vp[0] * (tau - F.vp[1]));
+    return s - 0.5 * F.Dt * (w + w);
+  };
   const double tau0 = F.t_min + F.ht * (double)line;
-  return edge_foot(F, e, tau0, tau0 + F.ht, 0.0, 0.0);  // time-independent fields
+  return 0.5 * (corner(tau0) + corner(tau0 + F.ht));
+}
+// The derivative's clamp of a foot on the end of the line (rare: kept out of
+// the kernels, whose single pass over their code is bound by fetching it).
+__device__ __noinline__ FootCell end_foot_cell(const SweepField &F, int line, int e) {
+  return foot_cell(F, line_foot(F, line, e), 1e-15);
 }
 
 // Remap of one cell over [fl, fr] (T2S4:306-347, 396-438), its left foot clamped
 // from below and its right one from above only: a left foot on the upper edge
 // itself lies in no cell and the right one still counts the last cell.
 template <typename T, typename V>
-__device__ __noinline__ T remap_at_end(const SweepField &F, const V &cells, double fl, double fr) {
+__device__ __noinline__ T remap_at_end(const SweepField &F, const V &cells, int line, int k) {
   const int L = F.L;
+  const double fl = line_foot(F, line, k), fr = line_foot(F, line, k + 1);
   if (fl > F.s_max || fr < F.s_min || fl == fr) return T(0);
   const double xl = fmax(fl, F.s_min + F.eps_remap), xr = fmin(fr, F.s_max - F.eps_remap);
   const int kl = (int)floor((xl - F.s_min) / F.h), kr = (int)floor((xr - F.s_min) / F.h);
@@ -219,36 +235,48 @@ constexpr int FOOT_BELOW = -1, FOOT_ON_END = -2, FOOT_ABOVE = 1 << 30;
 // All lanes of the warp call it (empty region: nothing but the barriers).
 template <typename T, int ES, bool REMAPPED, int HL>
 __device__ __forceinline__ void end_inputs(const SweepField &F, const StagedLine<T, ES> &cells,
-                                           int line, const EndRegion &R, int hc, T *phi, T *d,
-                                           T *tmp, int *kf) {
+                                           int line, int n0, double x0, const EndRegion &R, int hc,
+                                           T *phi, T *d, T *tmp, int *kf) {
+  tmp += 2;  // room for two ghosts on either side
   const int L = F.L;
   const T kbc = T(F.kb), inv12h = T(F.inv12h);
   const bool any = R.ka < R.kb;
   // feet of the edges [e0, e1]: PPM integral and cell, with a mark for feet
   // outside the line (zero inflow), and the derivative of the staged cells
   const int e0 = REMAPPED ? R.ra : R.ba, e1 = REMAPPED ? R.rb : R.bb;
-  // feet this far from the middle of the line are clamped by neither clamp
-  const double mid = 0.5 * (F.s_min + F.s_max), half = 0.5 * (F.s_max - F.s_min) - F.h;
+  // Every foot of a line sits at the same offset n0 + x0 from its edge: one
+  // clear of the ends needs no quotient of its own, one a cell beyond them lies
+  // in no cell and neither do those of its cell.
   if (any)
     for (int e = e0 + hc; e <= e1; e += HL) {
-      const double f = line_foot(F, line, e);
-      FootCell p = foot_cell(F, f, F.eps_remap);
-      if (!cells.near(p.k)) p.k = 0, p.xi = 0.0;
-      phi[e - e0] = p.k >= 0 && p.k < L ? ppm_to(cells, p.k, T(p.xi)) : T(0);
-      kf[e - e0] = f < F.s_min               ? FOOT_BELOW
-                   : f > F.s_max             ? FOOT_ABOVE + p.k
-                   : f < F.s_min + F.eps_remap || f > F.s_max - F.eps_remap ? FOOT_ON_END
-                                                                            : p.k;
-      if (!REMAPPED) {
-        T dv = T(0);
-        if (f >= F.s_min && f <= F.s_max) {
-          const FootCell q = F.eps_remap == 1e-15 || fabs(f - mid) < half ? p : foot_cell(F, f, 1e-15);
-          dv = derivative_at(cells, q.k, T(q.xi), L, inv12h);
+      const int j = e + n0;
+      int mark = j < 0 ? FOOT_BELOW : FOOT_ABOVE + L;
+      T ph = T(0), dv = T(0);
+      if (j > -2 && j < L + 1) {
+        FootCell p{j, x0};
+        bool in = true;
+        mark = j;
+        if (j < 2 || j > L - 4) {
+          const double f = line_foot(F, line, e);
+          p = foot_cell(F, f, F.eps_remap);
+          in = f >= F.s_min && f <= F.s_max;
+          mark = f < F.s_min               ? FOOT_BELOW
+                 : f > F.s_max             ? FOOT_ABOVE + p.k
+                 : f < F.s_min + F.eps_remap || f > F.s_max - F.eps_remap ? FOOT_ON_END
+                                                                          : p.k;
         }
-        d[e - e0] = dv;
-      } else {
-        d[e - e0] = T(p.xi);  // until the derivative of the remapped field
+        if (!cells.near(p.k)) p.k = 2;
+        if (p.k >= 0 && p.k < L) ph = ppm_to(cells, p.k, T(p.xi));
+        if (REMAPPED) {
+          dv = T(p.xi);  // until the derivative of the remapped field
+        } else if (in) {
+          if (mark == FOOT_ON_END && F.eps_remap != 1e-15) p = end_foot_cell(F, line, e);
+          dv = derivative_at(cells, p.k, T(p.xi), L, inv12h);
+        }
       }
+      phi[e - e0] = ph;
+      d[e - e0] = dv;
+      kf[e - e0] = mark;
     }
   __syncwarp();
   // remapped cells: whole cells between the feet plus the two integrals
@@ -260,7 +288,7 @@ __device__ __forceinline__ void end_inputs(const SweepField &F, const StagedLine
       const int kl = kf[k - e0], kr = kf[k + 1 - e0];
       T v = T(0);
       if (kl == FOOT_ON_END || kr == FOOT_ON_END) {
-        v = remap_at_end<T>(F, cells, line_foot(F, line, k), line_foot(F, line, k + 1));
+        v = remap_at_end<T>(F, cells, line, k);
       } else if (kl < FOOT_ABOVE && kr != FOOT_BELOW) {
         const int l = max(kl, 0), r = min(kr & (FOOT_ABOVE - 1), L);
         for (int j = l; j < r; ++j) v += cells(j);
@@ -273,29 +301,24 @@ __device__ __forceinline__ void end_inputs(const SweepField &F, const StagedLine
   if (REMAPPED) {
     // derivative of the remapped field at the edges of [ba, bb)
     // (T2S4:929-932), its ghosts from the three remapped end cells
-    auto remapped = [&](int k) -> T {
-      if (k < 0 || k >= L) {
-        T g1, g2;
-        if (k < 0) {
-          ghosts(tmp[0], tmp[1], tmp[2], g1, g2);  // ra = 0
-          return k == -1 ? g1 : g2;
-        }
-        const T *z = tmp + (L - 1 - R.ra);
-        ghosts(z[0], z[-1], z[-2], g1, g2);
-        return k == L ? g1 : g2;
-      }
-      return tmp[k - R.ra];
-    };
+    if (any && hc == 0) {
+      if (R.ra == 0) ghosts(tmp[0], tmp[1], tmp[2], tmp[-1], tmp[-2]);
+      T *z = tmp + (L - 1 - R.ra);
+      if (R.rb == L) ghosts(z[0], z[-1], z[-2], z[1], z[2]);
+    }
+    __syncwarp();
+    auto remapped = [&](int k) -> T { return tmp[k - R.ra]; };
     if (any)
       for (int e = R.ba + hc; e <= R.bb; e += HL) {
         int k = kf[e - e0];
         T xi = d[e - e0], dv = T(0);
         if (k == FOOT_ON_END) {  // inside [s_min, s_max], within the clamp
-          const FootCell q = foot_cell(F, line_foot(F, line, e), 1e-15);
+          const FootCell q = end_foot_cell(F, line, e);
           k = q.k;
           xi = T(q.xi);
         }
-        if (k >= 0 && k < FOOT_ABOVE) dv = derivative_at(remapped, k, xi, L, inv12h);
+        if (k >= 0 && k < FOOT_ABOVE)
+          dv = derivative_at(remapped, k, xi, L, inv12h);
         d[e - e0] = dv;
       }
     __syncwarp();
@@ -479,7 +502,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   const int line = line0 + warp * LPW + lw;
   const T mmu = T(-F.mu);
   const T *wt = reinterpret_cast<const T *>(F.wt) +  // padded past M
-                (size_t)line * (BND == 2 ? STREAM_TAPS_D : XX ? STREAM_TAPS_XX : 8);
+                (size_t)line *
+                    (BND == 2 ? STREAM_TAPS_D : BND == 1 ? STREAM_TAPS_C : XX ? STREAM_TAPS_XX : 8);
   T o[8];
   if (!ENDS) load_taps(o, wt);
   const int n0 = __ldg(F.nt + line);
@@ -557,8 +581,9 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     }
     __syncwarp();
     {
+      const double x0 = __ldg(wt + (BND == 2 ? STREAM_TAPS_D : STREAM_TAPS_C) - 1);
       T *h = sc + side * 3 * ends;
-      end_inputs<T, ES, BND == 2, LN / 2>(*D, cells, line, side ? hi : lo, c % (LN / 2), h,
+      end_inputs<T, ES, BND == 2, LN / 2>(*D, cells, line, n0, x0, side ? hi : lo, c % (LN / 2), h,
                                           h + ends, h + 2 * ends, kf);
     }
   }

@@ -1232,6 +1232,7 @@ __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__res
       };
       mass(wr, 6, om);
       mass(wd, 11, om + 8);
+      om[STREAM_TAPS_D - 1] = (f0 - F.s_min) / F.h - n0;
     }
     for (int m = 0; m < STREAM_TAPS_D; ++m) wt[(size_t)l * STREAM_TAPS_D + m] = T(om[m]);
     nt[l] = n0;
@@ -1249,14 +1250,20 @@ __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__res
     nt[l] = n0;
     return;
   }
+  const int nw = variant == SWEEP_COMPAT ? STREAM_TAPS_C : 8;
+  T *row = wt + (size_t)l * nw;
   if (l < F.M) {
     T om[8];
     int n0 = 0;
     filter_line_stencil<T>(F, l, 0.0, om, &n0);
-    for (int m = 0; m < 8; ++m) wt[(size_t)l * 8 + m] = om[m];
+    for (int m = 0; m < 8; ++m) row[m] = om[m];
     nt[l] = n0;
+    if (nw > 8) {
+      const double tau0 = F.t_min + F.ht * (double)l;
+      row[nw - 1] = T((edge_foot(F, 0, tau0, tau0 + F.ht, 0.0, 0.0) - F.s_min) / F.h - n0);
+    }
   } else {
-    for (int m = 0; m < 8; ++m) wt[(size_t)l * 8 + m] = T(0);
+    for (int m = 0; m < nw; ++m) row[m] = T(0);
     nt[l] = 0;
   }
 }
@@ -2023,10 +2030,10 @@ static FilterKernelT<T> filter_kernel_for(int variant) {
   }
 }
 
-// Programmatic dependent launch (the filter kernels wait for their predecessor
-// before reading cells) for the single-instance engine's launches: 1.4 % on
-// the 2048^2 Parareal solve, while the batched engine's back-to-back class
-// launches lost 14 % of their fine phase with it.  CCFV_PDL=0 turns it off.
+// Programmatic dependent launch: the filter kernels wait for their predecessor
+// before reading cells, after fetching what is constant.  Batch of 64 mixed
+// instances: 1323 ms without, 1276 ms with; 12 instances up to 583^2: 115 ms
+// without, 97 ms with.  CCFV_PDL=0 turns it off.
 static bool pdl_enabled() {
   static const bool on = [] {
     const char *e = std::getenv("CCFV_PDL");
@@ -2140,7 +2147,7 @@ cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, 
                                unsigned *d_status, cudaStream_t stream) {
   return launch_impl<T>(G, PlanFields(), d_fields, nfields, group_base, groups_total, 0.0,
                         FieldIo(), d_status,
-                        bs.jstep, bs.nslice, bs.nlo, bs.inplace, stream, bs.g0idx, false);
+                        bs.jstep, bs.nslice, bs.nlo, bs.inplace, stream, bs.g0idx, bs.pdl);
 }
 
 template cudaError_t launch_sweep<double>(const LaunchGeom &, const PlanFields &,
