@@ -135,21 +135,24 @@ enum { SWEEP_GENERAL = 0, SWEEP_FAST = 1, SWEEP_FILTER = 2, SWEEP_GENERAL_SRC = 
        SWEEP_FILTER_EXACT = 4, SWEEP_CELL = 5, SWEEP_CELL_EXACT = 6, SWEEP_CELL_COMPAT = 7,
        SWEEP_COMPAT = 8, SWEEP_COMPAT_D = 9, SWEEP_FILTER_XX = 10 };
 inline bool stream_variant(int v) {
-  return v == SWEEP_FILTER || v == SWEEP_COMPAT || v == SWEEP_COMPAT_D || v == SWEEP_FILTER_XX;
+  return v == SWEEP_FILTER || v == SWEEP_COMPAT || v == SWEEP_COMPAT_D ||
+         v == SWEEP_FILTER_XX || v == SWEEP_CELL;
 }
 // Variants run by the filter kernels (factored solve).
 inline bool filter_variant(int v) {
-  return stream_variant(v) || v == SWEEP_FILTER_EXACT || v == SWEEP_CELL ||
+  return stream_variant(v) || v == SWEEP_FILTER_EXACT ||
          v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT;
 }
 // Warm-up (segmented) forms: lines longer than MAX_CLUSTER segments are
 // allowed out of place.
 inline bool warm_filter_variant(int v) {
-  return stream_variant(v) || v == SWEEP_CELL || v == SWEEP_CELL_COMPAT;
+  return stream_variant(v) || v == SWEEP_CELL_COMPAT;
 }
 // Variants whose right-hand side is the per-line stencil table (SweepField::wt),
 // and its values per line.
-inline bool stencil_filter_variant(int v) { return stream_variant(v) || v == SWEEP_FILTER_EXACT; }
+inline bool stencil_filter_variant(int v) {
+  return (stream_variant(v) && v != SWEEP_CELL) || v == SWEEP_FILTER_EXACT;
+}
 constexpr int STREAM_TAPS_C = 10;   // 8 taps, the feet's offset in a cell last
 constexpr int STREAM_TAPS_D = 24;   // 8 + 13 taps, likewise
 constexpr int STREAM_TAPS_XX = 16;  // 15 taps, padded
@@ -256,8 +259,8 @@ cudaError_t launch_sweep_batch(const LaunchGeom &G, const SweepField *d_fields, 
 // The streaming form's launch (stream_variant), called by the two above.
 template <typename T>
 cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
-                          int nfields, int group_base, int groups_total, const FieldIo &io,
-                          unsigned *d_status,
+                          int nfields, int group_base, int groups_total, double toff,
+                          const FieldIo &io, unsigned *d_status,
                           int jstep, int nslice, const int *nlo, bool inplace,
                           cudaStream_t stream, const int *g0idx, bool pdl);
 

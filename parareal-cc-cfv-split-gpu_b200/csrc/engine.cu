@@ -404,7 +404,7 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
       if (inplace && G.cs > MAX_CLUSTER) {  // in place, a line's segments form one cluster
         G = general;
         if (uniform) G.variant = SWEEP_FAST;
-      } else if (uniform) {
+      } else {
         G.lc_fit = G.lc_max;
         G.halo_fit = G.halo;
         stream_geom(G, L, J, sh + 6, stream_lc(L, fp64));
@@ -412,10 +412,11 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
     } else if (uniform) {
       G.variant = SWEEP_FAST;
     }
-    if (cell_filter_variant(G.variant) &&
-        sweep_filter_smem_bytes(G.lc_max, G.halo, fp64, exact_filter_variant(G.variant), true) >
-            227 * 1024)
-      G = general;  // the per-cell form's two tiles do not fit: per-cell scan kernel
+    // the per-cell forms' tiles do not fit: per-cell scan kernel
+    if (G.variant == SWEEP_CELL_EXACT &&
+        sweep_filter_smem_bytes(G.lc_max, G.halo, fp64, true, true) > 227 * 1024)
+      G = general;
+    if (G.variant == SWEEP_CELL && stream_smem_bytes(G, fp64) > 227 * 1024) G = general;
   } else if (!g.source && g.bc == CCFV_BC_COMPAT) {
     // the reference's boundaries: the filter kernel's per-cell form with the
     // non-cyclic closure.  A line of at most one segment is solved exactly

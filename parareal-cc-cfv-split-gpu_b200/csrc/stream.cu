@@ -351,6 +351,102 @@ __device__ __forceinline__ StreamField stream_field(const SweepField &f) {
                      f.wt, f.nt};
 }
 
+// ---- feet that differ from edge to edge: the swirling field (BND 4) ----
+//
+// Speed along the line a(tau, t) sin^2(pi s): an edge's two corners share
+// sin(pi s) and cos(pi s) (a table of the CTA's edges), and the speed at the
+// predicted point s - Dt w is that of a small angle z away, so a corner foot is
+// a short series instead of a sine of its own: orders 5 and 4 below 2^-8 (5e-18
+// left out), 7 and 8 below 2^-5 (2e-18); longer steps call sinpi.  A loop over the
+// edges two at a time: unrolled whole, the kernel waits for its instructions
+// (23 us a sweep of 1024^2 against 18 us; the tile kernel, a sine per corner and
+// divisions per edge, took 51 us).
+template <int N>
+struct Series {
+  static constexpr int value = N;
+};
+struct CornerLine {
+  double wb, wa, z;  // a(tau, tb), a(tau, ta), pi Dt a(tau, tb)
+};
+__device__ __noinline__ double far_sine(double x) { return sinpi(x); }
+// w(s, tb) + w(s - Dt w, ta) of one corner; series: 2, 1 or 0 as above.
+template <int series>
+__device__ __forceinline__ double corner_speeds(const CornerLine &l, double S, double C, double s,
+                                                double Dt) {
+  const double s2 = S * S, w = l.wb * s2;
+  double q;
+  if (series) {
+    const double z = l.z * s2, z2 = z * z;
+    double a = 1.0 / 120, b = 1.0 / 24;
+    if (series == 1) {
+      a += z2 * (-1.0 / 5040);
+      b += z2 * (-1.0 / 720 + z2 * (1.0 / 40320));
+    }
+    const double sn = z + z * z2 * (-1.0 / 6 + z2 * a);
+    q = S + S * z2 * (-0.5 + z2 * b) - C * sn;
+  } else {
+    q = far_sine(s - Dt * w);
+  }
+  return w + l.wa * (q * q);
+}
+
+// One edge: its foot's cell, the PPM integral (T2S4:63-65, 260-304) and 12 h
+// times the derivative at the foot (T2S4:440-547), both as polynomials of the
+// offset in the cell, and the foot cell's value.  u: the foot in cells from its
+// edge e (not from the line's start, where it would round to 1e-13 of a cell on
+// a line of 1024).  A cell outside the staged rows (cannot happen) is replaced and
+// marked in `bad`.
+template <typename T>
+struct SwirlEdge {
+  int kf;
+  T phi, d, z;
+};
+template <typename T, int ES>
+__device__ __forceinline__ SwirlEdge<T> swirl_edge(int e, double u, const T *cells, int b0,
+                                                   int rows, int &bad) {
+  SwirlEdge<T> r;
+  // floor by the rounding of u - 1/2 + 1.5 2^52 (an exact cell edge may count
+  // as either cell's: the integrals meet there)
+  const double t = (u - 0.5) + 6755399441055744.0;
+  r.kf = e + __double2loint(t);
+  const T x = T(u - (t - 6755399441055744.0));
+  const int row = r.kf - b0, at = min(max(row, 2), rows - 3);
+  bad |= row ^ at;
+  const T *c = cells + at * ES;
+  const T m2 = c[-2 * ES], m1 = c[-ES], z = c[0], p1 = c[ES], p2 = c[2 * ES];
+  // left and right edge values, PPM integral x (cl + x (a + x b))
+  const T dm = z - m1, e0 = m2 - p1, s1 = m1 + p1;
+  const T cl = T(7.0 / 12.0) * (z + m1) - T(1.0 / 12.0) * (p1 + m2);
+  const T cr = T(7.0 / 12.0) * (p1 + z) - T(1.0 / 12.0) * (p2 + m1);
+  const T cs = cl + cr;
+  r.phi = x * (cl + x * ((T(3.0) * z - cs) - cl + x * (cs - T(2.0) * z)));
+  // derivative: c0 + x (3 c1 + x (-6 c2 + 2 x c3))
+  const T c0 = e0 + T(15.0) * dm, c2 = e0 + T(3.0) * dm;
+  const T c1 = (m2 - p2) + T(2.0) * m1 + T(6.0) * p1 - T(8.0) * z;
+  const T c3 = (m2 + p2) - T(4.0) * s1 + T(6.0) * z;
+  r.d = c0 + x * (T(3.0) * c1 + x * (T(2.0) * x * c3 - T(6.0) * c2));
+  r.z = z;
+  return r;
+}
+// Whole cells between two feet that are not one apart (compensated, signed).
+template <typename T, int ES>
+__device__ __noinline__ T cells_between(int kl, int kr, const T *cells, int b0, int rows,
+                                        unsigned *status) {
+  const int lo = min(kl, kr), hi = max(kl, kr);
+  if (lo < b0 || hi > b0 + rows) {
+    atomicOr(status, STATUS_HALO);
+    return T(0);
+  }
+  T s = T(0), comp = T(0);
+  for (int k = lo; k < hi; ++k) {
+    const T x = cells[(k - b0) * ES], t = s + x;
+    comp += (fabs(s) >= fabs(x)) ? ((s - t) + x) : ((x - t) + s);
+    s = t;
+  }
+  s += comp;
+  return kr > kl ? s : -s;
+}
+
 // BND 0: periodic lines; 1: the reference's boundaries, derivative of the sweep
 // input; 2: the reference's third sweep, which differentiates the remapped
 // field.  Its interior right-hand side R_k + sum_t wq_t R_{k+n0-2+t} with R_j =
@@ -364,11 +460,12 @@ __device__ __forceinline__ StreamField stream_field(const SweepField &f) {
 // recurrence is a few cells longer.  2048^2: one pass of 21.3 us for two of
 // 18.2 us (eight steps 317 -> 255 us).
 template <typename T, int DIR, int LN, int BND>
-__global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 : 6)
+__global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
+                                  BND == 4 ? (DIR == 0 ? 2 : 4) : (DIR == 0 ? 4 : 6))
     stream_kernel(const __grid_constant__ PlanFields plan, const SweepField *__restrict__ fields,
                   int nfields, int first, const FieldIo io, int rows, unsigned *status,
                   int jstep, int nslice, const int *nlo, int cs, int clustered,
-                  const int *g0idx, int ends) {
+                  const int *g0idx, int ends, double toff) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NT = StreamCta<DIR, LN>::warps * 32;
   constexpr int LPW = StreamCta<DIR, LN>::lpw;
@@ -377,6 +474,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   constexpr unsigned FULL = 0xffffffffu;
   constexpr bool ENDS = BND == 1 || BND == 2;  // the reference's boundaries
   constexpr bool XX = BND == 3;
+  constexpr bool SWIRL = BND == 4;
   T *tile_s = reinterpret_cast<T *>(smem_raw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
@@ -394,7 +492,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   void *vd;
   if (plan.tiles > 0) {
     F = stream_field(plan.f);
-    D = &plan.f;
+    // (the swirling field's times differ from slice to slice)
+    D = SWIRL ? fields + (first + (int)blockIdx.z) : &plan.f;
     tile = blockIdx.x;
     rank = blockIdx.y;
     field_io(plan.f, jstep, io, &vs, &vd);
@@ -408,6 +507,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
     const SweepField &f = fields[find_field(fields, g0idx, nfields, cta / cs)];
     F = stream_field(f);
     D = &f;
+    if (SWIRL) toff = field_time(f, toff, jstep, nslice);
     const int q = cta - F.cta0;
     rank = clustered ? q % cs : q / F.groups;
     tile = clustered ? q / cs : q - rank * F.groups;
@@ -505,15 +605,36 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
                 (size_t)line *
                     (BND == 2 ? STREAM_TAPS_D : BND == 1 ? STREAM_TAPS_C : XX ? STREAM_TAPS_XX : 8);
   T o[8];
-  if (!ENDS) load_taps(o, wt);
-  const int n0 = __ldg(F.nt + line);
+  if (!ENDS && !SWIRL) load_taps(o, wt);
+  const int n0 = SWIRL ? 0 : __ldg(F.nt + line);
+  // swirling field: sin and cos of the edges org-1 .. of the walked positions,
+  // and the speeds of the line's two corner lines
+  double2 *const sc_edge = reinterpret_cast<double2 *>(
+      tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows);
+  CornerLine c0{0, 0, 0}, c1{0, 0, 0};
+  int series = 0;
+  if (SWIRL) {
+    for (int i = threadIdx.x; i < act * SCH + 3; i += NT) {
+      const double s = D->s_min + D->h * (org - 1 + i);
+      sc_edge[i] = double2{sinpi(s), cospi(s)};
+    }
+    const double ca = cospi((toff + D->ta_rel) / D->vp[0]);
+    const double cb = cospi((toff + D->tb_rel) / D->vp[0]);
+    const double sg = DIR == 0 ? 1.0 : -1.0, Dt = D->Dt;
+    const double g0 = sg * sinpi(2.0 * (D->t_min + D->ht * (double)line));
+    const double g1 = sg * sinpi(2.0 * (D->t_min + D->ht * (double)(line + 1)));
+    const double pd = 3.14159265358979323846 * Dt;
+    c0 = CornerLine{g0 * cb, g0 * ca, pd * (g0 * cb)};
+    c1 = CornerLine{g1 * cb, g1 * ca, pd * (g1 * cb)};
+    series = pd <= 0.00390625 ? 2 : pd <= 0.03125 ? 1 : 0;  // |speed| <= 1
+  }
   static_assert(SCH == 17, "pw");
   T pw = mmu * mmu;  // (-mu)^17
   pw *= pw;
   pw *= pw;
   pw *= pw * mmu;
   cp_async_wait_all_committed();
-  if (DIR == 0) __syncthreads(); else __syncwarp();
+  if (DIR == 0 || SWIRL) __syncthreads(); else __syncwarp();
   // In place, the segments of a line are read (halo) by the neighbouring CTAs
   // of its cluster: no CTA stores before every CTA has staged.
   if (clustered) {
@@ -525,7 +646,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   T *const col = DIR == 0 ? tile_s + warp * LPW + lw : tile_s + (size_t)(warp * LPW + lw) * rows;
   const int k0 = (ENDS ? org - b0 : H - J) + c * SCH;  // staged row of this lane's first position
   const int r0 = XX ? k0 + 2 * n0 - 6 : k0 + n0 - 3;  // row of the first tap
-  bool ok = r0 >= 0 && r0 + SCH + (XX ? 14 : 7) <= rows;
+  bool ok = SWIRL || (r0 >= 0 && r0 + SCH + (XX ? 14 : 7) <= rows);
   if (BND == 2) ok = ok && k0 + 2 * n0 - 5 >= 0 && k0 + 2 * n0 + SCH + 8 <= rows;
   if (!ok && line < M) atomicOr(status, STATUS_HALO);
   // inputs of the positions next to the line's ends (BND): the left region is
@@ -595,7 +716,49 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
   if (ENDS && F.JD > 4 * SCH) ns = LN == 32 ? 5 : 4;
   T v[SCH];
   if (ENDS) load_taps(o, wt);
-  stencil<T, ES, 8, false>(col + (ok ? r0 : 0) * ES, o, v);
+  if (SWIRL) {
+    // b of the positions k0-1 .. k0+17 from the feet of their edges, then the
+    // mass matrix: v_i = (1/12c)(b_{i-1} + 10 b_i + b_{i+1})
+    if (c < act) {
+      const int kp = org + c * SCH;
+      const double s_min = D->s_min, h = D->h, Dt = D->Dt;
+      const double hd = 3.0 * Dt * D->inv12h;  // Dt / (4 h)
+      const T kbc = T(D->kb * D->inv12h), icw = T(D->sm_inv_den / 12.0);
+      int bad = 0;
+      T bl[SCH + 2];  // b, in a loop small enough for the instruction cache
+      auto cells_b = [&](auto order) {
+        constexpr int SERIES = decltype(order)::value;
+        auto edge = [&](int i) {  // edge kp - 1 + i
+          const double2 t = sc_edge[c * SCH + i];
+          const double s = SERIES ? 0.0 : s_min + h * (kp - 1 + i);
+          const double u = -hd * (corner_speeds<SERIES>(c0, t.x, t.y, s, Dt) +
+                                  corner_speeds<SERIES>(c1, t.x, t.y, s, Dt));
+          return swirl_edge<T, ES>(kp - 1 + i, u, col, b0, nr, bad);
+        };
+        SwirlEdge<T> l = edge(0);
+#pragma unroll 2
+        for (int i = 0; i < SCH + 2; ++i) {
+          const SwirlEdge<T> r = edge(i + 1);
+          T m = r.phi - l.phi;
+          if (r.kf == l.kf + 1) m += l.z;
+          else if (r.kf != l.kf) m += cells_between<T, ES>(l.kf, r.kf, col, b0, nr, status);
+          bl[i] = m + kbc * (r.d - l.d);
+          l = r;
+        }
+      };
+      if (series == 2) cells_b(Series<2>());
+      else if (series == 1) cells_b(Series<1>());
+      else cells_b(Series<0>());
+#pragma unroll
+      for (int i = 0; i < SCH; ++i) v[i] = icw * ((bl[i] + bl[i + 2]) + T(10.0) * bl[i + 1]);
+      if (bad && line < M) atomicOr(status, STATUS_HALO);
+    } else {
+#pragma unroll
+      for (int i = 0; i < SCH; ++i) v[i] = T(0);
+    }
+  } else {
+    stencil<T, ES, 8, false>(col + (ok ? r0 : 0) * ES, o, v);
+  }
   if (XX) {
     load_taps(o, wt + 8);
     stencil<T, ES, 7, true>(col + (ok ? r0 + 8 : 0) * ES, o, v);
@@ -748,7 +911,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32, DIR == 0 ? 4 :
 
 template <typename T>
 using StreamKernelT = void (*)(const PlanFields, const SweepField *, int, int, const FieldIo, int,
-                               unsigned *, int, int, const int *, int, int, const int *, int);
+                               unsigned *, int, int, const int *, int, int, const int *, int,
+                               double);
 
 template <typename T, int BND>
 StreamKernelT<T> stream_kernel_of(int dir, int lanes) {
@@ -757,6 +921,7 @@ StreamKernelT<T> stream_kernel_of(int dir, int lanes) {
 }
 template <typename T>
 StreamKernelT<T> stream_kernel_for(int variant, int dir, int lanes) {
+  if (variant == SWEEP_CELL) return stream_kernel_of<T, 4>(dir, lanes);
   if (variant == SWEEP_FILTER_XX) return stream_kernel<T, 0, 16, 3>;
   return variant == SWEEP_COMPAT     ? stream_kernel_of<T, 1>(dir, lanes)
          : variant == SWEEP_COMPAT_D ? stream_kernel_of<T, 2>(dir, lanes)
@@ -772,12 +937,13 @@ int stream_tile_lines(int dir, int lanes) {
 size_t stream_smem_bytes(const LaunchGeom &G, bool fp64) {
   const size_t el = fp64 ? 8 : 4, lines = stream_tile_lines(G.dir, G.lanes);
   return (G.dir == 0 ? (size_t)X_PITCH : lines) * G.rows * el +
-         lines * 2 * (size_t)G.ends * (3 * el + sizeof(int));
+         lines * 2 * (size_t)G.ends * (3 * el + sizeof(int)) +
+         (G.variant == SWEEP_CELL ? sizeof(double2) * ((size_t)G.lanes * STREAM_CH + 3) : 0);
 }
 
 template <typename T>
 cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const SweepField *d_fields,
-                          int nfields, int group_base, int groups_total, const FieldIo &io,
+                          int nfields, int group_base, int groups_total, double toff, const FieldIo &io,
                           unsigned *d_status, int jstep, int nslice, const int *nlo,
                           bool inplace, cudaStream_t stream, const int *g0idx, bool pdl) {
   // Function attributes apply to the device that is current when they are
@@ -791,7 +957,7 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   if (!configured[dev].load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lk(config_mu);
     if (!configured[dev].load(std::memory_order_relaxed)) {
-      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D, SWEEP_FILTER_XX})
+      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D, SWEEP_FILTER_XX, SWEEP_CELL})
         for (int l : {0, 16, 32}) {
           const void *fn = (const void *)stream_kernel_for<T>(v, l ? 1 : 0, l);
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -832,15 +998,15 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   count_launch();
   return cudaLaunchKernelEx(&cfg, stream_kernel_for<T>(G.variant, G.dir, G.lanes), plan, d_fields, nfields,
                             by_value ? group_base / plan.tiles : group_base * G.cs, io, G.rows,
-                            d_status, jstep, nslice, nlo, G.cs, clustered, g0idx, G.ends);
+                            d_status, jstep, nslice, nlo, G.cs, clustered, g0idx, G.ends, toff);
 }
 
 template cudaError_t launch_stream<double>(const LaunchGeom &, const PlanFields &,
-                                           const SweepField *, int, int, int, const FieldIo &, unsigned *,
+                                           const SweepField *, int, int, int, double, const FieldIo &, unsigned *,
                                            int, int, const int *, bool, cudaStream_t, const int *,
                                            bool);
 template cudaError_t launch_stream<float>(const LaunchGeom &, const PlanFields &,
-                                          const SweepField *, int, int, int, const FieldIo &, unsigned *,
+                                          const SweepField *, int, int, int, double, const FieldIo &, unsigned *,
                                           int, int, const int *, bool, cudaStream_t, const int *,
                                           bool);
 

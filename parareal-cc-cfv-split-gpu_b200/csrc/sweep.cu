@@ -2023,7 +2023,6 @@ template <typename T>
 static FilterKernelT<T> filter_kernel_for(int variant) {
   switch (variant) {
     case SWEEP_FILTER_EXACT: return sweep_filter_kernel<T, true, false, false>;
-    case SWEEP_CELL: return sweep_filter_kernel<T, false, true, false>;
     case SWEEP_CELL_EXACT: return sweep_filter_kernel<T, true, true, false>;
     case SWEEP_CELL_COMPAT: return sweep_filter_kernel<T, false, true, true>;
     default: return nullptr;
@@ -2050,7 +2049,7 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
                                bool inplace, cudaStream_t stream, const int *g0idx, bool pdl_ok) {
   const int variant = G.variant, cs = G.cs, lc_max = G.lc_max, halo = G.halo;
   if (stream_variant(variant))
-    return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, io, d_status,
+    return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, toff, io, d_status,
                             jstep, nslice, nlo, inplace, stream, g0idx, pdl_ok && pdl_enabled());
   const bool fast = (variant == SWEEP_FAST);
   const bool cell = cell_filter_variant(variant);
@@ -2077,7 +2076,6 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
         for (const void *fn :
              {(const void *)sweep_kernel<T>, (const void *)sweep_fast_kernel<T>,
               (const void *)filter_kernel_for<T>(SWEEP_FILTER_EXACT),
-              (const void *)filter_kernel_for<T>(SWEEP_CELL),
               (const void *)filter_kernel_for<T>(SWEEP_CELL_EXACT),
               (const void *)filter_kernel_for<T>(SWEEP_CELL_COMPAT)}) {
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,

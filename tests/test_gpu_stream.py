@@ -106,3 +106,22 @@ def test_step_sequences_match_oracle(oracle, ccfv, nx, ny, K, n):
     out = c.cpu().numpy()
     assert rel_l2(out, oracle.run(g, C0, 0.0, dt, n)) < TOL
     assert abs(out.sum() - C0.sum()) < 1e-12 * np.abs(C0).sum()
+
+
+@pytest.mark.parametrize("nx,ny", [(45, 46), (240, 239), (300, 270), (50, 1100)])
+@pytest.mark.parametrize("cfl", [0.8, 6.0, 20.0])
+def test_swirl_matches_oracle_at_small_and_large_steps(oracle, ccfv, nx, ny, cfl):
+    """Corner feet by a short series (fine steps), a longer one and sines of
+    their own (coarse steps on small grids); ragged tiles, one and several
+    segments, feet several cells from their edge."""
+    K, dt = 1e-4, cfl / max(nx, ny)
+    C0 = periodic_field(nx, nx + 2, ny=ny)
+    g = oracle.grid(nx, ny, bc=1, vel=3, vp=(1.5,), K=K, threads=THREADS, scheme=1)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=3, vel_params=(1.5,), K=K, scheme=1))
+    assert "cell" in [v for v, _ in s.sweep_plan(dt)]
+    c = dev(C0)
+    s.run(c, 0.2, dt, 3)
+    s.check()
+    out = c.cpu().numpy()
+    assert rel_l2(out, oracle.run(g, C0, 0.2, dt, 3)) < TOL
+    assert abs(out.sum() - C0.sum()) < 1e-12 * np.abs(C0).sum()
