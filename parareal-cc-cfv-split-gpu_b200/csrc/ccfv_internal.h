@@ -302,6 +302,9 @@ bool resident_g_fits(int nx, int ny, bool fp64, bool cell);
 cudaError_t launch_resident_g(bool fp64, bool cell, const ResidentG *d_rg, int n, size_t smem,
                               const int *nlo, cudaStream_t st);
 
+// Whether launches use programmatic dependent launch (CCFV_PDL).
+bool pdl_enabled();
+
 // Counts kernel launches made by the library.
 void count_launch(uint64_t n = 1);
 uint64_t launches();

@@ -1,6 +1,7 @@
 // engine.cu -- solver context, line-invariant tridiagonal factors, step plans,
 // propagators and the Parareal engine of libccfv.
 #include "engine.h"
+#include "reduce.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -787,68 +788,50 @@ __global__ void convert_kernel(const S *__restrict__ src, D *__restrict__ dst, l
 constexpr int RED_THREADS = 256;
 constexpr int RED_BLOCKS = 592;  // 4 x 148 SMs
 
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // U+[n+1] = G + (F - Gold)  (STANDARD; parareal_correction_kernel, T2S4:771-782)
 // U+[n+1] = F + G(e)        (DELTA)
 // fused with the update norms sum (U+ - U)^2 and sum U+^2, reduced
 // deterministically (fixed-order block partials, last block finishes).
 // STANDARD stores G into Gold; DELTA stores the new increment into Wd.  G is
-// read from Wg (the buffer the coarse sweep sequence ended in; Wg may be Wd).
+// read from Wg (the buffer the coarse sweep sequence ended in; Wg may be Wd;
+// null: G = 0).  Bound by latency between short coarse passes: launched as
+// their dependent, four cells a thread in flight, the last sum over all threads
+// of the last block (one thread summing 592 partials was 9 us).
 template <typename TG>
 __global__ void __launch_bounds__(RED_THREADS)
-    correction_kernel(int form, long long n, double *__restrict__ U, const double *__restrict__ Fv,
-                      double *__restrict__ Gold, const TG *Wg, TG *Wd,
-                      double *__restrict__ partial, unsigned *__restrict__ counter,
-                      double *__restrict__ out) {
+    correction_kernel(int form, long long n, double *U, const double *Fv, double *Gold,
+                      const TG *Wg, TG *Wd, double *partial, unsigned *counter, double *out) {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   double se = 0.0, su = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double uo = U[i];
-    const double gw = (double)Wg[i];
-    double un;
-    if (form == CCFV_FORM_STANDARD) {
-      un = gw + (Fv[i] - Gold[i]);
-      Gold[i] = gw;
-    } else {
-      un = Fv[i] + gw;
+  const bool standard = form == CCFV_FORM_STANDARD;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
+    double uo[4], gw[4], fv[4], go[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long i = i0 + j * stride;
+      if (i < n) {
+        uo[j] = U[i];
+        gw[j] = Wg ? (double)Wg[i] : 0.0;
+        fv[j] = Fv[i];
+        go[j] = standard ? Gold[i] : 0.0;
+      }
     }
-    const double d = un - uo;
-    U[i] = un;
-    if (form != CCFV_FORM_STANDARD) Wd[i] = (TG)d;
-    se += d * d;
-    su += un * un;
-  }
-  __shared__ double red[2][RED_THREADS / 32];
-  __shared__ bool last;
-  se = warp_sum(se);
-  su = warp_sum(su);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { red[0][w] = se; red[1][w] = su; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0, b = 0;
-    for (int k = 0; k < RED_THREADS / 32; ++k) { a += red[0][k]; b += red[1][k]; }
-    partial[2 * blockIdx.x] = a;
-    partial[2 * blockIdx.x + 1] = b;
-    __threadfence();
-    last = (atomicAdd(counter, 1u) == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    double a = 0, b = 0;
-    for (unsigned k = 0; k < gridDim.x; ++k) {
-      a += ((volatile double *)partial)[2 * k];
-      b += ((volatile double *)partial)[2 * k + 1];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long i = i0 + j * stride;
+      if (i < n) {
+        const double un = standard ? gw[j] + (fv[j] - go[j]) : fv[j] + gw[j];
+        const double d = un - uo[j];
+        U[i] = un;
+        if (standard) Gold[i] = gw[j]; else Wd[i] = (TG)d;
+        se += d * d;
+        su += un * un;
+      }
     }
-    out[0] = a;
-    out[1] = b;
-    *counter = 0;
   }
+  reduce_pair<RED_THREADS>(se, su, partial, counter, (int)gridDim.x, out);
 }
 
 static int grid_for(long long n) {
@@ -867,10 +850,18 @@ static int convert(ccfv_ctx *ctx, const S *src, D *dst, long long n, cudaStream_
 template <typename TG>
 static int correction(ccfv_ctx *ctx, int form, long long n, double *U, const double *Fv,
                       double *Gold, const TG *Wg, TG *Wd, double *out, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid_for(n), 1, 1);
+  cfg.blockDim = dim3(RED_THREADS, 1, 1);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
   count_launch();
-  correction_kernel<TG><<<grid_for(n), RED_THREADS, 0, st>>>(
-      form, n, U, Fv, Gold, Wg, Wd, ctx->partial.as<double>(), ctx->counter.as<unsigned>(), out);
-  CK(cudaGetLastError());
+  CK(cudaLaunchKernelEx(&cfg, correction_kernel<TG>, form, n, U, Fv, Gold, Wg, Wd,
+                        ctx->partial.as<double>(), ctx->counter.as<unsigned>(), out));
   return CCFV_OK;
 }
 
@@ -1010,8 +1001,7 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
         if ((rc = run_steps(ctx, cplan, g64, 0, 1, o->t0 + n * DT, dtc, m, st, io))) return rc;
         coarse_cu += (double)m * NN;
       } else if (n == nlo) {
-        CK(cudaMemsetAsync(W, 0, sizeof(TG) * NN, st));  // G(0) = 0
-        Gn = W;
+        Gn = nullptr;  // G(0) = 0
       } else {
         if ((rc = coarse_on_W(n, dplan))) return rc;
         coarse_cu += (double)m * NN;

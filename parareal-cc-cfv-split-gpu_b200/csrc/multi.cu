@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "multi.h"
+#include "reduce.cuh"
 
 namespace ccfv {
 namespace {
@@ -55,89 +56,70 @@ __global__ void __launch_bounds__(BT)
                       double *__restrict__ partial, unsigned *__restrict__ counters) {
   const int inst = blockIdx.y;
   const BElem b = d[inst];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int lo = nlo[inst];
   const long long cnt = b.NN;
   if (op == OP_LOAD_W_STD) {  // G-phase: only the standard form restarts G from U
     if (b.form != CCFV_FORM_STANDARD) return;
     op = OP_LOAD_W;
   }
-  switch (op) {
-    case OP_LOAD_W:
-    case OP_STORE_W:
-    case OP_CORRECT:
-      if (n >= b.S || n < lo) return;
-      break;
-  }
+  if (n >= b.S || n < lo) return;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  double se = 0.0, su = 0.0;
   if (op == OP_LOAD_W) {  // FP64 W: the first coarse sweep, standard-form G
-    const double *src = b.U + (long long)n * b.NN;
-    double *w = reinterpret_cast<double *>(b.W);
-    for (long long i = first; i < cnt; i += stride) w[i] = src[i];
+    const double *__restrict__ src = b.U + (long long)n * b.NN;
+    double *__restrict__ w = reinterpret_cast<double *>(b.W);
+#pragma unroll 4
+    for (long long i = first; i < cnt; i += stride) w[i] = __ldcg(src + i);
   } else if (op == OP_STORE_W) {
     double *dst = b.U + (long long)(n + 1) * b.NN;
     double *gd = b.Gold ? b.Gold + (long long)(n + 1) * b.NN : nullptr;
     const double *w = reinterpret_cast<const double *>(b.Wres);
+#pragma unroll 4
     for (long long i = first; i < cnt; i += stride) {
-      const double v = w[i];
+      const double v = __ldcg(w + i);
       dst[i] = v;
       if (gd) gd[i] = v;
     }
   } else {
+    if (b.pad) return;  // resident coarse propagator: corrected in its own kernel
     double *U = b.U + (long long)(n + 1) * b.NN;
     const double *Fv = b.F + (long long)(n + 1) * b.NN;
-    double *Go = b.Gold ? b.Gold + (long long)(n + 1) * b.NN : nullptr;
-    if (b.pad) return;  // resident coarse propagator: corrected in its own kernel
-    const bool zero_g = (b.form == CCFV_FORM_DELTA && n == lo);  // G(0) = 0
+    const bool standard = b.form == CCFV_FORM_STANDARD;
+    double *Go = standard ? b.Gold + (long long)(n + 1) * b.NN : nullptr;
+    const bool zero_g = !standard && n == lo;  // G(0) = 0
+    double se = 0.0, su = 0.0;
     // G is read from Wres; the new increment goes to W (elementwise, so the
-    // two may be the same buffer)
-    for (long long i = first; i < cnt; i += stride) {
-      const double uo = U[i];
-      const double gw = zero_g ? 0.0 : wload(b, i);
-      double un;
-      if (b.form == CCFV_FORM_STANDARD) {
-        un = gw + (Fv[i] - Go[i]);  // parareal_correction_kernel, T2S4:771-782
-        Go[i] = gw;
-      } else {
-        un = Fv[i] + gw;
-        wstore(b, i, un - uo);
+    // two may be the same buffer); four cells a thread in flight
+    for (long long i0 = first; i0 < cnt; i0 += 4 * stride) {
+      double uo[4], gw[4], fv[4], go[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const long long i = i0 + j * stride;
+        if (i < cnt) {
+          uo[j] = U[i];
+          gw[j] = zero_g ? 0.0 : wload(b, i);
+          fv[j] = Fv[i];
+          go[j] = standard ? Go[i] : 0.0;
+        }
       }
-      const double dd = un - uo;
-      U[i] = un;
-      se += dd * dd;
-      su += un * un;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      se += __shfl_down_sync(0xffffffffu, se, o);
-      su += __shfl_down_sync(0xffffffffu, su, o);
-    }
-    __shared__ double red[2][BT / 32];
-    __shared__ bool last;
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { red[0][w] = se; red[1][w] = su; }
-    __syncthreads();
-    double *part = partial + (size_t)inst * 2 * gridDim.x;
-    if (threadIdx.x == 0) {
-      double a = 0, c = 0;
-      for (int k = 0; k < BT / 32; ++k) { a += red[0][k]; c += red[1][k]; }
-      part[2 * blockIdx.x] = a;
-      part[2 * blockIdx.x + 1] = c;
-      __threadfence();
-      last = (atomicAdd(&counters[inst], 1u) == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-      __threadfence();
-      double a = 0, c = 0;
-      for (unsigned k = 0; k < gridDim.x; ++k) {
-        a += ((volatile double *)part)[2 * k];
-        c += ((volatile double *)part)[2 * k + 1];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const long long i = i0 + j * stride;
+        if (i < cnt) {
+          // parareal_correction_kernel, T2S4:771-782
+          const double un = standard ? gw[j] + (fv[j] - go[j]) : fv[j] + gw[j];
+          const double dd = un - uo[j];
+          U[i] = un;
+          if (standard) Go[i] = gw[j]; else wstore(b, i, dd);
+          se += dd * dd;
+          su += un * un;
+        }
       }
-      b.norms[2 * (n + 1)] = a;
-      b.norms[2 * (n + 1) + 1] = c;
-      counters[inst] = 0;
     }
+    reduce_pair<BT>(se, su, partial + (size_t)inst * 2 * gridDim.x, &counters[inst],
+                    (int)gridDim.x, b.norms + 2 * (n + 1));
   }
 }
 
@@ -654,10 +636,19 @@ bool MultiEngine::elem_active(int op, int n) const {
 int MultiEngine::elem(int op, int slice) {
   const int n = (int)slots_.size();
   if (!n || !elem_active(op, slice)) return CCFV_OK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(148, (unsigned)n, 1);
+  cfg.blockDim = dim3(BT, 1, 1);
+  cfg.stream = st_;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
   count_launch();
-  batch_elem_kernel<<<dim3(148, n), BT, 0, st_>>>(op, elems_.as<BElem>(), slice, nlo_d_.as<int>(),
-                                                   partial_.as<double>(), counters_.as<unsigned>());
-  MCK(cudaGetLastError());
+  MCK(cudaLaunchKernelEx(&cfg, batch_elem_kernel, op, (const BElem *)elems_.as<BElem>(), slice,
+                         (const int *)nlo_d_.as<int>(), partial_.as<double>(),
+                         counters_.as<unsigned>()));
   return CCFV_OK;
 }
 

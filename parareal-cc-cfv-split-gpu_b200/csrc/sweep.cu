@@ -2033,7 +2033,7 @@ static FilterKernelT<T> filter_kernel_for(int variant) {
 // before reading cells, after fetching what is constant.  Batch of 64 mixed
 // instances: 1323 ms without, 1276 ms with; 12 instances up to 583^2: 115 ms
 // without, 97 ms with.  CCFV_PDL=0 turns it off.
-static bool pdl_enabled() {
+bool pdl_enabled() {
   static const bool on = [] {
     const char *e = std::getenv("CCFV_PDL");
     return !(e && e[0] == '0');
