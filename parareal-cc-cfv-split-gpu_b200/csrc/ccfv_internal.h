@@ -92,6 +92,10 @@ struct SweepField {
                            // filter kernel: 1 / c
   const void *tab;         // T[3L]: alpha_k | g_k | z_k (solver factors)
   double rk_a;             // compat: mu^2 / (1 - mu^(2L+2)), rank-one closure
+  // exact form, q = -mu: q^n of a whole segment and of the line's last one,
+  // 1/(1 - q^2), 1/(1 - q^L), and q^-(positions that the last segment's last
+  // lane walks behind it)
+  double ex[5];
   // Filter kernel: per-line stencil of w's input, computed once per plan
   // (the velocity fields it serves do not depend on time); null: computed
   // per tile.  wt: T[groups*LPG][8] taps -3..4; nt: int[groups*LPG] shifts.
@@ -136,22 +140,23 @@ enum { SWEEP_GENERAL = 0, SWEEP_FAST = 1, SWEEP_FILTER = 2, SWEEP_GENERAL_SRC = 
        SWEEP_COMPAT = 8, SWEEP_COMPAT_D = 9, SWEEP_FILTER_XX = 10 };
 inline bool stream_variant(int v) {
   return v == SWEEP_FILTER || v == SWEEP_COMPAT || v == SWEEP_COMPAT_D ||
-         v == SWEEP_FILTER_XX || v == SWEEP_CELL;
+         v == SWEEP_FILTER_XX || v == SWEEP_CELL || v == SWEEP_FILTER_EXACT ||
+         v == SWEEP_CELL_EXACT;
 }
 // Variants run by the filter kernels (factored solve).
 inline bool filter_variant(int v) {
-  return stream_variant(v) || v == SWEEP_FILTER_EXACT ||
-         v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT;
+  return stream_variant(v) || v == SWEEP_CELL_COMPAT;
 }
 // Warm-up (segmented) forms: lines longer than MAX_CLUSTER segments are
 // allowed out of place.
 inline bool warm_filter_variant(int v) {
-  return stream_variant(v) || v == SWEEP_CELL_COMPAT;
+  return (stream_variant(v) && v != SWEEP_FILTER_EXACT && v != SWEEP_CELL_EXACT) ||
+         v == SWEEP_CELL_COMPAT;
 }
 // Variants whose right-hand side is the per-line stencil table (SweepField::wt),
 // and its values per line.
 inline bool stencil_filter_variant(int v) {
-  return (stream_variant(v) && v != SWEEP_CELL) || v == SWEEP_FILTER_EXACT;
+  return stream_variant(v) && v != SWEEP_CELL && v != SWEEP_CELL_EXACT;
 }
 constexpr int STREAM_TAPS_C = 10;   // 8 taps, the feet's offset in a cell last
 constexpr int STREAM_TAPS_D = 24;   // 8 + 13 taps, likewise
@@ -167,7 +172,7 @@ inline bool cell_filter_variant(int v) {
 }
 // The filter kernel's cluster form (exact periodic closure, out of place).
 inline bool exact_filter_variant(int v) { return v == SWEEP_FILTER_EXACT || v == SWEEP_CELL_EXACT; }
-constexpr int FILTER_JMAX = 64;  // longest recurrence warm-up of the filter kernel
+constexpr int FILTER_JMAX = 64;  // longest recurrence warm-up with 16 lanes per line
 
 // Launch geometry shared by all fields of one sweep launch.
 struct LaunchGeom {
@@ -177,6 +182,7 @@ struct LaunchGeom {
   int rows = 0;           // streaming form: staged positions per line (at most)
   int ends = 0;           // streaming form, reference's boundaries: scratch values per
                           // line end (edges and cells next to it)
+  bool strong = false;    // streaming form: warm-up past FILTER_JMAX
   int lc_fit = 0, halo_fit = 0;  // tile of the scan kernels: a step whose scan tile
                                  // does not fit is refused whatever form runs it
 };
@@ -204,7 +210,12 @@ struct PlanFields {
 // of L cells in cs segments (even: pairs of cells stay aligned); lines per CTA;
 // shared memory of a launch.
 constexpr int STREAM_CH = 17;
+constexpr int FILTER_JLONG = 8 * STREAM_CH;  // longest warm-up with 32 lanes per line
 __host__ __device__ inline int stream_seg(int L, int cs) { return ((L + cs - 1) / cs + 1) & ~1; }
+// Exact form: whole walks, or one segment.
+__host__ __device__ inline int exact_seg(int L, int cs, int lanes) {
+  return cs > 1 ? lanes * STREAM_CH : (L + 1) & ~1;
+}
 int stream_tile_lines(int dir, int lanes);
 size_t stream_smem_bytes(const LaunchGeom &G, bool fp64);
 // Lines per CTA of a launch geometry.

@@ -313,14 +313,17 @@ bool class_tuned(int L, bool fp64) {
 // segments repeat less of it), or as the tuner found; a y line takes 32 lanes
 // unless 16 cover it with much fewer lanes in all (lines of one short segment):
 // a lane of the 16-lane kernel issues 1.37 times the instructions of one of the
-// 32-lane kernel (two lines' copies per warp, spills).  reach: cells a
-// right-hand side reads on either side.
+// 32-lane kernel (two lines' copies per warp, spills).  An x line takes 32 only
+// for a warm-up past FILTER_JMAX: a warp of one line reads its tile with twofold
+// bank conflicts (2048^2, eight steps at a diffusion number of 1 per x sweep:
+// 280 us with 16 lanes, 326 us with 32; at 5, J = 62, 352 us either way).
+// reach: cells a right-hand side reads on either side.
 static void stream_geom(LaunchGeom &G, int L, int J, int reach, int lc) {
   auto segs = [&](int lanes) {
-    const int seg = std::min((lanes * STREAM_CH - 2 * J) & ~1, std::max(32, lc + (lc & 1)));
+    const int seg = std::max(2, std::min((lanes * STREAM_CH - 2 * J) & ~1, std::max(32, lc + (lc & 1))));
     return (L + seg - 1) / seg;
   };
-  G.lanes = G.dir == 1 && 3 * segs(32) <= 2 * segs(16) ? 32 : 16;
+  G.lanes = (G.dir == 0 ? J > FILTER_JMAX : 3 * segs(32) <= 2 * segs(16)) ? 32 : 16;
   G.cs = segs(G.lanes);
   G.lc_max = stream_seg(L, G.cs);
   G.halo = (J + reach + 1) & ~1;
@@ -383,15 +386,46 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
     int J = 0;
     const bool warm = filter_params(g, dir, Dt, fp64, nullptr, nullptr, &J, theta) && L > 2 * J;
     const int seg_exact = filter_segment_max(0);  // cells per CTA without warm-up
-    if (!warm && !inplace && (L + seg_exact - 1) / seg_exact <= MAX_CLUSTER) {
-      // strong diffusion, out of place: the filter kernel's cluster form
-      // (exact periodic closure across the segments, no warm-up)
+    const bool closed = !inplace && (L + seg_exact - 1) / seg_exact <= MAX_CLUSTER;
+    // Strong diffusion.  Lines longer than one segment, the same stencil all
+    // along: a warm-up of up to a quarter of the 32 lanes' positions (eight
+    // steps at a diffusion number of 10 per x sweep and 20 per y sweep, the
+    // segments of a line as a cluster that closes it exactly against the
+    // warm-up: 1024^2 214 -> 162 us, 2048^2 555 -> 409 us, 4096^2 2434 -> 1461
+    // us; y sweeps at 28, J = 146: 2048^2 445 us closed, 477 us warmed up).
+    // Whole lines, longer warm-ups and the per-cell right-hand sides (far more
+    // work per position): closed.
+    LaunchGeom S = G;
+    S.variant = SWEEP_FILTER;
+    S.strong = true;
+    S.lc_fit = G.lc_max;
+    S.halo_fit = G.halo;
+    if (closed) {
       const int lc = std::min(seg_exact, std::max({32, (L + MAX_CLUSTER - 1) / MAX_CLUSTER,
                                                    std::min(L, filter_lc(L, fp64))}));
+      S.cs = (L + lc - 1) / lc;
+      S.lc_fit = (L + S.cs - 1) / S.cs;
+      S.halo_fit = sh + 6;
+    }
+    bool longer = !warm && uniform && L > (dir == 0 ? 16 : 32) * STREAM_CH && J <= FILTER_JLONG &&
+                  L > 2 * J;
+    if (longer) {
+      LaunchGeom W = S;
+      stream_geom(W, L, J, sh + 6, L);
+      longer = !(inplace && W.cs > MAX_CLUSTER);
+      if (longer) G = W;
+    }
+    if (longer) {
+    } else if (!warm && closed) {
+      // no warm-up, the segments of a line form one cluster
+      G = S;
+      G.strong = false;
       G.variant = uniform ? SWEEP_FILTER_EXACT : SWEEP_CELL_EXACT;
-      G.cs = (L + lc - 1) / lc;
-      G.lc_max = (L + G.cs - 1) / G.cs;
-      G.halo = sh + 6;
+      G.lanes = dir == 1 && L > seg_exact ? 32 : 16;
+      G.cs = (L + G.lanes * STREAM_CH - 1) / (G.lanes * STREAM_CH);
+      G.lc_max = exact_seg(L, G.cs, G.lanes);
+      G.halo = (sh + 7) & ~1;
+      G.rows = (G.lanes * STREAM_CH + 2 * G.halo + 2) & ~1;
     } else if (warm) {
       G.variant = uniform ? SWEEP_FILTER : SWEEP_CELL;
       G.halo = J + sh + 6;
@@ -414,10 +448,9 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
       G.variant = SWEEP_FAST;
     }
     // the per-cell forms' tiles do not fit: per-cell scan kernel
-    if (G.variant == SWEEP_CELL_EXACT &&
-        sweep_filter_smem_bytes(G.lc_max, G.halo, fp64, true, true) > 227 * 1024)
+    if ((G.variant == SWEEP_CELL || G.variant == SWEEP_CELL_EXACT) &&
+        stream_smem_bytes(G, fp64) > 227 * 1024)
       G = general;
-    if (G.variant == SWEEP_CELL && stream_smem_bytes(G, fp64) > 227 * 1024) G = general;
   } else if (!g.source && g.bc == CCFV_BC_COMPAT) {
     // the reference's boundaries: the filter kernel's per-cell form with the
     // non-cyclic closure.  A line of at most one segment is solved exactly
@@ -469,7 +502,7 @@ bool fused_x_geom(const ccfv_grid &g, double dt, bool fp64, bool inplace, double
   double mu = 0;
   filter_params(g, 0, 0.5 * dt, fp64, &mu, nullptr, nullptr, theta);
   const int J = double_warm_up(mu, fp64);
-  if (g.nx <= 2 * J || 2 * J + 64 > 16 * STREAM_CH) return false;
+  if (g.nx <= 2 * J || 2 * J + 64 > 32 * STREAM_CH) return false;
   G->variant = SWEEP_FILTER_XX;
   stream_geom(*G, g.nx, J, 2 * shift_cells(g, 0, 0.5 * dt) + 10, stream_lc(g.nx, fp64));
   if (inplace && G->cs > MAX_CLUSTER) return false;
@@ -573,9 +606,18 @@ void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom
   f.sm_inv_den = ic;
   if (G.variant == SWEEP_FILTER_XX) J = double_warm_up(mu, fp64);
   f.jd = J;
-  // compat lines of one segment: the non-cyclic recurrences start exactly at
-  // the line's ends (no warm-up)
-  f.jf = (g.bc == CCFV_BC_COMPAT && G.cs == 1) ? 0 : J;
+  // no warm-up: compat lines of one segment (the non-cyclic recurrences start
+  // exactly at the line's ends) and the exact form
+  f.jf = (g.bc == CCFV_BC_COMPAT && G.cs == 1) || exact_filter_variant(G.variant) ? 0 : J;
+  if (exact_filter_variant(G.variant)) {
+    const double q = -mu;
+    const int seg = exact_seg(f.L, G.cs, G.lanes), end = f.L - (G.cs - 1) * seg;
+    f.ex[0] = std::pow(q, seg);
+    f.ex[1] = std::pow(q, end);
+    f.ex[2] = 1.0 / (1.0 - q * q);
+    f.ex[3] = 1.0 / (1.0 - std::pow(q, f.L));
+    f.ex[4] = std::pow(q, end - (end + STREAM_CH - 1) / STREAM_CH * STREAM_CH);
+  }
   f.rk_a = mu * mu / (1.0 - std::pow(mu * mu, f.L + 1));
   f.rk_tail = std::pow(std::fabs(mu), f.L) >= std::ldexp(1.0, -60) ? 1 : 0;
 }

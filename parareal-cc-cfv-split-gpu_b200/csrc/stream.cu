@@ -31,6 +31,8 @@
 // against 41.0 us for the copy rate and 62 us for the tile kernel this
 // replaced (8-byte copies, 16 lanes per line, carries added afterwards, two
 // CTA barriers; it issued 69 instructions per cell, this one about 26).
+#include <cooperative_groups.h>
+
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -39,6 +41,8 @@
 #include "sweep_device.cuh"
 #include "sweep_math.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace ccfv {
 
 namespace {
@@ -46,13 +50,12 @@ namespace {
 constexpr int SCH = STREAM_CH;     // positions per lane
 constexpr int X_LINES = 16;        // lines per CTA of an x sweep
 constexpr int X_PITCH = X_LINES + 2;
-constexpr int X_WARPS = X_LINES / 2;
 constexpr int Y_WARPS = 4;
 
 template <int DIR, int LN>
 struct StreamCta {
-  static constexpr int warps = DIR == 0 ? X_WARPS : Y_WARPS;
-  static constexpr int lpw = DIR == 0 ? 2 : 32 / LN;  // lines per warp
+  static constexpr int warps = DIR == 0 ? X_LINES * LN / 32 : Y_WARPS;
+  static constexpr int lpw = 32 / LN;  // lines per warp
   static constexpr int lines = warps * lpw;
 };
 
@@ -459,9 +462,21 @@ __device__ __noinline__ T cells_between(int kl, int kr, const T *cells, int b0, 
 // recurrence runs twice, then the backward one; the warm-up of such a double
 // recurrence is a few cells longer.  2048^2: one pass of 21.3 us for two of
 // 18.2 us (eight steps 317 -> 255 us).
-template <typename T, int DIR, int LN, int BND>
+//
+// EXACT (BND 0 and 4; any diffusion number): no warm-up.  Every segment of a
+// line runs both recurrences over its own cells from zero, which leaves it an
+// affine map of its carries, w_end = q^np w_in + E and x_start = q^np x_in + X
+// (q = -mu); the segments, one cluster, write E and X to each other and close
+// the periodic line exactly.  Segments are whole walks and a shorter last one;
+// a y line of 544 cells is one warp's and needs no exchange.  Bound by the
+// clusters' latency: 64 registers for the y kernel too, so that the next
+// launch's clusters find room beside this one's (1024^2, eight steps at
+// K dt / h^2 = 20: 264 us with 80 registers, 213 us with 64).  Against the tile
+// kernel: 256^2 163 -> 110 us, 1024^2 211 -> 213 us, 4096^2 2474 -> 2434 us;
+// swirling field, 1024^2 782 -> 420 us, 2048^2 2980 -> 1511 us.
+template <typename T, int DIR, int LN, int BND, bool EXACT>
 __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
-                                  BND == 4 ? (DIR == 0 ? 2 : 4) : (DIR == 0 ? 4 : 6))
+                                  BND == 4 ? (DIR == 0 ? 2 : 4) : DIR == 0 ? 64 / LN : EXACT ? 8 : 6)
     stream_kernel(const __grid_constant__ PlanFields plan, const SweepField *__restrict__ fields,
                   int nfields, int first, const FieldIo io, int rows, unsigned *status,
                   int jstep, int nslice, const int *nlo, int cs, int clustered,
@@ -470,7 +485,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   constexpr int NT = StreamCta<DIR, LN>::warps * 32;
   constexpr int LPW = StreamCta<DIR, LN>::lpw;
   constexpr int ES = DIR == 0 ? X_PITCH : 1;    // element stride of a position
-  constexpr int LS = DIR == 0 ? 2 : 1;          // lane stride of a chunk
+  constexpr int LS = DIR == 0 ? LPW : 1;        // lane stride of a chunk
   constexpr unsigned FULL = 0xffffffffu;
   constexpr bool ENDS = BND == 1 || BND == 2;  // the reference's boundaries
   constexpr bool XX = BND == 3;
@@ -516,11 +531,19 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (!field_active(f, jstep, nslice, nlo)) return;  // uniform over a cluster
   }
+  // exact form: its constants, then the values that the cluster exchanges
+  T *exs = tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows +
+           (SWIRL ? 2 * (LN * SCH + 3) * (sizeof(double) / sizeof(T)) : 0);
+  if (EXACT) {
+    if (threadIdx.x < 5) exs[threadIdx.x] = T(D->ex[threadIdx.x]);
+    // the peers may write to this CTA once it runs
+    if (cs > 1) asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");
+  }
   const T *src = reinterpret_cast<const T *>(vs);
   T *dst = reinterpret_cast<T *>(vd);
   const int L = F.L, M = F.M, J = F.J, H = F.H;
   const long long s_line = F.s_line, s_pos = F.s_pos;
-  const int Lc = plan.tiles > 0 ? plan.seg : stream_seg(L, cs);
+  const int Lc = plan.tiles > 0 ? plan.seg : EXACT ? exact_seg(L, cs, LN) : stream_seg(L, cs);
   const int p0 = min(L, rank * Lc), p1 = min(L, p0 + Lc), np = p1 - p0;
   const int line0 = tile * StreamCta<DIR, LN>::lines;        // first line of the CTA
   if (np <= 0 && !clustered) return;
@@ -597,8 +620,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   }
   cp_async_commit();
   // this lane's line and its stencil, while the cells arrive
-  const int c = DIR == 0 ? lane >> 1 : lane % LN;            // chunk
-  const int lw = DIR == 0 ? (lane & 1) : lane / LN;          // line within the warp
+  const int c = DIR == 0 ? lane / LPW : lane % LN;           // chunk
+  const int lw = DIR == 0 ? lane % LPW : lane / LN;          // line within the warp
   const int line = line0 + warp * LPW + lw;
   const T mmu = T(-F.mu);
   const T *wt = reinterpret_cast<const T *>(F.wt) +  // padded past M
@@ -634,10 +657,10 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   pw *= pw;
   pw *= pw * mmu;
   cp_async_wait_all_committed();
-  if (DIR == 0 || SWIRL) __syncthreads(); else __syncwarp();
+  if (DIR == 0 || SWIRL || EXACT) __syncthreads(); else __syncwarp();
   // In place, the segments of a line are read (halo) by the neighbouring CTAs
   // of its cluster: no CTA stores before every CTA has staged.
-  if (clustered) {
+  if (clustered && !EXACT) {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");
   }
@@ -712,8 +735,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   // one more, so that what is left out, |mu|^J of it at every chunk start, is
   // far below a rounding and not a share of one with the same sign everywhere)
   // (the reference's lines of one segment: no warm-up, any decay length).
-  int ns = (F.JD <= SCH ? 0 : F.JD <= 2 * SCH ? 1 : 2) + (sizeof(T) == 4 ? 1 : 0);
-  if (ENDS && F.JD > 4 * SCH) ns = LN == 32 ? 5 : 4;
+  int ns = (F.JD <= SCH ? 0 : F.JD <= 2 * SCH ? 1 : F.JD <= 4 * SCH ? 2 : F.JD <= 8 * SCH ? 3 : 4) + (sizeof(T) == 4 ? 1 : 0);
+  if (EXACT || (ENDS && F.JD > 4 * SCH)) ns = LN == 32 ? 5 : 4;
   T v[SCH];
   if (ENDS) load_taps(o, wt);
   if (SWIRL) {
@@ -832,14 +855,107 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
       v[i] = x;
     }
   }
-  T x = backward_carry();
+  T x, rise = T(0);  // rise (EXACT): the forward carry's share, before this lane's first position
+  if (!EXACT) {
+    x = backward_carry();
+  } else {
+    constexpr int W = DIR == 0 ? 32 : LN;      // shuffle width of a line
+    const int l0 = DIR == 0 ? lane % LPW : 0;  // its first lane
+    auto from = [&](T a, int ch) { return __shfl_sync(FULL, a, l0 + LS * ch, W); };
+    // E; nothing behind the segment for the backward recurrence
+    T E = v[SCH - 1];
+    if (np < LN * SCH) {
+      const int mine = np - c * SCH;  // positions of this lane
+#pragma unroll
+      for (int i = 0; i < SCH; ++i) {
+        if (i == mine - 1) E = v[i];
+        if (i >= mine) v[i] = T(0);
+      }
+    }
+    x = T(0);
+#pragma unroll
+    for (int i = SCH - 1; i >= 0; --i) x = v[i] + mmu * x;
+    // with the scan: q^(17 c), q^(17 (act-1-c))
+    T pd = pw, up = T(1), down = T(1);
+#pragma unroll
+    for (int b = 0; b < (LN == 32 ? 5 : 4); ++b) {
+      const T t = __shfl_down_sync(FULL, x, LS << b, W);
+      if (c + (1 << b) < LN) x += pd * t;
+      if (c >> b & 1) up *= pd;
+      if ((act - 1 - c) >> b & 1) down *= pd;
+      pd *= pd;
+    }
+    // The forward carry cr into a segment adds cr q^(j+1) to w_j (q = -mu),
+    // which the backward recurrence turns into A q^(j+1) - A q^(np+1) q^(np-j),
+    // A = cr / (1 - mu^2); the backward carry d from the right adds d q^(np-j).
+    const T whole = exs[0], last = exs[1], inv1m = exs[2], inv_line = exs[3];
+    T cr, d;  // this segment's carries
+    if (cs == 1) {
+      cr = from(E, act - 1) * inv_line;
+      d = (from(x, 0) + cr * (mmu * (T(1) - last * last) * inv1m)) * inv_line;
+    } else {
+      // every CTA writes its E and X to all of its cluster
+      T *ex = exs + 8 + 2 * MAX_CLUSTER * (warp * LPW + lw);
+      E = from(E, act - 1);
+      const T X = from(x, 0);
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+      if (c < cs) {
+        T *p = cg::this_cluster().map_shared_rank(ex, c) + 2 * rank;
+        p[0] = E;
+        p[1] = X;
+      }
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");
+      asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+      // lane r: segment r.  All but the last are Lc long, q^Lc = whole
+      const T e = c < cs ? ex[2 * c] : T(0), xr = c < cs ? ex[2 * c + 1] : T(0);
+      T S = e, pc = T(1), ps = whole;  // S: w at the end of segment r from a zero line start
+      for (int b = 0; (1 << b) < cs; ++b) {
+        const T t = __shfl_up_sync(FULL, S, LS << b, W);
+        if (c >= (1 << b)) S += ps * t;
+        if (c >> b & 1) pc *= ps;
+        ps *= ps;
+      }
+      const T w0 = (last * from(S, cs - 2) + from(e, cs - 1)) * inv_line;
+      S = __shfl_up_sync(FULL, S, LS, W);
+      const T cr_c = pc * w0 + (c > 0 ? S : T(0));
+      const T pr = c == cs - 1 ? last : whole;
+      T R = c < cs ? xr + cr_c * (mmu * (T(1) - pr * pr) * inv1m) : T(0);
+      ps = whole;
+      for (int b = 0; (1 << b) < cs; ++b) {
+        const T t = __shfl_down_sync(FULL, R, LS << b, W);
+        if (c + (1 << b) < LN) R += ps * t;
+        ps *= ps;
+      }
+      const T x0 = from(R, 0) * inv_line;  // x at the line's start
+      cr = from(cr_c, rank);
+      const T dn = from(R, min(rank + 1, cs - 1)) + from(pc, max(cs - 2 - rank, 0)) * last * x0;
+      d = rank + 1 < cs ? dn : x0;
+    }
+    const bool end = rank + 1 == cs;
+    rise = cr * inv1m * up;
+    const T far = d - cr * inv1m * mmu * (end ? last : whole);
+    x = __shfl_down_sync(FULL, x, LS, W);
+    if (c == LN - 1) x = T(0);
+    // carry into this lane; the last one, where it ends behind the segment,
+    // starts with as much more (q^-16 at most)
+    if (c < act) x += far * down * (end ? exs[4] : T(1));
+  }
   __syncwarp();  // every lane of the line has read its cells
   T *xp = col + k0 * ES;
 #pragma unroll
   for (int i = SCH - 1; i >= 0; --i) {
     x = v[i] + mmu * x;
-    if (ENDS) v[i] = x;
-    xp[i * ES] = x;
+    if (ENDS || EXACT) v[i] = x;
+    if (!EXACT) xp[i * ES] = x;
+  }
+  if (EXACT) {
+#pragma unroll
+    for (int i = 0; i < SCH; ++i) {
+      rise *= mmu;
+      xp[i * ES] = v[i] + rise;
+    }
   }
   if (ENDS && p0 == 0) {
     // non-cyclic system: A = c (1 + mu S^-1)(1 + mu S) + c mu^2 e_0 e_0^T, so
@@ -871,7 +987,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     }
   }
   if (DIR == 0) __syncthreads(); else __syncwarp();
-  if (clustered) asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+  if (clustered && !EXACT) asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
 
   // ---- store positions p0 .. p1-1 ----
   if (DIR == 0) {
@@ -914,15 +1030,20 @@ using StreamKernelT = void (*)(const PlanFields, const SweepField *, int, int, c
                                unsigned *, int, int, const int *, int, int, const int *, int,
                                double);
 
-template <typename T, int BND>
+template <typename T, int BND, bool EXACT = false>
 StreamKernelT<T> stream_kernel_of(int dir, int lanes) {
-  if (dir == 0) return stream_kernel<T, 0, 16, BND>;
-  return lanes == 32 ? stream_kernel<T, 1, 32, BND> : stream_kernel<T, 1, 16, BND>;
+  if constexpr (BND == 0 && !EXACT)
+    if (dir == 0 && lanes == 32) return stream_kernel<T, 0, 32, 0, false>;
+  if (dir == 0) return stream_kernel<T, 0, 16, BND, EXACT>;
+  return lanes == 32 ? stream_kernel<T, 1, 32, BND, EXACT> : stream_kernel<T, 1, 16, BND, EXACT>;
 }
 template <typename T>
 StreamKernelT<T> stream_kernel_for(int variant, int dir, int lanes) {
   if (variant == SWEEP_CELL) return stream_kernel_of<T, 4>(dir, lanes);
-  if (variant == SWEEP_FILTER_XX) return stream_kernel<T, 0, 16, 3>;
+  if (variant == SWEEP_FILTER_XX)
+    return lanes == 32 ? stream_kernel<T, 0, 32, 3, false> : stream_kernel<T, 0, 16, 3, false>;
+  if (variant == SWEEP_FILTER_EXACT) return stream_kernel_of<T, 0, true>(dir, lanes);
+  if (variant == SWEEP_CELL_EXACT) return stream_kernel_of<T, 4, true>(dir, lanes);
   return variant == SWEEP_COMPAT     ? stream_kernel_of<T, 1>(dir, lanes)
          : variant == SWEEP_COMPAT_D ? stream_kernel_of<T, 2>(dir, lanes)
                                      : stream_kernel_of<T, 0>(dir, lanes);
@@ -938,7 +1059,8 @@ size_t stream_smem_bytes(const LaunchGeom &G, bool fp64) {
   const size_t el = fp64 ? 8 : 4, lines = stream_tile_lines(G.dir, G.lanes);
   return (G.dir == 0 ? (size_t)X_PITCH : lines) * G.rows * el +
          lines * 2 * (size_t)G.ends * (3 * el + sizeof(int)) +
-         (G.variant == SWEEP_CELL ? sizeof(double2) * ((size_t)G.lanes * STREAM_CH + 3) : 0);
+         (exact_filter_variant(G.variant) ? (8 + (G.cs > 1 ? lines * 2 * MAX_CLUSTER : 0)) * el : 0) +
+         (G.variant == SWEEP_CELL || G.variant == SWEEP_CELL_EXACT ? sizeof(double2) * ((size_t)G.lanes * STREAM_CH + 3) : 0);
 }
 
 template <typename T>
@@ -957,9 +1079,10 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   if (!configured[dev].load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lk(config_mu);
     if (!configured[dev].load(std::memory_order_relaxed)) {
-      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D, SWEEP_FILTER_XX, SWEEP_CELL})
-        for (int l : {0, 16, 32}) {
-          const void *fn = (const void *)stream_kernel_for<T>(v, l ? 1 : 0, l);
+      for (int v : {SWEEP_FILTER, SWEEP_COMPAT, SWEEP_COMPAT_D, SWEEP_FILTER_XX, SWEEP_CELL,
+                    SWEEP_FILTER_EXACT, SWEEP_CELL_EXACT})
+        for (int i = 0; i < 4; ++i) {
+          const void *fn = (const void *)stream_kernel_for<T>(v, i / 2, i % 2 ? 32 : 16);
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
           if (err != cudaSuccess) return err;
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -974,13 +1097,14 @@ cudaError_t launch_stream(const LaunchGeom &G, const PlanFields &plan, const Swe
   cfg.gridDim = by_value ? dim3((unsigned)plan.tiles, (unsigned)G.cs,
                                 (unsigned)(groups_total / plan.tiles))
                          : dim3((unsigned)(groups_total * G.cs), 1, 1);
-  cfg.blockDim = dim3((unsigned)((G.dir == 0 ? X_WARPS : Y_WARPS) * 32), 1, 1);
+  cfg.blockDim = dim3((unsigned)(G.dir == 0 ? X_LINES * G.lanes : Y_WARPS * 32), 1, 1);
   cfg.dynamicSmemBytes = stream_smem_bytes(G, sizeof(T) == 8);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   unsigned na = 0;
-  // in place with several segments per line: they form one cluster
-  const int clustered = inplace && G.cs > 1 ? 1 : 0;
+  // in place, or closed exactly, with several segments per line: they form one
+  // cluster
+  const int clustered = (inplace || exact_filter_variant(G.variant)) && G.cs > 1 ? 1 : 0;
   if (clustered) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
     attr[na].val.clusterDim.x = by_value ? 1 : (unsigned)G.cs;

@@ -125,3 +125,24 @@ def test_swirl_matches_oracle_at_small_and_large_steps(oracle, ccfv, nx, ny, cfl
     out = c.cpu().numpy()
     assert rel_l2(out, oracle.run(g, C0, 0.2, dt, 3)) < TOL
     assert abs(out.sum() - C0.sum()) < 1e-12 * np.abs(C0).sum()
+
+
+@pytest.mark.parametrize("nx,ny", [(19, 18), (255, 256), (271, 273), (273, 543), (288, 546),
+                                   (34, 1089), (1089, 33), (40, 4352)])
+@pytest.mark.parametrize("vel,vp", [(1, (0.9, -1.7)), (3, (1.5,))], ids=["const", "swirl"])
+@pytest.mark.parametrize("nu", [20.0, 90.0])
+def test_strong_diffusion(oracle, ccfv, nx, ny, vel, vp, nu):
+    """Strong diffusion: whole lines (no warm-up), long warm-ups with 32 lanes
+    per line (uniform field) and lines closed by clusters of up to 16 segments,
+    a last segment of one position, whole and ragged lanes, missing lines."""
+    N = max(nx, ny)
+    dt, K = 0.4 / N, nu / (0.4 * N)
+    C0 = periodic_field(nx, nx + ny, ny=ny)
+    # K dt / h^2 = nu in the long direction
+    g = oracle.grid(nx, ny, bc=1, vel=vel, vp=vp, K=K, threads=THREADS, scheme=1)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=vel, vel_params=vp, K=K, scheme=1))
+    assert ("filter_exact" if vel == 1 else "cell_exact") in [v for v, _ in s.sweep_plan(dt)]
+    c = dev(C0)
+    s.run(c, 0.0, dt, 2)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
