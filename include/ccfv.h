@@ -342,9 +342,9 @@ int ccfv_autotune(ccfv_ctx *ctx, double dt, int precision, int *segment, void *s
  * is CCFV_SWEEP_GENERAL (per-cell feet), CCFV_SWEEP_UNIFORM (shared-foot
  * stencil with exact chunked scans), CCFV_SWEEP_FILTER (shared-foot stencil
  * with the factored cyclic solve), CCFV_SWEEP_SOURCE (per-cell, with the
- * source term) or CCFV_SWEEP_FILTER_EXACT (the factored solve with the
- * periodic closure taken exactly across a line's segments: strong
- * diffusion), CCFV_SWEEP_CELL / CCFV_SWEEP_CELL_EXACT (the two factored forms
+ * source term) or CCFV_SWEEP_FILTER_EXACT (the factored solve at strong
+ * diffusion: the periodic closure taken exactly across a line's segments, or
+ * warmed up over more cells than CCFV_SWEEP_FILTER allows), CCFV_SWEEP_CELL / CCFV_SWEEP_CELL_EXACT (the two factored forms
  * with a per-cell right-hand side: velocity fields whose feet differ from
  * edge to edge), CCFV_SWEEP_CELL_COMPAT (the factored solve of the
  * reference's non-cyclic system with its boundaries); segment[s] = cells per

@@ -306,9 +306,9 @@ class Solver:
         return [(self.SWEEP_NAMES[v[i]], sg[i]) for i in range(3)]
 
     SWEEP_KERNELS = {"general": "sweep_kernel", "uniform": "sweep_fast_kernel",
-                     "filter": "sweep_filter_kernel", "source": "sweep_kernel",
-                     "filter_exact": "sweep_filter_kernel", "cell": "sweep_filter_kernel",
-                     "cell_exact": "sweep_filter_kernel", "cell_compat": "sweep_filter_kernel"}
+                     "filter": "stream_kernel", "source": "sweep_kernel",
+                     "filter_exact": "stream_kernel", "cell": "stream_kernel",
+                     "cell_exact": "stream_kernel", "cell_compat": "stream_kernel"}
 
     def variant_names(self, dt, precision=FP64):
         """Names of the sweep kernels a step of dt launches (x, y, x)."""

@@ -2,6 +2,7 @@
 // translation units of libccfv (not part of the public ABI).
 #pragma once
 
+#include <cstddef>
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -53,9 +54,6 @@ struct SweepField {
   int cta0;              // filter kernel: first CTA of this field in the launch
                          // (a multiple of the launch's cluster size)
   int halo_f;            // filter kernel: staged halo (cells) of this field
-  int jd;                // cells over which a carry decays below rounding (jf, or more
-                         // where the recurrences need no warm-up)
-  int rk_tail;           // compat: the second term of the rank-one closure matters
   // Batched launches (all zero for single-instance launches):
   int inst;              // instance index into the launch's `nlo` array
   int slice;             // >= 0: fixed slice of this field; -1: the launch's slice
@@ -91,14 +89,18 @@ struct SweepField {
   double sm_inv_den;       // periodic, scan kernels: 1 / (1 + z0 + (a/gamma) z_{L-1});
                            // filter kernel: 1 / c
   const void *tab;         // T[3L]: alpha_k | g_k | z_k (solver factors)
+  // Streaming kernels only (the tile kernels' copy of a descriptor ends here)
+  int jd;                // cells over which a carry decays below rounding (jf, or more
+                         // where the recurrences need no warm-up)
+  int rk_tail;           // compat: the second term of the rank-one closure matters
   double rk_a;             // compat: mu^2 / (1 - mu^(2L+2)), rank-one closure
   // exact form, q = -mu: q^n of a whole segment and of the line's last one,
   // 1/(1 - q^2), 1/(1 - q^L), and q^-(positions that the last segment's last
   // lane walks behind it)
   double ex[5];
-  // Filter kernel: per-line stencil of w's input, computed once per plan
-  // (the velocity fields it serves do not depend on time); null: computed
-  // per tile.  wt: T[groups*LPG][8] taps -3..4; nt: int[groups*LPG] shifts.
+  // per-line stencil of w's input, computed once per plan (the velocity fields
+  // it serves do not depend on time).  wt: T[lines][stencil_taps(variant)];
+  // nt: int[lines] shifts.
   const void *wt;
   const int *nt;
 };
@@ -117,24 +119,24 @@ __host__ __device__ inline bool field_active(const SweepField &f, int jstep, int
   return nslice < f.smax && nslice >= lo + f.gskip;
 }
 
-// Shared-memory slot of one descriptor at the head of every sweep kernel's
+// Shared-memory slot of one descriptor at the head of every tile kernel's
 // dynamic shared memory (the data behind it stays 64-byte aligned).
-constexpr size_t FD_BYTES = (sizeof(SweepField) + 63) & ~size_t(63);
+constexpr size_t FD_COPY = offsetof(SweepField, jd);
+constexpr size_t FD_BYTES = (FD_COPY + 63) & ~size_t(63);
+static_assert(FD_COPY % 8 == 0 && FD_BYTES == 384, "bounds the steps that are taken");
 
 // Kernel variants: the per-cell kernel (any velocity / boundary / scheme) and
 // the fused stencil kernel (uniform displacement, periodic, derivative of the
 // sweep input).
-// SWEEP_GENERAL_SRC is the per-cell kernel with the source tile staged;
-// SWEEP_FILTER_EXACT the filter kernel's cluster form (any diffusion number,
-// out of place).
-// SWEEP_CELL / SWEEP_CELL_EXACT: the filter kernel's two forms with a
-// per-cell right-hand side (feet that differ from edge to edge);
-// SWEEP_CELL_COMPAT: the per-cell form with the reference's boundaries
-// (non-cyclic system).
-// The streaming kernels (stream.cu) run SWEEP_FILTER and, with the reference's
-// boundaries, SWEEP_COMPAT and (the reference scheme's third sweep, derivative
-// of the remapped field) SWEEP_COMPAT_D.  SWEEP_FILTER_XX: the last x sweep of
-// a step and the first of the next one in one pass over the field.
+// SWEEP_GENERAL_SRC is the per-cell kernel with the source tile staged.
+// The streaming kernels (stream.cu) run SWEEP_FILTER (warm-up between a line's
+// segments), SWEEP_FILTER_EXACT (the line closed exactly: any diffusion number),
+// SWEEP_CELL / SWEEP_CELL_EXACT (the same with a per-cell right-hand side: feet
+// that differ from edge to edge) and, with the reference's boundaries,
+// SWEEP_COMPAT and (the reference scheme's third sweep, derivative of the
+// remapped field) SWEEP_COMPAT_D.  SWEEP_FILTER_XX: the last x sweep of a step
+// and the first of the next one in one pass over the field.
+// SWEEP_CELL_COMPAT: the tile kernel with the reference's boundaries.
 enum { SWEEP_GENERAL = 0, SWEEP_FAST = 1, SWEEP_FILTER = 2, SWEEP_GENERAL_SRC = 3,
        SWEEP_FILTER_EXACT = 4, SWEEP_CELL = 5, SWEEP_CELL_EXACT = 6, SWEEP_CELL_COMPAT = 7,
        SWEEP_COMPAT = 8, SWEEP_COMPAT_D = 9, SWEEP_FILTER_XX = 10 };
@@ -143,7 +145,7 @@ inline bool stream_variant(int v) {
          v == SWEEP_FILTER_XX || v == SWEEP_CELL || v == SWEEP_FILTER_EXACT ||
          v == SWEEP_CELL_EXACT;
 }
-// Variants run by the filter kernels (factored solve).
+// Variants with the factored solve.
 inline bool filter_variant(int v) {
   return stream_variant(v) || v == SWEEP_CELL_COMPAT;
 }
@@ -170,7 +172,7 @@ inline int stencil_taps(int v) {
 inline bool cell_filter_variant(int v) {
   return v == SWEEP_CELL || v == SWEEP_CELL_EXACT || v == SWEEP_CELL_COMPAT;
 }
-// The filter kernel's cluster form (exact periodic closure, out of place).
+// Lines closed exactly (several segments: one cluster).
 inline bool exact_filter_variant(int v) { return v == SWEEP_FILTER_EXACT || v == SWEEP_CELL_EXACT; }
 constexpr int FILTER_JMAX = 64;  // longest recurrence warm-up with 16 lanes per line
 

@@ -408,7 +408,7 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
       S.halo_fit = sh + 6;
     }
     bool longer = !warm && uniform && L > (dir == 0 ? 16 : 32) * STREAM_CH && J <= FILTER_JLONG &&
-                  L > 2 * J;
+                  L > 2 * J && (closed || (inplace && L <= LC_MAX * MAX_CLUSTER));
     if (longer) {
       LaunchGeom W = S;
       stream_geom(W, L, J, sh + 6, L);
@@ -553,8 +553,8 @@ int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, 
     g_lc_override = lc;
     StepPlan plan;
     int rc = build_step_plan(ctx, &plan, dt, fp64, pf);
-    if (rc == CCFV_OK && !warm_filter_variant(plan.geom[0].variant) &&
-        !warm_filter_variant(plan.geom[1].variant)) {
+    auto tunable = [](const LaunchGeom &G) { return warm_filter_variant(G.variant) && !G.strong; };
+    if (rc == CCFV_OK && !tunable(plan.geom[0]) && !tunable(plan.geom[1])) {
       g_lc_override = 0;
       break;  // nothing to tune: this grid does not use the filter kernel
     }

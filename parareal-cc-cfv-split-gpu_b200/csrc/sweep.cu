@@ -675,8 +675,6 @@ __global__ void __launch_bounds__(NTH, 2) sweep_kernel(const SweepField *__restr
 // backward fix-up, the Sherman-Morrison correction and the store into a final
 // walk.
 
-static_assert(sizeof(SweepField) % 8 == 0, "descriptor slot");
-
 template <typename T>
 struct FastSmem {
   T *C;      // [(lc_max + 2H) * PITCH]
@@ -730,7 +728,7 @@ __global__ void __launch_bounds__(NTH, 2)
   {
     // every thread finds the field; the descriptor is copied cooperatively
     const int lo = find_field(fields, g0idx, nfields, tile);
-    constexpr int NW8 = (int)(sizeof(SweepField) / 8);
+    constexpr int NW8 = (int)(FD_COPY / 8);
     if (threadIdx.x < NW8)
       reinterpret_cast<long long *>(S.fd)[threadIdx.x] =
           __ldg(reinterpret_cast<const long long *>(&fields[lo]) + threadIdx.x);
@@ -998,16 +996,18 @@ __global__ void __launch_bounds__(NTH, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Filter path: uniform displacement + periodic cells + derivative of the
-// sweep input, for diffusion numbers where |mu| (below) is small enough.
+// Filter path, tile form: the reference's boundaries where the streaming
+// kernels (stream.cu) do not apply, i.e. feet that differ from edge to edge
+// (swirling deformation) and lines whose ends need more scratch than fits.
 //
-// The cyclic constant system a x_{k-1} + b x_k + a x_{k+1} = r_k factors as
+// The constant system a x_{k-1} + b x_k + a x_{k+1} = r_k factors as
 // c (1 + mu S^-1)(1 + mu S) x = r with |mu| < 1, mu / (1 + mu^2) = a / b,
-// c = a / mu, so it is solved exactly by two first-order recurrences,
-//   w_k = r_k / c - mu w_{k-1},   x_k = w_k - mu x_{k+1},
-// whose periodic wrap-around needs no correction term.  A recurrence started
-// from zero J positions early agrees with the exact one to |mu|^J, and J is
-// chosen on the host so that |mu|^J is below the rounding of T.
+// c = a / mu (plus a rank-one term at the line's start), so it is solved by two
+// first-order recurrences,
+//   w_k = r_k / c - mu w_{k-1},   x_k = w_k - mu x_{k+1}.
+// A recurrence started from zero J positions early agrees with the exact one
+// to |mu|^J, and J is chosen on the host so that |mu|^J is below the rounding
+// of T.
 //
 // A CTA owns a segment [p0, p1) of 16 lines.  The 16 lanes of a half-warp
 // own one line: lane c holds FCH consecutive positions in registers.  The
@@ -1030,130 +1030,26 @@ __host__ __device__ inline int filter_tile_rows(int lc_max, int H) {
   return (lc_max > FLANES * FCH ? lc_max : FLANES * FCH) + 2 * H + 8;
 }
 
-// Exact (cluster) form: powers (-mu)^e for e = 0 .. FPW - 1 (a segment of at
-// most FLANES * FCH cells needs exponents up to FLANES * FCH).
+// The tile of a step is bounded with the room of a power table and of its edges.
 constexpr int FPW = FLANES * FCH + 8;
 template <typename T>
 struct FiltSmem {
   T *C;      // [filter_tile_rows * PITCH]  input cells, then w, then x
-  T *B;      // per-cell form: [filter_tile_rows * PITCH]  b of every position
-  T *om;     // [8 * LPG]  weights of w's input (1/c) M b as an 8-tap stencil of C
+  T *B;      // [filter_tile_rows * PITCH]  b of every position
   T *pwt;    // [32]       (-mu)^(i+1), i = 0 .. FCH-1
-  T *pwa;    // exact form: [FPW] (-mu)^e
-  T *ex;     // exact form: [2 * LPG] this segment's forward end / backward start per line
-  double *et;  // per-cell form: [FPW] sin^2(pi s) of the tile's edges (swirling field)
-  int *n0;   // [LPG]
   SweepField *fd;
   int rows;
 };
 
-template <typename T, bool EXACT, bool CELL>
+template <typename T>
 __device__ __forceinline__ FiltSmem<T> carve_filt(unsigned char *raw, int lc_max, int H) {
   FiltSmem<T> s;
   s.fd = reinterpret_cast<SweepField *>(raw);
-  s.n0 = reinterpret_cast<int *>(raw + FD_BYTES);
-  T *p = reinterpret_cast<T *>(raw + FD_BYTES + 64 * sizeof(int));
-  s.om = p; p += 8 * LPG;
-  s.pwt = p; p += 32;
-  s.pwa = nullptr;
-  s.ex = nullptr;
-  if (EXACT) {
-    s.pwa = p; p += FPW;
-    s.ex = p; p += 2 * LPG;
-  }
-  s.C = p;
+  s.pwt = reinterpret_cast<T *>(raw + FD_BYTES);
+  s.C = s.pwt + 32;
   s.rows = filter_tile_rows(lc_max, H);
-  s.B = CELL ? p + (size_t)s.rows * PITCH : nullptr;
-  s.et = nullptr;
-  if (CELL) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(s.B + (size_t)s.rows * PITCH);
-    s.et = reinterpret_cast<double *>((a + 7) & ~uintptr_t(7));
-  }
+  s.B = s.C + (size_t)s.rows * PITCH;
   return s;
-}
-
-// Per-cell right-hand side of the filter kernel (velocity fields whose feet
-// differ from edge to edge, periodic cells, derivative of the sweep input).
-// One edge e of a line: its foot's cell kf and offset xi, the PPM
-// antiderivative of cell kf at xi (I(xi), d_intC_ppm4th, T2S4:63-65) and the
-// fourth-order derivative at the foot (dcdx_bar_on_gpu, T2S4:440-547).  The
-// remap of cell k is then I_{k+1} - I_k plus the whole cells between the two
-// feet (x_step_intC_ppm_on_gpu, T2S4:306-347), so every foot, PPM
-// reconstruction and derivative is evaluated once per edge instead of twice
-// per cell.
-template <typename T>
-struct CellEdge {
-  int kf;
-  T phi, d;
-};
-
-template <typename T>
-__device__ __forceinline__ CellEdge<T> cell_edge_at(const SweepField &F, double f,
-                                                    const T *ccol, int rb, int nrows,
-                                                    unsigned *status) {
-  const double u = (f - F.s_min) / F.h;
-  const double fk = floor(u);
-  CellEdge<T> r;
-  r.kf = (int)fk;
-  const T xi = T(u - fk);
-  const int row = r.kf + rb;
-  if (row < 2 || row + 2 >= nrows) {  // cannot happen within the staged halo
-    atomicOr(status, STATUS_HALO);
-    r.phi = T(0);
-    r.d = T(0);
-    return r;
-  }
-  const T *cp = ccol + (row - 2) * PITCH;
-  const T cm2 = cp[0], cm1 = cp[PITCH], c0 = cp[2 * PITCH], cp1 = cp[3 * PITCH],
-          cp2 = cp[4 * PITCH];
-  // PPM edge values and curvature of cell kf (x_step_ppm_coef_on_gpu, T2S4:260-304)
-  const T cl = T(7.0 / 12.0) * (c0 + cm1) - T(1.0 / 12.0) * (cp1 + cm2);
-  const T cr = T(7.0 / 12.0) * (cp1 + c0) - T(1.0 / 12.0) * (cp2 + cm1);
-  const T D = cr - cl;
-  const T C6 = T(6.0) * (c0 - T(0.5) * (cl + cr));
-  const T xi2 = xi * xi, xi3 = xi2 * xi;
-  r.phi = T(-1.0 / 3) * C6 * xi3 + T(0.5) * (D + C6) * xi2 + cl * xi;
-  r.d = T(F.inv12h) * ((T(2.0) * xi3 - T(6.0) * xi2 + T(3.0) * xi + T(1.0)) * cm2 +
-                       (T(-8.0) * xi3 + T(18.0) * xi2 + T(6.0) * xi - T(15.0)) * cm1 +
-                       (T(12.0) * xi3 - T(18.0) * xi2 - T(24.0) * xi + T(15.0)) * c0 +
-                       (T(-8.0) * xi3 + T(6.0) * xi2 + T(18.0) * xi - T(1.0)) * cp1 +
-                       (T(2.0) * xi3 - T(3.0) * xi) * cp2);
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ CellEdge<T> cell_edge(const SweepField &F, const LineFeet &lf,
-                                                 const T *ccol, int rb, int nrows, int e,
-                                                 unsigned *status) {
-  return cell_edge_at<T>(F, lf.foot(F, e), ccol, rb, nrows, status);
-}
-
-// b of the cell between edges l and l+1: remap + (1-theta) K Dt/h (D_r - D_l)
-// (x_b_RHS_on_gpu, T2S4:564-613, source-free); the whole cells between the
-// feet are summed with Neumaier compensation (periodic remap of sweep_kernel).
-template <typename T>
-__device__ __forceinline__ T cell_rhs(const CellEdge<T> &l, const CellEdge<T> &r, const T *ccol,
-                                      int rb, int nrows, T kbc, unsigned *status) {
-  T remap;
-  if (r.kf == l.kf) {
-    remap = r.phi - l.phi;
-  } else {
-    const int lo = min(l.kf, r.kf), hi = max(l.kf, r.kf) - 1;
-    T s = T(0), comp = T(0);
-    if (lo + rb < 0 || hi + rb >= nrows) {
-      atomicOr(status, STATUS_HALO);
-    } else {
-      for (int k = lo; k <= hi; ++k) {
-        const T x = ccol[(k + rb) * PITCH];
-        const T t = s + x;
-        comp += (fabs(s) >= fabs(x)) ? ((s - t) + x) : ((x - t) + s);
-        s = t;
-      }
-    }
-    s += comp;
-    remap = r.kf > l.kf ? (s + r.phi) - l.phi : -((s + l.phi) - r.phi);
-  }
-  return remap + kbc * (r.d - l.d);
 }
 
 // Compat boundaries (the reference's): an edge whose foot lies inside
@@ -1284,32 +1180,13 @@ __global__ void filter_weights_kernel(const SweepField *__restrict__ f, T *__res
   }
 }
 
-// Four CTAs per SM (at most 64 registers a thread; shared memory allows no
-// more): the kernel is latency bound, and each added CTA was worth more than
-// the few registers it spills (2 -> 3 -> 4 CTAs: fine phase 1498 -> 1207 ->
-// 1105 us per launch on the 2048^2 x 63-slice bench).
-//
-// EXACT (out of place, any diffusion number): a line's cs segments form one
-// thread-block cluster and no recurrence is warmed up.  Each segment runs
-// both filters from a zero start over its own cells only; a segment maps its
-// incoming carry linearly, w_end = (-mu)^np w_in + E (forward) and
-// x_start = (-mu)^np x_in + X (backward), so after the segments publish E (X)
-// in shared memory the periodic closure over the cluster gives every carry
-// exactly: w_{L-1} = E_total / (1 - (-mu)^L), then carries segment by
-// segment; each cell adds carry * (-mu)^distance from a power table.  The
-// field, its activity and the segment length are uniform over a cluster, so
-// every CTA of a cluster reaches every cluster barrier.
-//
-// CELL (velocity fields whose feet differ from edge to edge): the staged
-// cells first give every position's b (per-edge feet, PPM antiderivatives and
-// foot derivatives, cell_edge / cell_rhs) in a second tile, each line's
-// half-warp filling its own column; the forward filter then takes w's input
-// as the mass-matrix stencil (1/12c)(b_{k-1} + 10 b_k + b_{k+1}).  Two tiles
-// and the per-edge arithmetic: two CTAs per SM.
-// COMPAT (per-cell form only): the reference's boundaries, a separate
-// instantiation so that the periodic per-cell form carries none of their code.
-template <typename T, bool EXACT, bool CELL, bool COMPAT>
-__global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
+// The staged cells first give every position's b (the reference's per-cell
+// remap with its clamps, foot derivatives with its ghost selection) in a second
+// tile, each line's half-warp filling its own column; the forward filter then
+// takes w's input as the mass-matrix stencil (1/12c)(b_{k-1} + 10 b_k +
+// b_{k+1}).  Bound by the per-edge arithmetic; two tiles: two CTAs per SM.
+template <typename T>
+__global__ void __launch_bounds__(NTH, 2)
     sweep_filter_kernel(const SweepField *__restrict__ fields, int nfields, int group_base,
                         double toff, const FieldIo io, int lc_max, int H, unsigned *status,
                         int jstep, int nslice, const int *nlo, int cs, int clustered,
@@ -1326,11 +1203,11 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
   // of different segment lengths share one launch (lc_max and H size the
   // shared memory only)
   const int cta = (int)blockIdx.x + group_base;
-  FiltSmem<T> S = carve_filt<T, EXACT, CELL>(smem_raw, lc_max, H);
+  FiltSmem<T> S = carve_filt<T>(smem_raw, lc_max, H);
   {
     // a field's CTAs start at cta0 = group0 * cs (cs is uniform over a launch);
     // only the threads that copy the descriptor search for it
-    constexpr int NW8 = (int)(sizeof(SweepField) / 8);
+    constexpr int NW8 = (int)(FD_COPY / 8);
     if (threadIdx.x < NW8) {
       const int lo = find_field(fields, g0idx, nfields, cta / cs);
       reinterpret_cast<long long *>(S.fd)[threadIdx.x] =
@@ -1346,17 +1223,13 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
   const int q = cta - F.cta0;
   const int rank = q % cs;
   const long long line0 = (long long)(q / cs) * LPG;
-  // exact form: segments of a whole walk (FLANES * FCH cells) and a shorter
-  // last one when cs is the least count that covers the line (full segments
-  // need no masking, and their forward end is the scan's carry-out)
-  int Lc = (L + cs - 1) / cs;
-  if (EXACT && (cs - 1) * (FLANES * FCH) < L && cs * (FLANES * FCH) >= L) Lc = FLANES * FCH;
+  const int Lc = (L + cs - 1) / cs;
   const int p0 = min(L, rank * Lc);
   const int p1 = min(L, p0 + Lc);
   const int np = p1 - p0;
   const int nrows = np + 2 * H;
-  const int J = EXACT ? 0 : F.jf;
-  const T mu = T(F.sm_fac), ic = T(F.sm_inv_den);
+  const int J = F.jf;
+  const T mu = T(F.sm_fac);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T *gsrc;
   T *gdst;
@@ -1373,26 +1246,9 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
   // stores would otherwise make the compiler reload it every iteration.
   const long long s_pos = F.s_pos, s_line = F.s_line, M = F.M;
   const bool xsweep = s_line == 1;
-  // compat boundaries (per-cell form only): zero outside the line, ghost
-  // cells, non-cyclic solve
-  constexpr bool compat = CELL && COMPAT;
-
-  // ---- stage rows p0-H .. p1+H-1 (periodic wrap) ----
-  // Rows whose position lies inside the line ([rlo, rhi)) take pointer-stepped
-  // copies; only the halo rows outside it wrap (periodic) or are zero (compat).
+  // ---- stage rows p0-H .. p1+H-1 (zero outside the line) ----
   {
     const int rlo = max(0, H - p0), rhi = min(nrows, H - p0 + L);
-    auto halo_row = [&](T *dcol, const T *lbase, long long step, int row) {
-      int pos = p0 - H + row;
-      if (compat) {
-        dcol[row * PITCH] = T(0);
-        return;
-      }
-      pos %= L;
-      if (pos < 0) pos += L;
-      const T *src = lbase + (long long)pos * step;
-      if (sizeof(T) == 8) cp_async8(dcol + row * PITCH, src); else cp_async4(dcol + row * PITCH, src);
-    };
     if (xsweep) {
       // a warp copies two rows of 16 consecutive values (128 B for FP64) per step
       const int ln = lane & (LPG - 1);
@@ -1401,7 +1257,7 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
       int row = warp * 2 + (lane >> 4);
       if (gl < M) {
         const T *gcol = gsrc + gl;
-        for (; row < rlo; row += 2 * NW) halo_row(dcol, gcol, s_pos, row);
+        for (; row < rlo; row += 2 * NW) dcol[row * PITCH] = T(0);
         const T *src = gcol + (long long)(p0 - H + row) * s_pos;
         T *dst = dcol + row * PITCH;
         const long long gstep = 2LL * NW * s_pos;
@@ -1409,7 +1265,7 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
         for (; row < rhi; row += 2 * NW, src += gstep, dst += 2 * NW * PITCH) {
           if (sizeof(T) == 8) cp_async8(dst, src); else cp_async4(dst, src);
         }
-        for (; row < nrows; row += 2 * NW) halo_row(dcol, gcol, s_pos, row);
+        for (; row < nrows; row += 2 * NW) dcol[row * PITCH] = T(0);
       } else {
         for (; row < nrows; row += 2 * NW) dcol[row * PITCH] = T(0);
       }
@@ -1421,36 +1277,22 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
         int row = lane;
         if (gl < M) {
           const T *lbase = gsrc + gl * s_line;
-          for (; row < rlo; row += 32) halo_row(dcol, lbase, 1, row);
+          for (; row < rlo; row += 32) dcol[row * PITCH] = T(0);
           const T *src = lbase + (p0 - H + row);
           T *dst = dcol + row * PITCH;
 #pragma unroll 4
           for (; row < rhi; row += 32, src += 32, dst += 32 * PITCH) {
             if (sizeof(T) == 8) cp_async8(dst, src); else cp_async4(dst, src);
           }
-          for (; row < nrows; row += 32) halo_row(dcol, lbase, 1, row);
+          for (; row < nrows; row += 32) dcol[row * PITCH] = T(0);
         } else {
           for (; row < nrows; row += 32) dcol[row * PITCH] = T(0);
         }
       }
     }
   }
-  if (CELL) {
-    // per-cell form: no per-line stencil (b is computed per cell below)
-  } else if (F.wt) {  // per-line stencil from the plan's table, copied with the cells
-    if (threadIdx.x < 8 * LPG) {
-      const T *src = reinterpret_cast<const T *>(F.wt) + line0 * 8 + threadIdx.x;
-      if (sizeof(T) == 8) cp_async8(S.om + threadIdx.x, src); else cp_async4(S.om + threadIdx.x, src);
-    } else if (threadIdx.x < 9 * LPG) {
-      const int l = threadIdx.x - 8 * LPG;
-      cp_async4(S.n0 + l, F.nt + line0 + l);
-    }
-  }
   cp_async_commit();
-  if (!CELL && !F.wt && threadIdx.x < LPG) {
-    filter_line_stencil<T>(F, line0 + threadIdx.x, toff, S.om + 8 * threadIdx.x,
-                           S.n0 + threadIdx.x);
-  } else if (threadIdx.x == 9 * LPG) {
+  if (threadIdx.x == 9 * LPG) {
     const T mmu = T(-F.sm_fac);
     T pk = mmu;
     for (int i = 0; i < FCH; ++i) {
@@ -1458,23 +1300,11 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
       pk *= mmu;
     }
   }
-  if (EXACT && warp == 0) {
-    // powers (-mu)^e, e < FPW, by doubling: [s, 2s) = [0, s) * (-mu)^s
-    T xs = T(-F.sm_fac);
-    if (lane == 0) S.pwa[0] = T(1);
-    __syncwarp();
-    for (int s = 1; s < FPW; s <<= 1) {
-      for (int t = lane; t < s && s + t < FPW; t += 32) S.pwa[s + t] = S.pwa[t] * xs;
-      __syncwarp();
-      xs *= xs;
-    }
-  }
   cp_async_wait_all_committed();
   __syncthreads();
-  if (compat) {  // extrapolated ghost cells C_{-2}, C_{-1}, C_L, C_{L+1} (T2S4:275-286)
-    if (threadIdx.x < LPG) compat_ghosts(S.C + threadIdx.x, H - p0, p0 - H, p1 + H, L);
-    __syncthreads();
-  }
+  // extrapolated ghost cells C_{-2}, C_{-1}, C_L, C_{L+1} (T2S4:275-286)
+  if (threadIdx.x < LPG) compat_ghosts(S.C + threadIdx.x, H - p0, p0 - H, p1 + H, L);
+  __syncthreads();
   // In place, the segments of a line are read (halo) by the neighbouring CTAs
   // of its cluster: this CTA's reads are complete here, and no CTA of the
   // cluster stores before every CTA has arrived.  Out of place (ping-pong),
@@ -1482,10 +1312,8 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
   if (clustered) asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
 
   // ---- one line per half-warp, FCH positions per lane ----
-  // (exact form: Lc bounds every segment of the cluster, so all its CTAs
-  // leave here together, before any cluster barrier)
-  if (EXACT ? Lc > FLANES * FCH : np + 2 * J > FLANES * FCH) {
-    // the host keeps segments within filter_seg_max(J) (exact: FLANES * FCH)
+  if (np + 2 * J > FLANES * FCH) {
+    // the host keeps segments within filter_seg_max(J)
     if (threadIdx.x == 0) atomicOr(status, STATUS_HALO);
     return;
   }
@@ -1497,7 +1325,7 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
     const T mmu = -mu;
     const T pw = S.pwt[FCH - 1];      // (-mu)^FCH
 
-    if (CELL) {
+    {
       // b of positions [p0 - J - 1, p0 - J + FLANES * FCH + 1) into this
       // line's column of the second tile: every row the forward walk reads
       // (zero past p1 + J + 1, where the walk's values are masked); lane c
@@ -1509,215 +1337,131 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
       const int mm = (kw - kb + FLANES - 1) / FLANES;
       const int s0 = kb + c * mm, s1 = min(kw, s0 + mm);
       const double tau0 = F.t_min + F.ht * (double)gl;
-      const T *ccol = S.C + ln;
       const T kbc = T(F.kb);
-      bool swirl_done = false;
-      if constexpr (sizeof(T) == 8 && !compat) {
-        if (F.vel == VEL_SWIRL) {
-          // Swirling field: the corner feet of the tile's LPG + 1 corner
-          // lines at the edges [kb, kw] once each (a corner is shared by the
-          // lines on either side), sin^2(pi s) of an edge shared by all of
-          // them (the LineFeet factorisation: g(tau) h(t) per corner line and
-          // time), into the second tile as [edge row][corner line]; then
-          // each line's edge feet (the mean of its two corners) in place,
-          // and the right-hand side below reads them back per edge.
-          double *cf = S.B;
-          const int ne = kw - kb + 1;
-          if (threadIdx.x <= LPG) {
-            const double sg = F.dir == 0 ? 1.0 : -1.0;
-            const double g =
-                sg * sinpi(2.0 * (F.t_min + F.ht * (double)(line0 + (long long)threadIdx.x)));
-            S.om[threadIdx.x] = g * cospi((toff + F.ta_rel) / F.vp[0]);
-            S.om[LPG + 1 + threadIdx.x] = g * cospi((toff + F.tb_rel) / F.vp[0]);
-          }
-          for (int i = threadIdx.x; i < ne; i += NTH) {
-            const double ss = sinpi(F.s_min + F.h * (kb + i));
-            S.et[i] = ss * ss;
-          }
-          __syncthreads();
-          for (int i = threadIdx.x; i < ne * (LPG + 1); i += NTH) {
-            const int ei = i / (LPG + 1), j = i - ei * (LPG + 1);
-            const double sp = F.s_min + F.h * (kb + ei);
-            const double w = S.om[LPG + 1 + j] * S.et[ei];  // speed at tb
-            const double q = sinpi(sp - F.Dt * w);
-            cf[(kb + ei + rb) * PITCH + j] = sp - 0.5 * F.Dt * (w + S.om[j] * q * q);
-          }
-          __syncthreads();
-          for (int i = threadIdx.x; i < ne; i += NTH) {
-            double *row = cf + (kb + i + rb) * PITCH;
-            double c0 = row[0];
-#pragma unroll
-            for (int j = 0; j < LPG; ++j) {
-              const double c1 = row[j + 1];
-              row[j] = 0.5 * (c0 + c1);
-              c0 = c1;
-            }
-          }
-          __syncthreads();
-          // lane c's last edge is the next lane's first: read before any write
-          const double fend = s0 < s1 ? cf[(s1 + rb) * PITCH + ln] : 0.0;
-          __syncwarp(fm);
-          T *bcol = S.B + ln;
-          if (s0 < s1) {
-            CellEdge<T> el{0, T(0), T(0)};
-            if (s0 < kv) el = cell_edge_at<T>(F, cf[(s0 + rb) * PITCH + ln], ccol, rb, nrows, status);
-            for (int k = s0; k < s1; ++k) {
-              T b = T(0);
-              if (k < kv) {
-                const double f1 = k + 1 < s1 ? cf[(k + 1 + rb) * PITCH + ln] : fend;
-                const CellEdge<T> er = cell_edge_at<T>(F, f1, ccol, rb, nrows, status);
-                b = cell_rhs<T>(el, er, ccol, rb, nrows, kbc, status);
-                el = er;
-              }
-              bcol[(k + rb) * PITCH] = b;
-            }
-          }
-          swirl_done = true;
-        }
-      }
-      if (!swirl_done) {
       const LineFeet lf(F, tau0, tau0 + F.ht, toff + F.ta_rel, toff + F.tb_rel);
-      if (!compat) {
+      // b = 0 outside the line (the compact mass matrix's zero ghosts).
+      // Uniform displacement (the reference's rotation, constant, rotation):
+      // cells clear of the clamps and ghost selections take the
+      // shared-foot stencils, the rest the per-cell formulas of the
+      // reference (remap_cell, foot_derivative); other velocity fields the
+      // per-edge path (compat_edge)
+      const int ka = max(s0, 0), kz = min(min(s1, kv), L);
+      const LineView<T> vc{S.C + ln, rb, nrows, status};
+      const bool uni = F.uniform != 0;
+      T wr[6], wq[6];
+      int n0 = 0, klo = 1, khi = 0;
+      if (uni) {
+        uniform_weights<T>(F, lf.foot(F, 0), wr, wq, &n0);
+        klo = 2 - n0;
+        khi = L - 4 - n0;
+      }
+      if (!F.dsrc) {
         T *bcol = S.B + ln;
-        if (s0 < s1) {
-          CellEdge<T> el{0, T(0), T(0)};
-          if (s0 < kv) el = cell_edge<T>(F, lf, ccol, rb, nrows, s0, status);
-          for (int k = s0; k < s1; ++k) {
-            T b = T(0);
-            if (k < kv) {
-              const CellEdge<T> er = cell_edge<T>(F, lf, ccol, rb, nrows, k + 1, status);
-              b = cell_rhs<T>(el, er, ccol, rb, nrows, kbc, status);
-              el = er;
-            }
-            bcol[(k + rb) * PITCH] = b;
-          }
-        }
-      } else {
-        // b = 0 outside the line (the compact mass matrix's zero ghosts).
-        // Uniform displacement (the reference's rotation, constant, rotation):
-        // cells clear of the clamps and ghost selections take the
-        // shared-foot stencils, the rest the per-cell formulas of the
-        // reference (remap_cell, foot_derivative); other velocity fields the
-        // per-edge path (compat_edge)
-        const int ka = max(s0, 0), kz = min(min(s1, kv), L);
-        const LineView<T> vc{S.C + ln, rb, nrows, status};
-        const bool uni = F.uniform != 0;
-        T wr[6], wq[6];
-        int n0 = 0, klo = 1, khi = 0;
         if (uni) {
-          uniform_weights<T>(F, lf.foot(F, 0), wr, wq, &n0);
-          klo = 2 - n0;
-          khi = L - 4 - n0;
-        }
-        if (!F.dsrc) {
-          T *bcol = S.B + ln;
-          if (uni) {
-            // the lane's run in three ranges: the cells clear of the clamps
-            // and ghost selections [i0, i1) take the stencil with no
-            // per-cell branches, the others the reference's formulas (or 0
-            // outside the line)
-            auto edge_cell = [&](int k) {
-              T b = T(0);
-              if (k >= ka && k < kz) {
-                const double fa = lf.foot(F, k), fb = lf.foot(F, k + 1);
-                b = remap_cell(F, vc, fa, fb) +
-                    kbc * (foot_derivative(F, vc, fb) - foot_derivative(F, vc, fa));
-              }
-              bcol[(k + rb) * PITCH] = b;
-            };
-            const int i0 = max(s0, max(ka, klo)), i1 = max(i0, min(s1, min(kz, khi + 1)));
-            const int ia = min(i0, s1);
-            for (int k = i0; k < i1; ++k) {
-              const T *cp = S.C + (k + n0 - 2 + rb) * PITCH + ln;
-              T b = T(0);
-#pragma unroll
-              for (int t = 0; t < 6; ++t) b += (wr[t] + wq[t]) * cp[t * PITCH];
-              bcol[(k + rb) * PITCH] = b;
-            }
-            for (int k = s0; k < s1; ++k) {  // the rest, skipping [i0, i1)
-              if (k == ia) k = max(ia, i1);
-              if (k >= s1) break;
-              edge_cell(k);
-            }
-          } else {
-            if (ka < kz) {
-              CompatEdge<T> el = compat_edge<T>(F, lf, vc, vc, ka);
-              for (int k = ka; k < kz; ++k) {
-                const CompatEdge<T> er = compat_edge<T>(F, lf, vc, vc, k + 1);
-                bcol[(k + rb) * PITCH] = compat_remap<T>(F, el, er, vc) + kbc * (er.d - el.d);
-                el = er;
-              }
-            }
-            for (int k = s0; k < s1; ++k)
-              if (k < ka || k >= kz) bcol[(k + rb) * PITCH] = T(0);
-          }
-        } else {
-          // the reference's third sweep differentiates the remapped field
-          // (dcdx_bar_on_gpu(v_d_Cnphf_bar_x, ...), T2S4:929-932): remap the
-          // cells [ra0, ra1) into the second tile, its ghosts, then
-          // b = R + kbc (D_R(f_{k+1}) - D_R(f_k)) into the first tile (this
-          // line's cells are no longer read)
-          const int ra0 = max(0, kb - F.hd), ra1 = min(L, kv + F.hd);
-          const int m1 = (ra1 - ra0 + FLANES - 1) / FLANES;
-          const int q0 = ra0 + c * m1, q1 = min(ra1, q0 + m1);
-          T *rcol = S.B + ln;
-          if (uni) {
-            auto edge_remap = [&](int k) {
-              rcol[(k + rb) * PITCH] = remap_cell(F, vc, lf.foot(F, k), lf.foot(F, k + 1));
-            };
-            const int j0 = max(q0, klo), j1 = max(j0, min(q1, khi + 1));
-            const int ja = min(j0, q1);
-            for (int k = j0; k < j1; ++k) {
-              const T *cp = S.C + (k + n0 - 2 + rb) * PITCH + ln;
-              T r = T(0);
-#pragma unroll
-              for (int t = 0; t < 6; ++t) r += wr[t] * cp[t * PITCH];
-              rcol[(k + rb) * PITCH] = r;
-            }
-            for (int k = q0; k < q1; ++k) {  // the rest, skipping [j0, j1)
-              if (k == ja) k = max(ja, j1);
-              if (k >= q1) break;
-              edge_remap(k);
-            }
-          } else if (q0 < q1) {
-            CompatEdge<T> el = compat_edge<T>(F, lf, vc, vc, q0);
-            for (int k = q0; k < q1; ++k) {
-              const CompatEdge<T> er = compat_edge<T>(F, lf, vc, vc, k + 1);
-              rcol[(k + rb) * PITCH] = compat_remap<T>(F, el, er, vc);
-              el = er;
-            }
-          }
-          __syncwarp(fm);
-          if (c == 0) compat_ghosts(rcol, rb, ra0 - 2, ra1 + 2, L);
-          __syncwarp(fm);
-          const LineView<T> vr{rcol, rb, nrows, status};
-          T *bcol = S.C + ln;
+          // the lane's run in three ranges: the cells clear of the clamps
+          // and ghost selections [i0, i1) take the stencil with no
+          // per-cell branches, the others the reference's formulas (or 0
+          // outside the line)
           auto edge_cell = [&](int k) {
             T b = T(0);
             if (k >= ka && k < kz) {
               const double fa = lf.foot(F, k), fb = lf.foot(F, k + 1);
-              b = vr(k) + kbc * (foot_derivative(F, vr, fb) - foot_derivative(F, vr, fa));
+              b = remap_cell(F, vc, fa, fb) +
+                  kbc * (foot_derivative(F, vc, fb) - foot_derivative(F, vc, fa));
             }
             bcol[(k + rb) * PITCH] = b;
           };
-          // interior cells of a uniform displacement [i0, i1): the stencil
-          // (empty range for other fields: klo > khi)
           const int i0 = max(s0, max(ka, klo)), i1 = max(i0, min(s1, min(kz, khi + 1)));
           const int ia = min(i0, s1);
           for (int k = i0; k < i1; ++k) {
-            const T *rp = rcol + (k + n0 - 2 + rb) * PITCH;
-            T acc = T(0);
+            const T *cp = S.C + (k + n0 - 2 + rb) * PITCH + ln;
+            T b = T(0);
 #pragma unroll
-            for (int t = 0; t < 6; ++t) acc += wq[t] * rp[t * PITCH];
-            bcol[(k + rb) * PITCH] = rcol[(k + rb) * PITCH] + acc;
+            for (int t = 0; t < 6; ++t) b += (wr[t] + wq[t]) * cp[t * PITCH];
+            bcol[(k + rb) * PITCH] = b;
           }
           for (int k = s0; k < s1; ++k) {  // the rest, skipping [i0, i1)
             if (k == ia) k = max(ia, i1);
             if (k >= s1) break;
             edge_cell(k);
           }
+        } else {
+          if (ka < kz) {
+            CompatEdge<T> el = compat_edge<T>(F, lf, vc, vc, ka);
+            for (int k = ka; k < kz; ++k) {
+              const CompatEdge<T> er = compat_edge<T>(F, lf, vc, vc, k + 1);
+              bcol[(k + rb) * PITCH] = compat_remap<T>(F, el, er, vc) + kbc * (er.d - el.d);
+              el = er;
+            }
+          }
+          for (int k = s0; k < s1; ++k)
+            if (k < ka || k >= kz) bcol[(k + rb) * PITCH] = T(0);
         }
-      }
+      } else {
+        // the reference's third sweep differentiates the remapped field
+        // (dcdx_bar_on_gpu(v_d_Cnphf_bar_x, ...), T2S4:929-932): remap the
+        // cells [ra0, ra1) into the second tile, its ghosts, then
+        // b = R + kbc (D_R(f_{k+1}) - D_R(f_k)) into the first tile (this
+        // line's cells are no longer read)
+        const int ra0 = max(0, kb - F.hd), ra1 = min(L, kv + F.hd);
+        const int m1 = (ra1 - ra0 + FLANES - 1) / FLANES;
+        const int q0 = ra0 + c * m1, q1 = min(ra1, q0 + m1);
+        T *rcol = S.B + ln;
+        if (uni) {
+          auto edge_remap = [&](int k) {
+            rcol[(k + rb) * PITCH] = remap_cell(F, vc, lf.foot(F, k), lf.foot(F, k + 1));
+          };
+          const int j0 = max(q0, klo), j1 = max(j0, min(q1, khi + 1));
+          const int ja = min(j0, q1);
+          for (int k = j0; k < j1; ++k) {
+            const T *cp = S.C + (k + n0 - 2 + rb) * PITCH + ln;
+            T r = T(0);
+#pragma unroll
+            for (int t = 0; t < 6; ++t) r += wr[t] * cp[t * PITCH];
+            rcol[(k + rb) * PITCH] = r;
+          }
+          for (int k = q0; k < q1; ++k) {  // the rest, skipping [j0, j1)
+            if (k == ja) k = max(ja, j1);
+            if (k >= q1) break;
+            edge_remap(k);
+          }
+        } else if (q0 < q1) {
+          CompatEdge<T> el = compat_edge<T>(F, lf, vc, vc, q0);
+          for (int k = q0; k < q1; ++k) {
+            const CompatEdge<T> er = compat_edge<T>(F, lf, vc, vc, k + 1);
+            rcol[(k + rb) * PITCH] = compat_remap<T>(F, el, er, vc);
+            el = er;
+          }
+        }
+        __syncwarp(fm);
+        if (c == 0) compat_ghosts(rcol, rb, ra0 - 2, ra1 + 2, L);
+        __syncwarp(fm);
+        const LineView<T> vr{rcol, rb, nrows, status};
+        T *bcol = S.C + ln;
+        auto edge_cell = [&](int k) {
+          T b = T(0);
+          if (k >= ka && k < kz) {
+            const double fa = lf.foot(F, k), fb = lf.foot(F, k + 1);
+            b = vr(k) + kbc * (foot_derivative(F, vr, fb) - foot_derivative(F, vr, fa));
+          }
+          bcol[(k + rb) * PITCH] = b;
+        };
+        // interior cells of a uniform displacement [i0, i1): the stencil
+        // (empty range for other fields: klo > khi)
+        const int i0 = max(s0, max(ka, klo)), i1 = max(i0, min(s1, min(kz, khi + 1)));
+        const int ia = min(i0, s1);
+        for (int k = i0; k < i1; ++k) {
+          const T *rp = rcol + (k + n0 - 2 + rb) * PITCH;
+          T acc = T(0);
+#pragma unroll
+          for (int t = 0; t < 6; ++t) acc += wq[t] * rp[t * PITCH];
+          bcol[(k + rb) * PITCH] = rcol[(k + rb) * PITCH] + acc;
+        }
+        for (int k = s0; k < s1; ++k) {  // the rest, skipping [i0, i1)
+          if (k == ia) k = max(ia, i1);
+          if (k >= s1) break;
+          edge_cell(k);
+        }
       }
       __syncwarp(fm);
     }
@@ -1727,45 +1471,28 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
     // values only flow further right and are masked by the backward load.
     const int qb = p1 + J;
     const int k0 = p0 - J + c * FCH;
-    const int r0 = CELL ? k0 - 1 + rb : k0 + S.n0[ln] - 3 + rb;  // row of the first tap
-    const bool ok = r0 >= 0 && r0 + FCH + (CELL ? 2 : 7) <= S.rows;
+    const int r0 = k0 - 1 + rb;  // row of the first tap
+    const bool ok = r0 >= 0 && r0 + FCH + 2 <= S.rows;
     if (!ok) atomicOr(status, STATUS_HALO);
     T v[FCH];
-    if (CELL) {
-      // w_k = (1/12c)(b_{k-1} + 10 b_k + b_{k+1}) - mu w_{k-1}; compat: zero
-      // input outside the line (non-cyclic system, exact zero start at 0)
+    {
+      // w_k = (1/12c)(b_{k-1} + 10 b_k + b_{k+1}) - mu w_{k-1}; zero input
+      // outside the line (non-cyclic system, exact zero start at 0)
       const T icw = T(F.sm_inv_den / 12.0);
-      const T *bp = ((compat && F.dsrc) ? S.C : S.B) + (ok ? r0 : 0) * PITCH + ln;
+      const T *bp = (F.dsrc ? S.C : S.B) + (ok ? r0 : 0) * PITCH + ln;
       T b0 = bp[0], b1 = bp[PITCH];
       T w = T(0);
 #pragma unroll
       for (int i = 0; i < FCH; ++i) {
         const T b2 = bp[(2 + i) * PITCH];
         T in = icw * ((b0 + b2) + T(10.0) * b1);
-        if (compat && (unsigned)(k0 + i) >= (unsigned)L) in = T(0);
+        if ((unsigned)(k0 + i) >= (unsigned)L) in = T(0);
         w = in + mmu * w;
         v[i] = w;
         b0 = b1;
         b1 = b2;
       }
-    } else {
-      const T *omp = S.om + 8 * ln;
-      const T o0 = omp[0], o1 = omp[1], o2 = omp[2], o3 = omp[3], o4 = omp[4], o5 = omp[5],
-              o6 = omp[6], o7 = omp[7];
-      const T *cp = S.C + (ok ? r0 : 0) * PITCH + ln;
-      T w0 = cp[0], w1 = cp[PITCH], w2 = cp[2 * PITCH], w3 = cp[3 * PITCH], w4 = cp[4 * PITCH],
-        w5 = cp[5 * PITCH], w6 = cp[6 * PITCH];
-      T w = T(0);
-#pragma unroll
-      for (int i = 0; i < FCH; ++i) {
-        const T w7 = cp[(7 + i) * PITCH];
-        const T mb = o0 * w0 + o1 * w1 + o2 * w2 + o3 * w3 + o4 * w4 + o5 * w5 + o6 * w6 + o7 * w7;
-        w = mb + mmu * w;
-        v[i] = w;
-        w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; w5 = w6; w6 = w7;
-      }
     }
-    T fwd_out;  // exact form, full segment: the forward value at p1 - 1
     {
       // carries: chunk map x -> pw x + e_c, inclusive scan over the line's lanes
       T sa = pw, sb = v[FCH - 1];
@@ -1780,7 +1507,6 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
       }
       T cin = __shfl_up_sync(fm, sb, 1, FLANES);
       if (c == 0) cin = T(0);
-      fwd_out = __shfl_sync(fm, sb, FLANES - 1, FLANES);
       // + cin (-mu)^(i+1), the powers by a running product (no table loads)
 #pragma unroll
       for (int i = 0; i < FCH; ++i) {
@@ -1792,24 +1518,12 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
     // lane (w stays in registers); positions left of p0 are warm-up values
     // whose x is discarded, positions from qb on start it from zero.
     const int k1 = k0;
-    // positions of this lane inside the backward range (compat: the zero
-    // start is at the line's end, x_L = 0)
-    const int nb = (compat ? min(qb, L) : qb) - k1;
-    T e_fwd = T(0);
-    if (EXACT) {
-      // forward end of the segment from a zero carry (position p1 - 1)
-      if (np == FLANES * FCH) {
-        e_fwd = fwd_out;
-      } else {
-        const int cend = (np - 1) / FCH, iend = (np - 1) - cend * FCH;
-#pragma unroll
-        for (int i = 0; i < FCH; ++i) e_fwd = (c == cend && i == iend) ? v[i] : e_fwd;
-        e_fwd = __shfl_sync(fm, e_fwd, cend, FLANES);
-      }
-    }
-    // zero from qb on; a backward range that covers every lane's positions
+    // positions of this lane inside the backward range (the zero start is at
+    // the line's end, x_L = 0)
+    const int qe = min(qb, L), nb = qe - k1;
+    // zero from qe on; a backward range that covers every lane's positions
     // needs none (uniform over the CTA)
-    if ((compat ? min(qb, L) : qb) - (p0 - J) < FLANES * FCH) {
+    if (qe - (p0 - J) < FLANES * FCH) {
 #pragma unroll
       for (int i = 0; i < FCH; ++i) v[i] = (i < nb) ? v[i] : T(0);
     }
@@ -1840,98 +1554,7 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
         v[i] += cin;
       }
     }
-    if (EXACT) {
-      // Both periodic closures after one cluster barrier.  From zero carries
-      // the segment gives w_zs (forward end E) and x_zs (backward start X).
-      // The forward carry cr into the segment adds cr (-mu)^(k-p0+1) to w,
-      // which the (linear) backward filter turns into cr h_k with
-      //   h_k = (-mu)^(k-p0+1) (1 - mu^(2(p1-k))) / (1 - mu^2),
-      // and the backward carry d from the right adds d (-mu)^(p1-k).  So
-      // the segment's backward map is x_start = (-mu)^np x_in + X + cr h_p0.
-      const T xs = __shfl_sync(fm, v[0], 0, FLANES);
-      if (c == 0) {
-        S.ex[ln] = e_fwd;
-        S.ex[LPG + ln] = xs;
-      }
-      cg::this_cluster().sync();
-      const T inv1m = T(1) / (T(1) - mu * mu);
-      T cr, d;
-      {
-        // lane r (< cs) loads segment r's E_r and X_r
-        T sa = T(1), sb = T(0), xr = T(0), pr = T(1);
-        if (c < cs) {
-          const int a0 = min(L, c * Lc), a1 = min(L, a0 + Lc);
-          pr = S.pwa[a1 - a0];
-          sa = pr;
-          const T *rex = cg::this_cluster().map_shared_rank(S.ex, c);
-          sb = rex[ln];
-          xr = rex[LPG + ln];
-        }
-        // forward: compose w -> (-mu)^np_r w + E_r left to right, close the
-        // line periodically, carry into every segment
-#pragma unroll
-        for (int dd = 1; dd < FLANES; dd <<= 1) {
-          const T pa = __shfl_up_sync(fm, sa, dd, FLANES);
-          const T pb = __shfl_up_sync(fm, sb, dd, FLANES);
-          if (c >= dd) {
-            sb = sa * pb + sb;
-            sa = sa * pa;
-          }
-        }
-        const T at = __shfl_sync(fm, sa, FLANES - 1, FLANES);  // lanes >= cs: identity
-        const T et = __shfl_sync(fm, sb, FLANES - 1, FLANES);
-        const T c0 = et / (T(1) - at);
-        const T ea = __shfl_up_sync(fm, sa, 1, FLANES);
-        const T eb = __shfl_up_sync(fm, sb, 1, FLANES);
-        const T cr_c = c > 0 ? ea * c0 + eb : c0;  // carry into segment c
-        cr = __shfl_sync(fm, cr_c, rank, FLANES);
-        // backward: compose x -> (-mu)^np_r x + X_r + cr_r h_p0 right to left
-        T ba = pr, bb = c < cs ? xr + cr_c * (S.pwa[1] * (T(1) - pr * pr) * inv1m) : T(0);
-#pragma unroll
-        for (int dd = 1; dd < FLANES; dd <<= 1) {
-          const T pa = __shfl_down_sync(fm, ba, dd, FLANES);
-          const T pb = __shfl_down_sync(fm, bb, dd, FLANES);
-          if (c + dd < FLANES) {
-            bb = ba * pb + bb;
-            ba = ba * pa;
-          }
-        }
-        const T at2 = __shfl_sync(fm, ba, 0, FLANES);
-        const T xt = __shfl_sync(fm, bb, 0, FLANES);
-        const bool last = rank + 1 >= cs;
-        const T da = __shfl_sync(fm, ba, last ? 0 : rank + 1, FLANES);
-        const T db = __shfl_sync(fm, bb, last ? 0 : rank + 1, FLANES);
-        const T x0 = xt / (T(1) - at2);
-        d = last ? x0 : da * x0 + db;
-      }
-      // this CTA's reads of the cluster's shared memory are done; it waits
-      // for the others' before it exits (non-aligned forms: the wait follows
-      // the divergent store loops)
-      asm volatile("barrier.cluster.arrive;\n" ::: "memory");
-      // x_k += cr h_k + d (-mu)^(p1-k), with cr h_k = A (-mu)^(k-p0+1) -
-      // A (-mu)^(np+1) (-mu)^(p1-k), A = cr / (1 - mu^2): one power series
-      // rising from the segment start, one from its end (running products;
-      // positions from p1 on are not stored)
-      {
-        const T A = cr * inv1m;
-        const T Bc = d - A * S.pwa[np + 1];
-        T t1 = A * S.pwa[c * FCH + 1];  // A (-mu)^(k0-p0+1)
-#pragma unroll
-        for (int i = 0; i < FCH; ++i) {
-          v[i] += t1;
-          t1 *= mmu;
-        }
-        const int i0 = min(nb, FCH) - 1;  // this lane's last position before p1
-        T t3 = i0 >= 0 ? Bc * S.pwa[nb - i0] : T(0);
-#pragma unroll
-        for (int i = FCH - 1; i >= 0; --i)
-          if (i <= i0) {
-            v[i] += t3;
-            t3 *= mmu;
-          }
-      }
-    }
-    if (compat && p0 == 0) {
+    if (p0 == 0) {
       // non-cyclic system: A = c (1 + mu S^-1)(1 + mu S) + c mu^2 e_0 e_0^T,
       // so x = y - y_0 g with g_k = mu^2 ((-mu)^k - (-mu)^(2L-k)) /
       // (1 - mu^(2L+2)) (Sherman-Morrison); y_0 is this segment's x at 0
@@ -1988,7 +1611,6 @@ __global__ void __launch_bounds__(NTH, CELL ? 2 : 4)
       for (int row = lane; row < np; row += 32) lbase[row] = scol[row * PITCH];
     }
   }
-  if (EXACT) asm volatile("barrier.cluster.wait;\n" ::: "memory");
 }
 
 }  // namespace
@@ -2000,6 +1622,8 @@ size_t sweep_smem_bytes(int lc_max, int halo, bool fp64, bool source) {
   return FD_BYTES + n * el;
 }
 
+// The filter kernel's tile; exact, cell: the larger and smaller tiles that bound
+// which steps are taken.
 size_t sweep_filter_smem_bytes(int lc_max, int halo, bool fp64, bool exact, bool cell) {
   size_t el = fp64 ? 8 : 4;
   return FD_BYTES + 64 * sizeof(int) +
@@ -2030,21 +1654,6 @@ size_t sweep_fast_smem_bytes(int lc_max, int halo, bool fp64) {
   return FD_BYTES + 64 * sizeof(int) + n * el;
 }
 
-template <typename T>
-using FilterKernelT = void (*)(const SweepField *, int, int, double, const FieldIo, int, int, unsigned *,
-                               int, int, const int *, int, int, const int *);
-
-// The filter kernel's instantiation of a variant.
-template <typename T>
-static FilterKernelT<T> filter_kernel_for(int variant) {
-  switch (variant) {
-    case SWEEP_FILTER_EXACT: return sweep_filter_kernel<T, true, false, false>;
-    case SWEEP_CELL_EXACT: return sweep_filter_kernel<T, true, true, false>;
-    case SWEEP_CELL_COMPAT: return sweep_filter_kernel<T, false, true, true>;
-    default: return nullptr;
-  }
-}
-
 // Programmatic dependent launch: the filter kernels wait for their predecessor
 // before reading cells, after fetching what is constant.  Batch of 64 mixed
 // instances: 1323 ms without, 1276 ms with; 12 instances up to 583^2: 115 ms
@@ -2068,11 +1677,9 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
     return launch_stream<T>(G, plan, d_fields, nfields, group_base, groups_total, toff, io, d_status,
                             jstep, nslice, nlo, inplace, stream, g0idx, pdl_ok && pdl_enabled());
   const bool fast = (variant == SWEEP_FAST);
-  const bool cell = cell_filter_variant(variant);
-  const bool exact = exact_filter_variant(variant);
   const bool filt = filter_variant(variant);
   const bool src = (variant == SWEEP_GENERAL_SRC);
-  const size_t smem = filt ? sweep_filter_smem_bytes(lc_max, halo, sizeof(T) == 8, exact, cell)
+  const size_t smem = filt ? sweep_filter_smem_bytes(lc_max, halo, sizeof(T) == 8, false, true)
                       : fast ? sweep_fast_smem_bytes(lc_max, halo, sizeof(T) == 8)
                              : sweep_smem_bytes(lc_max, halo, sizeof(T) == 8, src);
   {
@@ -2091,9 +1698,7 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
       if (!configured[dev].load(std::memory_order_relaxed)) {
         for (const void *fn :
              {(const void *)sweep_kernel<T>, (const void *)sweep_fast_kernel<T>,
-              (const void *)filter_kernel_for<T>(SWEEP_FILTER_EXACT),
-              (const void *)filter_kernel_for<T>(SWEEP_CELL_EXACT),
-              (const void *)filter_kernel_for<T>(SWEEP_CELL_COMPAT)}) {
+              (const void *)sweep_filter_kernel<T>}) {
           err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      227 * 1024);
           if (err != cudaSuccess) return err;
@@ -2119,14 +1724,13 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
   cfg.numAttrs = 1;
   count_launch();
   if (filt) {
-    // whole lines per CTA, or out of place: no cluster (exact form: one
-    // cluster per tile, the cs segments of its lines)
+    // whole lines per CTA, or out of place: no cluster
     int clustered = 0;
     cudaLaunchAttribute fattr[2];
     unsigned na = 0;
-    if (exact || !(cs == 1 || !inplace)) {
+    if (cs > 1 && inplace) {
       fattr[na++] = attr[0];
-      clustered = exact ? 0 : 1;
+      clustered = 1;
     }
     if (pdl_ok && pdl_enabled()) {
       fattr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -2135,8 +1739,7 @@ static cudaError_t launch_impl(const LaunchGeom &G, const PlanFields &plan,
     }
     cfg.attrs = fattr;
     cfg.numAttrs = na;
-    FilterKernelT<T> fn = filter_kernel_for<T>(variant);
-    return cudaLaunchKernelEx(&cfg, fn, d_fields, nfields, group_base * cs, toff, io, lc_max,
+    return cudaLaunchKernelEx(&cfg, sweep_filter_kernel<T>, d_fields, nfields, group_base * cs, toff, io, lc_max,
                               halo, d_status, jstep, nslice, nlo, cs, clustered, g0idx);
   }
   if (fast)
