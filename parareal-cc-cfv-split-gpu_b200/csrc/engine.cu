@@ -711,7 +711,8 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
     const SweepField *hk = h.data() + (size_t)kind * nf;
     PlanFields &pv = plan->by_value[kind];
     pv.f = hk[0];
-    pv.tiles = hk[0].groups;
+    // (fields and segments are grid dimensions of at most 65535 there)
+    pv.tiles = nf <= 65535 && plan->geom[kind].cs <= 65535 ? hk[0].groups : 0;
     pv.seg = plan->geom[kind].lc_max;
     // buffers a constant stride apart (slices of one allocation)
     auto at = [](const void *p) { return reinterpret_cast<long long>(p); };

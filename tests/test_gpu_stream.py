@@ -146,3 +146,35 @@ def test_strong_diffusion(oracle, ccfv, nx, ny, vel, vp, nu):
     s.run(c, 0.0, dt, 2)
     s.check()
     assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
+
+
+@pytest.mark.parametrize("nx,ny", [(4, 4), (5, 7), (9, 17)])
+@pytest.mark.parametrize("vel,vp,bc,scheme", [(1, (0.9, -1.7), 1, 1), (3, (1.5,), 1, 1),
+                                              (1, (0.9, -1.7), 0, 0), (1, (0.9, -1.7), 0, 1)],
+                         ids=["const", "swirl", "compat_ref", "compat"])
+def test_smallest_grids(oracle, ccfv, nx, ny, vel, vp, bc, scheme):
+    """Lines shorter than one lane's positions: periodic (closed exactly) and
+    with the reference's boundaries, where every cell is next to a line end."""
+    K, dt = 1e-3, 0.8 / max(nx, ny) / 1.7
+    C0 = periodic_field(nx, nx + ny, ny=ny)
+    g = oracle.grid(nx, ny, bc=bc, vel=vel, vp=vp, K=K, threads=1, scheme=scheme)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=bc, velocity=vel, vel_params=vp, K=K,
+                                   scheme=scheme))
+    c = dev(C0)
+    s.run(c, 0.0, dt, 3)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 3)) < TOL
+
+
+def test_more_fields_than_a_grid_dimension_holds(ccfv):
+    """65,537 slices in one launch: the fields' launch index is flat there."""
+    n, N, DT = 65537, 40, 0.02
+    s = ccfv.Solver(ccfv.make_grid(N, bc=1, velocity=1, vel_params=(0.9, -1.7), K=1e-3, scheme=1))
+    assert [v for v, _ in s.sweep_plan(DT / 2)] == ["filter"] * 3
+    C0 = dev(periodic_field(N, 7))
+    f = C0.repeat(n, 1, 1).contiguous()
+    s.fine_slices(f, 0.0, DT, DT, 2)
+    s.run(C0, 0.0, DT / 2, 2)
+    s.check()
+    # the same sweeps of the same values but for the fused x pass's rounding
+    assert float((f - C0).abs().max()) < 1e-13 * float(C0.abs().max())
