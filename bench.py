@@ -259,19 +259,16 @@ def measured_peak():
     return 6650.0, "fallback"
 
 
-# DRAM bytes per cell per sweep of the fine sweep kernel, from one-launch ncu
-# captures (dram__bytes_read.sum + dram__bytes_write.sum / cells) of a 4096^2
-# FP64 sweep of each kernel form (warm-up form: the rotation field at
-# nu = 1e-3; cluster form: nu = 0.02).
-NCU_BYTES_PER_CELL_SWEEP = {"filter": 13.28, "filter_exact": 13.27}
+# DRAM bytes per cell per pass of the streaming kernel, from ncu captures
+# (dram__bytes_read.sum + dram__bytes_write.sum / cells) of 4096^2 FP64 passes
+# over the rotation field (x and y alike).
+NCU_BYTES_PER_CELL_SWEEP = {"filter": 13.4}
 
 
 def ncu_traffic(N, variants=()):
-    """Measured DRAM bytes per cell per sweep of the kernel form the fine
-    sweeps run (the exact cluster form when any sub-step runs it); scaled by
-    the caller to a launch.  None for forms without a capture."""
-    if "filter_exact" in variants:
-        return NCU_BYTES_PER_CELL_SWEEP["filter_exact"]
+    """Measured DRAM bytes per cell per pass of the kernel form the fine
+    sweeps run; scaled by the caller to a launch.  None for forms without a
+    capture."""
     if variants and all(v == "filter" for v in variants):
         return NCU_BYTES_PER_CELL_SWEEP["filter"]
     return None
@@ -731,8 +728,9 @@ def measure_batch(a, ws, rank, local, steps, warmup):
     th = coarse_theta_arg(a)
     plain = plain_rate(sample, local)
     plain_th = plain_rate(sample, local, th) if th != 0.5 else plain
-    # the batch's shared F phases: 48 algorithmic bytes per executed fine
-    # cell-update (3 FP64 sweeps, read + write)
+    # the batch's shared F phases: 48 bytes per executed fine cell-update (3 FP64
+    # sweeps, read + write); problems whose neighbouring x sweeps share a pass
+    # move a third less, so this is the rate of the scheme, not of the bus
     fine_cu = float(sum(x["fine_cell_updates"] for x in st))
     peak, peak_kind = measured_peak()
     f_gbs = 48.0 * fine_cu / (st[0]["fine_ms"] * 1e-3) / 1e9 if st[0]["fine_ms"] else None
@@ -943,7 +941,7 @@ def run_step(a, w, ws, rank, local):
         hn = solver.run(hn, i * n * dt, dt, n)
     e_s = reduce_max(time.perf_counter() - e0, ws)
     peak, peak_kind = measured_peak()
-    sweeps = 3 * n * a.steps
+    sweeps = launches  # passes over the field: neighbouring x sweeps share one
     achieved = N * N * sweeps * BYTES_PER_FINE_CELL_SWEEP / (ms * 1e-3) / 1e9
     tpc = ncu_traffic(N, [v for v, _ in solver.sweep_plan(dt)])
     cpu = None
