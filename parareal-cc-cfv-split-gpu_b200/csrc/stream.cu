@@ -233,53 +233,79 @@ __device__ __noinline__ T remap_at_end(const SweepField &F, const V &cells, int 
 // and within the clamp of one of its ends (remap_at_end).
 constexpr int FOOT_BELOW = -1, FOOT_ON_END = -2, FOOT_ABOVE = 1 << 30;
 
+// Feet of the edges that the region's positions need, by HL lanes (this one:
+// hc): kf, the cell with a mark for feet outside the line (zero inflow); d, the
+// offset in the cell `at`, which is NO_CELL where the foot lies in no cell.
+// They depend on the plan alone: done before the launch waits for its
+// predecessor.
+constexpr double NO_CELL = -4096.0;
+template <typename T, bool REMAPPED, int HL>
+__device__ __forceinline__ void end_feet(const SweepField &F, int line, int n0, double x0,
+                                         const EndRegion &R, int hc, T *at, T *d, int *kf) {
+  const int L = F.L, e0 = REMAPPED ? R.ra : R.ba, e1 = REMAPPED ? R.rb : R.bb;
+  if (R.ka >= R.kb) return;
+  // Every foot of a line sits at the same offset n0 + x0 from its edge: one
+  // clear of the ends needs no quotient of its own, one a cell beyond them lies
+  // in no cell and neither do those of its cell.
+  for (int e = e0 + hc; e <= e1; e += HL) {
+    const int j = e + n0;
+    int mark = j < 0 ? FOOT_BELOW : FOOT_ABOVE + L;
+    FootCell p{j, x0};
+    const bool cell = j > -2 && j < L + 1;
+    if (cell) {
+      mark = j;
+      if (j < 2 || j > L - 4) {
+        const double f = line_foot(F, line, e);
+        p = foot_cell(F, f, F.eps_remap);
+        mark = f < F.s_min               ? FOOT_BELOW
+               : f > F.s_max             ? FOOT_ABOVE + p.k
+               : f < F.s_min + F.eps_remap || f > F.s_max - F.eps_remap ? FOOT_ON_END
+                                                                        : p.k;
+      }
+    }
+    at[e - e0] = cell ? T(p.k) : T(NO_CELL);
+    d[e - e0] = T(p.xi);
+    kf[e - e0] = mark;
+  }
+}
+
 // r_k = (1/12c)(b_{k-1} + 10 b_k + b_{k+1}) of the region's positions into
-// `r`, by HL lanes (this one: hc).  phi / d / tmp / kf: scratch of the half.
-// All lanes of the warp call it (empty region: nothing but the barriers).
+// `d`, from the feet that end_feet left (phi: their cells).  phi / d / tmp / kf:
+// scratch of the half.  All lanes of the warp call it (empty region: nothing but
+// the barriers).
 template <typename T, int ES, bool REMAPPED, int HL>
 __device__ __forceinline__ void end_inputs(const SweepField &F, const StagedLine<T, ES> &cells,
-                                           int line, int n0, double x0, const EndRegion &R, int hc,
+                                           int line, int n0, const EndRegion &R, int hc,
                                            T *phi, T *d, T *tmp, int *kf) {
   tmp += 2;  // room for two ghosts on either side
   const int L = F.L;
   const T kbc = T(F.kb), inv12h = T(F.inv12h);
   const bool any = R.ka < R.kb;
-  // feet of the edges [e0, e1]: PPM integral and cell, with a mark for feet
-  // outside the line (zero inflow), and the derivative of the staged cells
+  // PPM integral of the feet's cells and derivative of the staged cells
   const int e0 = REMAPPED ? R.ra : R.ba, e1 = REMAPPED ? R.rb : R.bb;
-  // Every foot of a line sits at the same offset n0 + x0 from its edge: one
-  // clear of the ends needs no quotient of its own, one a cell beyond them lies
-  // in no cell and neither do those of its cell.
   if (any)
-    for (int e = e0 + hc; e <= e1; e += HL) {
-      const int j = e + n0;
-      int mark = j < 0 ? FOOT_BELOW : FOOT_ABOVE + L;
+    for (int e = e0 + hc; e <= e1; e += HL) {  // this lane's own edges
+      const T at = phi[e - e0];
       T ph = T(0), dv = T(0);
-      if (j > -2 && j < L + 1) {
-        FootCell p{j, x0};
-        bool in = true;
-        mark = j;
-        if (j < 2 || j > L - 4) {
-          const double f = line_foot(F, line, e);
-          p = foot_cell(F, f, F.eps_remap);
-          in = f >= F.s_min && f <= F.s_max;
-          mark = f < F.s_min               ? FOOT_BELOW
-                 : f > F.s_max             ? FOOT_ABOVE + p.k
-                 : f < F.s_min + F.eps_remap || f > F.s_max - F.eps_remap ? FOOT_ON_END
-                                                                          : p.k;
-        }
-        if (!cells.near(p.k)) p.k = 2;
-        if (p.k >= 0 && p.k < L) ph = ppm_to(cells, p.k, T(p.xi));
+      if (at != T(NO_CELL)) {
+        const int mark = kf[e - e0];
+        int k = (int)at;
+        T xi = d[e - e0];
+        if (!cells.near(k)) k = 2;
+        if (k >= 0 && k < L) ph = ppm_to(cells, k, xi);
         if (REMAPPED) {
-          dv = T(p.xi);  // until the derivative of the remapped field
-        } else if (in) {
-          if (mark == FOOT_ON_END && F.eps_remap != 1e-15) p = end_foot_cell(F, line, e);
-          dv = derivative_at(cells, p.k, T(p.xi), L, inv12h);
+          dv = xi;  // until the derivative of the remapped field
+        } else if (mark != FOOT_BELOW && mark < FOOT_ABOVE) {
+          if (mark == FOOT_ON_END && F.eps_remap != 1e-15) {
+            const FootCell q = end_foot_cell(F, line, e);
+            k = q.k;
+            xi = T(q.xi);
+          }
+          dv = derivative_at(cells, k, xi, L, inv12h);
         }
       }
       phi[e - e0] = ph;
       d[e - e0] = dv;
-      kf[e - e0] = mark;
     }
   __syncwarp();
   // remapped cells: whole cells between the feet plus the two integrals
@@ -515,8 +541,6 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     const long long off = (first + (int)blockIdx.z) * plan.stride;
     vs = static_cast<const char *>(vs) + off;
     vd = static_cast<char *>(vd) + off;
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   } else {
     const int cta = (int)blockIdx.x + first;
     const SweepField &f = fields[find_field(fields, g0idx, nfields, cta / cs)];
@@ -564,6 +588,97 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   const bool inside = b0 >= 0 && b0 + nr <= L;
   const bool pairs = ((DIR == 0 ? s_pos : s_line) & 1) == 0 && (DIR == 0 || (L & 1) == 0) &&
                      (((size_t)src | (size_t)dst) & (2 * sizeof(T) - 1)) == 0;
+  // What depends on the plan alone comes before the wait, beside the launch
+  // before this one: the line's shift, the feet of its ends, the swirl's tables.
+  // Small grids are chains of dependent launches, bound by each one's latency:
+  // one step of the reference's setting at 128^2 28.5 -> 20.6 us, ten at 600^2
+  // 259 -> 226 us, its Parareal at 256^2 20.4 -> 19.1 ms, six swirl steps of
+  // 1024^2 323 -> 311 us.  (Batched launches have waited: their tables may be
+  // this launch's predecessor's work.)
+  // this lane's line
+  const int c = DIR == 0 ? lane / LPW : lane % LN;           // chunk
+  const int lw = DIR == 0 ? lane % LPW : lane / LN;          // line within the warp
+  const int line = line0 + warp * LPW + lw;
+  const T mmu = T(-F.mu);
+  const T *wt = reinterpret_cast<const T *>(F.wt) +  // padded past M
+                (size_t)line *
+                    (BND == 2 ? STREAM_TAPS_D : BND == 1 ? STREAM_TAPS_C : XX ? STREAM_TAPS_XX : 8);
+  // whether positions next to the line's ends are walked here (both regions are
+  // shorter than their scratch): other segments copy first and skip them (2048^2,
+  // eight steps: 513 us with the feet before every segment's copies, 492 us so)
+  const bool near = ENDS && (org < ends || org + act * SCH > L - ends);
+  int n0 = 0;
+  if (!SWIRL && (!ENDS || near)) n0 = __ldg(F.nt + line);
+  // swirling field: sin and cos of the edges org-1 .. of the walked positions,
+  // and the speeds of the line's two corner lines
+  double2 *const sc_edge = reinterpret_cast<double2 *>(
+      tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows);
+  CornerLine c0{0, 0, 0}, c1{0, 0, 0};
+  int series = 0;
+  if (SWIRL) {
+    for (int i = threadIdx.x; i < act * SCH + 3; i += NT) {
+      const double s = D->s_min + D->h * (org - 1 + i);
+      sc_edge[i] = double2{sinpi(s), cospi(s)};
+    }
+    const double ca = cospi((toff + D->ta_rel) / D->vp[0]);
+    const double cb = cospi((toff + D->tb_rel) / D->vp[0]);
+    const double sg = DIR == 0 ? 1.0 : -1.0, Dt = D->Dt;
+    const double g0 = sg * sinpi(2.0 * (D->t_min + D->ht * (double)line));
+    const double g1 = sg * sinpi(2.0 * (D->t_min + D->ht * (double)(line + 1)));
+    const double pd = 3.14159265358979323846 * Dt;
+    c0 = CornerLine{g0 * cb, g0 * ca, pd * (g0 * cb)};
+    c1 = CornerLine{g1 * cb, g1 * ca, pd * (g1 * cb)};
+    series = pd <= 0.00390625 ? 2 : pd <= 0.03125 ? 1 : 0;  // |speed| <= 1
+  }
+  // inputs of the positions next to the line's ends (BND): the left region is
+  // r[k - lo.ka], k in [lo.ka, lo.kb), the right one likewise
+  EndRegion lo{}, hi{};
+  hi.ka = L;
+  T *rl = nullptr, *rr = nullptr, *half = nullptr;
+  int *kf = nullptr;
+  if (near) {
+    const int kend = org + act * SCH;  // first position not walked
+    // positions whose stencil, with the mass matrix's neighbours, stays clear
+    // of clamps and ghosts: [sl, sr)
+    int bl = max(2 - n0, 0), bh = min(L - 4 - n0, L - 1);
+    if (BND == 2) {
+      bl = max(bl, 4 - 2 * n0);
+      bh = min(bh, L - 7 - 2 * n0);
+    }
+    const int sl = min(bl + 1, L), sr = min(max(bh, sl), L);
+    auto region = [&](int ka, int kb) {
+      EndRegion e;
+      e.ka = ka;
+      e.kb = kb;
+      e.ba = max(0, ka - 1);
+      e.bb = min(L, kb + 1);
+      e.ra = max(0, min(e.ba, e.ba + n0 - 4));
+      e.rb = min(L, max(e.bb, e.bb + n0 + 5));
+      if (e.ra < 3) e.ra = 0;  // with the cells its ghosts come from
+      if (e.rb > L - 3) e.rb = L;
+      return e;
+    };
+    lo = region(max(0, org), min(sl, kend));
+    hi = region(max(sr, org), min(L, kend));
+    if (line >= M) lo.kb = lo.ka, hi.kb = hi.ka;
+    // scratch: per line and end 3 arrays of `ends` values and one of cells
+    T *sc = tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows;
+    kf = reinterpret_cast<int *>(sc + (size_t)StreamCta<DIR, LN>::lines * 6 * ends);
+    const int li = warp * LPW + lw, side = c >= LN / 2;
+    sc += (size_t)li * 6 * ends;
+    kf += (size_t)(2 * li + side) * ends;
+    rl = sc + ends;
+    rr = sc + 4 * ends;
+    half = sc + side * 3 * ends;
+    const double x0 = __ldg(wt + (BND == 2 ? STREAM_TAPS_D : STREAM_TAPS_C) - 1);
+    end_feet<T, BND == 2, LN / 2>(*D, line, n0, x0, side ? hi : lo, c % (LN / 2), half,
+                                  half + ends, kf);
+  }
+  if (plan.tiles > 0) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  }
+
   if (DIR == 0) {
     constexpr int G = X_LINES / 2;
     const int g = pairs ? 2 * ((int)threadIdx.x % G) : (int)threadIdx.x % X_LINES;
@@ -619,38 +734,10 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     }
   }
   cp_async_commit();
-  // this lane's line and its stencil, while the cells arrive
-  const int c = DIR == 0 ? lane / LPW : lane % LN;           // chunk
-  const int lw = DIR == 0 ? lane % LPW : lane / LN;          // line within the warp
-  const int line = line0 + warp * LPW + lw;
-  const T mmu = T(-F.mu);
-  const T *wt = reinterpret_cast<const T *>(F.wt) +  // padded past M
-                (size_t)line *
-                    (BND == 2 ? STREAM_TAPS_D : BND == 1 ? STREAM_TAPS_C : XX ? STREAM_TAPS_XX : 8);
+  if (ENDS && !near) n0 = __ldg(F.nt + line);
+  // the stencil, while the cells arrive
   T o[8];
   if (!ENDS && !SWIRL) load_taps(o, wt);
-  const int n0 = SWIRL ? 0 : __ldg(F.nt + line);
-  // swirling field: sin and cos of the edges org-1 .. of the walked positions,
-  // and the speeds of the line's two corner lines
-  double2 *const sc_edge = reinterpret_cast<double2 *>(
-      tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows);
-  CornerLine c0{0, 0, 0}, c1{0, 0, 0};
-  int series = 0;
-  if (SWIRL) {
-    for (int i = threadIdx.x; i < act * SCH + 3; i += NT) {
-      const double s = D->s_min + D->h * (org - 1 + i);
-      sc_edge[i] = double2{sinpi(s), cospi(s)};
-    }
-    const double ca = cospi((toff + D->ta_rel) / D->vp[0]);
-    const double cb = cospi((toff + D->tb_rel) / D->vp[0]);
-    const double sg = DIR == 0 ? 1.0 : -1.0, Dt = D->Dt;
-    const double g0 = sg * sinpi(2.0 * (D->t_min + D->ht * (double)line));
-    const double g1 = sg * sinpi(2.0 * (D->t_min + D->ht * (double)(line + 1)));
-    const double pd = 3.14159265358979323846 * Dt;
-    c0 = CornerLine{g0 * cb, g0 * ca, pd * (g0 * cb)};
-    c1 = CornerLine{g1 * cb, g1 * ca, pd * (g1 * cb)};
-    series = pd <= 0.00390625 ? 2 : pd <= 0.03125 ? 1 : 0;  // |speed| <= 1
-  }
   static_assert(SCH == 17, "pw");
   T pw = mmu * mmu;  // (-mu)^17
   pw *= pw;
@@ -672,43 +759,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   bool ok = SWIRL || (r0 >= 0 && r0 + SCH + (XX ? 14 : 7) <= rows);
   if (BND == 2) ok = ok && k0 + 2 * n0 - 5 >= 0 && k0 + 2 * n0 + SCH + 8 <= rows;
   if (!ok && line < M) atomicOr(status, STATUS_HALO);
-  // inputs of the positions next to the line's ends (BND): the left region is
-  // r[k - lo.ka], k in [lo.ka, lo.kb), the right one likewise
-  EndRegion lo, hi;
-  T *rl = nullptr, *rr = nullptr;
-  if (ENDS) {
-    const int kend = org + act * SCH;  // first position not walked
-    // positions whose stencil, with the mass matrix's neighbours, stays clear
-    // of clamps and ghosts: [sl, sr)
-    int bl = max(2 - n0, 0), bh = min(L - 4 - n0, L - 1);
-    if (BND == 2) {
-      bl = max(bl, 4 - 2 * n0);
-      bh = min(bh, L - 7 - 2 * n0);
-    }
-    const int sl = min(bl + 1, L), sr = min(max(bh, sl), L);
-    auto region = [&](int ka, int kb) {
-      EndRegion e;
-      e.ka = ka;
-      e.kb = kb;
-      e.ba = max(0, ka - 1);
-      e.bb = min(L, kb + 1);
-      e.ra = max(0, min(e.ba, e.ba + n0 - 4));
-      e.rb = min(L, max(e.bb, e.bb + n0 + 5));
-      if (e.ra < 3) e.ra = 0;  // with the cells its ghosts come from
-      if (e.rb > L - 3) e.rb = L;
-      return e;
-    };
-    lo = region(max(0, org), min(sl, kend));
-    hi = region(max(sr, org), min(L, kend));
-    if (line >= M) lo.kb = lo.ka, hi.kb = hi.ka;
-    // scratch: per line and end 3 arrays of `ends` values and one of cells
-    T *sc = tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows;
-    int *kf = reinterpret_cast<int *>(sc + (size_t)StreamCta<DIR, LN>::lines * 6 * ends);
-    const int li = warp * LPW + lw, side = c >= LN / 2;
-    sc += (size_t)li * 6 * ends;
-    kf += (size_t)(2 * li + side) * ends;
-    rl = sc + ends;
-    rr = sc + 4 * ends;
+  if (near) {
     const StagedLine<T, ES> cells{col - b0 * ES, b0, b0 + nr, status};
     if (c == 0 && line < M) {  // ghost cells of the staged line
       T g1, g2;
@@ -724,12 +775,8 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
       }
     }
     __syncwarp();
-    {
-      const double x0 = __ldg(wt + (BND == 2 ? STREAM_TAPS_D : STREAM_TAPS_C) - 1);
-      T *h = sc + side * 3 * ends;
-      end_inputs<T, ES, BND == 2, LN / 2>(*D, cells, line, n0, x0, side ? hi : lo, c % (LN / 2), h,
-                                          h + ends, h + 2 * ends, kf);
-    }
+    end_inputs<T, ES, BND == 2, LN / 2>(*D, cells, line, n0, c < LN / 2 ? lo : hi, c % (LN / 2),
+                                        half, half + ends, half + 2 * ends, kf);
   }
   // doubling steps that bring a carry in from every chunk of the warm-up (FP32:
   // one more, so that what is left out, |mu|^J of it at every chunk start, is
