@@ -560,6 +560,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
            (SWIRL ? 2 * (LN * SCH + 3) * (sizeof(double) / sizeof(T)) : 0);
   if (EXACT) {
     if (threadIdx.x < 5) exs[threadIdx.x] = T(D->ex[threadIdx.x]);
+    __syncwarp();  // an aligned cluster barrier takes converged warps only
     // the peers may write to this CTA once it runs
     if (cs > 1) asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");
   }
