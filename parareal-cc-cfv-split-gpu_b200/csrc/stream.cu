@@ -580,9 +580,11 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   // (The reference's lines end: nothing is walked past position L - 1.)
   const int walked = ENDS ? min(np + 2 * J, L - p0 + J) : np + 2 * J;
   const int act = min(LN, (walked + SCH - 1) / SCH);
-  // first position of the first lane: p0 - J, or (BND) as much earlier as makes
-  // the last lane end with the line, so that nothing is masked there either
-  const int org = ENDS && p1 == L ? L - act * SCH : p0 - J;
+  // first position of the first lane: p0 - J, or (the reference's lines) as much
+  // earlier as makes the last lane end with the line, so that nothing is masked
+  // there either (also where the line ends within the warm-up of a segment
+  // before the last one)
+  const int org = ENDS ? min(p0 - J, L - act * SCH) : p0 - J;
   const int nr = (act * SCH + 2 * (H - J) + (ENDS ? 2 : 1)) & ~1;
   // position of staged row 0, row of position p0 (both even with p0 and H)
   const int b0 = ENDS ? (org - (H - J)) & ~1 : p0 - H, h0 = ENDS ? p0 - b0 : H;

@@ -1,0 +1,51 @@
+"""Sweep kernels at the ends of what they take: last segments shorter than the
+recurrence's warm-up, backward steps, the shortest lines in FP32, displacements
+of hundreds of cells, lone steps, short tuned segments."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2, seeded_field
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # FP64 parity bar of the sweeps against the oracle
+THREADS = min(32, os.cpu_count() or 1)
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64)).cuda()
+
+
+def warm_up(nu):
+    """Positions after which a start from zero has decayed below FP64 rounding,
+    for a sweep of diffusion number nu (half of it on either side)."""
+    r = (1 / 12 - 0.5 * nu) / (10 / 12 + nu)
+    mu = 2 * r / (1 + np.sqrt(1 - 4 * r * r))
+    return int(np.ceil(np.log(2.0 ** -56) / np.log(abs(mu))))
+
+
+@pytest.mark.parametrize("dir,L,last", [(0, 10225, 1), (0, 10230, 6), (0, 5966, 62),
+                                        (1, 86113, 1), (1, 86118, 6)])
+@pytest.mark.parametrize("scheme", [0, 1])
+def test_reference_boundaries_last_segment_shorter_than_the_warm_up(oracle, ccfv, dir, L, last,
+                                                                    scheme):
+    """The segment before such a last one reaches the line's end with its
+    warm-up: it stops there."""
+    nu = 5.4
+    J = warm_up(nu)
+    h, vel = 2.0 / L, (3.0, -3.7)
+    Dt = 0.8 * h / abs(vel[dir])
+    dt = 2 * Dt if dir == 0 else Dt
+    nx, ny = (L, 24) if dir == 0 else (24, L)
+    K = nu * h * h / Dt
+    C0 = seeded_field(nx, 5, ny=ny)
+    g = oracle.grid(nx, ny, K=K, vel=1, vp=vel, threads=THREADS, scheme=scheme)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, K=K, velocity=1, vel_params=vel, scheme=scheme))
+    name, seg = s.sweep_plan(dt)[dir]
+    assert name == "cell_compat" and L - (L - 1) // seg * seg == last < J
+    c = dev(C0)
+    s.run(c, 0.0, dt, 2)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
