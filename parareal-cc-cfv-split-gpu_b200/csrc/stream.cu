@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     const double pd = 3.14159265358979323846 * Dt;
     c0 = CornerLine{g0 * cb, g0 * ca, pd * (g0 * cb)};
     c1 = CornerLine{g1 * cb, g1 * ca, pd * (g1 * cb)};
-    series = pd <= 0.00390625 ? 2 : pd <= 0.03125 ? 1 : 0;  // |speed| <= 1
+    series = fabs(pd) <= 0.00390625 ? 2 : fabs(pd) <= 0.03125 ? 1 : 0;  // |speed| <= 1
   }
   // inputs of the positions next to the line's ends (BND): the left region is
   // r[k - lo.ka], k in [lo.ka, lo.kb), the right one likewise

@@ -6,7 +6,7 @@ import os
 import numpy as np
 import pytest
 
-from conftest import rel_l2, seeded_field
+from conftest import periodic_field, rel_l2, seeded_field
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-12  # FP64 parity bar of the sweeps against the oracle
@@ -49,3 +49,18 @@ def test_reference_boundaries_last_segment_shorter_than_the_warm_up(oracle, ccfv
     s.run(c, 0.0, dt, 2)
     s.check()
     assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.0, dt, 2)) < TOL
+
+
+@pytest.mark.parametrize("nx,ny", [(45, 46), (64, 64), (128, 120), (300, 270)])
+@pytest.mark.parametrize("cfl", [0.8, 6.0, 20.0])
+def test_swirl_backward_steps_match_oracle(oracle, ccfv, nx, ny, cfl):
+    """Corner feet of backward steps: the series is chosen by the step's length,
+    not its sign."""
+    dt = -cfl / max(nx, ny)
+    C0 = periodic_field(nx, nx + 2, ny=ny)
+    g = oracle.grid(nx, ny, bc=1, vel=3, vp=(1.5,), threads=THREADS, scheme=1)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=3, vel_params=(1.5,), scheme=1))
+    c = dev(C0)
+    s.run(c, 0.4, dt, 3)
+    s.check()
+    assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.4, dt, 3)) < TOL
