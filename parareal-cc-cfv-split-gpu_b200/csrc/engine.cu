@@ -616,7 +616,7 @@ void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom
     f.ex[1] = std::pow(q, end);
     f.ex[2] = 1.0 / (1.0 - q * q);
     f.ex[3] = 1.0 / (1.0 - std::pow(q, f.L));
-    f.ex[4] = std::pow(q, end - (end + STREAM_CH - 1) / STREAM_CH * STREAM_CH);
+    f.ex[4] = std::pow(q, (end - 1) % STREAM_CH + 1);
   }
   f.rk_a = mu * mu / (1.0 - std::pow(mu * mu, f.L + 1));
   f.rk_tail = std::pow(std::fabs(mu), f.L) >= std::ldexp(1.0, -60) ? 1 : 0;

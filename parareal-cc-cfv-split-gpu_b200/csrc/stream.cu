@@ -912,10 +912,10 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     constexpr int W = DIR == 0 ? 32 : LN;      // shuffle width of a line
     const int l0 = DIR == 0 ? lane % LPW : 0;  // its first lane
     auto from = [&](T a, int ch) { return __shfl_sync(FULL, a, l0 + LS * ch, W); };
+    const int mine = np - c * SCH;  // positions from this lane's first one on
     // E; nothing behind the segment for the backward recurrence
     T E = v[SCH - 1];
     if (np < LN * SCH) {
-      const int mine = np - c * SCH;  // positions of this lane
 #pragma unroll
       for (int i = 0; i < SCH; ++i) {
         if (i == mine - 1) E = v[i];
@@ -925,14 +925,14 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     x = T(0);
 #pragma unroll
     for (int i = SCH - 1; i >= 0; --i) x = v[i] + mmu * x;
-    // with the scan: q^(17 c), q^(17 (act-1-c))
+    // with the scan: q^(17 c), and q^(17 (act-2-c)) for the lanes before the last
     T pd = pw, up = T(1), down = T(1);
 #pragma unroll
     for (int b = 0; b < (LN == 32 ? 5 : 4); ++b) {
       const T t = __shfl_down_sync(FULL, x, LS << b, W);
       if (c + (1 << b) < LN) x += pd * t;
       if (c >> b & 1) up *= pd;
-      if ((act - 1 - c) >> b & 1) down *= pd;
+      if ((act - 2 - c) >> b & 1) down *= pd;
       pd *= pd;
     }
     // The forward carry cr into a segment adds cr q^(j+1) to w_j (q = -mu),
@@ -988,9 +988,18 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     const T far = d - cr * inv1m * mmu * (end ? last : whole);
     x = __shfl_down_sync(FULL, x, LS, W);
     if (c == LN - 1) x = T(0);
-    // carry into this lane; the last one, where it ends behind the segment,
-    // starts with as much more (q^-16 at most)
-    if (c < act) x += far * down * (end ? exs[4] : T(1));
+    // carry into this lane; into the last one right behind the segment's last
+    // position (scaled up to the lane's end it would leave FP32's range on the
+    // shortest lines: q^-13 at 4 cells)
+    if (mine > SCH) {
+      x += far * down * (end ? exs[4] : pw);
+    } else if (mine == SCH) {
+      x += far;
+    } else {
+#pragma unroll
+      for (int i = 1; i < SCH; ++i)
+        if (i == mine) v[i] = far;
+    }
   }
   __syncwarp();  // every lane of the line has read its cells
   T *xp = col + k0 * ES;

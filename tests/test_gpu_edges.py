@@ -64,3 +64,27 @@ def test_swirl_backward_steps_match_oracle(oracle, ccfv, nx, ny, cfl):
     s.run(c, 0.4, dt, 3)
     s.check()
     assert rel_l2(c.cpu().numpy(), oracle.run(g, C0, 0.4, dt, 3)) < TOL
+
+
+@pytest.mark.parametrize("L", [4, 5, 6])
+@pytest.mark.parametrize("dir", [0, 1])
+@pytest.mark.parametrize("mu", [2.0 ** -14, -2.0 ** -12, 2.0 ** -11, -2.0 ** -9.5])
+@pytest.mark.parametrize("vel,vp", [(1, (0.9, -1.7)), (3, (1.5,))], ids=["const", "swirl"])
+def test_fp32_coarse_steps_on_the_shortest_lines(oracle, ccfv, L, dir, mu, vel, vp):
+    """Lines of a few cells whose system is next to diagonal (K Dt / h^2 near
+    1/6): carries of many orders of magnitude less than one."""
+    nx, ny = (L, 8) if dir == 0 else (8, L)
+    Dt = 0.3 / 8
+    r = mu / (1 + mu * mu)
+    nu = (1 / 12 - r * 10 / 12) / (0.5 + r)  # (1/12 - nu/2) / (10/12 + nu) = r
+    K = nu / (L * L * Dt)
+    dt = 2 * Dt if dir == 0 else Dt
+    C0 = periodic_field(nx, L, ny=ny)
+    g = oracle.grid(nx, ny, bc=1, vel=vel, vp=vp, K=K, threads=1, scheme=1)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=vel, vel_params=vp, K=K, scheme=1))
+    c = dev(C0)
+    s.coarse(c, 0.0, dt, 1, precision=ccfv.FP32)
+    s.check()
+    # three sweeps of at most 20 roundings of 2^-24 each, on values of the
+    # field's size
+    assert rel_l2(c.cpu().numpy(), oracle.coarse(g, C0, 0.0, dt, 1)) < 60 * 2.0 ** -24
