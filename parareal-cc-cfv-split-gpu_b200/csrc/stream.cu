@@ -38,6 +38,7 @@
 #include <mutex>
 
 #include "ccfv_internal.h"
+#include "line_ends.cuh"
 #include "sweep_device.cuh"
 #include "sweep_math.cuh"
 
@@ -139,48 +140,7 @@ struct StagedLine {
   }
 };
 
-// Ghost cells C_{-2}, C_{-1} (left) or C_L, C_{L+1} (3-point extrapolation,
-// T2S4:275-286) of the line ends: near to far cells a, b, d; ghosts at `g`.
-template <typename T>
-__device__ __forceinline__ void ghosts(T a, T b, T d, T &g1, T &g2) {
-  const T e = T(1.0 / 11.0);
-  g1 = e * (-d + T(3) * b + T(9) * a);
-  g2 = e * (T(-15) * d + T(56) * b - T(30) * a);
-}
-
-// PPM integral of a cell from its left edge to xi (d_intC_ppm4th, T2S4:63-65,
-// with the coefficients of T2S4:260-304).
-template <typename T, typename V>
-__device__ __forceinline__ T ppm_to(const V &c, int k, T xi) {
-  const T m2 = c(k - 2), m1 = c(k - 1), z = c(k), p1 = c(k + 1), p2 = c(k + 2);
-  const T cl = T(7.0 / 12.0) * (z + m1) - T(1.0 / 12.0) * (p1 + m2);
-  const T cr = T(7.0 / 12.0) * (p1 + z) - T(1.0 / 12.0) * (p2 + m1);
-  const T D = cr - cl, C6 = T(6.0) * (z - T(0.5) * (cl + cr));
-  const T xi2 = xi * xi;
-  return T(-1.0 / 3) * C6 * (xi2 * xi) + T(0.5) * (D + C6) * xi2 + cl * xi;
-}
-
-// Fourth-order derivative at a foot in cell k (T2S4:440-547) with the
-// reference's choice of ghosts at k = 1 (-2 tap reads C_{-2}) and k = L - 2
-// (+2 tap reads C_{L+1}).
-template <typename T, typename V>
-__device__ __forceinline__ T derivative_at(const V &c, int k, T xi, int L, T inv12h) {
-  const T m2 = c(k == 1 ? -2 : k - 2), m1 = c(k - 1), z = c(k), p1 = c(k + 1),
-          p2 = c(k == L - 2 ? L + 1 : k + 2);
-  const T xi2 = xi * xi, xi3 = xi2 * xi;
-  return inv12h * ((T(2.0) * xi3 - T(6.0) * xi2 + T(3.0) * xi + T(1.0)) * m2 +
-                   (T(-8.0) * xi3 + T(18.0) * xi2 + T(6.0) * xi - T(15.0)) * m1 +
-                   (T(12.0) * xi3 - T(18.0) * xi2 - T(24.0) * xi + T(15.0)) * z +
-                   (T(-8.0) * xi3 + T(6.0) * xi2 + T(18.0) * xi - T(1.0)) * p1 +
-                   (T(2.0) * xi3 - T(3.0) * xi) * p2);
-}
-
-// A foot in cell units: cell and offset, clamped by eps to the line
-// (T2S4:322-324, 414-415, 452-455).
-struct FootCell {
-  int k;
-  double xi;
-};
+// FootCell of a foot, clamped by eps to the line (T2S4:322-324, 414-415, 452-455).
 __device__ __forceinline__ FootCell foot_cell(const SweepField &F, double f, double eps) {
   const double x = fmin(fmax(f, F.s_min + eps), F.s_max - eps);
   FootCell r;
@@ -228,17 +188,11 @@ __device__ __noinline__ T remap_at_end(const SweepField &F, const V &cells, int 
   return v + ir;
 }
 
-// Marks of the feet that are in no cell of the line: below it (clamped to cell
-// 0), above it (added to the cell it is clamped to: L - 1, or L by rounding),
-// and within the clamp of one of its ends (remap_at_end).
-constexpr int FOOT_BELOW = -1, FOOT_ON_END = -2, FOOT_ABOVE = 1 << 30;
-
 // Feet of the edges that the region's positions need, by HL lanes (this one:
 // hc): kf, the cell with a mark for feet outside the line (zero inflow); d, the
 // offset in the cell `at`, which is NO_CELL where the foot lies in no cell.
 // They depend on the plan alone: done before the launch waits for its
 // predecessor.
-constexpr double NO_CELL = -4096.0;
 template <typename T, bool REMAPPED, int HL>
 __device__ __forceinline__ void end_feet(const SweepField &F, int line, int n0, double x0,
                                          const EndRegion &R, int hc, T *at, T *d, int *kf) {
@@ -285,27 +239,13 @@ __device__ __forceinline__ void end_inputs(const SweepField &F, const StagedLine
   const int e0 = REMAPPED ? R.ra : R.ba, e1 = REMAPPED ? R.rb : R.bb;
   if (any)
     for (int e = e0 + hc; e <= e1; e += HL) {  // this lane's own edges
-      const T at = phi[e - e0];
-      T ph = T(0), dv = T(0);
-      if (at != T(NO_CELL)) {
-        const int mark = kf[e - e0];
-        int k = (int)at;
-        T xi = d[e - e0];
-        if (!cells.near(k)) k = 2;
-        if (k >= 0 && k < L) ph = ppm_to(cells, k, xi);
-        if (REMAPPED) {
-          dv = xi;  // until the derivative of the remapped field
-        } else if (mark != FOOT_BELOW && mark < FOOT_ABOVE) {
-          if (mark == FOOT_ON_END && F.eps_remap != 1e-15) {
-            const FootCell q = end_foot_cell(F, line, e);
-            k = q.k;
-            xi = T(q.xi);
-          }
-          dv = derivative_at(cells, k, xi, L, inv12h);
-        }
-      }
-      phi[e - e0] = ph;
-      d[e - e0] = dv;
+      const int i = e - e0;
+      T ph = phi[i], dv = d[i];
+      if (!foot_inputs<REMAPPED>(cells, L, inv12h, kf[i], F.eps_remap != 1e-15,
+                                 [&] { return end_foot_cell(F, line, e); }, ph, dv))
+        kf[i] = FOOT_ABOVE;
+      phi[i] = ph;
+      d[i] = dv;
     }
   __syncwarp();
   // remapped cells: whole cells between the feet plus the two integrals
