@@ -295,12 +295,15 @@ int filter_lc(int L, bool fp64) {
 // Streaming form: the tuned length of exactly these lines, else no limit (its
 // longest segment is the fastest but for rounding up to whole segments).  A
 // line class does not bound it, so a problem splits its lines alike alone and
-// in a batch and FP32 increments round alike.
-static int stream_lc(int L, bool fp64) {
-  if (g_lc_override > 0) return g_lc_override;
+// in a batch and FP32 increments round alike.  Lengths are tuned out of place;
+// in place a line's segments form one cluster, so they are no shorter than
+// MAX_CLUSTER of them need.
+static int stream_lc(int L, bool fp64, bool inplace) {
+  const int least = inplace ? (L + MAX_CLUSTER - 1) / MAX_CLUSTER : 0;
+  if (g_lc_override > 0) return std::max(least, g_lc_override);
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_filter_lc.find({L, fp64 ? 1 : 0});
-  return it != g_filter_lc.end() ? it->second : L;
+  return it != g_filter_lc.end() ? std::max(least, it->second) : L;
 }
 
 bool class_tuned(int L, bool fp64) {
@@ -357,7 +360,7 @@ static bool stream_compat_geom(LaunchGeom &G, int L, int J, bool jok, int sh, in
     S.halo = (reach + 1) & ~1;
     S.rows = (S.lanes * STREAM_CH + 2 * S.halo + 2) & ~1;
   } else if (jok) {
-    stream_geom(S, L, J, reach, stream_lc(L, fp64));
+    stream_geom(S, L, J, reach, stream_lc(L, fp64, inplace));
     if (inplace && S.cs > MAX_CLUSTER) return false;
   } else {
     return false;
@@ -442,7 +445,7 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
       } else {
         G.lc_fit = G.lc_max;
         G.halo_fit = G.halo;
-        stream_geom(G, L, J, sh + 6, stream_lc(L, fp64));
+        stream_geom(G, L, J, sh + 6, stream_lc(L, fp64, inplace));
       }
     } else if (uniform) {
       G.variant = SWEEP_FAST;
@@ -504,7 +507,7 @@ bool fused_x_geom(const ccfv_grid &g, double dt, bool fp64, bool inplace, double
   const int J = double_warm_up(mu, fp64);
   if (g.nx <= 2 * J || 2 * J + 64 > 32 * STREAM_CH) return false;
   G->variant = SWEEP_FILTER_XX;
-  stream_geom(*G, g.nx, J, 2 * shift_cells(g, 0, 0.5 * dt) + 10, stream_lc(g.nx, fp64));
+  stream_geom(*G, g.nx, J, 2 * shift_cells(g, 0, 0.5 * dt) + 10, stream_lc(g.nx, fp64, inplace));
   if (inplace && G->cs > MAX_CLUSTER) return false;
   return stream_smem_bytes(*G, fp64) <= 227 * 1024;
 }

@@ -88,3 +88,32 @@ def test_fp32_coarse_steps_on_the_shortest_lines(oracle, ccfv, L, dir, mu, vel, 
     # three sweeps of at most 20 roundings of 2^-24 each, on values of the
     # field's size
     assert rel_l2(c.cpu().numpy(), oracle.coarse(g, C0, 0.0, dt, 1)) < 60 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("bc,scheme", [(1, 1), (0, 0)], ids=["periodic", "reference"])
+@pytest.mark.parametrize("dir,L", [(0, 3602), (1, 3598)])
+def test_slices_in_place_after_short_segments_were_tuned(oracle, ccfv, bc, scheme, dir, L):
+    """Lengths are tuned out of place; in place a line's segments form one
+    cluster of at most 16, whatever the tuned length."""
+    vp = (0.9, -1.7)
+    dt = 0.8 / L / 1.7
+
+    def solver(nx, ny):
+        return ccfv.Solver(ccfv.make_grid(nx, ny, bc=bc, velocity=1, vel_params=vp, scheme=scheme))
+
+    least = (L + 15) // 16
+    for m in (24, 40, 24, 96, 160):  # few x lines: short segments fill more of the GPU
+        seg = solver(L, m).autotune(dt)
+        if seg < least:
+            break
+    assert seg < least
+    nx, ny = (L, 20) if dir == 0 else (20, L)
+    s = solver(nx, ny)
+    assert s.sweep_plan(dt)[dir][1] <= seg
+    C0 = np.stack([periodic_field(nx, 3 + i, ny=ny) for i in range(2)])
+    f = dev(C0)
+    s.fine_slices(f, 0.0, 2 * dt, 2 * dt, 2)
+    s.check()
+    g = oracle.grid(nx, ny, bc=bc, vel=1, vp=vp, threads=THREADS, scheme=scheme)
+    for i in range(2):
+        assert rel_l2(f[i].cpu().numpy(), oracle.run(g, C0[i], 2 * i * dt, dt, 2)) < TOL
