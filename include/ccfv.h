@@ -344,15 +344,27 @@ int ccfv_autotune(ccfv_ctx *ctx, double dt, int precision, int *segment, void *s
  * with the factored cyclic solve), CCFV_SWEEP_SOURCE (per-cell, with the
  * source term) or CCFV_SWEEP_FILTER_EXACT (the factored solve at strong
  * diffusion: the periodic closure taken exactly across a line's segments, or
- * warmed up over more cells than CCFV_SWEEP_FILTER allows), CCFV_SWEEP_CELL / CCFV_SWEEP_CELL_EXACT (the two factored forms
- * with a per-cell right-hand side: velocity fields whose feet differ from
- * edge to edge), CCFV_SWEEP_CELL_COMPAT (the factored solve of the
- * reference's non-cyclic system with its boundaries); segment[s] = cells per
- * CTA along a line (either may be NULL).  No device work. */
+ * warmed up over more cells than CCFV_SWEEP_FILTER allows), CCFV_SWEEP_CELL /
+ * CCFV_SWEEP_CELL_EXACT (the two factored forms with a per-cell right-hand
+ * side: velocity fields whose feet differ from edge to edge),
+ * CCFV_SWEEP_CELL_COMPAT (the factored solve of the reference's non-cyclic
+ * system with its boundaries); segment[s] = cells per CTA along a line (either
+ * may be NULL).  No device work. */
 enum { CCFV_SWEEP_GENERAL = 0, CCFV_SWEEP_UNIFORM = 1, CCFV_SWEEP_FILTER = 2,
        CCFV_SWEEP_SOURCE = 3, CCFV_SWEEP_FILTER_EXACT = 4, CCFV_SWEEP_CELL = 5,
        CCFV_SWEEP_CELL_EXACT = 6, CCFV_SWEEP_CELL_COMPAT = 7 };
 int ccfv_sweep_plan(ccfv_ctx *ctx, double dt, int precision, int variant[3], int segment[3]);
+
+/* The kernels behind ccfv_sweep_plan's variants, which several share and
+ * CCFV_SWEEP_CELL_COMPAT and CCFV_SWEEP_FILTER_EXACT have two forms of:
+ * kernel[s] = CCFV_KERNEL_*; lanes[s] = lanes per line of the streaming
+ * kernel, 0 for the others; warm_up[s] = positions that its recurrences run
+ * before and behind a segment, 0 for lines closed exactly (any may be NULL).
+ * No device work. */
+enum { CCFV_KERNEL_SWEEP = 0, CCFV_KERNEL_SWEEP_FAST = 1, CCFV_KERNEL_SWEEP_FILTER = 2,
+       CCFV_KERNEL_STREAM = 3 };
+int ccfv_sweep_kernels(ccfv_ctx *ctx, double dt, int precision, int kernel[3], int lanes[3],
+                       int warm_up[3]);
 
 /* ---- library info ---------------------------------------------------- */
 /* Number of kernels this library launched since load (all contexts). */

@@ -146,6 +146,8 @@ _SIGS = {
     "ccfv_autotune": (C.c_int, [C.c_void_p, C.c_double, C.c_int, C.POINTER(C.c_int), C.c_void_p]),
     "ccfv_sweep_plan": (C.c_int, [C.c_void_p, C.c_double, C.c_int, C.POINTER(C.c_int),
                                   C.POINTER(C.c_int)]),
+    "ccfv_sweep_kernels": (C.c_int, [C.c_void_p, C.c_double, C.c_int, C.POINTER(C.c_int),
+                                     C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "ccfv_step_noalloc": (C.c_int, [C.POINTER(Grid), C.c_void_p, C.c_double, C.c_double,
                                     C.c_void_p]),
 }
@@ -305,14 +307,19 @@ class Solver:
         self._chk(lib().ccfv_sweep_plan(self._h, dt, int(precision), v, sg))
         return [(self.SWEEP_NAMES[v[i]], sg[i]) for i in range(3)]
 
-    SWEEP_KERNELS = {"general": "sweep_kernel", "uniform": "sweep_fast_kernel",
-                     "filter": "stream_kernel", "source": "sweep_kernel",
-                     "filter_exact": "stream_kernel", "cell": "stream_kernel",
-                     "cell_exact": "stream_kernel", "cell_compat": "stream_kernel"}
+    KERNEL_NAMES = ("sweep_kernel", "sweep_fast_kernel", "sweep_filter_kernel", "stream_kernel")
+
+    def sweep_kernels(self, dt, precision=FP64):
+        """Kernel, lanes per line and recurrence warm-up of the three sub-steps
+        of a step of dt: [(kernel name, lanes, positions)] * 3 (0, 0 for kernels
+        other than the streaming one; warm-up 0: lines closed exactly)."""
+        k, ln, w = (C.c_int * 3)(), (C.c_int * 3)(), (C.c_int * 3)()
+        self._chk(lib().ccfv_sweep_kernels(self._h, dt, int(precision), k, ln, w))
+        return [(self.KERNEL_NAMES[k[i]], ln[i], w[i]) for i in range(3)]
 
     def variant_names(self, dt, precision=FP64):
         """Names of the sweep kernels a step of dt launches (x, y, x)."""
-        return "/".join(self.SWEEP_KERNELS[n] for n, _ in self.sweep_plan(dt, precision))
+        return "/".join(n for n, _, _ in self.sweep_kernels(dt, precision))
 
     # -- fields and diagnostics --------------------------------------------
     def exact_ref(self, C_dev, t, stream=None):

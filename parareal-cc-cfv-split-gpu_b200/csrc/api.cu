@@ -36,6 +36,16 @@ int last_launch(ccfv_ctx *ctx) {
 
 }  // namespace
 
+// Geometry of sub-step `kind` of a step of dt as ccfv_step / ccfv_run and the
+// Parareal engines sweep it: out of place.
+static LaunchGeom planned_geom(const ccfv_ctx *ctx, int kind, double dt, int precision) {
+  const int dsrc = (kind == 2 && ctx->grid.scheme == CCFV_SCHEME_REFERENCE) ? 1 : 0;
+  LaunchGeom G = step_geom(ctx->grid, kind == 1 ? 1 : 0, kind == 1 ? dt : 0.5 * dt, dsrc,
+                           precision == CCFV_FP64, false);
+  if (ctx->force_general && G.variant != SWEEP_GENERAL_SRC) G.variant = SWEEP_GENERAL;
+  return G;
+}
+
 extern "C" {
 
 const char *ccfv_strerror(int status) {
@@ -255,18 +265,39 @@ int ccfv_sweep_plan(ccfv_ctx *ctx, double dt, int precision, int variant[3], int
   if (!ctx || !(dt > 0.0) || (precision != CCFV_FP64 && precision != CCFV_FP32))
     return CCFV_ERR_INVALID;
   for (int kind = 0; kind < 3; ++kind) {
-    const int dir = kind == 1 ? 1 : 0;
-    const double Dt = kind == 1 ? dt : 0.5 * dt;
-    const int dsrc = (kind == 2 && ctx->grid.scheme == CCFV_SCHEME_REFERENCE) ? 1 : 0;
-    // as ccfv_step/ccfv_run and the Parareal engines sweep: out of place
-    const LaunchGeom G = step_geom(ctx->grid, dir, Dt, dsrc, precision == CCFV_FP64, false);
+    const LaunchGeom G = planned_geom(ctx, kind, dt, precision);
     if (variant)
-      variant[kind] = (ctx->force_general && G.variant != SWEEP_GENERAL_SRC) ? SWEEP_GENERAL
-                      : G.variant == SWEEP_COMPAT || G.variant == SWEEP_COMPAT_D
+      variant[kind] = G.variant == SWEEP_COMPAT || G.variant == SWEEP_COMPAT_D
                           ? CCFV_SWEEP_CELL_COMPAT
                       : G.strong ? CCFV_SWEEP_FILTER_EXACT
                           : G.variant;
     if (segment) segment[kind] = G.lc_max;
+  }
+  return CCFV_OK;
+}
+
+int ccfv_sweep_kernels(ccfv_ctx *ctx, double dt, int precision, int kernel[3], int lanes[3],
+                       int warm_up[3]) {
+  if (!ctx || !(dt > 0.0) || (precision != CCFV_FP64 && precision != CCFV_FP32))
+    return CCFV_ERR_INVALID;
+  for (int kind = 0; kind < 3; ++kind) {
+    const LaunchGeom G = planned_geom(ctx, kind, dt, precision);
+    const bool stream = stream_variant(G.variant);
+    if (kernel)
+      kernel[kind] = stream                       ? CCFV_KERNEL_STREAM
+                     : filter_variant(G.variant)  ? CCFV_KERNEL_SWEEP_FILTER
+                     : G.variant == SWEEP_FAST    ? CCFV_KERNEL_SWEEP_FAST
+                                                  : CCFV_KERNEL_SWEEP;
+    if (lanes) lanes[kind] = stream ? G.lanes : 0;
+    if (warm_up) {
+      SweepField f{};
+      f.dir = G.dir;
+      f.Dt = kind == 1 ? dt : 0.5 * dt;
+      f.L = G.dir == 0 ? ctx->grid.nx : ctx->grid.ny;
+      f.theta = 0.5;
+      if (stream) filter_field(ctx->grid, f, precision == CCFV_FP64, G);
+      warm_up[kind] = f.jf;
+    }
   }
   return CCFV_OK;
 }

@@ -117,3 +117,35 @@ def test_slices_in_place_after_short_segments_were_tuned(oracle, ccfv, bc, schem
     g = oracle.grid(nx, ny, bc=bc, vel=1, vp=vp, threads=THREADS, scheme=scheme)
     for i in range(2):
         assert rel_l2(f[i].cpu().numpy(), oracle.run(g, C0[i], 2 * i * dt, dt, 2)) < TOL
+
+
+@pytest.mark.parametrize("kw,dt,want", [
+    # the reference's boundaries: lines of one segment, of several, the swirl
+    (dict(nx=300, ny=270, K=2e-3), 0.8 / 600, [(16, True), (16, False), (16, True)]),
+    (dict(nx=64, K=1e-3, velocity=3, vel_params=(1.5,)), 1e-3, "sweep_filter_kernel"),
+    (dict(nx=64, K=1e-3), 2.0,  # the third sweep's line ends need more scratch than fits
+     "stream_kernel/stream_kernel/sweep_filter_kernel"),
+    # periodic: weak diffusion, a long warm-up, closed lines, the swirl
+    (dict(nx=300, bc=1, K=1e-4, velocity=1, vel_params=(0.9, -1.7), scheme=1), 1e-3,
+     [(16, True), (32, True), (16, True)]),
+    (dict(nx=600, bc=1, K=0.1, velocity=1, vel_params=(0.9, -1.7), scheme=1), 5e-4,
+     [(32, True)] * 3),
+    (dict(nx=600, bc=1, K=1.0, velocity=1, vel_params=(0.9, -1.7), scheme=1), 1e-3,
+     [(16, False), (32, False), (16, False)]),
+    (dict(nx=64, bc=1, velocity=3, vel_params=(1.5,), scheme=1), 1e-3, "stream_kernel"),
+    (dict(nx=64, bc=1, velocity=1, vel_params=(0.9, -1.7)), 1e-3,
+     "stream_kernel/stream_kernel/sweep_kernel"),
+    (dict(nx=64, bc=1, source=1, source_params=(0.5, 0.5, 1.0, 0.1, 0.0)), 1e-3, "sweep_kernel"),
+])
+def test_the_plan_names_the_kernels_that_run(ccfv, kw, dt, want):
+    """Kernel, lanes per line and whether the recurrences are warmed up."""
+    s = ccfv.Solver(ccfv.make_grid(**kw))
+    got = s.sweep_kernels(dt)
+    if isinstance(want, str):
+        names = want.split("/") * (1 if "/" in want else 3)
+        assert [k for k, _, _ in got] == names
+        assert s.variant_names(dt) == "/".join(names)
+    else:
+        assert got == [("stream_kernel", n, w) for (n, _), (_, _, w) in zip(want, got)]
+        assert [w > 0 for _, _, w in got] == [w for _, w in want]
+        assert s.variant_names(dt) == "/".join(["stream_kernel"] * 3)
