@@ -555,7 +555,7 @@ int autotune(ccfv_ctx *ctx, double dt, bool fp64, cudaStream_t st, int *chosen, 
     if (lc > std::max(g.nx, g.ny) && lc != cand[0]) break;
     g_lc_override = lc;
     StepPlan plan;
-    int rc = build_step_plan(ctx, &plan, dt, fp64, pf);
+    int rc = build_step_plan(ctx, &plan, dt, fp64, pf, 5);
     auto tunable = [](const LaunchGeom &G) { return warm_filter_variant(G.variant) && !G.strong; };
     if (rc == CCFV_OK && !tunable(plan.geom[0]) && !tunable(plan.geom[1])) {
       g_lc_override = 0;
@@ -634,18 +634,64 @@ static void sweep_kind(int kind, double dt, int *dir, double *Dt, double *ta, do
 }
 
 int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
-                    const std::vector<std::pair<void *, double>> &fields, bool homogeneous,
-                    double theta) {
+                    const std::vector<std::pair<void *, double>> &fields, int nsteps,
+                    bool homogeneous, double theta) {
   std::vector<PlanField> pf(fields.size());
   for (size_t i = 0; i < fields.size(); ++i) {
     pf[i].A = fields[i].first;
     pf[i].t0 = fields[i].second;
   }
-  return build_step_plan(ctx, plan, dt, fp64, pf, homogeneous, theta);
+  return build_step_plan(ctx, plan, dt, fp64, pf, nsteps, homogeneous, theta);
+}
+
+// Bytes of a stencil table's taps in a plan, and of all of it (the shifts behind).
+static size_t taps_bytes(const StepPlan &plan, int kind, bool fp64) {
+  const size_t b = (fp64 ? 8 : 4) * (size_t)stencil_taps(plan.geom[kind].variant) * plan.lines[kind];
+  return (b + 255) & ~size_t(255);
+}
+static size_t table_bytes(const StepPlan &plan, int kind, bool fp64) {
+  return taps_bytes(plan, kind, fp64) +
+         ((sizeof(int) * (size_t)plan.lines[kind] + 255) & ~size_t(255));
+}
+static void point_to_table(const StepPlan &plan, int kind, bool fp64, char *at, SweepField *f) {
+  f->wt = at;
+  f->nt = reinterpret_cast<const int *>(at + taps_bytes(plan, kind, fp64));
+}
+
+// Fills the stencil table of a sub-step kind, from the descriptor of kind `like`.
+static cudaError_t fill_table(const StepPlan &plan, int kind, int like, bool fp64,
+                              cudaStream_t st) {
+  const SweepField &f = plan.by_value[kind].f;
+  return launch_filter_weights(fp64, plan.mem.as<SweepField>() + (size_t)like * plan.nf,
+                               const_cast<void *>(f.wt), const_cast<int *>(f.nt),
+                               plan.lines[kind], st, plan.geom[kind].variant);
+}
+
+// The fused pass's table of a plan that was built for a lone step, from the
+// descriptor of the first x sweep (the same line systems).  Filled once, before
+// any stream's sequence; a captured sequence fills it at each replay.
+static int make_fused_table(ccfv_ctx *ctx, StepPlan &plan, bool fp64, cudaStream_t st) {
+  if (!plan.fmem.p) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // allocates under capture too
+    CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = plan.fmem.alloc(table_bytes(plan, 3, fp64));
+    CK(cudaThreadExchangeStreamCaptureMode(&mode));
+    CK(e);
+    point_to_table(plan, 3, fp64, plan.fmem.as<char>(), &plan.by_value[3].f);
+  }
+  cudaStreamCaptureStatus capture;
+  CK(cudaStreamIsCapturing(st, &capture));
+  CK(fill_table(plan, 3, 0, fp64, st));
+  if (capture == cudaStreamCaptureStatusNone) {
+    CK(cudaStreamSynchronize(st));
+    plan.fused_filled = true;
+  }
+  return CCFV_OK;
 }
 
 int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
-                    const std::vector<PlanField> &fields, bool homogeneous, double theta) {
+                    const std::vector<PlanField> &fields, int nsteps, bool homogeneous,
+                    double theta) {
   ccfv_grid g = ctx->grid;
   if (homogeneous) g.source = CCFV_SRC_NONE;
   const int nf = (int)fields.size();
@@ -697,19 +743,30 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
   plan->pp = plan_pp;
   // filter sub-steps: one per-line stencil table per kind, shared by the
   // plan's fields (same grid and sub-step; the velocity fields of the filter
-  // kernel do not depend on time)
-  int lines[4] = {0, 0, 0, 0};
-  for (int kind = 0; kind < kinds && nf > 0; ++kind) {
-    if (!stencil_filter_variant(plan->geom[kind].variant)) continue;
-    lines[kind] = h[(size_t)kind * nf].groups * tile_lines(plan->geom[kind]);
-    CK(plan->wt[kind].alloc((fp64 ? 8 : 4) * stencil_taps(plan->geom[kind].variant) *
-                            (size_t)lines[kind]));
-    CK(plan->nt[kind].alloc(sizeof(int) * (size_t)lines[kind]));
-    for (int i = 0; i < nf; ++i) {
-      h[(size_t)kind * nf + i].wt = plan->wt[kind].p;
-      h[(size_t)kind * nf + i].nt = plan->nt[kind].as<int>();
+  // kernel do not depend on time) and by the two x sweeps where both take the
+  // same form.  A lone step of a new dt is bound by what its plan allocates and
+  // launches (330 us for every 2 MB): descriptors and tables are one
+  // allocation, and the fused pass's table waits for a sequence (descriptors
+  // that the kernels read themselves need theirs at once).
+  for (int kind = 0; kind < kinds && nf > 0; ++kind)
+    if (stencil_filter_variant(plan->geom[kind].variant))
+      plan->lines[kind] = h[(size_t)kind * nf].groups * tile_lines(plan->geom[kind]);
+  const bool shared = plan->geom[2].variant == plan->geom[0].variant;
+  plan->fused_filled = plan->fused && (nsteps > 1 || nf != 1 || plan->geom[3].cs > 65535);
+  auto own_table = [&](int kind) {
+    return plan->lines[kind] > 0 && !(kind == 2 && shared) && !(kind == 3 && !plan->fused_filled);
+  };
+  size_t bytes = (sizeof(SweepField) * h.size() + 255) & ~size_t(255), at[4] = {};
+  for (int kind = 0; kind < kinds; ++kind)
+    if (own_table(kind)) {
+      at[kind] = bytes;
+      bytes += table_bytes(*plan, kind, fp64);
     }
-  }
+  at[2] = shared ? at[0] : at[2];
+  CK(plan->mem.alloc(bytes));
+  for (int kind = 0; kind < kinds; ++kind)
+    for (int i = 0; at[kind] && i < nf; ++i)
+      point_to_table(*plan, kind, fp64, plan->mem.as<char>() + at[kind], &h[(size_t)kind * nf + i]);
   for (int kind = 0; kind < kinds && nf > 0; ++kind) {
     const SweepField *hk = h.data() + (size_t)kind * nf;
     PlanFields &pv = plan->by_value[kind];
@@ -726,30 +783,29 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
                         at(hk[i].in0) - at(hk[0].in0) != i * pv.stride || hk[i].par != hk[0].par)))
         pv.tiles = 0;
   }
-  CK(plan->fields.alloc(sizeof(SweepField) * h.size()));
-  CK(cudaMemcpy(plan->fields.p, h.data(), sizeof(SweepField) * h.size(), cudaMemcpyHostToDevice));
+  if (!h.empty())
+    CK(cudaMemcpy(plan->mem.p, h.data(), sizeof(SweepField) * h.size(), cudaMemcpyHostToDevice));
   for (int kind = 0; kind < kinds; ++kind)
-    if (lines[kind])
-      CK(launch_filter_weights(fp64, plan->fields.as<SweepField>() + (size_t)kind * nf,
-                               plan->wt[kind].p, plan->nt[kind].as<int>(), lines[kind], 0,
-                               plan->geom[kind].variant));
+    if (own_table(kind)) CK(fill_table(*plan, kind, kind, fp64, 0));
   CK(cudaStreamSynchronize(0));
   return CCFV_OK;
 }
 
-int run_steps(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int count, double t0,
+int run_steps(ccfv_ctx *ctx, StepPlan &plan, bool fp64, int first, int count, double t0,
               double dt, int nsteps, cudaStream_t st, const FieldIo &io0, bool y_in_place) {
   unsigned *status = ctx->status.as<unsigned>();
   auto launch = [&](int kind, int n, const FieldIo &io, bool inplace) {
     const LaunchGeom &G = plan.geom[kind];
     const int gpf = plan.groups_per_field[kind];
-    const SweepField *fk = plan.fields.as<SweepField>() + (size_t)kind * plan.nf;
+    const SweepField *fk = plan.mem.as<SweepField>() + (size_t)kind * plan.nf;
     const double toff = t0 + n * dt;
     return fp64 ? launch_sweep<double>(G, plan.by_value[kind], fk, plan.nf, first * gpf,
                                        count * gpf, toff, io, status, st, n, inplace)
                 : launch_sweep<float>(G, plan.by_value[kind], fk, plan.nf, first * gpf,
                                       count * gpf, toff, io, status, st, n, inplace);
   };
+  if (plan.fused && nsteps > 1 && !plan.fused_filled)
+    if (int rc = make_fused_table(ctx, plan, fp64, st)) return rc;
   for (int n = 0; n < nsteps; ++n) {
     const bool last = n == nsteps - 1;
     FieldIo io = io0;
@@ -764,7 +820,8 @@ int run_steps(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int cou
 
 // Plan of one field for the single-field calls: an out-of-place sequence
 // between the caller's field (passed per launch) and a context scratch field.
-static StepPlan *single_plan(ccfv_ctx *ctx, double dt, bool fp64, int *status, double theta) {
+static StepPlan *single_plan(ccfv_ctx *ctx, double dt, bool fp64, int nsteps, int *status,
+                             double theta) {
   auto key = std::make_tuple(dt, fp64 ? 1 : 0, 0, theta);
   auto it = ctx->step_plans.find(key);
   if (it != ctx->step_plans.end()) return it->second.get();
@@ -781,7 +838,7 @@ static StepPlan *single_plan(ccfv_ctx *ctx, double dt, bool fp64, int *status, d
   auto plan = std::make_unique<StepPlan>();
   std::vector<PlanField> f(1);
   f[0].B = scratch.p;  // A and in0: the caller's field (launch override)
-  int st = build_step_plan(ctx, plan.get(), dt, fp64, f, false, theta);
+  int st = build_step_plan(ctx, plan.get(), dt, fp64, f, nsteps, false, theta);
   if (st != CCFV_OK) {
     *status = st;
     return nullptr;
@@ -807,7 +864,7 @@ int steps(ccfv_ctx *ctx, void *d_C, bool fp64, double t0, double dt, int nsteps,
     if (src) CK(cudaMemcpyAsync(d_C, src, bytes, cudaMemcpyDeviceToDevice, st));
     return CCFV_OK;
   }
-  StepPlan *plan = single_plan(ctx, dt, fp64, &status, theta);
+  StepPlan *plan = single_plan(ctx, dt, fp64, nsteps, &status, theta);
   if (!plan) return status;
   const bool odd = plan_passes(plan->fused, nsteps) & 1;
   FieldIo io;
@@ -964,7 +1021,7 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
       fl[n].in0 = U + (size_t)n * NN;
       fl[n].ends = J;
     }
-    int rc = build_step_plan(ctx, plan.get(), dt, true, fl);
+    int rc = build_step_plan(ctx, plan.get(), dt, true, fl, J);
     if (rc) return rc;
     ctx->fine_plan = std::move(plan);
     std::memcpy(ctx->fine_plan_key, key, sizeof(key));
@@ -988,12 +1045,12 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
     f[0].A = W;
     f[0].B = W2;
     f[0].in0 = W;
-    int rc = build_step_plan(ctx, &cplan, dtc, g64, f, false, th);
+    int rc = build_step_plan(ctx, &cplan, dtc, g64, f, m, false, th);
     if (!rc && o->form == CCFV_FORM_DELTA && g.source != CCFV_SRC_NONE)
-      rc = build_step_plan(ctx, &hplan, dtc, g64, f, true, th);
+      rc = build_step_plan(ctx, &hplan, dtc, g64, f, m, true, th);
     if (rc) return rc;
   }
-  const StepPlan *dplan =
+  StepPlan *dplan =
       (o->form == CCFV_FORM_DELTA && g.source != CCFV_SRC_NONE) ? &hplan : &cplan;
   const TG *Wres = (plan_passes(dplan->fused, m) & 1) ? W2 : W;
 
@@ -1004,7 +1061,7 @@ static int parareal_impl(ccfv_ctx *ctx, const ccfv_parareal_opts *o, const doubl
   const cudaMemcpyKind k_in = o->mem == CCFV_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   CK(cudaMemcpyAsync(U, C0, fb, k_in, st));
 
-  auto coarse_on_W = [&](int n, const StepPlan *plan) -> int {
+  auto coarse_on_W = [&](int n, StepPlan *plan) -> int {
     return run_steps(ctx, *plan, g64, 0, 1, o->t0 + n * DT, dtc, m, st);
   };
 
@@ -1150,7 +1207,7 @@ int fine_slices(ccfv_ctx *ctx, double *d_fields, int n, double t0, double slice_
   StepPlan plan;
   std::vector<std::pair<void *, double>> fl;
   for (int i = 0; i < n; ++i) fl.push_back({d_fields + (size_t)i * NN, t0 + i * slice_dt});
-  int rc = build_step_plan(ctx, &plan, dt, true, fl);
+  int rc = build_step_plan(ctx, &plan, dt, true, fl, J);
   if (rc) return rc;
   if ((rc = run_steps(ctx, plan, true, 0, n, 0.0, dt, J, st))) return rc;
   CK(cudaStreamSynchronize(st));  // the plan's descriptors are released on return

@@ -42,14 +42,19 @@ struct SolverTable {
 // y(dt), x(dt/2), and, where the x sweeps of neighbouring steps fuse
 // (SWEEP_FILTER_XX), the last one of a step with the first of the next.
 struct StepPlan {
-  DevBuf fields;          // SweepField[kinds][nf]
+  DevBuf mem;             // descriptors SweepField[kinds][nf], then the stencil tables
   int nf = 0;
   bool fused = false;     // steps run x y (xx y)* x: 2 n + 1 passes, else 3 n
   int groups_per_field[4] = {0, 0, 0, 0};
   LaunchGeom geom[4];
   PlanFields by_value[4];  // the same fields as a kernel argument
   bool pp = false;        // out-of-place sequence (SweepField::pp)
-  DevBuf wt[4], nt[4];    // filter kernel: per-line stencil tables per sub-step kind
+  // lines of the per-line stencil tables per sub-step kind (0: none), which the
+  // descriptors point to.  The fused pass's table (fmem) is made by the first
+  // sequence of several steps.
+  int lines[4] = {0, 0, 0, 0};
+  DevBuf fmem;
+  bool fused_filled = false;
 };
 
 // One field of a plan: swept in place on A (B == nullptr), or an out-of-place
@@ -122,17 +127,18 @@ int batch_solve(int n, const ccfv_problem *probs, ccfv_stats *stats, int device,
                 cudaStream_t st, std::string *errmsg);
 // homogeneous: the source term is left out (the linear part of the step,
 // which the delta form of Parareal applies to slice increments).
+// nsteps: steps of the sequence that it is built for (it serves others too).
 int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
-                    const std::vector<std::pair<void *, double>> &fields,
+                    const std::vector<std::pair<void *, double>> &fields, int nsteps,
                     bool homogeneous = false, double theta = 0.5);
 int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
-                    const std::vector<PlanField> &fields, bool homogeneous = false,
+                    const std::vector<PlanField> &fields, int nsteps, bool homogeneous = false,
                     double theta = 0.5);
 // nsteps steps of dt from t0 on fields first .. first+count-1 of a plan.  io:
 // buffers of a single field that replace the plan's; y_in_place: the last
 // step's y sweep writes over its input, so that the sequence ends in the
 // other buffer than its number of passes says.
-int run_steps(ccfv_ctx *ctx, const StepPlan &plan, bool fp64, int first, int count, double t0,
+int run_steps(ccfv_ctx *ctx, StepPlan &plan, bool fp64, int first, int count, double t0,
               double dt, int nsteps, cudaStream_t st, const FieldIo &io = FieldIo(),
               bool y_in_place = false);
 // nsteps steps of the field `src` into d_C (null: d_C in place).

@@ -149,3 +149,45 @@ def test_the_plan_names_the_kernels_that_run(ccfv, kw, dt, want):
         assert got == [("stream_kernel", n, w) for (n, _), (_, _, w) in zip(want, got)]
         assert [w > 0 for _, _, w in got] == [w for _, w in want]
         assert s.variant_names(dt) == "/".join(["stream_kernel"] * 3)
+
+
+def test_a_lone_step_prepares_no_pass_that_it_does_not_launch(ccfv):
+    """The first step of a new dt fills the tables of its x and y sweeps; the pass
+    that joins neighbouring steps gets its own from the first sequence, also a
+    captured one."""
+    import torch
+    N = 200
+    s = ccfv.Solver(ccfv.make_grid(N, bc=1, velocity=1, vel_params=(0.9, -1.7), K=1e-3, scheme=1))
+    C0 = dev(periodic_field(N, 11))
+
+    def launches(f):
+        n = ccfv.kernel_launches()
+        f()
+        return ccfv.kernel_launches() - n
+
+    a, b = C0.clone(), C0.clone()
+    assert launches(lambda: s.step(a, 0.0, 1e-3)) == 2 + 3
+    assert launches(lambda: s.step(a, 1e-3, 1e-3)) == 3
+    # two steps x y xx y x, captured before any other sequence
+    cap = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=cap):
+        s.run(b, 0.0, 1e-3, 2)
+    graph.replay()
+    torch.cuda.synchronize()
+    once = b.clone()
+    assert float((once - a).abs().max()) < 1e-13 * float(a.abs().max())  # one pass for two
+    # eagerly: filled once more, then kept; the same values as replayed
+    for n in (5 + 1, 5):
+        b.copy_(C0)
+        assert launches(lambda: s.run(b, 0.0, 1e-3, 2)) == n
+        assert torch.equal(b, once)
+    b.copy_(C0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(b, once)
+    # a plan that starts with a sequence serves lone steps as well
+    c = C0.clone()
+    assert launches(lambda: s.run(c, 0.0, 5e-4, 3)) == 3 + 7
+    assert launches(lambda: s.step(c, 0.0, 5e-4)) == 3
+    s.check()
