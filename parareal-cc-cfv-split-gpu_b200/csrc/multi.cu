@@ -151,17 +151,20 @@ static void prepare_field(std::vector<PreparedField> &out, int kind, const ccfv_
   pf.f.groups = (pf.f.M + tile_lines(pf.G) - 1) / tile_lines(pf.G);
   if (filt) filter_field(g, pf.f, fp64, pf.G);
   if (stencil_filter_variant(pf.G.variant)) {
+    if (kind == 2 && !f0.dsrc) std::get<0>(tkey) = 0;  // the first x sweep's
     FilterTable &T = (*tabs)[tkey];  // shared by every field of this key
     if (!T.lines) {
       T.lines = pf.f.groups * tile_lines(pf.G);
       T.fp64 = fp64;
       T.variant = pf.G.variant;
       T.level = pf.level;
-      T.wt.alloc((fp64 ? 8 : 4) * stencil_taps(pf.G.variant) * (size_t)T.lines);
-      T.nt.alloc(sizeof(int) * (size_t)T.lines);
+      const size_t taps =
+          ((fp64 ? 8 : 4) * stencil_taps(pf.G.variant) * (size_t)T.lines + 255) & ~size_t(255);
+      if (T.buf.alloc(taps + sizeof(int) * (size_t)T.lines) == cudaSuccess)
+        T.nt = reinterpret_cast<int *>(T.buf.as<char>() + taps);
     }
-    pf.f.wt = T.wt.p;
-    pf.f.nt = T.nt.as<int>();
+    pf.f.wt = T.buf.p;
+    pf.f.nt = T.nt;
     pf.T = &T;
   }
   out.push_back(pf);
@@ -536,7 +539,7 @@ int MultiEngine::rebuild() {
   for (FilterTable *T : pending) {  // a descriptor of each new table, after the sort
     const SweepClass &K = (T->level == 0 ? fine_ : coarse_).at(T->cls);
     size_t i = 0;
-    while (i < K.h.size() && K.h[i].wt != T->wt.p) ++i;
+    while (i < K.h.size() && K.h[i].wt != T->buf.p) ++i;
     if (i == K.h.size()) return fail(CCFV_ERR_CUDA, "stencil table without a field");
     T->idx = i;
   }
@@ -549,10 +552,10 @@ int MultiEngine::rebuild() {
                         cudaMemcpyHostToDevice, st_));
   }
   for (FilterTable *T : pending) {  // stencil tables first needed by this rebuild
-    if (!T->wt.p || !T->nt.p) return fail(CCFV_ERR_NOMEM, "stencil table allocation failed");
+    if (!T->buf.p) return fail(CCFV_ERR_NOMEM, "stencil table allocation failed");
     const SweepClass &K = (T->level == 0 ? fine_ : coarse_).at(T->cls);
-    MCK(launch_filter_weights(T->fp64, classbuf_.as<SweepField>() + K.off + T->idx, T->wt.p,
-                              T->nt.as<int>(), T->lines, st_, T->variant));
+    MCK(launch_filter_weights(T->fp64, classbuf_.as<SweepField>() + K.off + T->idx, T->buf.p,
+                              T->nt, T->lines, st_, T->variant));
     T->ready = true;
   }
   const int eb = 148;
@@ -592,6 +595,7 @@ int MultiEngine::rebuild() {
         for (const SweepField &f : hr[q][i].f) {
           if (!f.wt || !f.nt) return fail(CCFV_ERR_NOMEM, "stencil table allocation failed");
           const size_t k = &f - hr[q][i].f;
+          if (k == 2 && f.wt == hr[q][i].f[0].wt) continue;
           MCK(launch_filter_weights(q == 1, rgbuf_[q].as<ResidentG>()[i].f + k,
                                     const_cast<void *>(f.wt), const_cast<int *>(f.nt), f.M, st_));
         }

@@ -15,9 +15,12 @@ namespace ccfv {
 // Per-line stencil table of the filter kernel for one (sub-step kind, level,
 // precision) of a problem; `cls`/`idx` locate a descriptor that uses it in
 // the launch classes of the rebuild that first needs it (the weights are
-// computed once, then kept while the problem lives).
+// computed once, then kept while the problem lives).  Taps and, behind them,
+// shifts are one allocation; both x sweeps of a step share a table where they
+// are alike.
 struct FilterTable {
-  DevBuf wt, nt;
+  DevBuf buf;
+  int *nt = nullptr;
   int lines = 0;
   bool fp64 = true;
   int variant = SWEEP_FILTER;  // form whose taps it holds

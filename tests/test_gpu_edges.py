@@ -191,3 +191,24 @@ def test_a_lone_step_prepares_no_pass_that_it_does_not_launch(ccfv):
     assert launches(lambda: s.run(c, 0.0, 5e-4, 3)) == 3 + 7
     assert launches(lambda: s.step(c, 0.0, 5e-4)) == 3
     s.check()
+
+
+def test_a_batch_fills_one_table_per_form_of_pass(ccfv):
+    """Problems of one size share every launch but those of their own tables:
+    x, y and joined x passes, fine and coarse."""
+    import torch
+    N = 300  # too large for the coarse propagator that keeps a field in one SM
+    grid = ccfv.make_grid(N, bc=1, velocity=1, vel_params=(0.9, -1.7), K=1e-3, scheme=1)
+    opts = dict(t0=0.0, t1=0.02, nt_fine=16, n_slices=2, coarse_ratio=2, kmax=1)
+    C0 = dev(periodic_field(N, 3))
+
+    def launches(n):
+        probs = [dict(grid=grid, C0=C0.clone(), C_T=torch.empty_like(C0), **opts)
+                 for _ in range(n)]
+        before = ccfv.kernel_launches()
+        ccfv.batch_solve(probs)
+        assert all(torch.equal(p["C_T"], probs[0]["C_T"]) for p in probs)
+        return ccfv.kernel_launches() - before
+
+    one = launches(1)
+    assert launches(2) - one == 6 and launches(4) - one == 18
