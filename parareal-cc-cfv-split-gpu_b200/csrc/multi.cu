@@ -197,11 +197,12 @@ static int step_bound(const SweepField &f) { return f.jmax > 0 ? f.jmax : INT_MA
 
 // Sorts a class by step bound (descending, stable: problem and slice order
 // kept within a bound) and numbers its tiles.
-static void finish_class(SweepClass &K) {
+void finish_class(SweepClass &K) {
   std::stable_sort(K.h.begin(), K.h.end(), [](const SweepField &a, const SweepField &b) {
     return step_bound(a) > step_bound(b);
   });
   K.groups = 0;
+  K.steps.clear();
   K.bound.resize(K.h.size());
   K.gpre.assign(K.h.size() + 1, 0);
   for (size_t i = 0; i < K.h.size(); ++i) {
@@ -211,7 +212,33 @@ static void finish_class(SweepClass &K) {
     K.groups += f.groups;
     K.bound[i] = step_bound(f);
     K.gpre[i + 1] = K.groups;
+    const std::pair<int, int> r{f.jmin, K.bound[i]};
+    if (std::find(K.steps.rbegin(), K.steps.rend(), r) == K.steps.rend()) K.steps.push_back(r);
   }
+}
+
+bool active_fields(const SweepClass &K, int jstep, int nslice, const int *nlo, int *lo, int *hi) {
+  if (K.smax_all > 0 && nslice >= K.smax_all) return false;
+  if (std::none_of(K.steps.begin(), K.steps.end(), [&](const std::pair<int, int> &r) {
+        return r.first <= jstep && jstep < r.second;
+      }))
+    return false;
+  // fields with a step bound above jstep: a prefix of the sorted class
+  *hi = (int)(std::partition_point(K.bound.begin(), K.bound.end(),
+                                   [&](int b) { return b > jstep; }) -
+              K.bound.begin());
+  auto active = [&](int i) { return field_active(K.h[i], jstep, nslice, nlo); };
+  if (K.kind == 2) {
+    // the last x sweep of fused sequences: a short range at the prefix's end
+    while (*hi > 0 && !active(*hi - 1)) --*hi;
+    *lo = 0;
+    while (*lo < *hi && !active(*lo)) ++*lo;
+    return *lo < *hi;
+  }
+  *lo = 0;
+  for (int i = 0; i < *hi; ++i)
+    if (active(i)) return true;
+  return false;
 }
 
 size_t problem_bytes(const ccfv_grid &g, const ccfv_parareal_opts &o) {
@@ -667,21 +694,8 @@ int MultiEngine::sweeps(std::map<KKey, SweepClass> &classes, int kind, int jstep
   for (auto &kv : classes) {
     SweepClass &K = kv.second;
     if (K.kind != kind) continue;
-    if (K.smax_all > 0 && nslice >= K.smax_all) continue;
-    // fields with a step bound above jstep: a prefix of the sorted class
-    const int np = (int)(std::partition_point(K.bound.begin(), K.bound.end(),
-                                              [&](int b) { return b > jstep; }) -
-                         K.bound.begin());
-    // first and last field that take part: the kernel's own guard, evaluated
-    // here on the host copy of nlo (the last x sweep of fused sequences is
-    // active in one step only: a short range at the prefix's end)
-    int lo = 0, hi = np;
-    while (lo < hi && !field_active(K.h[lo], jstep, nslice, nlo_.data())) ++lo;
-    if (lo == hi) continue;
-    if (K.kind == 2)
-      while (!field_active(K.h[hi - 1], jstep, nslice, nlo_.data())) --hi;
-    else
-      lo = 0;
+    int lo = 0, hi = 0;
+    if (!active_fields(K, jstep, nslice, nlo_.data(), &lo, &hi)) continue;
     bs.g0idx = idxbuf_.as<int>() + K.ioff;
     const SweepField *fd = classbuf_.as<SweepField>() + K.off;
     cudaError_t e =

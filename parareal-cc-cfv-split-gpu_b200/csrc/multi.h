@@ -6,6 +6,7 @@
 #include <memory>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "engine.h"
@@ -99,10 +100,20 @@ struct SweepClass {
   int groups = 0;
   std::vector<int> bound;  // step bound per field (jmax, 0 -> INT_MAX), descending
   std::vector<int> gpre;   // gpre[i]: tiles of fields [0, i)
+  // the distinct step ranges [first, bound) of the fields: a step in none of
+  // them is not launched (the last x sweep of fused sequences runs in one step
+  // of each, and looking at every field to find that out costs host time)
+  std::vector<std::pair<int, int>> steps;
   // slice bound over the fields (0: some field has none): a launch with
   // nslice >= smax_all has no active field
   int smax_all = -1;
 };
+
+// Fields [*lo, *hi) of a class hold every field that takes part in a launch
+// (the kernels' own guard, on the host copy of nlo); false: none does.
+bool active_fields(const SweepClass &K, int jstep, int nslice, const int *nlo, int *lo, int *hi);
+// Sorts a class by step bound and numbers its tiles.
+void finish_class(SweepClass &K);
 
 class MultiEngine {
  public:
