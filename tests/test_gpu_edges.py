@@ -1,6 +1,6 @@
 """Sweep kernels at the ends of what they take: last segments shorter than the
-recurrence's warm-up, backward steps, the shortest lines in FP32, displacements
-of hundreds of cells, lone steps, short tuned segments."""
+recurrence's warm-up, backward steps, the shortest lines in FP32, short tuned
+segments, slices in place, what plans and batches prepare."""
 import os
 
 import numpy as np
@@ -212,3 +212,69 @@ def test_a_batch_fills_one_table_per_form_of_pass(ccfv):
 
     one = launches(1)
     assert launches(2) - one == 6 and launches(4) - one == 18
+
+
+@pytest.mark.parametrize("nx,ny", [(48, 50), (300, 270), (600, 44), (40, 1100)])
+@pytest.mark.parametrize("bc,vel,vp,scheme,nu", [
+    (0, 0, (), 0, 0.2), (0, 0, (), 1, 0.2), (0, 1, (3.0, -3.7), 0, 3.0), (0, 3, (1.5,), 0, 0.2),
+    (1, 3, (1.5,), 1, 0.2), (1, 3, (1.5,), 1, 20.0), (1, 1, (0.9, -1.7), 1, 20.0),
+    (1, 1, (0.9, -1.7), 0, 0.2)],
+    ids=["ref", "ref_consistent", "ref_const", "ref_swirl", "swirl", "swirl_strong", "strong",
+         "third_sweep"])
+def test_slices_in_place_by_form(oracle, ccfv, nx, ny, bc, vel, vp, scheme, nu):
+    """Slices swept over their input, a line's segments as one cluster: each form
+    of sweep, lines of one and of several segments, times from slice to slice."""
+    N = max(nx, ny)
+    h = (2.0 if bc == 0 else 1.0) / N
+    dt = 0.8 * h / 4.0
+    K = nu * h * h / dt
+    C0 = np.stack([seeded_field(nx, 5 + i, ny=ny) if bc == 0 else periodic_field(nx, 5 + i, ny=ny)
+                   for i in range(3)])
+    g = oracle.grid(nx, ny, bc=bc, K=K, vel=vel, vp=vp, threads=THREADS, scheme=scheme)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=bc, K=K, velocity=vel, vel_params=vp, scheme=scheme))
+    f = dev(C0)
+    s.fine_slices(f, 0.1, 0.25, 3 * dt, 3)
+    s.check()
+    for i in range(3):
+        assert rel_l2(f[i].cpu().numpy(), oracle.run(g, C0[i], 0.1 + 0.25 * i, dt, 3)) < TOL
+
+
+@pytest.mark.parametrize("nx,ny", [(40, 41), (271, 258), (272, 520), (500, 44), (42, 1025),
+                                   (1100, 66), (65, 233)])
+@pytest.mark.parametrize("vel,vp", [(1, (0.9, -1.7)), (3, (1.5,))], ids=["const", "swirl"])
+@pytest.mark.parametrize("nu", [0.1, 20.0, 90.0])
+def test_fp32_forms_at_the_sizes_of_their_tiles(oracle, ccfv, nx, ny, vel, vp, nu):
+    """FP32 coarse steps: warmed up over one and several segments, long warm-ups
+    of 32 lanes, lines closed alone and by clusters, odd rows."""
+    N = max(nx, ny)
+    dt = 0.4 / N
+    K = nu / (0.4 * N)  # K dt / h^2 = nu in the long direction
+    C0 = periodic_field(nx, nx + ny, ny=ny)
+    g = oracle.grid(nx, ny, bc=1, vel=vel, vp=vp, K=K, threads=THREADS, scheme=1)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=vel, vel_params=vp, K=K, scheme=1))
+    c = dev(C0)
+    s.coarse(c, 0.2, 2 * dt, 2, precision=ccfv.FP32)
+    s.check()
+    r = (1 / 12 - 0.5 * nu) / (10 / 12 + nu)
+    mu = abs(2 * r / (1 + np.sqrt(1 - 4 * r * r)))
+    # six sweeps; in each the right-hand side's ten roundings and those of the two
+    # recurrences, which add up over 1 / (1 - |mu|) positions (and the carries')
+    tol = 6 * (10 + 3 / (1 - mu)) * 2.0 ** -24
+    assert rel_l2(c.cpu().numpy(), oracle.coarse(g, C0, 0.2, 2 * dt, 2)) < tol
+
+
+@pytest.mark.parametrize("bc,vel,vp,scheme", [(1, 1, (0.9, -1.7), 1), (0, 0, (), 0)],
+                         ids=["const", "ref"])
+def test_plans_of_several_step_lengths_take_turns(oracle, ccfv, bc, vel, vp, scheme):
+    """One solver, three step lengths, lone steps and sequences in turn."""
+    nx, ny, K = 300, 130, 1e-3
+    C0 = seeded_field(nx, 9, ny=ny) if bc == 0 else periodic_field(nx, 9, ny=ny)
+    g = oracle.grid(nx, ny, bc=bc, K=K, vel=vel, vp=vp, threads=THREADS, scheme=scheme)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=bc, K=K, velocity=vel, vel_params=vp, scheme=scheme))
+    c, want, t = dev(C0), C0, 0.0
+    for dt, n in ((1e-3, 1), (2e-3, 3), (1e-3, 2), (5e-4, 1), (2e-3, 1), (5e-4, 4), (1e-3, 3)):
+        s.run(c, t, dt, n)
+        want = oracle.run(g, want, t, dt, n)
+        t += n * dt
+    s.check()
+    assert rel_l2(c.cpu().numpy(), want) < TOL
