@@ -752,7 +752,7 @@ int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
     if (stencil_filter_variant(plan->geom[kind].variant))
       plan->lines[kind] = h[(size_t)kind * nf].groups * tile_lines(plan->geom[kind]);
   const bool shared = plan->geom[2].variant == plan->geom[0].variant;
-  plan->fused_filled = plan->fused && (nsteps > 1 || nf != 1 || plan->geom[3].cs > 65535);
+  plan->fused_filled = plan->fused && (nsteps != 1 || nf != 1 || plan->geom[3].cs > 65535);
   auto own_table = [&](int kind) {
     return plan->lines[kind] > 0 && !(kind == 2 && shared) && !(kind == 3 && !plan->fused_filled);
   };
@@ -860,12 +860,13 @@ int steps(ccfv_ctx *ctx, void *d_C, bool fp64, double t0, double dt, int nsteps,
   int status = CCFV_OK;
   const size_t bytes =
       (fp64 ? sizeof(double) : sizeof(float)) * (size_t)ctx->grid.nx * ctx->grid.ny;
+  // (no steps: dt is checked and its plan made all the same)
+  StepPlan *plan = single_plan(ctx, dt, fp64, nsteps, &status, theta);
+  if (!plan) return status;
   if (nsteps <= 0) {
     if (src) CK(cudaMemcpyAsync(d_C, src, bytes, cudaMemcpyDeviceToDevice, st));
     return CCFV_OK;
   }
-  StepPlan *plan = single_plan(ctx, dt, fp64, nsteps, &status, theta);
-  if (!plan) return status;
   const bool odd = plan_passes(plan->fused, nsteps) & 1;
   FieldIo io;
   io.data = d_C;

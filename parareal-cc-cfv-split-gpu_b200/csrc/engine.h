@@ -127,7 +127,8 @@ int batch_solve(int n, const ccfv_problem *probs, ccfv_stats *stats, int device,
                 cudaStream_t st, std::string *errmsg);
 // homogeneous: the source term is left out (the linear part of the step,
 // which the delta form of Parareal applies to slice increments).
-// nsteps: steps of the sequence that it is built for (it serves others too).
+// nsteps: steps of the sequence that it is built for (it serves others too; not
+// 1: any sequence).
 int build_step_plan(ccfv_ctx *ctx, StepPlan *plan, double dt, bool fp64,
                     const std::vector<std::pair<void *, double>> &fields, int nsteps,
                     bool homogeneous = false, double theta = 0.5);

@@ -278,3 +278,20 @@ def test_plans_of_several_step_lengths_take_turns(oracle, ccfv, bc, vel, vp, sch
         t += n * dt
     s.check()
     assert rel_l2(c.cpu().numpy(), want) < TOL
+
+
+@pytest.mark.parametrize("bc,scheme", [(1, 1), (0, 0)], ids=["periodic", "reference"])
+def test_a_run_of_no_steps_makes_the_plan_and_refuses_what_steps_refuse(ccfv, bc, scheme):
+    s = ccfv.Solver(ccfv.make_grid(64, bc=bc, K=1e-3, velocity=1, vel_params=(0.9, -1.7),
+                                   scheme=scheme))
+    C0 = dev(periodic_field(64, 3))
+    c = C0.clone()
+    before = ccfv.kernel_launches()
+    s.run(c, 0.0, 1e-3, 0)
+    made = ccfv.kernel_launches()
+    assert made > before and bool((c == C0).all())
+    s.run(c, 0.0, 1e-3, 2)
+    assert ccfv.kernel_launches() - made == (5 if bc == 1 else 6)  # nothing left to prepare
+    for n in (0, 1):
+        with pytest.raises(ccfv.CcfvError):
+            s.run(c, 0.0, 50.0, n)  # feet too far for any kernel's tile
