@@ -95,8 +95,9 @@ struct SweepField {
   int rk_tail;           // compat: the second term of the rank-one closure matters
   double rk_a;             // compat: mu^2 / (1 - mu^(2L+2)), rank-one closure
   // exact form, q = -mu: q^n of a whole segment and of the line's last one,
-  // 1/(1 - q^2), 1/(1 - q^L), and q^n of the last lane of the last one
-  double ex[5];
+  // 1/(1 - q^2), 1/(1 - q^L), q^n of the last lane of the last one, and
+  // q^-(positions that this lane walks behind it), 0 where that is above 2^24
+  double ex[6];
   // per-line stencil of w's input, computed once per plan (the velocity fields
   // it serves do not depend on time).  wt: T[lines][stencil_taps(variant)];
   // nt: int[lines] shifts.

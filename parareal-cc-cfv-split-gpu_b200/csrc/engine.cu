@@ -619,7 +619,11 @@ void filter_field(const ccfv_grid &g, SweepField &f, bool fp64, const LaunchGeom
     f.ex[1] = std::pow(q, end);
     f.ex[2] = 1.0 / (1.0 - q * q);
     f.ex[3] = 1.0 / (1.0 - std::pow(q, f.L));
-    f.ex[4] = std::pow(q, (end - 1) % STREAM_CH + 1);
+    const int mine = (end - 1) % STREAM_CH + 1;
+    f.ex[4] = std::pow(q, mine);
+    // (q = 0: the system is diagonal, nothing is carried)
+    f.ex[5] = mine == STREAM_CH ? 1.0 : std::pow(q, mine - STREAM_CH);
+    if (!(std::fabs(f.ex[5]) <= std::ldexp(1.0, 24))) f.ex[5] = 0.0;
   }
   f.rk_a = mu * mu / (1.0 - std::pow(mu * mu, f.L + 1));
   f.rk_tail = std::pow(std::fabs(mu), f.L) >= std::ldexp(1.0, -60) ? 1 : 0;

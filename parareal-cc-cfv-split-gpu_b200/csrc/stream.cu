@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
   T *exs = tile_s + (size_t)(DIR == 0 ? X_PITCH : StreamCta<DIR, LN>::lines) * rows +
            (SWIRL ? 2 * (LN * SCH + 3) * (sizeof(double) / sizeof(T)) : 0);
   if (EXACT) {
-    if (threadIdx.x < 5) exs[threadIdx.x] = T(D->ex[threadIdx.x]);
+    if (threadIdx.x < 6) exs[threadIdx.x] = T(D->ex[threadIdx.x]);
     __syncwarp();  // an aligned cluster barrier takes converged warps only
     // the peers may write to this CTA once it runs
     if (cs > 1) asm volatile("barrier.cluster.arrive.aligned;\n" ::: "memory");
@@ -865,14 +865,14 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     x = T(0);
 #pragma unroll
     for (int i = SCH - 1; i >= 0; --i) x = v[i] + mmu * x;
-    // with the scan: q^(17 c), and q^(17 (act-2-c)) for the lanes before the last
+    // with the scan: q^(17 c), q^(17 (act-1-c))
     T pd = pw, up = T(1), down = T(1);
 #pragma unroll
     for (int b = 0; b < (LN == 32 ? 5 : 4); ++b) {
       const T t = __shfl_down_sync(FULL, x, LS << b, W);
       if (c + (1 << b) < LN) x += pd * t;
       if (c >> b & 1) up *= pd;
-      if ((act - 2 - c) >> b & 1) down *= pd;
+      if ((act - 1 - c) >> b & 1) down *= pd;
       pd *= pd;
     }
     // The forward carry cr into a segment adds cr q^(j+1) to w_j (q = -mu),
@@ -928,13 +928,15 @@ __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
     const T far = d - cr * inv1m * mmu * (end ? last : whole);
     x = __shfl_down_sync(FULL, x, LS, W);
     if (c == LN - 1) x = T(0);
-    // carry into this lane; into the last one right behind the segment's last
-    // position (scaled up to the lane's end it would leave FP32's range on the
-    // shortest lines: q^-13 at 4 cells)
-    if (mine > SCH) {
-      x += far * down * (end ? exs[4] : pw);
-    } else if (mine == SCH) {
-      x += far;
+    // Carry into this lane.  The last one, where it ends behind the segment,
+    // starts with q^-(positions behind) as much.  Where that factor is large
+    // (lines of a few cells and |q| far below one: q^-13 at 4 cells leaves FP32's
+    // range) the carry enters right behind the segment's last position.
+    const T back = end ? exs[5] : T(1);
+    if (back != T(0)) {
+      if (c < act) x += far * down * back;
+    } else if (c < act - 1) {
+      x += far * exs[4] * T(powi(-F.mu, SCH * (act - 2 - c)));
     } else {
 #pragma unroll
       for (int i = 1; i < SCH; ++i)

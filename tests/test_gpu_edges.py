@@ -295,3 +295,33 @@ def test_a_run_of_no_steps_makes_the_plan_and_refuses_what_steps_refuse(ccfv, bc
     for n in (0, 1):
         with pytest.raises(ccfv.CcfvError):
             s.run(c, 0.0, 50.0, n)  # feet too far for any kernel's tile
+
+
+@pytest.mark.parametrize("L", [5, 17, 18, 20, 33, 34, 35, 50])
+@pytest.mark.parametrize("dir", [0, 1])
+@pytest.mark.parametrize("nu", [0.05, 1 / 6 + 1e-3, 0.5, 2.0, 2.2, 4.0])
+def test_closed_lines_of_a_few_lanes(oracle, ccfv, L, dir, nu):
+    """Short closed lines on either side of where the carry into the last lane is
+    scaled to its end (|q| = 0.35), in FP64 and FP32."""
+    nx, ny = (L, 8) if dir == 0 else (8, L)
+    Dt = 0.3 / L
+    K = nu / (L * L * Dt)
+    dt = 2 * Dt if dir == 0 else Dt
+    C0 = periodic_field(nx, L, ny=ny)
+    g = oracle.grid(nx, ny, bc=1, vel=1, vp=(0.9, -1.7), K=K, threads=1, scheme=1)
+    s = ccfv.Solver(ccfv.make_grid(nx, ny, bc=1, velocity=1, vel_params=(0.9, -1.7), K=K, scheme=1))
+    want = oracle.coarse(g, C0, 0.0, dt, 1)
+    # a sweep's right-hand side has ten roundings, its recurrences add theirs up
+    # over 1 / (1 - |mu|) positions; the other direction's sweep has a mu of its own
+    other = nu * (8 / L) ** 2 * (2 if dir == 0 else 0.5)
+
+    def roundings(n):
+        r = (1 / 12 - 0.5 * n) / (10 / 12 + n)
+        return 10 + 3 / (1 - abs(2 * r / (1 + np.sqrt(1 - 4 * r * r))))
+
+    n = 2 * roundings(nu) + 2 * roundings(other)
+    for precision, tol in ((ccfv.FP64, TOL), (ccfv.FP32, n * 2.0 ** -24)):
+        c = dev(C0)
+        s.coarse(c, 0.0, dt, 1, precision=precision)
+        s.check()
+        assert rel_l2(c.cpu().numpy(), want) < tol
