@@ -1041,8 +1041,9 @@ StreamKernelT<T> stream_kernel_of(int dir, int lanes) {
 template <typename T>
 StreamKernelT<T> stream_kernel_for(int variant, int dir, int lanes) {
   if (variant == SWEEP_CELL) return stream_kernel_of<T, 4>(dir, lanes);
-  if (variant == SWEEP_FILTER_XX)
-    return lanes == 32 ? stream_kernel<T, 0, 32, 3, false> : stream_kernel<T, 0, 16, 3, false>;
+  if constexpr (sizeof(T) == 8)  // (fused_x_geom: FP64 only)
+    if (variant == SWEEP_FILTER_XX)
+      return lanes == 32 ? stream_kernel<T, 0, 32, 3, false> : stream_kernel<T, 0, 16, 3, false>;
   if (variant == SWEEP_FILTER_EXACT) return stream_kernel_of<T, 0, true>(dir, lanes);
   if (variant == SWEEP_CELL_EXACT) return stream_kernel_of<T, 4, true>(dir, lanes);
   return variant == SWEEP_COMPAT     ? stream_kernel_of<T, 1>(dir, lanes)
