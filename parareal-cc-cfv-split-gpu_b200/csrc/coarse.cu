@@ -100,9 +100,9 @@ __device__ __forceinline__ T rg_rhs(const RgEdge<T> &l, const RgEdge<T> &r, cons
 
 // Threads of a resident CTA.  One CTA runs a chain of dependent sweeps, so its
 // time is the latency of a round of lines times the rounds: as many half-warps
-// as the register file holds (batch of 12 instances of up to 583^2: 171 ms with
-// 256 threads, 107 ms with these and dependent launches).  The per-cell form
-// keeps 16 lines a round, whose right-hand sides have a scratch row each.
+// as the register file holds (batch of 12 instances of up to 583^2: 127 ms with
+// 256 threads, 101 ms with these).  The per-cell form keeps 16 lines a round,
+// whose right-hand sides have a scratch row each.
 template <typename T, bool CELL>
 constexpr int rg_threads() {
   return CELL ? 256 : sizeof(T) == 4 ? 1024 : 512;

@@ -394,7 +394,7 @@ LaunchGeom step_geom(const ccfv_grid &g, int dir, double Dt, int dsrc, bool fp64
     // along: a warm-up of up to a quarter of the 32 lanes' positions (eight
     // steps at a diffusion number of 10 per x sweep and 20 per y sweep, the
     // segments of a line as a cluster that closes it exactly against the
-    // warm-up: 1024^2 214 -> 162 us, 2048^2 555 -> 409 us, 4096^2 2434 -> 1461
+    // warm-up: 1024^2 212 -> 174 us, 2048^2 556 -> 422 us, 4096^2 2455 -> 1485
     // us; y sweeps at 28, J = 146: 2048^2 445 us closed, 477 us warmed up).
     // Whole lines, longer warm-ups and the per-cell right-hand sides (far more
     // work per position): closed.
@@ -857,8 +857,8 @@ static StepPlan *single_plan(ccfv_ctx *ctx, double dt, bool fp64, int nsteps, in
 // in d_C.  In place, an odd number of passes would end in the scratch field:
 // the last y sweep then writes over its input (a line's segments form one
 // cluster), which costs nothing where copying the result back was one more
-// pass over the field (4096^2 step: 208 us with the copy, 172 us without);
-// lines of more segments than a cluster holds are copied.
+// pass over the field (36 us of a lone 4096^2 step); lines of more segments than
+// a cluster holds are copied.
 int steps(ccfv_ctx *ctx, void *d_C, bool fp64, double t0, double dt, int nsteps, cudaStream_t st,
           double theta, const void *src) {
   int status = CCFV_OK;

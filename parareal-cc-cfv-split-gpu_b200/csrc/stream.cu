@@ -27,10 +27,11 @@
 // decay by (-mu)^17 per lane, so the scan over lanes needs only as many
 // doubling steps as the warm-up has chunks (0, 1 or 2 instead of 4).
 //
-// What bounds it: HBM.  One FP64 sweep of 4096^2 (268 MB): y 41.2 us, x 47 us,
-// against 41.0 us for the copy rate and 62 us for the tile kernel this
-// replaced (8-byte copies, 16 lanes per line, carries added afterwards, two
-// CTA barriers; it issued 69 instructions per cell, this one about 26).
+// What bounds it: HBM, then issue.  A lone FP64 step of 4096^2, three passes of
+// 268 MB (123 us at the copy rate), takes 183 us against 230 us for the tile
+// kernel this replaced (8-byte copies, 16 lanes per line, carries added
+// afterwards, two CTA barriers).  Instructions per cell: 50 an x sweep, 41 a y
+// sweep, 68 two x sweeps in one pass; the tile kernel 69 a sweep.
 #include <cooperative_groups.h>
 
 #include <atomic>
@@ -436,10 +437,11 @@ __device__ __noinline__ T cells_between(int kl, int kr, const T *cells, int b0, 
 // the periodic line exactly.  Segments are whole walks and a shorter last one;
 // a y line of 544 cells is one warp's and needs no exchange.  Bound by the
 // clusters' latency: 64 registers for the y kernel too, so that the next
-// launch's clusters find room beside this one's (1024^2, eight steps at
-// K dt / h^2 = 20: 264 us with 80 registers, 213 us with 64).  Against the tile
-// kernel: 256^2 163 -> 110 us, 1024^2 211 -> 213 us, 4096^2 2474 -> 2434 us;
-// swirling field, 1024^2 782 -> 420 us, 2048^2 2980 -> 1511 us.
+// launch's clusters find room beside this one's (1024^2, eight steps with every
+// sweep closed: 264 us with 80 registers, 213 us with 64).  Eight steps at
+// K dt / h^2 = 90 against the tile kernel: 256^2 175 -> 122 us, 1024^2 222 -> 212
+// us, 2048^2 602 -> 556 us, 4096^2 2491 -> 2455 us; swirling field at 20, 1024^2
+// 792 -> 405 us, 2048^2 2988 -> 1510 us.
 template <typename T, int DIR, int LN, int BND, bool EXACT>
 __global__ void __launch_bounds__(StreamCta<DIR, LN>::warps * 32,
                                   BND == 4 ? (DIR == 0 ? 2 : 4) : DIR == 0 ? 64 / LN : EXACT ? 8 : 6)

@@ -1656,8 +1656,8 @@ size_t sweep_fast_smem_bytes(int lc_max, int halo, bool fp64) {
 
 // Programmatic dependent launch: the filter kernels wait for their predecessor
 // before reading cells, after fetching what is constant.  Batch of 64 mixed
-// instances: 1323 ms without, 1276 ms with; 12 instances up to 583^2: 115 ms
-// without, 97 ms with.  CCFV_PDL=0 turns it off.
+// instances: 1323 ms without, 1276 ms with; 12 instances up to 583^2: 120 ms
+// without, 101 ms with.  CCFV_PDL=0 turns it off.
 bool pdl_enabled() {
   static const bool on = [] {
     const char *e = std::getenv("CCFV_PDL");
